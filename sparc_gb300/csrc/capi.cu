@@ -234,6 +234,7 @@ int sgpu_destroy(sgpu_ctx *ctx)
     nonlocal_free(ctx->nl);
     if (ctx->veff64) cudaFree(ctx->veff64);
     if (ctx->veff32) cudaFree(ctx->veff32);
+    if (ctx->veff_fx) cudaFree(ctx->veff_fx);
     for (auto &w : ctx->ws)
         if (w.ptr) cudaFree(w.ptr);
     if (ctx->cublas) cublasDestroy(ctx->cublas);
@@ -271,16 +272,22 @@ int sgpu_set_veff(sgpu_ctx *ctx, int nspin, const double *veff)
         if (ctx->veff64) cudaFree(ctx->veff64);
         if (ctx->veff32) cudaFree(ctx->veff32);
         ctx->veff64 = nullptr;
+        if (ctx->veff_fx) cudaFree(ctx->veff_fx);
         ctx->veff32 = nullptr;
+        ctx->veff_fx = nullptr;
         ctx->nspin_veff = 0;
         SGPU_CUDA_TRY(cudaMalloc(&ctx->veff64, n * sizeof(double)));
         SGPU_CUDA_TRY(cudaMalloc(&ctx->veff32, n * sizeof(float)));
+        SGPU_CUDA_TRY(cudaMalloc(&ctx->veff_fx, (n + 1) * sizeof(int2)));
         ctx->nspin_veff = nspin;
     }
     SGPU_CUDA_TRY(cudaMemcpyAsync(ctx->veff64, veff, n * sizeof(double), cudaMemcpyDefault,
                                   ctx->stream));
     SGPU_TRY(convert_cols<double, float>(ctx->veff64, (long)n, ctx->veff32, (long)n, (long)n, 1,
                                          ctx->stream));
+    SGPU_TRY(fx_potential(ctx, ctx->veff64, 1.0, (long)n, ctx->veff_fx,
+                          reinterpret_cast<unsigned *>(ctx->veff_fx + n), &ctx->veff_key,
+                          ctx->stream));
     SGPU_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     return SGPU_OK;
 }
@@ -592,7 +599,7 @@ int sgpu_poisson_residual(sgpu_ctx *ctx, double c, const double *x, const double
     SGPU_TRY(stage_in(ctx, WS_STAGE_B, r, (int)ctx->Nd, 1, false, &dr, &lr));
     // r = 1 * (Lap + c) x + 1 * b
     SGPU_TRY(launch_stencil<double>(ctx, 1, 1.0, 0.0, c, nullptr, dx, lx, dr, lr, 1.0, 1.0, db,
-                                    lb, ctx->stream));
+                                    lb, ctx->stream, nullptr, false));
     SGPU_TRY(stage_out(ctx, dr, lr, r, (int)ctx->Nd, 1));
     SGPU_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     return SGPU_OK;

@@ -50,8 +50,9 @@ int hamiltonian_dev(sgpu_ctx *ctx, int spin, int ncol, double c, const T *x, lon
         SGPU_TRY(launch_nonlocal_project<T>(ctx, ncol, x, ldx, a, lda, st));
         alpha = a;
     }
+    const FxPot pot{ctx->veff_fx + (long)spin * ctx->Nd, ctx->veff_key};
     SGPU_TRY(launch_stencil<T>(ctx, ncol, -0.5, 1.0, c, veff_of<T>(ctx, spin), x, ldx, hx, ldh,
-                               s1, s2, z, ldz, st));
+                               s1, s2, z, ldz, st, &pot));
     if (!alpha) return SGPU_OK;
     if constexpr (sizeof(T) == 4) {
         if (alpha_out) {

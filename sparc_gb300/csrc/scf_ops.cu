@@ -551,7 +551,7 @@ int aar_dev(sgpu_ctx *ctx, double c, double *x, const double *b, double omega, d
     if (std::fabs(minv) < 1e-14) minv = 1.0;
     minv = -1.0 / minv;
     // r = b + (Lap + c) x
-    SGPU_TRY(launch_stencil<double>(ctx, 1, 1.0, 0.0, c, nullptr, x, N, r, N, 1.0, 1.0, b, N, st));
+    SGPU_TRY(launch_stencil<double>(ctx, 1, 1.0, 0.0, c, nullptr, x, N, r, N, 1.0, 1.0, b, N, st, nullptr, false));
     tol *= std::sqrt(bnorm2);
     double rnorm = tol + 1.0;
     int it = 0;
@@ -568,13 +568,13 @@ int aar_dev(sgpu_ctx *ctx, double c, double *x, const double *b, double omega, d
                                                  nullptr);
             ctx->launches++;
             SGPU_TRY(launch_stencil<double>(ctx, 1, 1.0, 0.0, c, nullptr, x, N, r, N, 1.0, 1.0,
-                                            b, N, st));
+                                            b, N, st, nullptr, false));
             double r2 = 0.0;
             SGPU_TRY(dot_host(ctx, r, r, N, &r2, st));
             rnorm = std::sqrt(r2);
         } else {
             SGPU_TRY(launch_stencil<double>(ctx, 1, 1.0, 0.0, c, nullptr, x, N, r, N, 1.0, 1.0,
-                                            b, N, st));
+                                            b, N, st, nullptr, false));
         }
         it++;
     }
@@ -611,7 +611,7 @@ int kerker_dev(sgpu_ctx *ctx, const double *f, double a, double kTF, double idie
     double *Lf = nullptr;
     SGPU_TRY(ws_get(ctx, WS_RHS, sizeof(double) * (size_t)N, (void **)&Lf));
     SGPU_TRY(launch_stencil<double>(ctx, 1, 1.0, 0.0, -kTF * kTF * idiemac, nullptr, f, N, Lf, N,
-                                    1.0, 0.0, nullptr, 0, st));
+                                    1.0, 0.0, nullptr, 0, st, nullptr, false));
     int rc = aar_dev(ctx, -kTF * kTF, Pf, Lf, 0.6, 0.6, 7, 6, tol, 1000, nullptr, st);
     if (rc != SGPU_OK && rc != SGPU_ERR_NOT_CONVERGED) return rc;
     if (std::fabs(kTF) < 1e-14) SGPU_TRY(remove_mean_dev(ctx, Pf, st));

@@ -109,6 +109,13 @@ struct Nonlocal {
     float *tc_chi = nullptr;    // Chi values of the merged entries, range_jp per entry
 };
 
+// A potential as fixed-point digits (fixed64.cuh) for the FP64 stencil; key: the exponent key of its
+// largest magnitude, which sets the digits' scale (0: all zero)
+struct FxPot {
+    const int2 *vd = nullptr;
+    unsigned key = 0;
+};
+
 struct Workspace {
     void *ptr = nullptr;
     size_t bytes = 0;
@@ -159,6 +166,8 @@ struct sgpu_ctx {
     int nspin_veff = 0;
     double *veff64 = nullptr;  // Nd * nspin
     float *veff32 = nullptr;
+    int2 *veff_fx = nullptr;   // digits of veff64 (all spins at one scale), key after them
+    unsigned veff_key = 0;
     sgpu::Nonlocal nl;
     bool has_nl = false;
     cublasHandle_t cublas = nullptr;
@@ -168,7 +177,7 @@ struct sgpu_ctx {
     size_t xhost_bytes = 0;
     int rr_batched = 1;                     // k-point CheFSI pass: batched Rayleigh-Ritz step
                                             // for blocks of one width (sgpu_set_rr_batched)
-    sgpu::Workspace ws[16];    // grow-only scratch slots (see enum WsSlot)
+    sgpu::Workspace ws[24];    // grow-only scratch slots (see enum WsSlot)
     sgpu::MixState *mix = nullptr;
     sgpu::KpointState *kp = nullptr;  // cell lengths and image coordinates (k-point calls)
     sgpu::SetupState *setup = nullptr;  // pseudopotential tables (set-up calls)
@@ -221,7 +230,7 @@ namespace sgpu {
 enum WsSlot {
     WS_STAGE_A = 0, WS_STAGE_B, WS_STAGE_C, WS_ALPHA, WS_MISC, WS_EIG, WS_POIS, WS_MIX,
     WS_RED, WS_RHS, WS_SCF, WS_SCF2, WS_ALPHA2, WS_SPLIT_A, WS_SPLIT_B, WS_TC_PART,
-    WS_COUNT
+    WS_FXPOT, WS_COUNT
 };
 
 // grow-only device scratch
@@ -250,10 +259,16 @@ bool is_device_ptr(const void *p);
 // ---- stencil (stencil.cu)
 // out[:, n] = s1 * ( a*Lap + bv*diag(v) + c*I ) x[:, n]  +  s2 * z[:, n]
 // (z may be null; v may be null). All arrays column-major with the given leading dims.
+// FP64: pot are the digits of v where the caller keeps them; fixed = false asks for the FP64
+// kernel. The AAR solves do: an iterate's rounding decides what the next Anderson step
+// extrapolates, so another kernel's rounding moves a solution within its tolerance (1e-8 of it
+// at 77^3, far above the rounding itself), and one column of one vector is latency-bound.
 template <typename T>
 int launch_stencil(sgpu_ctx *ctx, int ncol, double a, double bv, double c, const T *v,
                    const T *x, long ldx, T *out, long ldo, double s1, double s2, const T *z,
-                   long ldz, cudaStream_t st);
+                   long ldz, cudaStream_t st, const FxPot *pot = nullptr, bool fixed = true);
+int fx_potential(sgpu_ctx *ctx, const double *v, double bv, long n, int2 *vd, unsigned *key,
+                 unsigned *hkey, cudaStream_t st);
 
 // ---- nonlocal (nonlocal.cu)
 // alpha is (ntot x lda) projector-major: alpha[row * lda + n]; lda from nonlocal_alpha_ld

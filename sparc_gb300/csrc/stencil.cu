@@ -19,6 +19,7 @@
 #include "sgpu_internal.h"
 #include "mbarrier.cuh"
 #include "cpasync.cuh"
+#include "stencil_fx.cuh"
 
 namespace sgpu {
 namespace {
@@ -42,7 +43,9 @@ __device__ __forceinline__ int wrapi(int i, int n)
     return i < 0 ? i + n : i;
 }
 
-// FP64 (and generic) kernel: one point per thread. On GB300 the FP64 pipe, not HBM, bounds it.
+// FP64 kernel: one point per thread. The FP64 pipe (2 lanes per clock and SM) bounds it, 37.3 ms per
+// launch at 96^3 x 512 against 4.75 of the fixed-point form (stencil_fx.cuh); it serves the AAR
+// solves and the coefficients and potentials that the fixed-point form does not take.
 template <typename T, int R, int BX, int BY>
 __global__ void __launch_bounds__(BX *BY)
     k_stencil_orth(const StencilParams<T> p)
@@ -1038,12 +1041,88 @@ int launch_bulk(const StencilParams<float> &q, dim3 grid, cudaStream_t st)
     return SGPU_OK;
 }
 
+// FP64 stencil in block fixed point; *done false when the coefficients are out of its range
+int launch_stencil_fx(sgpu_ctx *ctx, int ncol, const StencilParams<double> &q, const FxPot *pot,
+                      bool *done, cudaStream_t st)
+{
+    *done = false;
+    if (ctx->Nd >= (1L << 28)) return SGPU_OK;  // 32-bit byte offsets in a column
+    constexpr int R = kMaxFDn;
+    StencilFxParams p{};
+    p.x = q.x; p.out = q.out; p.z = q.z; p.v = q.v;
+    p.ldx = q.ldx; p.ldo = q.ldo; p.ldz = q.ldz;
+    p.Nx = q.Nx; p.Ny = q.Ny; p.Nz = q.Nz;
+    p.c0 = q.c0; p.bv = q.bv; p.s1 = q.s1; p.s2 = q.s2;
+    for (int r = 0; r < R; r++) {
+        p.w[0][r] = q.wx[r + 1];
+        p.w[1][r] = q.wy[r + 1];
+        p.w[2][r] = q.wz[r + 1];
+    }
+    FxPot own{};
+    if (q.v && !pot) {  // a caller's potential: its digits for this call
+        char *w = nullptr;
+        SGPU_TRY(ws_get(ctx, WS_FXPOT, sizeof(int2) * (size_t)ctx->Nd + 16, (void **)&w));
+        SGPU_TRY(fx_potential(ctx, q.v, q.bv, ctx->Nd, reinterpret_cast<int2 *>(w + 16),
+                              reinterpret_cast<unsigned *>(w), &own.key, st));
+        SGPU_CUDA_TRY(cudaStreamSynchronize(st));
+        own.vd = reinterpret_cast<int2 *>(w + 16);
+        pot = &own;
+    }
+    const unsigned vkey = q.v ? pot->key : 0u;
+    p.vd = vkey ? pot->vd : nullptr;
+    if (!fx_setup(p, R, vkey)) return SGPU_OK;
+    *done = true;
+    const bool cube = std::equal(p.w[0], p.w[0] + R, p.w[1]) &&
+                      std::equal(p.w[0], p.w[0] + R, p.w[2]);
+    int nslab = 1, nsm = 152;
+    SGPU_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device));
+    fx_plan(p.Nx, p.Ny, p.Nz, ncol, nsm, p.TX, p.TY, nslab);
+    p.hx = 2 * R * p.TY;
+    p.hy = 2 * R * p.TX;
+    const int tilesx = (p.Nx + p.TX - 1) / p.TX, tilesy = (p.Ny + p.TY - 1) / p.TY;
+    const int nthr = fx_threads(p.TX, p.TY), ns = (p.hx + p.hy + nthr - 1) / nthr;
+    p.zlen = (p.Nz + nslab - 1) / nslab;
+    p.nslab = nslab;
+    const size_t smem = 2 * sizeof(int2) * (size_t)kFxPitch * (p.TY + 2 * R);
+    const int maxz = 65535 / nslab;
+    for (int c0i = 0; c0i < ncol; c0i += maxz) {
+        const int nc = std::min(ncol - c0i, maxz);
+        StencilFxParams b = p;
+        b.x = p.x + (long)c0i * p.ldx;
+        b.out = p.out + (long)c0i * p.ldo;
+        if (b.z) b.z = p.z + (long)c0i * p.ldz;
+        const dim3 grid(tilesx, tilesy, nc * nslab);
+        ProfScope ps(ctx, SGPU_KERNEL_STENCIL, st);
+        auto kern = ns <= 2 ? (cube ? k_stencil_fx<2, true> : k_stencil_fx<2, false>)
+                    : ns == 3 ? (cube ? k_stencil_fx<3, true> : k_stencil_fx<3, false>)
+                              : (cube ? k_stencil_fx<4, true> : k_stencil_fx<4, false>);
+        kern<<<grid, nthr, smem, st>>>(b);
+    }
+    SGPU_CUDA_TRY(cudaGetLastError());
+    return SGPU_OK;
+}
+
 }  // namespace
+
+// digits of bv v into vd and the exponent key of the largest |bv v|, on the device (*key) and, after
+// the stream's next synchronisation, on the host (*hkey)
+int fx_potential(sgpu_ctx *ctx, const double *v, double bv, long n, int2 *vd, unsigned *key,
+                 unsigned *hkey, cudaStream_t st)
+{
+    const int nb = (int)std::min<long>((n + 255) / 256, 152L * 8);
+    SGPU_CUDA_TRY(cudaMemsetAsync(key, 0, sizeof(unsigned), st));
+    k_fx_key<<<nb, 256, 0, st>>>(v, bv, n, key);
+    k_fx_digits<<<nb, 256, 0, st>>>(v, bv, n, key, vd);
+    ctx->launches += 2;
+    SGPU_CUDA_TRY(cudaGetLastError());
+    SGPU_CUDA_TRY(cudaMemcpyAsync(hkey, key, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+    return SGPU_OK;
+}
 
 template <typename T>
 int launch_stencil(sgpu_ctx *ctx, int ncol, double a, double bv, double c, const T *v,
                    const T *x, long ldx, T *out, long ldo, double s1, double s2, const T *z,
-                   long ldz, cudaStream_t st)
+                   long ldz, cudaStream_t st, const FxPot *pot, bool fixed)
 {
     constexpr int R = 6, BX = 32, BY = 8;       // FP64 tile (one point per thread)
     constexpr int BXP = 32, BYP = 16;          // FP32 tile (two points per thread)
@@ -1075,6 +1154,12 @@ int launch_stencil(sgpu_ctx *ctx, int ncol, double a, double bv, double c, const
     p.status = ctx->kstatus;
     if (!v || fabs(bv) < 1e-14) p.v = nullptr;
     if (!z || s2 == 0.0) p.z = nullptr;
+
+    if constexpr (sizeof(T) == 8) {
+        bool done = false;
+        if (fixed) SGPU_TRY(launch_stencil_fx(ctx, ncol, p, pot, &done, st));
+        if (done) return SGPU_OK;
+    }
 
     const bool f32 = sizeof(T) == 4;
     // FP32 variants (autotune.cu): 0 paired 32x16, 1 2x2-blocked 32x16, 2 2x2-blocked 64x8,
@@ -1204,9 +1289,9 @@ int wait_bound_check(sgpu_ctx *ctx)
 
 template int launch_stencil<double>(sgpu_ctx *, int, double, double, double, const double *,
                                     const double *, long, double *, long, double, double,
-                                    const double *, long, cudaStream_t);
+                                    const double *, long, cudaStream_t, const FxPot *, bool);
 template int launch_stencil<float>(sgpu_ctx *, int, double, double, double, const float *,
                                    const float *, long, float *, long, double, double,
-                                   const float *, long, cudaStream_t);
+                                   const float *, long, cudaStream_t, const FxPot *, bool);
 
 }  // namespace sgpu

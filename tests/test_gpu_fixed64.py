@@ -1,0 +1,97 @@
+"""FP64 kernels in block fixed point (csrc/fixed64.cuh) at the sizes and values where they can go
+wrong: tiles cut by the grid edge, rows that wrap several times, slabs, fields whose largest value
+grows along z (a new block scale), columns that the fixed-point range does not cover."""
+import numpy as np
+import pytest
+
+import sparc_gb300 as sg
+from oracle.oracle import Oracle
+from sparc_gb300.synthetic import fd_d2_coeffs
+
+pytestmark = pytest.mark.gpu
+
+
+def _fields(N, rng):
+    Nd = N[0] * N[1] * N[2]
+    z = np.arange(Nd) // (N[0] * N[1])
+    u = rng.uniform(-1, 1, (2, Nd))
+    return {"uniform": u, "growing": u * 2.0 ** (1.5 * z), "falling": u * 2.0 ** (-1.5 * z),
+            "one point": np.eye(1, Nd, Nd // 2) * 3.7, "zero": np.zeros((1, Nd)),
+            "wide": u * 10.0 ** rng.uniform(-12, 0, (2, Nd)), "tiny": u * 1e-290,
+            "huge": u * 1e290}
+
+
+@pytest.mark.parametrize("N", [(14, 14, 14), (6, 7, 9), (31, 17, 23), (45, 33, 12), (34, 12, 70),
+                               (77, 20, 13)])
+@pytest.mark.parametrize("h", [(0.4, 0.4, 0.4), (0.4, 0.37, 0.45)])
+def test_stencil_fields(gpu_available, N, h):
+    """Both weight forms (equal and different spacings). Each result is off by at most the
+    rounding of the oracle's 37-term sum and the two final operations, 40 units of 2^-53 of the
+    sum of |coefficient| times the column's largest value."""
+    rng = np.random.default_rng(sum(N))
+    c = [fd_d2_coeffs(6, x) for x in h]
+    grid = dict(Nx=N[0], Ny=N[1], Nz=N[2], FDn=6, cx=c[0], cy=c[1], cz=c[2], dV=float(np.prod(h)))
+    ctx = sg.Context(*N, 6, *c, grid["dV"])
+    o = Oracle(grid, None)
+    Nd = N[0] * N[1] * N[2]
+    v = rng.normal(size=Nd)
+    S = 0.5 * sum(abs(w[0]) + 2 * np.abs(w[1:]).sum() for w in c) + 3.1 + np.abs(v).max()
+    for name, x in _fields(N, rng).items():
+        y = np.full_like(x, np.nan)
+        ctx.Lap_plus_diag_vec_mult_orth(-0.5, 1.0, -3.1, v, x, y)
+        ref = o.lap_plus_diag(-0.5, 1.0, -3.1, v, x)
+        for n in range(x.shape[0]):
+            assert np.abs(y[n] - ref[n]).max() <= 40 * 2.0 ** -53 * S * np.abs(x[n]).max(), name
+    ctx.close()
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e3, 1e9, 0.0])
+def test_stencil_potential_range(gpu_available, scale):
+    """A potential of the stencil's own size, one far above it (the FP64 kernel takes over) and
+    none; the filter's recurrence term; a few columns and enough columns for whole-z slabs."""
+    N, h = (20, 18, 26), 0.4
+    rng = np.random.default_rng(5)
+    c = fd_d2_coeffs(6, h)
+    grid = dict(Nx=N[0], Ny=N[1], Nz=N[2], FDn=6, cx=c, cy=c, cz=c, dV=h ** 3)
+    ctx = sg.Context(*N, 6, c, c, c, h ** 3)
+    o = Oracle(grid, None)
+    Nd = N[0] * N[1] * N[2]
+    v = rng.normal(size=Nd) * scale
+    ctx.set_veff(v)
+    S = 1.5 * (abs(c[0]) + 2 * np.abs(c[1:]).sum()) + 20 + np.abs(v).max()
+    for ncol in (1, 3, 300):
+        x = rng.uniform(-1, 1, (ncol, Nd))
+        y = np.zeros_like(x)
+        ctx.Hamiltonian_vectors_mult(-20.0, x, y)
+        k = min(ncol, 3)
+        assert np.abs(y[:k] - o.hamiltonian(v, -20.0, x[:k])).max() <= 40 * 2.0 ** -53 * S
+        b = 2.0 * S  # above the spectrum: the recurrence keeps the block near its input's size
+        X, Y = x.copy(), np.zeros_like(x)
+        ctx.ChebyshevFiltering(X, Y, 4, 0.1 * S, b, -b)
+        Xo, Yo = o.chebyshev(v, 4, 0.1 * S, b, -b, x[:k])
+        # four applies, each scaled to at most 4, on iterates at most 8 times the input
+        assert np.abs(Y[:k] - Yo).max() <= 4 * 4 * 8 * 40 * 2.0 ** -53
+        assert np.abs(X[:k] - Xo).max() <= 4 * 4 * 8 * 40 * 2.0 ** -53
+    ctx.close()
+
+
+def test_stencil_nonfinite(gpu_available):
+    """An infinity and a NaN reach exactly the points whose stencil touches them."""
+    N, h = (33, 21, 30), 0.4
+    rng = np.random.default_rng(6)
+    c = fd_d2_coeffs(6, h)
+    grid = dict(Nx=N[0], Ny=N[1], Nz=N[2], FDn=6, cx=c, cy=c, cz=c, dV=h ** 3)
+    ctx = sg.Context(*N, 6, c, c, c, h ** 3)
+    Nd = N[0] * N[1] * N[2]
+    x = rng.uniform(-1, 1, (3, Nd))
+    x[0, Nd // 3] = np.nan
+    x[1, Nd // 2] = np.inf
+    x[2, 7] = -np.inf
+    y = np.zeros_like(x)
+    ctx.Lap_vec_mult(0.3, x, y)
+    ref = Oracle(grid, None).lap_plus_diag(1.0, 0.0, 0.3, None, x)
+    fin = np.isfinite(ref)
+    assert np.array_equal(np.isfinite(y), fin) and np.array_equal(np.isnan(y), np.isnan(ref))
+    S = 3 * (abs(c[0]) + 2 * np.abs(c[1:]).sum()) + 0.3
+    assert np.abs((y - ref)[fin]).max() <= 40 * 2.0 ** -53 * S
+    ctx.close()

@@ -29,8 +29,8 @@ const float *veff_of<float>(sgpu_ctx *ctx, int spin)
 }
 
 // alpha_in (optional): dV * Gamma * Chiᵀ x already formed (ld nonlocal_alpha_ld), so no
-// projection is launched; alpha_out (optional, FP32 with alpha_in): receives dV * Gamma * Chiᵀ
-// of the finished hx from the fused range apply, for the next filter degree.
+// projection is launched; alpha_out (optional, with alpha_in): receives dV * Gamma * Chiᵀ of the
+// finished hx from the fused range apply, for the next filter degree.
 template <typename T>
 int hamiltonian_dev(sgpu_ctx *ctx, int spin, int ncol, double c, const T *x, long ldx, T *hx,
                     long ldh, double s1, double s2, const T *z, long ldz, cudaStream_t st,
@@ -46,7 +46,8 @@ int hamiltonian_dev(sgpu_ctx *ctx, int spin, int ncol, double c, const T *x, lon
     if (!alpha && ctx->has_nl && ctx->nl.ntot > 0) {
         T *a = nullptr;
         SGPU_TRY(ws_get(ctx, WS_ALPHA, abytes, (void **)&a));
-        SGPU_CUDA_TRY(cudaMemsetAsync(a, 0, abytes, st));
+        if (sizeof(T) == 4 || !nonlocal_fx_ready(ctx))  // the fixed-point form writes alpha
+            SGPU_CUDA_TRY(cudaMemsetAsync(a, 0, abytes, st));
         SGPU_TRY(launch_nonlocal_project<T>(ctx, ncol, x, ldx, a, lda, st));
         alpha = a;
     }
@@ -60,6 +61,8 @@ int hamiltonian_dev(sgpu_ctx *ctx, int spin, int ncol, double c, const T *x, lon
             return launch_nonlocal_apply_project(ctx, ncol, alpha, lda, s1, hx, ldh, alpha_out,
                                                  st);
         }
+    } else if (alpha_out) {
+        return launch_nonlocal_fx_apply(ctx, ncol, alpha, lda, s1, hx, ldh, alpha_out, st);
     }
     return launch_nonlocal_apply<T>(ctx, ncol, alpha, lda, s1, hx, ldh, st);
 }
@@ -69,20 +72,22 @@ bool filter_fuses_projection(sgpu_ctx *ctx)
     return ctx->nl_fuse && ctx->has_nl && ctx->nl.ntot > 0 && ctx->nl.nrange > 0;
 }
 
-// The FP32 filter's projection buffers when the projections are carried across degrees:
+// The filter's projection buffers when the projections are carried across degrees:
 // A = dV * Gamma * Chiᵀ X (one projection launch), B the buffer the fused applies alternate
-// with. Both null when the filter does not fuse.
-static int carried_alpha(sgpu_ctx *ctx, int ncol, const float *X, long ldx, float **A, float **B,
+// with. Both null when the filter does not fuse: FP32 as tuned, FP64 whenever the fixed-point
+// tables exist (a fused launch saves the covered points' read and conversion of every degree).
+template <typename T>
+static int carried_alpha(sgpu_ctx *ctx, int ncol, const T *X, long ldx, T **A, T **B,
                          cudaStream_t st)
 {
     *A = *B = nullptr;
-    if (!filter_fuses_projection(ctx)) return SGPU_OK;
-    const long lda = nonlocal_alpha_ld(ncol, 4);
-    const size_t bytes = sizeof(float) * (size_t)ctx->nl.ntot * lda;
+    if (sizeof(T) == 4 ? !filter_fuses_projection(ctx) : !nonlocal_fx_ready(ctx)) return SGPU_OK;
+    const long lda = nonlocal_alpha_ld(ncol, (int)sizeof(T));
+    const size_t bytes = sizeof(T) * (size_t)ctx->nl.ntot * lda;
     SGPU_TRY(ws_get(ctx, WS_ALPHA, bytes, (void **)A));
     SGPU_TRY(ws_get(ctx, WS_ALPHA2, bytes, (void **)B));
-    SGPU_CUDA_TRY(cudaMemsetAsync(*A, 0, bytes, st));
-    return launch_nonlocal_project<float>(ctx, ncol, X, ldx, *A, lda, st);
+    if (sizeof(T) == 4) SGPU_CUDA_TRY(cudaMemsetAsync(*A, 0, bytes, st));
+    return launch_nonlocal_project<T>(ctx, ncol, X, ldx, *A, lda, st);
 }
 
 // On return the filtered block is in Y and the degree m-1 iterate in X, as in the reference.
@@ -109,10 +114,10 @@ int chebyshev_dev(sgpu_ctx *ctx, int spin, T *X, long ldx, T *Y, long ldy, int n
     const bool route = ((m - 1) % 2) == 1;
     if (route) SGPU_TRY(ws_get(ctx, WS_STAGE_C, sizeof(T) * (size_t)Nd * ncol, (void **)&W));
 
-    // FP32 with the fused range apply: each degree's apply also projects its finished output
-    // for the next degree, alternating between two projection buffers
+    // with the fused range apply each degree's apply also projects its finished output for the
+    // next degree, alternating between two projection buffers
     T *acur = nullptr, *anext = nullptr;
-    if constexpr (sizeof(T) == 4) SGPU_TRY(carried_alpha(ctx, ncol, X, ldx, &acur, &anext, st));
+    SGPU_TRY(carried_alpha(ctx, ncol, X, ldx, &acur, &anext, st));
 
     // Y_0 = (sigma1/e) (H - c I) X
     T *y0 = route ? W : Y;

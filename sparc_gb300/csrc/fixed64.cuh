@@ -45,12 +45,21 @@ __device__ __forceinline__ int2 to_digits(double x, int E)
     return make_int2(h * sg, l * sg);
 }
 
-// hh += h Wh, mid += h Wl + l Wh (l Wl is below 2^-58 of the product's scale)
+// hh += h Wh, mid += h Wl + l Wh (l Wl is below 2^-58 of the product's scale). The plain C product of
+// widened operands is not safe here: with a loop-invariant operand the compiler hoists its sign
+// extension and multiplies 64 by 64 bits (a nonlocal apply of 27 products took 119 multiply-pipe
+// instructions per entry).
+__device__ __forceinline__ long long mad_wide(int a, int b, long long c)
+{
+    long long d;
+    asm("mul.wide.s32 %0, %1, %2;" : "=l"(d) : "r"(a), "r"(b));
+    return c + d;
+}
 __device__ __forceinline__ void mac(long long &hh, long long &mid, int h, int l, int Wh, int Wl)
 {
-    hh += (long long)h * Wh;
-    mid += (long long)h * Wl;
-    mid += (long long)l * Wh;
+    hh = mad_wide(h, Wh, hh);
+    mid = mad_wide(h, Wl, mid);
+    mid = mad_wide(l, Wh, mid);
 }
 
 // the sum hh 2^58 + mid 2^29 in units of 2^(29 + kDrop)

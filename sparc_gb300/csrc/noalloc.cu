@@ -133,7 +133,8 @@ extern "C" int sgpu_Vnl_vec_mult_noalloc(sgpu_ctx *ctx, int ncol, const double *
     SGPU_TRY(noalloc_scratch(&alpha));
     // the array keeps the previous call's contents: clear the part this call accumulates into
     SGPU_CUDA_TRY(cudaMemsetAsync(alpha, 0, sizeof(double) * (size_t)need, ctx->stream));
-    SGPU_TRY(launch_nonlocal_project<double>(ctx, ncol, x, ldi, alpha, lda, ctx->stream));
+    SGPU_TRY(launch_nonlocal_project<double>(ctx, ncol, x, ldi, alpha, lda, ctx->stream,
+                                             false));
     SGPU_TRY(launch_nonlocal_apply<double>(ctx, ncol, alpha, lda, 1.0, Hx, ldo, ctx->stream));
     SGPU_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     return SGPU_OK;

@@ -916,7 +916,7 @@ int launch_nonlocal_project_plain(sgpu_ctx *ctx, int ncol, const double *x, long
 
 template <typename T>
 int launch_nonlocal_project(sgpu_ctx *ctx, int ncol, const T *x, long ldx, T *alpha, long lda,
-                            cudaStream_t st)
+                            cudaStream_t st, bool fixed)
 {
     const Nonlocal &nl = ctx->nl;
     if (!ctx->has_nl || nl.nimg == 0 || ncol <= 0) return SGPU_OK;
@@ -932,6 +932,9 @@ int launch_nonlocal_project(sgpu_ctx *ctx, int ncol, const T *x, long ldx, T *al
             return SGPU_OK;
         }
     }
+    if constexpr (sizeof(T) == 8)
+        if (fixed && nonlocal_fx_ready(ctx))
+            return launch_nonlocal_fx_project(ctx, ncol, x, ldx, alpha, lda, st);
     return project_segments<T>(ctx, ncol, x, ldx, alpha, lda, gamma_of<T>(nl), (T)ctx->dV, st);
 }
 
@@ -941,6 +944,9 @@ int launch_nonlocal_apply(sgpu_ctx *ctx, int ncol, const T *alpha, long lda, dou
 {
     const Nonlocal &nl = ctx->nl;
     if (!ctx->has_nl || nl.ncov == 0 || ncol <= 0) return SGPU_OK;
+    if constexpr (sizeof(T) == 8)
+        if (nonlocal_fx_ready(ctx))
+            return launch_nonlocal_fx_apply(ctx, ncol, alpha, lda, scale, out, ldo, nullptr, st);
     constexpr int CB = apply_cb<T>();
     constexpr int VW = sizeof(T) == 4 ? 4 : 2;
     constexpr int SCB = sizeof(T) == 4 ? 32 : 16;  // columns per block of the staged form
@@ -1041,9 +1047,9 @@ int launch_nonlocal_apply(sgpu_ctx *ctx, int ncol, const T *alpha, long lda, dou
 }
 
 template int launch_nonlocal_project<double>(sgpu_ctx *, int, const double *, long, double *,
-                                             long, cudaStream_t);
+                                             long, cudaStream_t, bool);
 template int launch_nonlocal_project<float>(sgpu_ctx *, int, const float *, long, float *, long,
-                                            cudaStream_t);
+                                            cudaStream_t, bool);
 int launch_nonlocal_apply_project(sgpu_ctx *ctx, int ncol, const float *alpha, long lda,
                                   double scale, float *out, long ldo, float *alpha_next,
                                   cudaStream_t st)
@@ -1108,7 +1114,9 @@ void nonlocal_free(Nonlocal &nl)
                     nl.rng_pt0,  nl.rng_ent0, nl.rng_item0, nl.item_e0, nl.item_row,
                     nl.item_wsplit,
                     nl.pe_lp,    nl.pe_chi32, nl.tc_pt0, nl.tc_pts, nl.tc_row0, nl.tc_rows,
-                    nl.tc_ent0,  nl.tc_ent,   nl.tc_chi};
+                    nl.tc_ent0,  nl.tc_ent,   nl.tc_chi,   nl.fx_pt0, nl.fx_pts, nl.fx_item0,
+                    nl.fx_ent0,  nl.fx_items, nl.fx_wsplit, nl.fx_lp, nl.fx_chi,  nl.fx_er,
+                    nl.fx_row0,  nl.fx_sum_ptr, nl.fx_sum_idx, nl.fx_rows};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     nl = Nonlocal();
@@ -1345,8 +1353,9 @@ int nonlocal_upload(sgpu_ctx *ctx, int natom, const int *ip_displ, const double 
     UP(pe_lp, pe_lp.data(), pe_lp.size());
     UP(pe_chi32, pe_chi.data(), pe_chi.size());
 #undef UP
-    if (rc == SGPU_OK)
-        rc = nonlocal_tc_build(nl, ctx->Nx, ctx->Ny, covpts, covptr, ent_chi, ent_meta, chi);
+    const std::vector<int> ord = compact_order(ctx->Nx, ctx->Ny, covpts);
+    if (rc == SGPU_OK) rc = nonlocal_tc_build(nl, ord, covpts, covptr, ent_chi, ent_meta, chi);
+    if (rc == SGPU_OK) rc = nonlocal_fx_build(nl, ord, covpts, covptr, ent_chi, ent_meta, chi);
     if (rc != SGPU_OK) {
         nonlocal_free(nl);
         return rc;

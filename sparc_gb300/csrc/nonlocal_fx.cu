@@ -1,0 +1,311 @@
+// FP64 nonlocal apply and projection in block fixed point: range tables and launches
+// (the kernel body is in nonlocal_fx.cuh).
+#include <algorithm>
+#include <cmath>
+#include <type_traits>
+#include <vector>
+
+#include "nonlocal_fx.cuh"
+
+namespace sgpu {
+namespace {
+
+template <bool APPLY, bool PROJ, int MAXJ>
+__global__ void __launch_bounds__(32 * nlfx::kWarps, 2)
+    k_nl_fx(const nlfx::Tables T, int ncol, const double *__restrict__ alpha, double scale,
+            double *out, const double *__restrict__ x, long ld, double *__restrict__ part,
+            long lda, long ldp)
+{
+    extern __shared__ __align__(16) unsigned char smem_nlfx[];
+    nlfx::block<false, APPLY, PROJ, MAXJ>(T, blockIdx.y, blockIdx.x, gridDim.x, ncol, alpha, scale,
+                                          out, x, ld, part, lda, ldp, nullptr, smem_nlfx);
+}
+
+// alpha[row] = dV Gamma[row] times the sum of the row's partial projections, in the order of ptr/idx;
+// n: doubles per row
+__global__ void k_fx_reduce(const int *__restrict__ ptr, const int *__restrict__ idx,
+                            const double *__restrict__ part, long ldp, int n, double dV,
+                            const double *__restrict__ gamma, double *__restrict__ alpha, long lda)
+{
+    const int row = blockIdx.y;
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= n) return;
+    const int e1 = ptr[row + 1];
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    int e = ptr[row];
+    for (; e + 4 <= e1; e += 4)
+#pragma unroll
+        for (int u = 0; u < 4; u++) s[u] += __ldg(part + (long)idx[e + u] * ldp + c);
+    for (; e < e1; e++) s[0] += __ldg(part + (long)idx[e] * ldp + c);
+    alpha[(long)row * lda + c] = dV * gamma[row] * ((s[0] + s[1]) + (s[2] + s[3]));
+}
+
+// Chi digits of the entries: value j of entry e is chi[src[e].x + j * src[e].y] scaled by its row's
+// 2^er, rounded to kChiBits bits
+__global__ void k_fx_chi(const long2 *__restrict__ src, const int2 *__restrict__ rows, long nent,
+                         int jp, const double *__restrict__ chi, const int *__restrict__ er,
+                         int2 *__restrict__ out)
+{
+    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < nent * jp;
+         i += (long)gridDim.x * blockDim.x) {
+        const long e = i / jp;
+        const int j = (int)(i - e * jp);
+        const int2 row = rows[e];  // (first projector row, count)
+        int2 d = make_int2(0, 0);
+        if (j < row.y) {
+            const long long C =
+                llrint(ldexp(chi[src[e].x + j * src[e].y], nlfx::kChiBits - er[row.x + j]));
+            const long long H = (C + (1ll << (fx::kDigit - 1))) >> fx::kDigit;
+            d = make_int2((int)H, (int)(C - (H << fx::kDigit)));
+        }
+        out[i] = d;
+    }
+}
+
+template <bool APPLY, bool PROJ>
+int launch(sgpu_ctx *ctx, int ncol, const double *alpha, double scale, double *out,
+           const double *x, long ld, double *alpha_next, long lda, cudaStream_t st)
+{
+    const Nonlocal &nl = ctx->nl;
+    const nlfx::Tables T = nonlocal_fx_tables(nl);
+    const size_t smem = nlfx::smem_bytes(T);
+    auto kern = nl.max_np <= 9 ? k_nl_fx<APPLY, PROJ, 9> : k_nl_fx<APPLY, PROJ, 18>;
+    SGPU_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)smem));
+    const int groups = (ncol + nlfx::kLanes - 1) / nlfx::kLanes;
+    const long ldp = (long)groups * nlfx::kLanes;
+    double *part = nullptr;
+    if (PROJ)
+        SGPU_TRY(ws_get(ctx, WS_NLPART, sizeof(double) * (size_t)nl.fx_nrows * ldp, (void **)&part));
+    {
+        ProfScope ps(ctx, APPLY ? SGPU_KERNEL_NL_APPLY : SGPU_KERNEL_NL_PROJECT, st);
+        for (int r0 = 0; r0 < nl.fx_nrange; r0 += 65535) {
+            nlfx::Tables R = T;
+            R.pt0 += r0;
+            R.item0 += r0;
+            R.row0 += r0;
+            // blocks of few ranges split the column groups, so that there are at least 8 per SM
+            const int gx = std::min(groups, std::max(1, 152 * 8 / nl.fx_nrange));
+            const dim3 grid(gx, std::min(65535, nl.fx_nrange - r0));
+            kern<<<grid, 32 * nlfx::kWarps, smem, st>>>(R, ncol, alpha, scale, out, x, ld, part,
+                                                        lda, ldp);
+        }
+        SGPU_CUDA_TRY(cudaGetLastError());
+    }
+    if (PROJ) {
+        ProfScope ps(ctx, SGPU_KERNEL_NL_PROJECT, st);
+        const int bx = ncol <= 64 ? 32 : 128;
+        k_fx_reduce<<<dim3((ncol + bx - 1) / bx, nl.ntot), bx, 0, st>>>(
+            nl.fx_sum_ptr, nl.fx_sum_idx, part, ldp, ncol, ctx->dV, nl.gamma64, alpha_next, lda);
+        SGPU_CUDA_TRY(cudaGetLastError());
+    }
+    return SGPU_OK;
+}
+
+}  // namespace
+
+nlfx::Tables nonlocal_fx_tables(const Nonlocal &nl)
+{
+    return {nl.fx_pt0, nl.fx_pts, nl.fx_item0, nl.fx_items, nl.fx_ent0, nl.fx_wsplit, nl.fx_lp,
+            nl.fx_chi, nl.fx_rows, nl.fx_row0, nl.fx_jp, nl.fx_max_rows, nl.fx_max_ent,
+            nl.fx_max_items};
+}
+
+bool nonlocal_fx_ready(const sgpu_ctx *ctx) { return ctx->has_nl && ctx->nl.fx_nrange > 0; }
+
+int launch_nonlocal_fx_project(sgpu_ctx *ctx, int ncol, const double *x, long ldx, double *alpha,
+                               long lda, cudaStream_t st)
+{
+    return launch<false, true>(ctx, ncol, nullptr, 0.0, nullptr, x, ldx, alpha, lda, st);
+}
+
+int launch_nonlocal_fx_apply(sgpu_ctx *ctx, int ncol, const double *alpha, long lda, double scale,
+                             double *out, long ldo, double *alpha_next, cudaStream_t st)
+{
+    if (alpha_next)
+        return launch<true, true>(ctx, ncol, alpha, scale, out, nullptr, ldo, alpha_next, lda, st);
+    return launch<true, false>(ctx, ncol, alpha, scale, out, nullptr, ldo, nullptr, lda, st);
+}
+
+// Range tables. A range takes covered points in the order of 32 x 4 x 4 blocks of the grid until it
+// holds `cap` of them or the next point's images would take its rows past kRows or its Chi digits
+// past kChiBytes; cap is the
+// largest of 128, 64 and 32 that still gives two blocks per SM for one column group, so small
+// cells spread over the chip. No tables (and the FP64 kernels stay) for more than 18 projectors
+// per atom, for a point under more than kPtRows projector rows (the 64-bit sums hold that many)
+// and for Chi values outside 1e-40 .. 1e40.
+int nonlocal_fx_build(Nonlocal &nl, const std::vector<int> &ord, const std::vector<int> &covpts,
+                      const std::vector<int> &covptr, const std::vector<long> &ent_chi,
+                      const std::vector<int4> &ent_meta, const double *chi)
+{
+    nl.fx_nrange = 0;
+    if (nl.max_np > 18 || nl.max_np < 1 || nl.ncov == 0) return SGPU_OK;
+    // exponent of each projector row's largest Chi value
+    std::vector<int> er(nl.ntot, 0);
+    {
+        std::vector<double> mx(nl.ntot, 0.0);
+        for (long e = 0; e < nl.nent; e++) {
+            const int4 m = ent_meta[e];
+            for (int j = 0; j < m.y; j++) {
+                const double v = std::fabs(chi[ent_chi[e] + (long)j * m.z]);
+                if (!(v < 1e40)) return SGPU_OK;  // NaN too
+                mx[m.x + j] = std::max(mx[m.x + j], v);
+            }
+        }
+        for (int i = 0; i < nl.ntot; i++) {
+            if (mx[i] == 0.0) continue;
+            if (mx[i] < 1e-40) return SGPU_OK;
+            std::frexp(mx[i], &er[i]);
+        }
+    }
+    int cap = nlfx::kPts;
+    while (cap > 32 && nl.ncov < cap * 304) cap /= 2;
+
+    std::vector<int> pt0(1, 0), pts, item0(1, 0), ent0(1, 0), row0(1, 0), wsplit;
+    std::vector<int4> items, rowinfo;
+    std::vector<unsigned char> lp;
+    std::vector<long2> src;
+    std::vector<int2> rows;
+    pts.reserve(nl.ncov);
+    lp.reserve(nl.nent);
+    src.reserve(nl.nent);
+    rows.reserve(nl.nent);
+    std::vector<int> slot(nl.nimg, -1);                 // image -> item of the current range
+    std::vector<std::vector<std::pair<int, int>>> bucket;  // per item: (point, entry)
+    nl.fx_jp = nl.max_np <= 9 ? 10 : 18;
+    const int max_ent = nlfx::kChiBytes / (8 * nl.fx_jp);
+    int k = 0;
+    nl.fx_max_rows = nl.fx_max_ent = nl.fx_max_items = 0;
+    while (k < nl.ncov) {
+        const int q0 = k;
+        int nrow = 0, nitem = 0, nent = 0;
+        std::vector<int> imgs;
+        while (k < nl.ncov && k - q0 < cap) {
+            const int c = ord[k];
+            int add = 0, here = 0;
+            for (int e = covptr[c]; e < covptr[c + 1]; e++) {
+                here += ent_meta[e].y;
+                if (slot[ent_meta[e].w] < 0) add += ent_meta[e].y;
+            }
+            if (here > nlfx::kPtRows) return SGPU_OK;
+            if (nrow + add > nlfx::kRows || nent + covptr[c + 1] - covptr[c] > max_ent) break;
+            nent += covptr[c + 1] - covptr[c];
+            for (int e = covptr[c]; e < covptr[c + 1]; e++) {
+                const int g = ent_meta[e].w;
+                if (slot[g] < 0) {
+                    slot[g] = nitem++;
+                    imgs.push_back(g);
+                    if ((int)bucket.size() < nitem) bucket.emplace_back();
+                    bucket[slot[g]].clear();
+                    nrow += ent_meta[e].y;
+                }
+                bucket[slot[g]].push_back({k - q0, e});
+            }
+            pts.push_back(covpts[c]);
+            k++;
+        }
+        if (k == q0) return SGPU_OK;
+        nl.fx_max_rows = std::max(nl.fx_max_rows, nrow);
+        nl.fx_max_ent = std::max(nl.fx_max_ent, nent);
+        nl.fx_max_items = std::max(nl.fx_max_items, nitem);
+        // owner warps of the apply: runs of points with about equal entry counts
+        int wb[nlfx::kWarps + 1];
+        {
+            long tot = 0, seen = 0;
+            for (int q = q0; q < k; q++) tot += covptr[ord[q] + 1] - covptr[ord[q]];
+            wb[0] = 0;
+            int q = q0;
+            for (int w = 1; w < nlfx::kWarps; w++) {
+                while (q < k && seen < tot * w / nlfx::kWarps) {
+                    seen += covptr[ord[q] + 1] - covptr[ord[q]];
+                    q++;
+                }
+                wb[w] = q - q0;
+            }
+            wb[nlfx::kWarps] = k - q0;
+        }
+        int off = 0;
+        for (int i = 0; i < nitem; i++) {
+            const int4 m0 = ent_meta[bucket[i][0].second];
+            items.push_back(make_int4(off, m0.x, m0.y, imgs[i]));
+            off += m0.y;
+            for (int j = 0; j < m0.y; j++)
+                rowinfo.push_back(make_int4(m0.x + j, imgs[i], er[m0.x + j], 0));
+            const int first = (int)lp.size();
+            for (const auto &b : bucket[i]) {
+                const int4 m = ent_meta[b.second];
+                lp.push_back((unsigned char)b.first);
+                src.push_back({ent_chi[b.second], (long)m.z});
+                rows.push_back(make_int2(m.x, m.y));
+            }
+            for (int w = 0, e = first; w <= nlfx::kWarps; w++) {
+                while (e < (int)lp.size() && (w == nlfx::kWarps || lp[e] < wb[w])) e++;
+                wsplit.push_back(e);
+            }
+            ent0.push_back((int)lp.size());
+            slot[imgs[i]] = -1;
+        }
+        pt0.push_back(k);
+        item0.push_back((int)items.size());
+        row0.push_back(row0.back() + nrow);
+    }
+    // per projector row, its rows of the partial buffer in range order
+    nl.fx_nrows = row0.back();
+    std::vector<int> sum_ptr(nl.ntot + 1, 0), sum_idx(nl.fx_nrows);
+    for (const int4 &I : items)
+        for (int j = 0; j < I.z; j++) sum_ptr[I.y + j + 1]++;
+    for (int i = 0; i < nl.ntot; i++) sum_ptr[i + 1] += sum_ptr[i];
+    {
+        std::vector<int> at(sum_ptr.begin(), sum_ptr.end() - 1);
+        for (size_t r = 0; r + 1 < item0.size(); r++)
+            for (int i = item0[r]; i < item0[r + 1]; i++)
+                for (int j = 0; j < items[i].z; j++)
+                    sum_idx[at[items[i].y + j]++] = row0[r] + items[i].x + j;
+    }
+    int rc = SGPU_OK;
+    auto up = [&](auto **dst, const auto &v) {
+        using T = std::remove_reference_t<decltype(v[0])>;
+        if (rc != SGPU_OK) return;
+        if (cudaMalloc((void **)dst, sizeof(T) * std::max<size_t>(v.size(), 1)) != cudaSuccess ||
+            (!v.empty() && cudaMemcpy((void *)*dst, v.data(), sizeof(T) * v.size(),
+                                      cudaMemcpyHostToDevice) != cudaSuccess)) {
+            set_error("set_nonlocal: device allocation of the fixed-point range tables failed");
+            rc = SGPU_ERR_CUDA;
+        }
+    };
+    long2 *dsrc = nullptr;
+    int2 *drows = nullptr;
+    up(&nl.fx_pt0, pt0);
+    up(&nl.fx_pts, pts);
+    up(&nl.fx_item0, item0);
+    up(&nl.fx_items, items);
+    up(&nl.fx_ent0, ent0);
+    up(&nl.fx_wsplit, wsplit);
+    up(&nl.fx_lp, lp);
+    up(&nl.fx_er, er);
+    up(&nl.fx_rows, rowinfo);
+    up(&nl.fx_row0, row0);
+    up(&nl.fx_sum_ptr, sum_ptr);
+    up(&nl.fx_sum_idx, sum_idx);
+    up(&dsrc, src);
+    up(&drows, rows);
+    const size_t cbytes = sizeof(int2) * (size_t)nl.nent * nl.fx_jp;
+    if (rc == SGPU_OK && cudaMalloc((void **)&nl.fx_chi, cbytes) != cudaSuccess) {
+        set_error("set_nonlocal: device allocation of the Chi digits failed");
+        rc = SGPU_ERR_CUDA;
+    }
+    if (rc == SGPU_OK) {
+        k_fx_chi<<<152 * 8, 256>>>(dsrc, drows, nl.nent, nl.fx_jp, nl.chi64, nl.fx_er,
+                                   reinterpret_cast<int2 *>(nl.fx_chi));
+        if (cudaDeviceSynchronize() != cudaSuccess) {
+            set_error("set_nonlocal: the Chi digit kernel failed");
+            rc = SGPU_ERR_CUDA;
+        }
+    }
+    if (dsrc) cudaFree(dsrc);
+    if (drows) cudaFree(drows);
+    if (rc == SGPU_OK) nl.fx_nrange = (int)pt0.size() - 1;
+    return rc;
+}
+
+}  // namespace sgpu

@@ -432,7 +432,23 @@ int launch_nonlocal_apply_project_tc(sgpu_ctx *ctx, int ncol, const float *alpha
 // one covered point alone needs more than kTcRows rows no tables are built and the form is
 // unavailable.
 constexpr int kTcBx = 32, kTcBy = 4, kTcBz = 4;
-int nonlocal_tc_build(Nonlocal &nl, int Nx, int Ny, const std::vector<int> &covpts,
+std::vector<int> compact_order(int Nx, int Ny, const std::vector<int> &covpts)
+{
+    const long nbx = (Nx + kTcBx - 1) / kTcBx, nby = (Ny + kTcBy - 1) / kTcBy;
+    std::vector<std::pair<long long, int>> key(covpts.size());
+    for (size_t c = 0; c < covpts.size(); c++) {
+        const long g = covpts[c];
+        const long x = g % Nx, y = (g / Nx) % Ny, z = g / ((long)Nx * Ny);
+        const long blk = ((z / kTcBz) * nby + y / kTcBy) * nbx + x / kTcBx;
+        const long in = ((z % kTcBz) * kTcBy + y % kTcBy) * kTcBx + x % kTcBx;
+        key[c] = {(long long)blk * (kTcBx * kTcBy * kTcBz) + in, (int)c};
+    }
+    std::sort(key.begin(), key.end());
+    std::vector<int> ord(covpts.size());
+    for (size_t c = 0; c < ord.size(); c++) ord[c] = key[c].second;
+    return ord;
+}
+int nonlocal_tc_build(Nonlocal &nl, const std::vector<int> &ord, const std::vector<int> &covpts,
                       const std::vector<int> &covptr, const std::vector<long> &ent_chi,
                       const std::vector<int4> &ent_meta, const double *chi)
 {
@@ -442,21 +458,6 @@ int nonlocal_tc_build(Nonlocal &nl, int Nx, int Ny, const std::vector<int> &covp
     if (nl.max_np > jp || nl.max_np > kTcRows) {  // an atom's rows exceed an entry or a range
         nl.tc_nrange = 0;
         return SGPU_OK;
-    }
-    // covered points in block order
-    std::vector<int> ord(nl.ncov);
-    {
-        const long nbx = (Nx + kTcBx - 1) / kTcBx, nby = (Ny + kTcBy - 1) / kTcBy;
-        std::vector<long long> key(nl.ncov);
-        for (int c = 0; c < nl.ncov; c++) {
-            const long g = covpts[c];
-            const long x = g % Nx, y = (g / Nx) % Ny, z = g / ((long)Nx * Ny);
-            const long blk = ((z / kTcBz) * nby + y / kTcBy) * nbx + x / kTcBx;
-            const long in = ((z % kTcBz) * kTcBy + y % kTcBy) * kTcBx + x % kTcBx;
-            key[c] = (long long)blk * (kTcBx * kTcBy * kTcBz) + in;
-            ord[c] = c;
-        }
-        std::sort(ord.begin(), ord.end(), [&](int a, int b) { return key[a] < key[b]; });
     }
     std::unordered_map<int, int> rowoff;  // atom (its first projector row) -> range row offset
     std::vector<double> acc(jp);

@@ -107,6 +107,16 @@ struct Nonlocal {
     int *tc_ent0 = nullptr;     // tc_nrange + 1: first merged entry of each range
     int *tc_ent = nullptr;      // point | row offset << 7 | projector count << 14
     float *tc_chi = nullptr;    // Chi values of the merged entries, range_jp per entry
+    // FP64 apply and projection in block fixed point (nonlocal_fx.cuh); fx_nrange 0: no tables
+    int fx_nrange = 0, fx_jp = 0, fx_max_rows = 0, fx_max_ent = 0, fx_max_items = 0,
+        fx_nrows = 0;
+    int *fx_pt0 = nullptr, *fx_pts = nullptr, *fx_item0 = nullptr, *fx_ent0 = nullptr;
+    int4 *fx_items = nullptr, *fx_rows = nullptr;
+    int *fx_wsplit = nullptr;
+    unsigned char *fx_lp = nullptr;
+    int4 *fx_chi = nullptr;
+    int *fx_er = nullptr, *fx_row0 = nullptr;
+    int *fx_sum_ptr = nullptr, *fx_sum_idx = nullptr;  // projector row -> its partial rows
 };
 
 // A potential as fixed-point digits (fixed64.cuh) for the FP64 stencil; key: the exponent key of its
@@ -230,7 +240,7 @@ namespace sgpu {
 enum WsSlot {
     WS_STAGE_A = 0, WS_STAGE_B, WS_STAGE_C, WS_ALPHA, WS_MISC, WS_EIG, WS_POIS, WS_MIX,
     WS_RED, WS_RHS, WS_SCF, WS_SCF2, WS_ALPHA2, WS_SPLIT_A, WS_SPLIT_B, WS_TC_PART,
-    WS_FXPOT, WS_COUNT
+    WS_FXPOT, WS_NLPART, WS_COUNT
 };
 
 // grow-only device scratch
@@ -273,9 +283,11 @@ int fx_potential(sgpu_ctx *ctx, const double *v, double bv, long n, int2 *vd, un
 // ---- nonlocal (nonlocal.cu)
 // alpha is (ntot x lda) projector-major: alpha[row * lda + n]; lda from nonlocal_alpha_ld
 long nonlocal_alpha_ld(int ncol, int elem_bytes);
+// (alpha += unless the FP64 fixed-point form runs, which writes it; fixed = false keeps to the
+// segment kernel, which needs no workspace)
 template <typename T>
 int launch_nonlocal_project(sgpu_ctx *ctx, int ncol, const T *x, long ldx, T *alpha, long lda,
-                            cudaStream_t st);
+                            cudaStream_t st, bool fixed = true);
 // alpha += Chi^T x (no dV, no Gamma: ones holds ntot ones), the segment kernel in FP64
 int launch_nonlocal_project_plain(sgpu_ctx *ctx, int ncol, const double *x, long ldx,
                                   double *alpha, long lda, const double *ones, cudaStream_t st);
@@ -299,9 +311,22 @@ int launch_nonlocal_apply_project_tc(sgpu_ctx *ctx, int ncol, const float *alpha
                                      cudaStream_t st);
 bool nonlocal_tc_ready(const sgpu_ctx *ctx);
 // builds the tensor-core range tables from the point CSR of nonlocal_upload
-int nonlocal_tc_build(Nonlocal &nl, int Nx, int Ny, const std::vector<int> &covpts,
+int nonlocal_tc_build(Nonlocal &nl, const std::vector<int> &ord, const std::vector<int> &covpts,
                       const std::vector<int> &covptr, const std::vector<long> &ent_chi,
                       const std::vector<int4> &ent_meta, const double *chi);
+// covered points in the order of compact blocks of the grid (nonlocal_tc.cu)
+std::vector<int> compact_order(int Nx, int Ny, const std::vector<int> &covpts);
+// FP64 in block fixed point (nonlocal_fx.cu): tables from the same CSR, projection (alpha is
+// written, not added to), and the apply into out with, when alpha_next is given, the projection
+// of the finished out
+bool nonlocal_fx_ready(const sgpu_ctx *ctx);
+int nonlocal_fx_build(Nonlocal &nl, const std::vector<int> &ord, const std::vector<int> &covpts,
+                      const std::vector<int> &covptr, const std::vector<long> &ent_chi,
+                      const std::vector<int4> &ent_meta, const double *chi);
+int launch_nonlocal_fx_project(sgpu_ctx *ctx, int ncol, const double *x, long ldx, double *alpha,
+                               long lda, cudaStream_t st);
+int launch_nonlocal_fx_apply(sgpu_ctx *ctx, int ncol, const double *alpha, long lda, double scale,
+                             double *out, long ldo, double *alpha_next, cudaStream_t st);
 int nonlocal_upload(sgpu_ctx *ctx, int natom, const int *ip_displ, const double *gamma,
                     int nimg, const int *img_atom, const int *img_ndc, const int *grid_pos,
                     const double *chi);

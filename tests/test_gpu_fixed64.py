@@ -6,7 +6,7 @@ import pytest
 
 import sparc_gb300 as sg
 from oracle.oracle import Oracle
-from sparc_gb300.synthetic import fd_d2_coeffs
+from sparc_gb300.synthetic import fd_d2_coeffs, synthetic_nonlocal
 
 pytestmark = pytest.mark.gpu
 
@@ -94,4 +94,81 @@ def test_stencil_nonfinite(gpu_available):
     assert np.array_equal(np.isfinite(y), fin) and np.array_equal(np.isnan(y), np.isnan(ref))
     S = 3 * (abs(c[0]) + 2 * np.abs(c[1:]).sum()) + 0.3
     assert np.abs((y - ref)[fin]).max() <= 40 * 2.0 ** -53 * S
+    ctx.close()
+
+
+def _nonlocal_case(N, h, natom, rc, lmax, seed, dup=1):
+    """Grid, potential and projectors; dup > 1 doubles the projectors of every atom."""
+    rng = np.random.default_rng(seed)
+    c = fd_d2_coeffs(6, h)
+    grid = dict(Nx=N[0], Ny=N[1], Nz=N[2], FDn=6, cx=c, cy=c, cz=c, dV=h ** 3)
+    nl = synthetic_nonlocal(rng, N, h, natom=natom, rc=rc, lmax=lmax)
+    if dup > 1:
+        np1 = (lmax + 1) ** 2
+        nl["ip_displ"] = nl["ip_displ"] * dup
+        nl["gamma"] = np.tile(nl["gamma"].reshape(natom, np1), (1, dup)).reshape(-1)
+        out, o = [], 0
+        for n in nl["img_ndc"]:
+            blk = nl["chi"][o:o + n * np1]
+            out += [blk] + [blk * 10.0 ** -(3 * k) for k in range(1, dup)]
+            o += n * np1
+        nl["chi"] = np.concatenate(out)
+    ctx = sg.Context(*N, 6, c, c, c, h ** 3)
+    ctx.set_nonlocal(nl["ip_displ"], nl["gamma"], nl["img_atom"], nl["img_ndc"], nl["grid_pos"],
+                     nl["chi"])
+    return ctx, Oracle(grid, nl), rng, nl
+
+
+@pytest.mark.parametrize("natom,rc,lmax,dup", [(1, 1.3, 0, 1), (5, 2.0, 2, 1), (6, 2.2, 2, 2),
+                                               (9, 4.5, 2, 1), (24, 4.5, 2, 2)])
+def test_nonlocal_products(gpu_available, natom, rc, lmax, dup):
+    """One projector, 9, 18 (the second half a thousandth of the first), spheres that wrap and
+    overlap, and more rows over a point than the fixed-point sums hold (the FP64 kernels stay);
+    column counts around the group of 32 and over columns of very different size. The error of a
+    column is at most that of the two FP64 contractions: n 2^-53 times the products' magnitudes,
+    with n the points of a sphere plus the rows over a point."""
+    N, h = (21, 18, 26), 0.45
+    ctx, o, rng, nl = _nonlocal_case(N, h, natom, rc, lmax, 3 + natom, dup)
+    Nd = N[0] * N[1] * N[2]
+    absnl = dict(nl, chi=np.abs(nl["chi"]), gamma=np.abs(nl["gamma"]))
+    oabs = Oracle(dict(Nx=N[0], Ny=N[1], Nz=N[2], FDn=6, cx=np.zeros(7), cy=np.zeros(7),
+                       cz=np.zeros(7), dV=h ** 3), absnl)
+    rows = np.bincount(nl["grid_pos"], minlength=Nd).max() * (lmax + 1) ** 2 * dup
+    n = nl["img_ndc"].max() + rows
+    for ncol in (1, 31, 33, 70):
+        x = rng.uniform(-1, 1, (ncol, Nd)) * 10.0 ** rng.uniform(-6, 6, (ncol, 1))
+        y = np.zeros_like(x)
+        ctx.Vnl_vec_mult(x, y)
+        ref = o.vnl(x)
+        size = oabs.vnl(np.abs(x)).max(axis=1)
+        assert np.all(np.abs(y - ref).max(axis=1) <= n * 2.0 ** -53 * size), ncol
+        if rows <= 128:  # the fixed-point form adds in a fixed order (the FP64 one by atomics)
+            y2 = np.zeros_like(x)
+            ctx.Vnl_vec_mult(x, y2)
+            assert np.array_equal(y, y2)
+    ctx.close()
+
+
+def test_nonlocal_nonfinite_columns(gpu_available):
+    """NaN, infinities and extreme exponents stay in their own columns."""
+    N, h = (21, 18, 26), 0.45
+    ctx, o, rng, _ = _nonlocal_case(N, h, 6, 2.4, 2, 11)
+    Nd = N[0] * N[1] * N[2]
+    x = rng.uniform(-1, 1, (40, Nd))
+    ref = o.vnl(x)
+    x[3] *= 1e-300
+    x[5, :] = np.nan
+    x[7, ::5] = np.inf
+    x[33] *= 1e290
+    x[36] = 0.0
+    y = np.zeros_like(x)
+    ctx.Vnl_vec_mult(x, y)
+    keep = [i for i in range(40) if i not in (3, 5, 7, 33, 36)]
+    big = np.abs(ref).max()
+    assert np.abs(y[keep] - ref[keep]).max() <= 1e-12 * big
+    assert np.abs(y[3] * 1e300 - ref[3]).max() <= 1e-12 * big
+    assert np.abs(y[33] * 1e-290 - ref[33]).max() <= 1e-12 * big
+    covered = np.abs(ref[0]) > 0
+    assert np.all(np.isnan(y[5][covered])) and not np.any(np.isfinite(y[7][covered]))
+    assert np.all(y[36] == 0.0) and np.all(y[:, ~covered] == 0.0)
     ctx.close()

@@ -616,8 +616,10 @@ int sgpu_set_gemm_emulation(sgpu_ctx *ctx, int mode);
  * products) for FP32 blocks (sgpu_Project_Hamiltonian_f32, sgpu_Subspace_Rotation_f32, the
  * mixed SCF's FP32 phase) and FP64-accurate (6 slices, 21 products) for the mixed SCF's FP64
  * phase after the switch; plain FP64 calls (sgpu_Project_Hamiltonian,
- * sgpu_Subspace_Rotation, the plain FP64 SCF) keep cuBLAS DSYRK/DGEMM, the drop-in.
- * mode 2: the FP64-accurate tensor-core products for the plain FP64 calls too.
+ * sgpu_Subspace_Rotation, the plain FP64 SCF) use 8 slices (36 products; every level summed
+ * apart, closer to the exact products than cuBLAS DSYRK/DGEMM), except rotations of fewer than
+ * 48 columns and blocks with infinities or NaN, which go to cuBLAS.
+ * mode 2: the 6-slice products for the plain FP64 calls too.
  * mode 0: cuBLAS everywhere (sgpu_set_gemm_emulation then picks the FP32-block form).
  * The Gram products compute the upper triangle and mirror it. No counterpart in the
  * reference (which calls cblas_dgemm). */

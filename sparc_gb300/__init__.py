@@ -758,8 +758,9 @@ class Context:
         return mode.value != 0, int(mode.value), [float(ms[0]), float(ms[1])]
 
     def set_rr_products(self, mode):
-        """Rayleigh-Ritz products: 1 tensor-core split slices for FP32 blocks and the mixed
-        SCF's FP64 phase, 2 also for plain FP64 calls, 0 cuBLAS (sgpu_set_rr_products)."""
+        """Rayleigh-Ritz products: 1 tensor-core split slices for FP32 blocks (3), the mixed
+        SCF's FP64 phase (6) and plain FP64 calls (8), 2 six slices for plain FP64 calls too,
+        0 cuBLAS (sgpu_set_rr_products)."""
         _check(lib().sgpu_set_rr_products(self._h, int(mode)))
 
     def set_eig_solver(self, mode):

@@ -777,6 +777,428 @@ int rotate_impl(sgpu_ctx *ctx, int ncol, const T *Y, long ldy, const double *Q, 
     return launch_gemm<NS>(ctx, p, p.nrbA * p.nrbB, st);
 }
 
+
+// ---------------------------------------------------------------------------------------------
+// Full FP64 products (the plain FP64 calls): eight slices, 56 bits, every level summed exactly.
+//
+// cuBLAS's FP64 GEMMs run at this part's FP64 tensor rate, 1 TFLOP/s. Eight 7-bit slices hold a
+// value to 2^-57 of its row's largest, below FP64's own rounding of that value, and the 36 slice
+// products of levels i + j < 8 leave out less than 2^-56 of |a||b|. All eight level sums stay
+// apart in tensor memory (64 columns each, 128 x 64 output tiles) and are exact over a 512-long
+// chunk up to level 4 (below 2^24 units; the rounding of the higher ones is under 2^-59); the
+// chunks add up in three compensated FP32 words (72 bits).
+//
+// Slices are laid out slice-major per K step, so the slices 0 .. 7 of a 64-row B block are one
+// 512-row operand in shared memory, and slice i of A times all the slices of B that it meets is
+// one wide product whose columns land on the levels i, i + 1, ...: 12 instructions of up to 256
+// columns per 16 K values instead of 36 of 64, which would be bound by shared-memory reads of A.
+// 77^3, 520 columns: projection 547 ms (DSYRK + DGEMM) -> 10.9, rotation 239 -> 8.9 ms; of the
+// exact products (uniform columns) Mp is off by 1.3e-16 (DSYRK 2.8e-15), X by 5e-17 (2.1e-16).
+constexpr int XS = 8;                              // slices
+constexpr int XN = 64;                             // output tile columns = rows of a B block
+constexpr int XG = 256;                            // elements of an 8-row group of a K step
+constexpr unsigned XA_BYTES = TM * TK * 2;         // one slice of A's 128 rows: 8 KB
+constexpr unsigned XB_BYTES = XN * TK * 2;         // one slice of B's 64 rows: 4 KB
+constexpr unsigned XSTAGE = XS * (XA_BYTES + XB_BYTES);  // 96 KB
+constexpr int XNST = 2;
+constexpr unsigned XBAR = XNST * XSTAGE;
+constexpr unsigned XSMEM = XBAR + 16 * XNST + 32 + 1024;
+
+struct TcxParams {
+    const __nv_bfloat16 *A;  // [kstep][slice][row group][256]
+    const __nv_bfloat16 *B;
+    long ngA, ngB;           // row groups of A and B
+    int mtiles, ntiles;      // 128-row and 64-column tiles
+    int ksteps, mode, ksplit, M, N;
+    const int *eA, *eB;
+    double *C;
+    long ldc;
+    int *status;
+};
+
+// instruction descriptor with n columns (kIdesc is the 128-column one)
+__device__ __forceinline__ void mma_bf16_n(unsigned tmem_d, unsigned long long adesc,
+                                           unsigned long long bdesc, int n, unsigned accumulate)
+{
+    const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(n >> 3) << 17) |
+                           ((unsigned)(TM >> 4) << 24);
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
+// Gram work item -> (row tile, column tile): the 128 x 64 tiles that touch the upper triangle
+__device__ __forceinline__ void upper_tile(int t, int ntiles, int &mt, int &nt)
+{
+    mt = 0;
+    while (t >= ntiles - 2 * mt) {
+        t -= ntiles - 2 * mt;
+        mt++;
+    }
+    nt = 2 * mt + t;
+}
+inline int upper_tiles(int mtiles, int ntiles)
+{
+    int n = 0;
+    for (int m = 0; m < mtiles; m++) n += std::max(0, ntiles - 2 * m);
+    return n;
+}
+
+__global__ void __launch_bounds__(NTHREADS, 1) k_tc_gemm_x(const TcxParams p, int nupper)
+{
+    extern __shared__ __align__(1024) unsigned char smem[];
+    const unsigned sbase = smem_u32(smem);
+    constexpr int NST = XNST;
+    const unsigned bar_full = sbase + XBAR;
+    const unsigned bar_empty = bar_full + 8 * NST;
+    const unsigned bar_accf = bar_empty + 8 * NST;
+    const unsigned bar_acce = bar_accf + 8;
+    const unsigned bar_done = bar_accf + 16;
+    unsigned *tmem_slot = reinterpret_cast<unsigned *>(smem + XBAR + 16 * NST + 24);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + XBAR + 16 * NST + 28);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    const int ntot = p.mode == 0 ? nupper * p.ksplit : p.mtiles * p.ntiles;
+    auto tile_of = [&](int t, int &mt, int &nt, int &ks0, int &ks1, int &split) {
+        if (p.mode == 0) {
+            split = t / nupper;
+            upper_tile(t - split * nupper, p.ntiles, mt, nt);
+            const int per = (p.ksteps + p.ksplit - 1) / p.ksplit;
+            ks0 = split * per;
+            ks1 = min(p.ksteps, ks0 + per);
+        } else {
+            mt = t / p.ntiles;
+            nt = t - mt * p.ntiles;
+            ks0 = 0;
+            ks1 = p.ksteps;
+            split = 0;
+        }
+        if (ks1 < ks0) ks1 = ks0;
+    };
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < NST; s++) {
+            mbar_init(bar_full + 8 * s, 1);
+            mbar_init(bar_empty + 8 * s, 1);
+        }
+        mbar_init(bar_accf, 1);
+        mbar_init(bar_acce, EPI_WARPS);
+        mbar_init(bar_done, 1);
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    if (warp == 1) {  // 512 TMEM columns: eight levels of 64
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;\n" ::"r"(
+                         smem_u32(tmem_slot))
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const unsigned tmem = *tmem_slot;
+    auto fail = [&]() {
+        *abort_flag = 1;
+        if (p.status) atomicOr(p.status, STATUS_TC_WAIT);
+    };
+
+    if (warp == 0) {
+        // ---------------- producer: the eight slices of A's and of B's rows per K step
+        if (lane == 0) {
+            int it = 0;
+            for (int t = blockIdx.x; t < ntot && !*abort_flag; t += gridDim.x) {
+                int mt, nt, ks0, ks1, split;
+                tile_of(t, mt, nt, ks0, ks1, split);
+                for (int s = ks0; s < ks1; s++, it++) {
+                    const int st = it % NST;
+                    if (it >= NST && !mbar_wait_bounded(bar_empty + 8 * st, (it / NST - 1) & 1)) {
+                        fail();
+                        break;
+                    }
+                    if (*abort_flag) break;
+                    const unsigned dst = sbase + st * XSTAGE;
+                    mbar_arrive_tx(bar_full + 8 * st, XSTAGE);
+                    for (int i = 0; i < XS; i++) {
+                        bulk_g2s(dst + i * XA_BYTES,
+                                 p.A + (((long)s * XS + i) * p.ngA + (long)mt * (TM / 8)) * XG,
+                                 XA_BYTES, bar_full + 8 * st);
+                        bulk_g2s(dst + XS * XA_BYTES + i * XB_BYTES,
+                                 p.B + (((long)s * XS + i) * p.ngB + (long)nt * (XN / 8)) * XG,
+                                 XB_BYTES, bar_full + 8 * st);
+                    }
+                }
+            }
+            // no copy may land after the block exits: wait for the last fill of each stage
+            const int issued = it;
+            for (int st = 0; st < NST; st++) {
+                const int last = issued - 1 - ((issued - 1 - st) % NST + NST) % NST;
+                if (last >= 0 && !mbar_wait_bounded(bar_full + 8 * st, (last / NST) & 1)) fail();
+            }
+        }
+    } else if (warp == 1) {
+        // ---------------- MMA issuer
+        if (lane == 0) {
+            int it = 0, cg = 0;
+            for (int t = blockIdx.x; t < ntot && !*abort_flag; t += gridDim.x) {
+                int mt, nt, ks0, ks1, split;
+                tile_of(t, mt, nt, ks0, ks1, split);
+                const int nsteps = ks1 - ks0;
+                const int nchunks = (nsteps + CHUNK_STEPS - 1) / CHUNK_STEPS;
+                for (int c = 0; c < nchunks && !*abort_flag; c++, cg++) {
+                    if (cg > 0 && !mbar_wait_bounded(bar_acce, (cg - 1) & 1)) {
+                        fail();
+                        break;
+                    }
+                    tc_fence_after();
+                    const int cend = min(nsteps, (c + 1) * CHUNK_STEPS);
+                    for (int k = c * CHUNK_STEPS; k < cend; k++, it++) {
+                        const int st = it % NST;
+                        if (!mbar_wait_bounded(bar_full + 8 * st, (it / NST) & 1)) {
+                            fail();
+                            break;
+                        }
+                        if (*abort_flag) break;
+                        tc_fence_after();
+                        const unsigned a0 = sbase + st * XSTAGE;
+                        const unsigned b0 = a0 + XS * XA_BYTES;
+#pragma unroll
+                        for (int kk = 0; kk < 2; kk++) {
+                            const unsigned fresh = k == c * CHUNK_STEPS && kk == 0;
+#pragma unroll
+                            for (int i = 0; i < XS; i++) {
+                                const unsigned accum = fresh && i == 0 ? 0u : 1u;
+                                // B slices j of this instruction: levels i + j
+#pragma unroll
+                                for (int j = 0; j < XS - i; j += 4) {
+                                    const int nj = XS - i - j < 4 ? XS - i - j : 4;
+                                    mma_bf16_n(tmem + (i + j) * XN,
+                                               smem_desc(a0 + i * XA_BYTES + kk * 256),
+                                               smem_desc(b0 + j * XB_BYTES + kk * 256), nj * XN,
+                                               accum);
+                                }
+                            }
+                        }
+                        mma_commit(bar_empty + 8 * st);
+                    }
+                    mma_commit(bar_accf);
+                }
+            }
+            mma_commit(bar_done);
+            if (!mbar_wait_bounded(bar_done, 0)) fail();  // nothing in flight at dealloc
+        }
+    } else {
+        // ---------------- epilogue: three compensated words per output element
+        const int q = warp & 3;         // TMEM lane quarter
+        const int h = (warp - 2) >> 2;  // column half: 32 columns per warp
+        const unsigned tl = tmem + ((unsigned)(32 * q) << 16) + (unsigned)(32 * h);
+        int cg = 0;
+        for (int t = blockIdx.x; t < ntot; t += gridDim.x) {
+            int mt, nt, ks0, ks1, split;
+            tile_of(t, mt, nt, ks0, ks1, split);
+            const int nchunks = (ks1 - ks0 + CHUNK_STEPS - 1) / CHUNK_STEPS;
+            float w0[32], w1[32], w2[32];
+#pragma unroll
+            for (int c = 0; c < 32; c++) w0[c] = w1[c] = w2[c] = 0.f;
+            for (int c = 0; c < nchunks; c++, cg++) {
+                if (*abort_flag) break;
+                if (!mbar_wait_bounded(bar_accf, cg & 1)) {
+                    fail();
+                    break;
+                }
+                tc_fence_after();
+#pragma unroll
+                for (int g = 0; g < 2; g++) {
+                    auto add = [&](const float *l) {
+#pragma unroll
+                        for (int e = 0; e < 16; e++) {
+                            float s0, e0, s1, e1;
+                            two_sum(w0[16 * g + e], l[e], s0, e0);
+                            two_sum(w1[16 * g + e], e0, s1, e1);
+                            w0[16 * g + e] = s0;
+                            w1[16 * g + e] = s1;
+                            w2[16 * g + e] += e1;
+                        }
+                    };
+                    float l5[16], l[16];
+                    tmem_ld16(tl + 5 * XN + 16 * g, l5);  // levels 5 and up need no care
+                    tmem_ld16(tl + 6 * XN + 16 * g, l);
+#pragma unroll
+                    for (int e = 0; e < 16; e++) l5[e] = __fadd_rn(l5[e], l[e]);
+                    tmem_ld16(tl + 7 * XN + 16 * g, l);
+#pragma unroll
+                    for (int e = 0; e < 16; e++) l5[e] = __fadd_rn(l5[e], l[e]);
+#pragma unroll
+                    for (int a = 0; a < 5; a++) {
+                        tmem_ld16(tl + a * XN + 16 * g, l);
+                        add(l);
+                    }
+                    add(l5);
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_acce);
+            }
+            if (*abort_flag) break;
+            const int m = mt * TM + 32 * q + lane;
+            if (m < p.M) {
+                const int em = p.eA[m];
+                const int n0 = nt * XN + 32 * h;
+                double *part = p.C + (p.mode == 0 ? (long)split * p.N * p.M : 0);
+#pragma unroll
+                for (int c = 0; c < 32; c++) {
+                    const int n = n0 + c;
+                    if (n >= p.N || (p.mode == 0 && m > n)) continue;
+                    const double v = scale2((f2d_exact(w0[c]) + f2d_exact(w1[c])) + f2d_exact(w2[c]),
+                                            em + p.eB[n]);
+                    if (p.mode == 0) {  // the upper triangle, mirrored
+                        part[(long)n * p.M + m] = v;
+                        part[(long)m * p.M + n] = v;
+                    } else {
+                        p.C[(long)n * p.ldc + m] = v;
+                    }
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 1)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;\n" ::"r"(tmem)
+                     : "memory");
+}
+
+// Eight balanced 7-bit digits of x 2^-e (|x 2^-e| < 1) as BF16 numbers d_i 2^(-7(i+1)). A bias of 64
+// per digit makes them plain bit fields; a digit becomes a float by placing it below the
+// exponent of 1.5 2^23 ulps (one add, no conversion instruction).
+__device__ __forceinline__ void split8x(Bits x, int e, float (&d)[XS])
+{
+    const int sh = x.p - e + 7 * XS;
+    long long V;
+    if (sh >= 0) V = x.m << min(sh, 62);
+    else if (sh > -62) V = (x.m + (1ll << (-sh - 1))) >> (-sh);
+    else V = 0;
+    constexpr long long bias = 64ll * (1ll + (1ll << 7) + (1ll << 14) + (1ll << 21) + (1ll << 28) +
+                                       (1ll << 35) + (1ll << 42));
+    V += bias;
+#pragma unroll
+    for (int i = 0; i < XS; i++) {
+        // unit 2^(-7(i+1)): the float 1.5 2^23 units has its last bit there
+        const int base = ((127 + 23 - 7 * (i + 1)) << 23) | 0x400000;
+        const int f = i == 0 ? (int)(V >> (7 * (XS - 1)))
+                             : (int)((V >> (7 * (XS - 1 - i))) & 127) - 64;
+        d[i] = __fsub_rn(__int_as_float(base + f), __int_as_float(base));
+    }
+}
+__device__ __forceinline__ void put8x(const float (&sl)[8][XS], __nv_bfloat16 *dst, long slice)
+{
+#pragma unroll
+    for (int i = 0; i < XS; i++) {
+        unsigned w[4];
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+            const __nv_bfloat162 b = __floats2bfloat162_rn(sl[2 * t][i], sl[2 * t + 1][i]);
+            w[t] = *reinterpret_cast<const unsigned *>(&b);
+        }
+        *reinterpret_cast<uint4 *>(dst + i * slice) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+}
+
+// as k_split_cols: tile row = column n of X, K = rows k0 .. of X; slice-major layout
+__global__ void __launch_bounds__(256) k_split_cols_x(const double *__restrict__ X, long ld,
+                                                      long krows, int ncols,
+                                                      const int *__restrict__ e, const int *ek,
+                                                      int ksign, int nrb,
+                                                      __nv_bfloat16 *__restrict__ out)
+{
+    const int s = blockIdx.x / nrb, rb = blockIdx.x - s * nrb;
+    const long slice = (long)nrb * (TM / 8) * XG;
+    __nv_bfloat16 *base = out + (long)s * XS * slice + (long)rb * (TM / 8) * XG;
+    for (int u = threadIdx.x; u < TM * 4; u += blockDim.x) {
+        const int r = u >> 2, g = u & 3;
+        const int n = rb * TM + r;
+        const long k0 = (long)s * TK + g * 8;
+        const int en = n < ncols ? e[n] : 0;
+        float sl[8][XS];
+#pragma unroll
+        for (int t = 0; t < 8; t++) {
+            const long k = k0 + t;
+            const bool in = n < ncols && k < krows;
+            split8x(bits_of(in ? X[(long)n * ld + k] : 0.0), en - (ek && in ? ksign * ek[k] : 0),
+                    sl[t]);
+        }
+        put8x(sl, base + tile_off(r, g * 8), slice);
+    }
+}
+// as k_split_rows: tile row = grid point, K = columns of X scaled by 2^-ec
+__global__ void __launch_bounds__(256) k_split_rows_x(const double *__restrict__ X, long ld,
+                                                      long rows, int kcols,
+                                                      const int *__restrict__ e,
+                                                      const int *__restrict__ ec, int nrb,
+                                                      __nv_bfloat16 *__restrict__ out)
+{
+    const int s = blockIdx.x / nrb, rb = blockIdx.x - s * nrb;
+    const long slice = (long)nrb * (TM / 8) * XG;
+    __nv_bfloat16 *base = out + (long)s * XS * slice + (long)rb * (TM / 8) * XG;
+    for (int u = threadIdx.x; u < TM * 4; u += blockDim.x) {
+        const int g = u >> 7, r = u & 127;  // a warp: 32 consecutive rows, one K group
+        const long m = (long)rb * TM + r;
+        const int em = m < rows ? e[m] : 0;
+        float sl[8][XS];
+#pragma unroll
+        for (int t = 0; t < 8; t++) {
+            const int k = s * TK + g * 8 + t;
+            const bool in = m < rows && k < kcols;
+            split8x(bits_of(in ? X[(long)k * ld + m] : 0.0), em + (in ? ec[k] : 0), sl[t]);
+        }
+        put8x(sl, base + tile_off(r, g * 8), slice);
+    }
+}
+
+// a scale beyond the finite exponents: an infinity or a NaN in that row or column
+__global__ void k_nonfinite(const int *__restrict__ e, int n, int *flag)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n && e[i] > 1024) *flag = 1;
+}
+
+int launch_gemm_x(sgpu_ctx *ctx, const TcxParams &p, cudaStream_t st)
+{
+    int nsm = 0;
+    SGPU_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device));
+    const int nupper = upper_tiles(p.mtiles, p.ntiles);
+    const int ntot = p.mode == 0 ? nupper * p.ksplit : p.mtiles * p.ntiles;
+    SGPU_CUDA_TRY(cudaFuncSetAttribute(k_tc_gemm_x, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)XSMEM));
+    ProfScope ps(ctx, SGPU_KERNEL_OTHER, st);
+    k_tc_gemm_x<<<std::max(1, std::min(ntot, nsm)), NTHREADS, XSMEM, st>>>(p, nupper);
+    SGPU_CUDA_TRY(cudaGetLastError());
+    return SGPU_OK;
+}
+
+// Workspaces are bounded: the products run over ranges of grid points whose slices of one operand
+// take at most this many bytes
+constexpr size_t kXOperand = (size_t)2 << 30;
+
+int x_row_blocks(int ncol)  // 128-row blocks that cover the 128- and the 64-row tiles
+{
+    return (ncol + TM - 1) / TM;
+}
+
+// the scales of ncol columns of X into e, their non-finite ones into flag
+int x_col_scales(sgpu_ctx *ctx, const double *X, long ld, long rows, int ncol, const int *ek,
+                 int ksign, int *e, int *flag, cudaStream_t st)
+{
+    ProfScope ps(ctx, SGPU_KERNEL_OTHER, st);
+    k_colmax_exp<double><<<ncol, 256, 0, st>>>(X, ld, rows, ek, ksign, e);
+    k_nonfinite<<<(ncol + 255) / 256, 256, 0, st>>>(e, ncol, flag);
+    SGPU_CUDA_TRY(cudaGetLastError());
+    ctx->launches++;
+    return SGPU_OK;
+}
+
 }  // namespace
 
 // Hp = Yᵀ HY and Mp = Yᵀ Y (ncol x ncol, ld ncol, symmetric) for column-major Nd x ncol blocks,
@@ -799,6 +1221,150 @@ int tc_rotate(sgpu_ctx *ctx, int ncol, const T *Y, long ldy, const double *Q, in
     if (ncol <= 0) return SGPU_OK;
     if (fp64_accurate) return rotate_impl<T, 6>(ctx, ncol, Y, ldy, Q, ldq, X, ldx, st);
     return rotate_impl<T, 3>(ctx, ncol, Y, ldy, Q, ldq, X, ldx, st);
+}
+
+// Whether the last products met an infinity or a NaN (synchronises the stream)
+static int x_nonfinite(const int *flag, bool *bad, cudaStream_t st)
+{
+    int h = 0;
+    SGPU_CUDA_TRY(cudaMemcpyAsync(&h, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+    SGPU_CUDA_TRY(cudaStreamSynchronize(st));
+    *bad = h != 0;
+    return SGPU_OK;
+}
+
+// Hp = Yᵀ HY and Mp = Yᵀ Y to full FP64 accuracy. *done false, with nothing written that a caller
+// would keep: an entry is not finite (the FP64 GEMM gives the right infinities and NaN).
+int tc_project_x(sgpu_ctx *ctx, int ncol, const double *Y, long ldy, const double *HY, long ldh,
+                 double *Hp, double *Mp, bool *done, cudaStream_t st)
+{
+    *done = false;
+    const long Nd = ctx->Nd;
+    const int nrb = x_row_blocks(ncol);
+    const int mt = nrb, nt = (ncol + XN - 1) / XN;
+    const int nupper = upper_tiles(mt, nt);
+    const size_t step_bytes = sizeof(__nv_bfloat16) * (size_t)XS * nrb * (TM / 8) * XG;
+    const int steps = (int)((Nd + TK - 1) / TK);
+    const int per = (int)std::max<size_t>(CHUNK_STEPS, std::min<size_t>(steps, kXOperand / step_bytes));
+    const int npass = (steps + per - 1) / per;
+    int ksplit = std::max(1, 152 / nupper);
+    ksplit = std::min(ksplit, std::max(1, per / CHUNK_STEPS));
+    char *wa = nullptr, *wb = nullptr;
+    double *part = nullptr;
+    const size_t ebytes = sizeof(int) * ((size_t)2 * ncol + 64);
+    SGPU_TRY(ws_get(ctx, WS_SPLIT_A, step_bytes * per + ebytes, (void **)&wa));
+    SGPU_TRY(ws_get(ctx, WS_SPLIT_B, step_bytes * per, (void **)&wb));
+    const size_t psz = (size_t)ncol * ncol;
+    SGPU_TRY(ws_get(ctx, WS_TC_PART, sizeof(double) * 2 * npass * ksplit * psz, (void **)&part));
+    int *ey = reinterpret_cast<int *>(wa + step_bytes * per), *eh = ey + ncol, *flag = eh + ncol;
+    SGPU_CUDA_TRY(cudaMemsetAsync(flag, 0, sizeof(int), st));
+    SGPU_TRY(x_col_scales(ctx, Y, ldy, Nd, ncol, nullptr, 0, ey, flag, st));
+    SGPU_TRY(x_col_scales(ctx, HY, ldh, Nd, ncol, nullptr, 0, eh, flag, st));
+    __nv_bfloat16 *ty = reinterpret_cast<__nv_bfloat16 *>(wa);
+    __nv_bfloat16 *th = reinterpret_cast<__nv_bfloat16 *>(wb);
+    for (int ps = 0; ps < npass; ps++) {
+        const long k0 = (long)ps * per * TK, rows = std::min<long>(Nd - k0, (long)per * TK);
+        const int ks = (int)((rows + TK - 1) / TK);
+        for (int w = 0; w < 2; w++) {
+            ProfScope sc(ctx, SGPU_KERNEL_OTHER, st);
+            k_split_cols_x<<<(unsigned)(ks * nrb), 256, 0, st>>>(
+                (w ? HY : Y) + k0, w ? ldh : ldy, rows, ncol, w ? eh : ey, nullptr, 0, nrb,
+                w ? th : ty);
+            SGPU_CUDA_TRY(cudaGetLastError());
+        }
+        for (int w = 0; w < 2; w++) {  // Mp, then Hp
+            TcxParams p{};
+            p.A = ty;
+            p.B = w ? th : ty;
+            p.ngA = p.ngB = (long)nrb * (TM / 8);
+            p.mtiles = mt;
+            p.ntiles = nt;
+            p.ksteps = ks;
+            p.ksplit = ksplit;
+            p.M = p.N = ncol;
+            p.eA = ey;
+            p.eB = w ? eh : ey;
+            p.C = part + ((size_t)w * npass + ps) * ksplit * psz;
+            p.status = ctx->kstatus;
+            SGPU_TRY(launch_gemm_x(ctx, p, st));
+        }
+    }
+    for (int w = 0; w < 2; w++) {
+        ProfScope sc(ctx, SGPU_KERNEL_OTHER, st);
+        k_reduce_parts<<<blocks_for((long)psz), 256, 0, st>>>(part + (size_t)w * npass * ksplit * psz,
+                                                              npass * ksplit, ncol, w ? Hp : Mp,
+                                                              ncol);
+        SGPU_CUDA_TRY(cudaGetLastError());
+    }
+    bool bad = false;
+    SGPU_TRY(x_nonfinite(flag, &bad, st));
+    *done = !bad;
+    return SGPU_OK;
+}
+
+// X = Y Q to full FP64 accuracy (Q ncol x ncol, ld ncol); *done as above
+int tc_rotate_x(sgpu_ctx *ctx, int ncol, const double *Y, long ldy, const double *Q, double *X,
+                long ldx, bool *done, cudaStream_t st)
+{
+    *done = false;
+    const long Nd = ctx->Nd;
+    const int ksteps = (ncol + TK - 1) / TK, nqb = x_row_blocks(ncol);
+    const size_t blk_bytes = sizeof(__nv_bfloat16) * (size_t)ksteps * XS * (TM / 8) * XG;
+    const long blocks = (Nd + TM - 1) / TM;
+    const long per = std::max<long>(1, std::min<long>(blocks, (long)(kXOperand / blk_bytes)));
+    char *wa = nullptr, *wb = nullptr;
+    const size_t qbytes = sizeof(__nv_bfloat16) * (size_t)ksteps * XS * nqb * (TM / 8) * XG;
+    SGPU_TRY(ws_get(ctx, WS_SPLIT_A, blk_bytes * per + sizeof(int) * ((size_t)per * TM + 64),
+                    (void **)&wa));
+    SGPU_TRY(ws_get(ctx, WS_SPLIT_B, qbytes + sizeof(int) * ((size_t)2 * ncol + 64), (void **)&wb));
+    int *er = reinterpret_cast<int *>(wa + blk_bytes * per);
+    int *ec = reinterpret_cast<int *>(wb + qbytes), *eq = ec + ncol, *flag = eq + ncol;
+    __nv_bfloat16 *ta = reinterpret_cast<__nv_bfloat16 *>(wa);
+    __nv_bfloat16 *tq = reinterpret_cast<__nv_bfloat16 *>(wb);
+    SGPU_CUDA_TRY(cudaMemsetAsync(flag, 0, sizeof(int), st));
+    // column balance of Y; row c of Q gets the inverse power of two
+    SGPU_TRY(x_col_scales(ctx, Y, ldy, Nd, ncol, nullptr, 0, ec, flag, st));
+    SGPU_TRY(x_col_scales(ctx, Q, ncol, ncol, ncol, nullptr, 0, eq, flag, st));
+    SGPU_TRY(x_col_scales(ctx, Q, ncol, ncol, ncol, ec, 1, eq, flag + 1, st));
+    {
+        ProfScope sc(ctx, SGPU_KERNEL_OTHER, st);
+        k_split_cols_x<<<(unsigned)(ksteps * nqb), 256, 0, st>>>(Q, ncol, ncol, ncol, eq, ec, 1, nqb,
+                                                                 tq);
+        SGPU_CUDA_TRY(cudaGetLastError());
+    }
+    for (long b0 = 0; b0 < blocks; b0 += per) {
+        const long m0 = b0 * TM, rows = std::min<long>(Nd - m0, per * TM);
+        const int nrb = (int)((rows + TM - 1) / TM);
+        {
+            ProfScope sc(ctx, SGPU_KERNEL_OTHER, st);
+            k_rowmax_exp<double><<<blocks_for(rows), 256, 0, st>>>(Y + m0, ldy, rows, ncol, ec, er);
+            k_split_rows_x<<<(unsigned)((long)ksteps * nrb), 256, 0, st>>>(Y + m0, ldy, rows, ncol,
+                                                                           er, ec, nrb, ta);
+            SGPU_CUDA_TRY(cudaGetLastError());
+        }
+        TcxParams p{};
+        p.A = ta;
+        p.B = tq;
+        p.ngA = (long)nrb * (TM / 8);
+        p.ngB = (long)nqb * (TM / 8);
+        p.mtiles = nrb;
+        p.ntiles = (ncol + XN - 1) / XN;
+        p.ksteps = ksteps;
+        p.mode = 1;
+        p.ksplit = 1;
+        p.M = (int)rows;
+        p.N = ncol;
+        p.eA = er;
+        p.eB = eq;
+        p.C = X + m0;
+        p.ldc = ldx;
+        p.status = ctx->kstatus;
+        SGPU_TRY(launch_gemm_x(ctx, p, st));
+    }
+    bool bad = false;
+    SGPU_TRY(x_nonfinite(flag, &bad, st));
+    *done = !bad;
+    return SGPU_OK;
 }
 
 template int tc_project<double>(sgpu_ctx *, int, const double *, long, const double *, long,

@@ -207,9 +207,10 @@ struct sgpu_ctx {
     int eig_mode = 0;   // subspace eigensolver: 0 dsygvd, 1 Cholesky reduction + dsyevd,
                         // 2 Cholesky reduction + Jacobi dsyevj (sgpu_set_eig_solver)
     int rr_tc = 1;      // Rayleigh-Ritz products on the library's own tcgen05 split-slice
-                        // kernels (rr_tc.cu): 1 (default) for FP32 blocks (FP32-accurate) and
-                        // the mixed SCF's FP64 phase (FP64-accurate), 2 also for plain FP64
-                        // calls; 0 cuBLAS
+                        // kernels (rr_tc.cu): 1 (default) for FP32 blocks (FP32-accurate),
+                        // the mixed SCF's FP64 phase (six slices) and plain FP64 calls (eight
+                        // slices, full FP64 accuracy), 2 six slices for plain FP64 calls too;
+                        // 0 cuBLAS
     int zpair_on = 1;   // complex64 stencil: the two-points-per-thread kernel (1) or the
                         // one-point kernel (0) (sgpu_set_zstencil_pairs)
     double tune_fused_ms = 0.0;  // last timing of the fused apply + projection (chosen form)
@@ -361,6 +362,11 @@ int tc_project(sgpu_ctx *ctx, int ncol, const T *Y, long ldy, const T *HY, long 
 template <typename T>
 int tc_rotate(sgpu_ctx *ctx, int ncol, const T *Y, long ldy, const double *Q, int ldq, T *X,
               long ldx, bool fp64_accurate, cudaStream_t st);
+// the same two products to full FP64 accuracy (eight slices); *done false: a value is not finite
+int tc_project_x(sgpu_ctx *ctx, int ncol, const double *Y, long ldy, const double *HY, long ldh,
+                 double *Hp, double *Mp, bool *done, cudaStream_t st);
+int tc_rotate_x(sgpu_ctx *ctx, int ncol, const double *Y, long ldy, const double *Q, double *X,
+                long ldx, bool *done, cudaStream_t st);
 int rotate_f64(sgpu_ctx *ctx, int ncol, const double *Y, long ldy, const double *Q, double *X,
                long ldx, cudaStream_t st);
 int cholqr_f64(sgpu_ctx *ctx, int ncol, double *Y, long ldy, cudaStream_t st);

@@ -11,8 +11,9 @@
 // GPU form: with rr_tc set (sgpu_set_rr_products), FP32 blocks (the mixed-precision filter)
 // and the mixed-precision SCF's FP64 phase use the library's own tcgen05 kernels (rr_tc.cu:
 // split-slice BF16 products with exact chunk accumulation, FP32- or FP64-accurate); the plain
-// FP64 drop-in keeps cuBLAS DSYRK/DGEMM, and with rr_tc = 0 FP32 blocks go to cuBLAS FP32
-// GEMMs (BF16x9 emulation requested; on this GB300 cuBLAS keeps its FP32 SIMT GEMM, 56
+// FP64 drop-in uses the same with eight slices (more accurate than an FP64 GEMM), cuBLAS DGEMM
+// for narrow rotations and blocks with non-finite values, and with rr_tc = 0 FP32 blocks go to
+// cuBLAS FP32 GEMMs (BF16x9 emulation requested; on this GB300 cuBLAS keeps its FP32 SIMT GEMM, 56
 // TFLOP/s at the Si216 shapes). The Ns x Ns generalized eigenproblem stays FP64 on cuSOLVER
 // (dsygvd).
 #include <algorithm>
@@ -64,11 +65,24 @@ __global__ void k_f32_to_f64(const float *__restrict__ a, double *__restrict__ b
 }
 }  // namespace
 
+// Columns from which the plain FP64 rotation goes to the eight-slice tensor-core kernels: at 32
+// columns cuBLAS DGEMM is ahead (26^3: 0.089 against 0.114 ms, 77^3: 0.94 against 1.10), at 64 behind
+// (0.198 against 0.117, 3.53 against 1.23; 520 columns of 77^3: 239 against 8.9). The projection
+// goes there at any width: DSYRK and DGEMM with a long inner dimension and a narrow result take
+// 5.2 ms at 26^3 x 8 and 133 ms at 77^3 x 32, the split products 0.17 and 1.8 ms.
+constexpr int kRotateTcCols = 48;
+
 // Hp = Yᵀ HY and Mp = Yᵀ Y (full symmetric Ns x Ns, column-major, ld = Ns), FP64 blocks.
 int project_f64(sgpu_ctx *ctx, int ncol, const double *Y, long ldy, const double *HY,
                 long ldh, double *Hp, double *Mp, cudaStream_t st)
 {
     if (ctx->rr_tc == 2) return tc_project<double>(ctx, ncol, Y, ldy, HY, ldh, Hp, Mp, true, st);
+    if (ctx->rr_tc == 1) {
+        bool done = false;
+        const int rc = tc_project_x(ctx, ncol, Y, ldy, HY, ldh, Hp, Mp, &done, st);
+        if (rc != SGPU_OK && rc != SGPU_ERR_NOMEM) return rc;
+        if (done) return SGPU_OK;
+    }
     SGPU_TRY(ensure_handles(ctx));
     SGPU_CUBLAS_TRY(cublasSetStream(ctx->cublas, st));
     const double one = 1.0, zero = 0.0;
@@ -400,6 +414,12 @@ int rotate_f64(sgpu_ctx *ctx, int ncol, const double *Y, long ldy, const double 
                long ldx, cudaStream_t st)
 {
     if (ctx->rr_tc == 2) return tc_rotate<double>(ctx, ncol, Y, ldy, Q, ncol, X, ldx, true, st);
+    if (ctx->rr_tc == 1 && ncol >= kRotateTcCols) {
+        bool done = false;
+        const int rc = tc_rotate_x(ctx, ncol, Y, ldy, Q, X, ldx, &done, st);
+        if (rc != SGPU_OK && rc != SGPU_ERR_NOMEM) return rc;
+        if (done) return SGPU_OK;
+    }
     SGPU_TRY(ensure_handles(ctx));
     SGPU_CUBLAS_TRY(cublasSetStream(ctx->cublas, st));
     const double one = 1.0, zero = 0.0;

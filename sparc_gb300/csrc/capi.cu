@@ -235,6 +235,7 @@ int sgpu_destroy(sgpu_ctx *ctx)
     if (ctx->veff64) cudaFree(ctx->veff64);
     if (ctx->veff32) cudaFree(ctx->veff32);
     if (ctx->veff_fx) cudaFree(ctx->veff_fx);
+    if (ctx->pinned) cudaFreeHost(ctx->pinned);
     for (auto &w : ctx->ws)
         if (w.ptr) cudaFree(w.ptr);
     if (ctx->cublas) cublasDestroy(ctx->cublas);

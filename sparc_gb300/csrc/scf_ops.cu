@@ -55,6 +55,74 @@ __global__ void k_sum_partials(const double *__restrict__ part, int np, double *
     if (threadIdx.x == 0) *out = sh[0];
 }
 
+// The dots of anderson_gamma in one launch: G[i][j] = F_i . F_j (j >= i) and F_i . f, each summed as
+// k_dot_partial sums one pair (the same elements per thread, the same tree), so the coefficients
+// keep their bits. A block reads its elements of the m + 1 vectors once; 256 threads leave
+// m (m + 3) / 2 partial sums each, and a warp reduces one pair at a time.
+template <int M>
+__global__ void __launch_bounds__(256) k_gram_partial(const double *__restrict__ F,
+                                                      const double *__restrict__ f, long n,
+                                                      double *__restrict__ part)
+{
+    constexpr int NP = M * (M + 3) / 2;
+    extern __shared__ double gsh[];  // [NP][256]
+    double s[NP];
+#pragma unroll
+    for (int p = 0; p < NP; p++) s[p] = 0.0;
+    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n;
+         i += (long)gridDim.x * blockDim.x) {
+        double v[M + 1];
+#pragma unroll
+        for (int a = 0; a < M; a++) v[a] = F[(long)a * n + i];
+        v[M] = f[i];
+        int p = 0;
+#pragma unroll
+        for (int a = 0; a < M; a++)
+#pragma unroll
+            for (int b = a; b <= M; b++) {
+                s[p] += v[a] * v[b];
+                p++;
+            }
+    }
+#pragma unroll
+    for (int p = 0; p < NP; p++) gsh[p * 256 + threadIdx.x] = s[p];
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int p = warp; p < NP; p += 8) {
+        const double *t = gsh + p * 256 + lane;
+        double a0 = t[0] + t[128], a1 = t[32] + t[160], a2 = t[64] + t[192], a3 = t[96] + t[224];
+        a0 += a2;
+        a1 += a3;
+        a0 += a1;
+        for (int o = 16; o > 0; o >>= 1) a0 += __shfl_down_sync(0xffffffffu, a0, o);
+        if (lane == 0) part[(long)p * gridDim.x + blockIdx.x] = a0;
+    }
+}
+// one block per pair: the sums of k_sum_partials, placed at ftf[a * m + b] and ftb[a]
+__global__ void k_gram_sum(const double *__restrict__ part, int np, int m, double *__restrict__ ftf,
+                           double *__restrict__ ftb)
+{
+    __shared__ double sh[256];
+    const double *q = part + (long)blockIdx.x * np;
+    double s = 0.0;
+    for (int i = threadIdx.x; i < np; i += blockDim.x) s += q[i];
+    sh[threadIdx.x] = s;
+    __syncthreads();
+    for (int o = 128; o > 0; o >>= 1) {
+        if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        int a = 0, p = blockIdx.x;
+        while (p >= m + 1 - a) {
+            p -= m + 1 - a;
+            a++;
+        }
+        if (p < m - a) ftf[a * m + a + p] = sh[0];
+        else ftb[a] = sh[0];
+    }
+}
+
 inline int egrid(long n)
 {
     long g = (n + 255) / 256;
@@ -193,28 +261,50 @@ __global__ void k_lsda_pw(const double *__restrict__ up_in, const double *__rest
     }
 }
 
-// AAR bookkeeping for one iteration (after the residual r is known):
-//   f = minv * r; if hist >= 0: X[:,hist] = x - x_old, F[:,hist] = f - f_old;
-//   x_old = x; f_old = f; if richardson: x = x_old + omega * f
-__global__ void k_aar_step(long n, double minv, double omega, int hist, int richardson,
-                           double *__restrict__ x, const double *__restrict__ r,
-                           double *__restrict__ f, double *__restrict__ x_old,
-                           double *__restrict__ f_old, double *__restrict__ X,
-                           double *__restrict__ F)
+// One AAR iteration in one launch: r = b + (Lap + c) x in the arithmetic of the FP64 stencil kernel
+// (three chains over the symmetric pair sums), then f = minv r, the history columns and, unless
+// an Anderson step follows, x_next = x + omega f. x_next is another buffer (neighbours still
+// read x). One point per thread straight from L1: the FP64 pipe
+// bounds it (44 instructions a point at two lanes per clock), and unlike a march along z it fills
+// the chip at any size (26^3: 47 + 4 us as stencil and step; 77^3: 68 + 9 us).
+struct AarParams {
+    const double *__restrict__ x;
+    const double *__restrict__ b;
+    double *__restrict__ x_next;
+    double *__restrict__ r;   // written when not null
+    double *__restrict__ f, *__restrict__ x_old, *__restrict__ f_old, *__restrict__ X, *__restrict__ F;
+    int Nx, Ny, Nz, hist, richardson;
+    double wx[kMaxFDn + 1], wy[kMaxFDn + 1], wz[kMaxFDn + 1], c0, minv, omega;
+};
+__global__ void __launch_bounds__(128) k_aar_iter(const AarParams p)
 {
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n;
-         i += (long)gridDim.x * blockDim.x) {
-        const double fi = minv * r[i];
-        const double xi = x[i];
-        if (hist >= 0) {
-            X[(long)hist * n + i] = xi - x_old[i];
-            F[(long)hist * n + i] = fi - f_old[i];
-        }
-        x_old[i] = xi;
-        f_old[i] = fi;
-        f[i] = fi;
-        if (richardson) x[i] = xi + omega * fi;
+    constexpr int R = kMaxFDn;
+    const int NxNy = p.Nx * p.Ny, n = NxNy * p.Nz;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int k = i / NxNy, jx = i - k * NxNy, j = jx / p.Nx, ix = jx - j * p.Nx;
+    const double xi = p.x[i];
+    double rx = p.c0 * xi, ry = 0.0, rz = 0.0;
+#pragma unroll
+    for (int q = 1; q <= R; q++) {
+        const int xm = i - q + (ix < q ? p.Nx : 0), xp = i + q - (ix + q >= p.Nx ? p.Nx : 0);
+        const int ym = i - q * p.Nx + (j < q ? NxNy : 0), yp = i + q * p.Nx - (j + q >= p.Ny ? NxNy : 0);
+        const int zm = i - q * NxNy + (k < q ? n : 0), zp = i + q * NxNy - (k + q >= p.Nz ? n : 0);
+        rx = fma(__ldg(p.x + xm) + __ldg(p.x + xp), p.wx[q], rx);
+        ry = fma(__ldg(p.x + ym) + __ldg(p.x + yp), p.wy[q], ry);
+        rz = fma(__ldg(p.x + zm) + __ldg(p.x + zp), p.wz[q], rz);
     }
+    const double r = (rx + (ry + rz)) + p.b[i];
+    if (p.r) p.r[i] = r;
+    const double fi = p.minv * r;
+    if (p.hist >= 0) {
+        p.X[(long)p.hist * n + i] = xi - p.x_old[i];
+        p.F[(long)p.hist * n + i] = fi - p.f_old[i];
+    }
+    p.x_old[i] = xi;
+    p.f_old[i] = fi;
+    p.f[i] = fi;
+    if (p.richardson) p.x_next[i] = xi + p.omega * fi;
 }
 
 struct Gam {
@@ -222,11 +312,12 @@ struct Gam {
 };
 
 // x_wavg = x_k - X*Gamma, f_wavg = f_k - F*Gamma; out = x_wavg + beta * f_wavg (AAR), or the
-// two averages separately (mixing, when xw / fw are given)
+// two averages separately (mixing, when xw / fw are given); out2 gets a copy of out
 __global__ void k_anderson(long n, int m, Gam gam, double beta, const double *__restrict__ xk,
                            const double *__restrict__ fk, const double *__restrict__ X,
                            const double *__restrict__ F, double *__restrict__ out,
-                           double *__restrict__ xw, double *__restrict__ fw)
+                           double *__restrict__ out2, double *__restrict__ xw,
+                           double *__restrict__ fw)
 {
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n;
          i += (long)gridDim.x * blockDim.x) {
@@ -235,7 +326,7 @@ __global__ void k_anderson(long n, int m, Gam gam, double beta, const double *__
             xa -= gam.g[j] * X[(long)j * n + i];
             fa -= gam.g[j] * F[(long)j * n + i];
         }
-        if (out) out[i] = xa + beta * fa;
+        if (out) out[i] = out2[i] = xa + beta * fa;
         if (xw) xw[i] = xa;
         if (fw) fw[i] = fa;
     }
@@ -502,23 +593,48 @@ int scf_error_dev(sgpu_ctx *ctx, const double *out, const double *in, double *er
 }
 
 // Anderson coefficients: Gamma = pinv(Fᵀ F) Fᵀ f (m x m normal equations on the host)
+// The m x m sums come over with one synchronisation; extra (device, optional) is a scalar that
+// comes with them into *extra_host.
 static int anderson_gamma(sgpu_ctx *ctx, long n, int m, const double *F, const double *f,
-                          Gam *gam, cudaStream_t st)
+                          Gam *gam, cudaStream_t st, const double *extra = nullptr,
+                          double *extra_host = nullptr)
 {
+    constexpr int kGramM = 7;  // the history length of AAR and the default of the mixing
+    constexpr int kGramPairs = kGramM * (kGramM + 3) / 2;
+    const size_t npart = m == kGramM ? (size_t)kRedBlocks * kGramPairs : (size_t)kRedBlocks * 2 + 8;
     double *part = nullptr;
-    SGPU_TRY(ws_get(ctx, WS_RED, sizeof(double) * (kRedBlocks * 2 + 8 + kMaxHist * (kMaxHist + 1)),
+    SGPU_TRY(ws_get(ctx, WS_RED, sizeof(double) * (npart + kMaxHist * (kMaxHist + 1)),
                     (void **)&part));
-    double *ftf = part + kRedBlocks * 2 + 8;
+    double *ftf = part + npart;
     double *ftb = ftf + kMaxHist * kMaxHist;
-    // Fᵀ F and Fᵀ f with deterministic device reductions
-    for (int i = 0; i < m; i++) {
-        for (int j = i; j < m; j++) SGPU_TRY(dot_dev(ctx, F + (long)i * n, F + (long)j * n, n, ftf + i * m + j, st));
-        SGPU_TRY(dot_dev(ctx, F + (long)i * n, f, n, ftb + i, st));
+    // Fᵀ F and Fᵀ f with deterministic device reductions; 35 pairs of launches of 7 + 4.5 us each
+    // at 77^3 as single dots, 2 launches here
+    if (m == kGramM) {
+        const size_t sm = sizeof(double) * 256 * kGramPairs;
+        SGPU_CUDA_TRY(cudaFuncSetAttribute(k_gram_partial<kGramM>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        k_gram_partial<kGramM><<<kRedBlocks, 256, sm, st>>>(F, f, n, part);
+        k_gram_sum<<<kGramPairs, 256, 0, st>>>(part, kRedBlocks, m, ftf, ftb);
+        ctx->launches += 2;
+        SGPU_CUDA_TRY(cudaGetLastError());
+    } else {
+        for (int i = 0; i < m; i++) {
+            for (int j = i; j < m; j++)
+                SGPU_TRY(dot_dev(ctx, F + (long)i * n, F + (long)j * n, n, ftf + i * m + j, st));
+            SGPU_TRY(dot_dev(ctx, F + (long)i * n, f, n, ftb + i, st));
+        }
     }
-    double h[kMaxHist * (kMaxHist + 1)];
+    if (!ctx->pinned)
+        SGPU_CUDA_TRY(cudaMallocHost((void **)&ctx->pinned,
+                                     sizeof(double) * (kMaxHist * (kMaxHist + 1) + 1)));
+    double *h = ctx->pinned;
     SGPU_CUDA_TRY(cudaMemcpyAsync(h, ftf, sizeof(double) * kMaxHist * (kMaxHist + 1),
                                   cudaMemcpyDeviceToHost, st));
+    if (extra)
+        SGPU_CUDA_TRY(cudaMemcpyAsync(h + kMaxHist * (kMaxHist + 1), extra, sizeof(double),
+                                      cudaMemcpyDeviceToHost, st));
     SGPU_CUDA_TRY(cudaStreamSynchronize(st));
+    if (extra) *extra_host = h[kMaxHist * (kMaxHist + 1)];
     double A[kMaxHist * kMaxHist], b[kMaxHist];
     for (int i = 0; i < m; i++) {
         for (int j = i; j < m; j++) A[(size_t)j * m + i] = A[(size_t)i * m + j] = h[i * m + j];
@@ -531,6 +647,12 @@ static int anderson_gamma(sgpu_ctx *ctx, long n, int m, const double *F, const d
 // AAR for  b + (Lap + c) x = 0  with the Jacobi preconditioner, restating AAR
 // (src/linearSolver.c:37-165) with poisson_residual and Jacobi_preconditioner. The residual
 // norm is evaluated at Anderson steps only, as in the reference. Returns the iteration count.
+//
+// An iteration is one launch (k_aar_iter: residual and step), an Anderson step three more and the
+// only synchronisation. The norm that an Anderson step ends with is formed by the next iteration's
+// launch and read at the next Anderson step, with its sums: the p - 1 iterations in between are
+// already running, and when the norm was below the tolerance the iterate kept from that step is
+// the result (up to p launches of a solve are for nothing, against one wait less per step).
 int aar_dev(sgpu_ctx *ctx, double c, double *x, const double *b, double omega, double beta,
             int m, int p, double tol, int max_iter, int *iters, cudaStream_t st)
 {
@@ -539,48 +661,82 @@ int aar_dev(sgpu_ctx *ctx, double c, double *x, const double *b, double omega, d
         return SGPU_ERR_ARG;
     }
     const long N = ctx->Nd;
+    if (N >= (1L << 31) - 128) {
+        set_error("AAR: the grid must hold fewer than 2^31 points");
+        return SGPU_ERR_ARG;
+    }
     double *w = nullptr;
-    SGPU_TRY(ws_get(ctx, WS_POIS, sizeof(double) * (size_t)N * (4 + 2 * m), (void **)&w));
+    SGPU_TRY(ws_get(ctx, WS_POIS, sizeof(double) * ((size_t)N * (6 + 2 * m) + 8), (void **)&w));
     double *r = w, *x_old = w + N, *f = w + 2 * N, *f_old = w + 3 * N;
-    double *X = w + 4 * N, *F = w + (4 + m) * N;
+    double *xb = w + 4 * N, *kept = w + 5 * N, *X = w + 6 * N, *F = w + (6 + m) * N;
+    double *r2 = w + (size_t)N * (6 + 2 * m);  // |r|^2 after the last Anderson step
     SGPU_CUDA_TRY(cudaMemsetAsync(X, 0, sizeof(double) * (size_t)N * 2 * m, st));
-    SGPU_CUDA_TRY(cudaMemcpyAsync(x_old, x, sizeof(double) * N, cudaMemcpyDeviceToDevice, st));
     double bnorm2 = 0.0;
     SGPU_TRY(dot_host(ctx, b, b, N, &bnorm2, st));
     double minv = ctx->cx[0] + ctx->cy[0] + ctx->cz[0] + c;
     if (std::fabs(minv) < 1e-14) minv = 1.0;
     minv = -1.0 / minv;
-    // r = b + (Lap + c) x
-    SGPU_TRY(launch_stencil<double>(ctx, 1, 1.0, 0.0, c, nullptr, x, N, r, N, 1.0, 1.0, b, N, st, nullptr, false));
     tol *= std::sqrt(bnorm2);
+    AarParams q{};
+    q.b = b;
+    q.f = f; q.x_old = x_old; q.f_old = f_old; q.X = X; q.F = F;
+    q.Nx = ctx->Nx; q.Ny = ctx->Ny; q.Nz = ctx->Nz;
+    for (int i = 0; i <= kMaxFDn; i++) { q.wx[i] = ctx->cx[i]; q.wy[i] = ctx->cy[i]; q.wz[i] = ctx->cz[i]; }
+    q.c0 = ctx->cx[0];
+    q.c0 += ctx->cy[0];
+    q.c0 += ctx->cz[0];
+    q.c0 += c;
+    q.minv = minv;
+    q.omega = omega;
+    const int nb = (int)((N + 127) / 128);
+    double *cur = x, *next = xb;
     double rnorm = tol + 1.0;
-    int it = 0;
+    bool pending = false;  // |r|^2 of the iterate after `done` iterations is in r2, it in `kept`
+    int it = 0, done = 0;
     while (rnorm > tol && it < max_iter) {
-        const int hist = it > 0 ? (it - 1) % m : -1;
         const bool anderson = ((it + 1) % p == 0) && it > 0;
-        k_aar_step<<<egrid(N), 256, 0, st>>>(N, minv, omega, hist, anderson ? 0 : 1, x, r, f,
-                                             x_old, f_old, X, F);
+        q.x = cur;
+        q.x_next = next;
+        q.hist = it > 0 ? (it - 1) % m : -1;
+        q.richardson = anderson ? 0 : 1;
+        q.r = pending && it == done ? r : nullptr;
+        k_aar_iter<<<nb, 128, 0, st>>>(q);
         ctx->launches++;
+        if (q.r) SGPU_TRY(dot_dev(ctx, r, r, N, r2, st));
         if (anderson) {
             Gam gam;
-            SGPU_TRY(anderson_gamma(ctx, N, m, F, f, &gam, st));
-            k_anderson<<<egrid(N), 256, 0, st>>>(N, m, gam, beta, x_old, f, X, F, x, nullptr,
+            double h = 0.0;
+            SGPU_TRY(anderson_gamma(ctx, N, m, F, f, &gam, st, pending ? r2 : nullptr, &h));
+            if (pending) rnorm = std::sqrt(h);
+            if (pending && !(rnorm > tol)) break;
+            k_anderson<<<egrid(N), 256, 0, st>>>(N, m, gam, beta, x_old, f, X, F, next, kept, nullptr,
                                                  nullptr);
             ctx->launches++;
-            SGPU_TRY(launch_stencil<double>(ctx, 1, 1.0, 0.0, c, nullptr, x, N, r, N, 1.0, 1.0,
-                                            b, N, st, nullptr, false));
-            double r2 = 0.0;
-            SGPU_TRY(dot_host(ctx, r, r, N, &r2, st));
-            rnorm = std::sqrt(r2);
-        } else {
-            SGPU_TRY(launch_stencil<double>(ctx, 1, 1.0, 0.0, c, nullptr, x, N, r, N, 1.0, 1.0,
-                                            b, N, st, nullptr, false));
+            pending = true;
+            done = it + 1;
         }
+        std::swap(cur, next);
         it++;
     }
     SGPU_CUDA_TRY(cudaGetLastError());
-    if (iters) *iters = it;
-    if (rnorm > tol) {
+    const bool early = pending && !(rnorm > tol);
+    if (pending && !early) {  // the iteration limit: the norm of the last Anderson step
+        if (it == done) {     // its residual was not formed yet
+            SGPU_TRY(launch_stencil<double>(ctx, 1, 1.0, 0.0, c, nullptr, cur, N, r, N, 1.0, 1.0, b,
+                                            N, st, nullptr, false));
+            SGPU_TRY(dot_dev(ctx, r, r, N, r2, st));
+        }
+        double h = 0.0;
+        SGPU_CUDA_TRY(cudaMemcpyAsync(&h, r2, sizeof(double), cudaMemcpyDeviceToHost, st));
+        SGPU_CUDA_TRY(cudaStreamSynchronize(st));
+        rnorm = std::sqrt(h);
+    }
+    const bool converged = pending && !(rnorm > tol);
+    const double *res = converged ? kept : cur;
+    if (iters) *iters = converged ? done : it;
+    if (res != x)
+        SGPU_CUDA_TRY(cudaMemcpyAsync(x, res, sizeof(double) * N, cudaMemcpyDeviceToDevice, st));
+    if (!converged && rnorm > tol) {
         set_error("AAR: no convergence in " + std::to_string(max_iter) + " iterations");
         return SGPU_ERR_NOT_CONVERGED;
     }
@@ -701,7 +857,7 @@ int mixing_step(sgpu_ctx *ctx, int iter_count, double *g, cudaStream_t st)
         Gam gam;
         SGPU_TRY(anderson_gamma(ctx, N, m, ms->F, ms->f_k, &gam, st));
         k_anderson<<<egrid(N), 256, 0, st>>>(N, m, gam, 0.0, ms->x_k, ms->f_k, ms->R, ms->F,
-                                             nullptr, ms->x_wavg, ms->f_wavg);
+                                             nullptr, nullptr, ms->x_wavg, ms->f_wavg);
         ctx->launches++;
     } else {
         SGPU_CUDA_TRY(cudaMemcpyAsync(ms->x_wavg, ms->x_k, sizeof(double) * N,

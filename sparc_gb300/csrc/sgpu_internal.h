@@ -187,6 +187,7 @@ struct sgpu_ctx {
     size_t xhost_bytes = 0;
     int rr_batched = 1;                     // k-point CheFSI pass: batched Rayleigh-Ritz step
                                             // for blocks of one width (sgpu_set_rr_batched)
+    double *pinned = nullptr;                // page-locked host scratch of the Anderson sums
     sgpu::Workspace ws[24];    // grow-only scratch slots (see enum WsSlot)
     sgpu::MixState *mix = nullptr;
     sgpu::KpointState *kp = nullptr;  // cell lengths and image coordinates (k-point calls)

@@ -20,6 +20,8 @@
 
 #include "sgpu_internal.h"
 #include "zmath.cuh"
+#include "nonlocal_fx.cuh"
+#include "stencil_fx_z.cuh"
 #include "zstencil_c64.cuh"
 
 namespace sgpu {
@@ -475,10 +477,13 @@ struct BBlock {
     double kL[3];           // k_d * L_d
     double2 bf[9];          // e^{i d k_a L_a}, index 3 a + d + 1 (a = x, y, z; d = -1, 0, 1)
     int ncol, spin;
+    CT *alpha2, *part;      // fixed-point form: the projections' other buffer, the ranges' partial
+    long ldp;               // projections and their row length
 };
 
 struct BCoef {
     double c0, s1, s2;      // centre weight (with the shift), output and recurrence scales
+    int c0h, c0l;           // digits of c0 (fixed-point form)
 };
 
 struct BConst {
@@ -512,6 +517,113 @@ __global__ void __launch_bounds__(zstencil_threads<CT>())
     p.c0 = cf.c0; p.bv = 1.0; p.s1 = cf.s1; p.s2 = cf.s2;
     p.k.kLx = B.kL[0]; p.k.kLy = B.kL[1]; p.k.kLz = B.kL[2];
     stencil_z_body<CT, R>(p, bc.y, slab);
+}
+
+// complex128 in block fixed point: one launch's columns of all blocks
+template <int NS, bool CUBE>
+__global__ void __launch_bounds__(kFxZThreads, 1)
+    k_stencil_fxzb(const BBlock<double2> *__restrict__ blocks, const BCoef *__restrict__ coef,
+                   const int2 *__restrict__ work, const __grid_constant__ FxZConst g,
+                   const double *__restrict__ veff, const int2 *__restrict__ veff_fx, long Nd, int m,
+                   int deg, int in_sel, int out_sel, int z_sel)
+{
+    extern __shared__ __align__(16) unsigned char fxz_smem[];
+    const int w = blockIdx.z / g.nslab, slab = blockIdx.z % g.nslab;
+    const int2 bc = work[w];
+    const BBlock<double2> &B = blocks[bc.x];
+    const BCoef &cf = coef[(long)bc.x * m + deg];
+    FxZCol c;
+    c.x = B.buf[in_sel] + (long)bc.y * B.ld[in_sel];
+    c.out = B.buf[out_sel] + (long)bc.y * B.ld[out_sel];
+    c.z = z_sel >= 0 ? B.buf[z_sel] + (long)bc.y * B.ld[z_sel] : nullptr;
+    c.v = veff ? veff + (long)B.spin * Nd : nullptr;
+    c.vd = veff_fx ? veff_fx + (long)B.spin * Nd : nullptr;
+    c.c0h = cf.c0h; c.c0l = cf.c0l;
+    c.c0 = cf.c0; c.s1 = cf.s1; c.s2 = cf.s2;
+    c.bf = B.bf;
+    stencil_fxz<NS, CUBE>(g, c, slab, fxz_smem);
+}
+// the same for the columns of one block with its numbers as parameters
+struct FxZOne {
+    FxZCol c;              // column 0
+    long ldx, ldo, ldz;
+    double2 bf[9];
+};
+template <int NS, bool CUBE>
+__global__ void __launch_bounds__(kFxZThreads, 1)
+    k_stencil_fxz(const __grid_constant__ FxZConst g, const __grid_constant__ FxZOne b)
+{
+    extern __shared__ __align__(16) unsigned char fxz_smem[];
+    const int col = blockIdx.z / g.nslab, slab = blockIdx.z % g.nslab;
+    FxZCol c = b.c;
+    c.x += (long)col * b.ldx;
+    c.out += (long)col * b.ldo;
+    if (c.z) c.z += (long)col * b.ldz;
+    c.bf = b.bf;
+    stencil_fxz<NS, CUBE>(g, c, slab, fxz_smem);
+}
+// complex128 nonlocal products in block fixed point: grid (block and column-group phase, range)
+template <bool APPLY, bool PROJ, int MAXJ>
+__global__ void __launch_bounds__(32 * nlfx::kWarps, 2)
+    k_nl_fx_zb(const nlfx::Tables T, const BBlock<double2> *__restrict__ blocks,
+               const BCoef *__restrict__ coef, int m, int deg, int sel, bool second, int gx)
+{
+    extern __shared__ __align__(16) unsigned char nlfxz_smem[];
+    const int b = blockIdx.x / gx, g0 = blockIdx.x - b * gx;
+    const BBlock<double2> &B = blocks[b];
+    double *buf = reinterpret_cast<double *>(B.buf[sel]);
+    nlfx::block<true, APPLY, PROJ, MAXJ>(
+        T, blockIdx.y, g0, gx, B.ncol, reinterpret_cast<const double *>(second ? B.alpha2 : B.alpha),
+        APPLY ? coef[(long)b * m + deg].s1 : 0.0, buf, buf, B.ld[sel],
+        reinterpret_cast<double *>(B.part), B.ncol, B.ldp, B.phase, nlfxz_smem);
+}
+template <bool APPLY, bool PROJ, int MAXJ>
+__global__ void __launch_bounds__(32 * nlfx::kWarps, 2)
+    k_nl_fx_z(const nlfx::Tables T, int ncol, const double2 *__restrict__ alpha, double scale,
+              double2 *buf, long ld, double2 *__restrict__ part, long lda, long ldp,
+              const double2 *__restrict__ phase)
+{
+    extern __shared__ __align__(16) unsigned char nlfxz_smem[];
+    double *d = reinterpret_cast<double *>(buf);
+    nlfx::block<true, APPLY, PROJ, MAXJ>(T, blockIdx.y, blockIdx.x, gridDim.x, ncol,
+                                         reinterpret_cast<const double *>(alpha), scale, d, d, ld,
+                                         reinterpret_cast<double *>(part), lda, ldp, phase,
+                                         nlfxz_smem);
+}
+// alpha row = dV Gamma times the sum of its partial rows, in their order; one component a thread
+__device__ __forceinline__ void fx_reduce_row(const int *__restrict__ ptr, const int *__restrict__ idx,
+                                              const double *__restrict__ part, long ldp, int c, int row,
+                                              double f, double *__restrict__ alpha, long lda)
+{
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    const int e1 = ptr[row + 1];
+    int e = ptr[row];
+    for (; e + 4 <= e1; e += 4)
+#pragma unroll
+        for (int u = 0; u < 4; u++) s[u] += __ldg(part + (long)idx[e + u] * ldp + c);
+    for (; e < e1; e++) s[0] += __ldg(part + (long)idx[e] * ldp + c);
+    alpha[(long)row * lda + c] = f * ((s[0] + s[1]) + (s[2] + s[3]));
+}
+__global__ void k_fx_reduce_zb(const BBlock<double2> *__restrict__ blocks, const int *__restrict__ ptr,
+                               const int *__restrict__ idx, double dV,
+                               const double *__restrict__ gamma, bool second)
+{
+    const BBlock<double2> &B = blocks[blockIdx.z];
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c < 2 * B.ncol)
+        fx_reduce_row(ptr, idx, reinterpret_cast<const double *>(B.part), 2 * B.ldp, c, blockIdx.y,
+                      dV * gamma[blockIdx.y],
+                      reinterpret_cast<double *>(second ? B.alpha2 : B.alpha), 2L * B.ncol);
+}
+__global__ void k_fx_reduce_z(const double2 *__restrict__ part, long ldp, const int *__restrict__ ptr,
+                              const int *__restrict__ idx, double dV,
+                              const double *__restrict__ gamma, int ncol, double2 *__restrict__ alpha,
+                              long lda)
+{
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c < 2 * ncol)
+        fx_reduce_row(ptr, idx, reinterpret_cast<const double *>(part), 2 * ldp, c, blockIdx.y,
+                      dV * gamma[blockIdx.y], reinterpret_cast<double *>(alpha), 2 * lda);
 }
 
 template <int R>
@@ -759,10 +871,46 @@ static int set_phases(sgpu_ctx *ctx, const double *k, cudaStream_t st)
     return SGPU_OK;
 }
 
+// Launch shape and constants of the complex128 fixed-point stencil; false where it does not apply
+// (coefficients or potential out of range, tiny grids, columns past 32-bit byte offsets). c0: the
+// largest centre weight of the launch's columns, w: a w_r per direction.
+struct FxZLaunch {
+    FxZConst g{};
+    int s, ns, threads, tilesx, tilesy;
+    bool cube;
+    size_t smem;
+};
+static bool fxz_launch(const sgpu_ctx *ctx, const double (&w)[3][kMaxFDn], double c0, unsigned vkey,
+                       long ncol, FxZLaunch *L)
+{
+    if (ctx->Nd >= (1L << 27)) return false;
+    StencilFxParams d{};
+    d.c0 = c0;
+    d.s1 = 1.0;
+    std::copy(&w[0][0], &w[0][0] + 3 * kMaxFDn, &d.w[0][0]);
+    if (!fx_setup(d, kMaxFDn, vkey)) return false;
+    fxz_const(L->g, d);
+    L->s = d.s;
+    FxZConst &g = L->g;
+    g.Nx = ctx->Nx; g.Ny = ctx->Ny; g.Nz = ctx->Nz;
+    if (!fxz_plan(g.Nx, g.Ny, g.Nz, ncol, 152, g.TX, g.TY, g.nslab)) return false;
+    g.zlen = (g.Nz + g.nslab - 1) / g.nslab;
+    g.hx = 2 * kMaxFDn * g.TY;
+    g.hy = 2 * kMaxFDn * g.TX;
+    L->threads = fxz_threads(g.TX, g.TY);
+    L->ns = (g.hx + g.hy + L->threads - 1) / L->threads;
+    L->tilesx = (g.Nx + g.TX - 1) / g.TX;
+    L->tilesy = (g.Ny + g.TY - 1) / g.TY;
+    L->smem = 2 * sizeof(int4) * (size_t)kFxZPitch * (g.TY + 2 * kMaxFDn);
+    L->cube = std::equal(w[0], w[0] + kMaxFDn, w[1]) && std::equal(w[0], w[0] + kMaxFDn, w[2]);
+    return true;
+}
+
 template <typename CT>
 static int stencil_z(sgpu_ctx *ctx, const double *k, int ncol, double a, double bv, double c,
                      const double *v, const float *v32, const CT *x, long ldx, CT *out,
-                     long ldo, double s1, double s2, const CT *z, long ldz, cudaStream_t st)
+                     long ldo, double s1, double s2, const CT *z, long ldz, cudaStream_t st,
+                     const FxPot *pot = nullptr)
 {
     constexpr int R = 6;
     if (ctx->FDn != R) {
@@ -791,6 +939,55 @@ static int stencil_z(sgpu_ctx *ctx, const double *k, int ncol, double a, double 
     p.k.kLx = k[0] * ks->L[0];
     p.k.kLy = k[1] * ks->L[1];
     p.k.kLz = k[2] * ks->L[2];
+    if constexpr (sizeof(CT) == 16) {  // complex128: block fixed point where it applies
+        FxZLaunch L;
+        double w[3][kMaxFDn];
+        for (int r = 0; r < kMaxFDn; r++) {
+            w[0][r] = p.wx[r + 1];
+            w[1][r] = p.wy[r + 1];
+            w[2][r] = p.wz[r + 1];
+        }
+        // (the kernel's own FP64 path takes bv = 1)
+        const bool can = !p.v || bv == 1.0;
+        FxPot own{};
+        if (can && p.v && !pot) {  // a caller's potential: its digits for this call
+            char *ws = nullptr;
+            SGPU_TRY(ws_get(ctx, WS_FXPOT, sizeof(int2) * (size_t)ctx->Nd + 16, (void **)&ws));
+            SGPU_TRY(fx_potential(ctx, p.v, bv, ctx->Nd, reinterpret_cast<int2 *>(ws + 16),
+                                  reinterpret_cast<unsigned *>(ws), &own.key, st));
+            SGPU_CUDA_TRY(cudaStreamSynchronize(st));
+            own.vd = reinterpret_cast<int2 *>(ws + 16);
+            pot = &own;
+        }
+        if (can && fxz_launch(ctx, w, c0, p.v ? pot->key : 0u, ncol, &L)) {
+            FxZOne b{};
+            b.c.x = x; b.c.out = out; b.c.z = p.z;
+            b.c.v = p.v;
+            b.c.vd = p.v && pot->key ? pot->vd : nullptr;
+            fx_coef(c0, L.s, b.c.c0h, b.c.c0l);
+            b.c.c0 = c0; b.c.s1 = s1; b.c.s2 = s2;
+            b.ldx = ldx; b.ldo = ldo; b.ldz = ldz;
+            const double kL[3] = {p.k.kLx, p.k.kLy, p.k.kLz};
+            for (int q = 0; q < 9; q++)
+                b.bf[q] = make_double2(std::cos((q % 3 - 1) * kL[q / 3]), std::sin((q % 3 - 1) * kL[q / 3]));
+            const int maxz = 65535 / L.g.nslab;
+            for (int c0i = 0; c0i < ncol; c0i += maxz) {
+                const int nc = std::min(maxz, ncol - c0i);
+                FxZOne q = b;
+                q.c.x = x + (long)c0i * ldx;
+                q.c.out = out + (long)c0i * ldo;
+                if (q.c.z) q.c.z = p.z + (long)c0i * ldz;
+                ProfScope ps(ctx, SGPU_KERNEL_STENCIL, st);
+                const dim3 grid(L.tilesx, L.tilesy, nc * L.g.nslab);
+                auto kern = L.ns <= 2 ? (L.cube ? k_stencil_fxz<2, true> : k_stencil_fxz<2, false>)
+                            : L.ns == 3 ? (L.cube ? k_stencil_fxz<3, true> : k_stencil_fxz<3, false>)
+                                        : (L.cube ? k_stencil_fxz<4, true> : k_stencil_fxz<4, false>);
+                kern<<<grid, L.threads, L.smem, st>>>(L.g, q);
+            }
+            SGPU_CUDA_TRY(cudaGetLastError());
+            return SGPU_OK;
+        }
+    }
     if constexpr (sizeof(CT) == 8) {  // complex64: the pair kernel where it applies
         int PX2, PY;
         zpair_tile(ctx->Nx, ctx->Ny, R, &PX2, &PY);
@@ -881,6 +1078,35 @@ static int nonlocal_z(sgpu_ctx *ctx, int ncol, const CT *x, long ldx, CT *out, l
     const long lda = ncol;
     CT *alpha = nullptr;
     SGPU_TRY(ws_get(ctx, WS_ALPHA, sizeof(CT) * (size_t)nl.ntot * lda, (void **)&alpha));
+    if constexpr (sizeof(CT) == 16)
+        if (nonlocal_fx_ready(ctx)) {
+            const int groups = (ncol + nlfx::kLanes / 2 - 1) / (nlfx::kLanes / 2);
+            const NlFx &X = nonlocal_fx_pick(nl, groups);
+            const nlfx::Tables T = nonlocal_fx_tables(nl, X);
+            const long ldp = (long)groups * (nlfx::kLanes / 2);
+            const int sm = (int)nlfx::smem_bytes(T);
+            CT *part = nullptr;
+            SGPU_TRY(ws_get(ctx, WS_NLPART, sizeof(CT) * (size_t)X.nrows * ldp, (void **)&part));
+            auto project = nl.max_np <= 9 ? k_nl_fx_z<false, true, 9> : k_nl_fx_z<false, true, 18>;
+            auto apply = nl.max_np <= 9 ? k_nl_fx_z<true, false, 9> : k_nl_fx_z<true, false, 18>;
+            if (X.nrange <= 65535) {
+                const dim3 grid(std::min(groups, std::max(1, 152 * 8 / X.nrange)), X.nrange);
+                SGPU_CUDA_TRY(cudaFuncSetAttribute(project, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+                SGPU_CUDA_TRY(cudaFuncSetAttribute(apply, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+                {
+                    ProfScope ps(ctx, SGPU_KERNEL_NL_PROJECT, st);
+                    project<<<grid, 32 * nlfx::kWarps, sm, st>>>(T, ncol, nullptr, 0.0,
+                        const_cast<CT *>(x), ldx, part, lda, ldp, ks->img_phase);
+                    k_fx_reduce_z<<<dim3((2 * ncol + 127) / 128, nl.ntot), 128, 0, st>>>(
+                        part, ldp, X.sum_ptr, X.sum_idx, ctx->dV, nl.gamma64, ncol, alpha, lda);
+                }
+                ProfScope ps(ctx, SGPU_KERNEL_NL_APPLY, st);
+                apply<<<grid, 32 * nlfx::kWarps, sm, st>>>(T, ncol, alpha, scale, out, ldo, nullptr, lda,
+                                                           ldp, ks->img_phase);
+                SGPU_CUDA_TRY(cudaGetLastError());
+                return SGPU_OK;
+            }
+        }
     SGPU_CUDA_TRY(cudaMemsetAsync(alpha, 0, sizeof(CT) * (size_t)nl.ntot * lda, st));
     const dim3 pg(nl.nimg, (ncol + 31) / 32);
     {
@@ -946,7 +1172,8 @@ int hamiltonian_z(sgpu_ctx *ctx, int spin, const double *k, int ncol, double c, 
     const bool f64 = sizeof(CT) == 16;
     const double *v = f64 ? ctx->veff64 + (long)spin * ctx->Nd : nullptr;
     const float *v32 = f64 ? nullptr : ctx->veff32 + (long)spin * ctx->Nd;
-    SGPU_TRY(stencil_z<CT>(ctx, k, ncol, -0.5, 1.0, c, v, v32, x, ldx, hx, ldh, s1, s2, z, ldz, st));
+    const FxPot pot{ctx->veff_fx + (long)spin * ctx->Nd, ctx->veff_key};
+    SGPU_TRY(stencil_z<CT>(ctx, k, ncol, -0.5, 1.0, c, v, v32, x, ldx, hx, ldh, s1, s2, z, ldz, st, &pot));
     SGPU_TRY(nonlocal_z<CT>(ctx, ncol, x, ldx, hx, ldh, s1, st));
     return SGPU_OK;
 }
@@ -1017,6 +1244,37 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
     if (route) SGPU_TRY(ws_get(ctx, WS_STAGE_C, sizeof(CT) * (size_t)Nd * totcols, (void **)&W));
     if (has_nl)
         SGPU_TRY(ws_get(ctx, WS_ALPHA, sizeof(CT) * (size_t)nl.ntot * totcols, (void **)&alpha));
+    // complex128 in block fixed point: the stencil's shape, and the projections' second buffer and
+    // partial rows (per block, in groups of 16 columns)
+    constexpr bool Z128 = sizeof(CT) == 16;
+    constexpr int FG = nlfx::kLanes / 2;
+    FxZLaunch fxl;
+    bool fx_st = false, fx_nl = false;
+    const NlFx *fxt = nullptr;
+    CT *alpha2 = nullptr, *part = nullptr;
+    std::vector<long> partoff(nblk + 1, 0);
+    if (Z128) {
+        double w[3][kMaxFDn], c0max = 0.0;
+        for (int r = 0; r < kMaxFDn; r++) {
+            w[0][r] = ctx->cx[r + 1] * -0.5;
+            w[1][r] = ctx->cy[r + 1] * -0.5;
+            w[2][r] = ctx->cz[r + 1] * -0.5;
+        }
+        for (int b = 0; b < nblk; b++)
+            c0max = std::max(c0max, std::fabs(-0.5 * (ctx->cx[0] + ctx->cy[0] + ctx->cz[0]) -
+                                              0.5 * (blk[b].a + blk[b].b)));
+        fx_st = fxz_launch(ctx, w, c0max * 1.0000001, ctx->veff_key, totcols, &fxl);
+        fx_nl = has_nl && nonlocal_fx_ready(ctx);
+    }
+    if (fx_nl) {
+        for (int b = 0; b < nblk; b++) partoff[b + 1] = partoff[b] + (blk[b].ncol + FG - 1) / FG * FG;
+        fxt = &nonlocal_fx_pick(nl, partoff[nblk] / FG);
+        fx_nl = fxt->nrange <= 65535;
+    }
+    if (fx_nl) {
+        SGPU_TRY(ws_get(ctx, WS_ALPHA2, sizeof(CT) * (size_t)nl.ntot * totcols, (void **)&alpha2));
+        SGPU_TRY(ws_get(ctx, WS_NLPART, sizeof(CT) * (size_t)fxt->nrows * partoff[nblk], (void **)&part));
+    }
 
     // host copies of the tables: blocks | coef | work | column groups | phases
     std::vector<BBlock<CT>> hb(nblk);
@@ -1040,6 +1298,9 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
                 B.bf[3 * a + d + 1] = make_double2(std::cos(d * B.kL[a]), std::sin(d * B.kL[a]));
         B.ncol = f.ncol;
         B.spin = f.spin;
+        B.alpha2 = fx_nl ? alpha2 + (size_t)nl.ntot * coloff[b] : nullptr;
+        B.part = fx_nl ? part + (size_t)fxt->nrows * partoff[b] : nullptr;
+        B.ldp = partoff[b + 1] - partoff[b];
         // recurrence scalars of ChebyshevFiltering_kpt (src/eigenSolverKpt.c:458-550)
         const double e = 0.5 * (f.b - f.a), c = 0.5 * (f.b + f.a);
         double sigma = e / (f.a0 - c);
@@ -1051,6 +1312,8 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
         for (int j = 0; j < m; j++) {
             BCoef &q = hc[(size_t)b * m + j];
             q.c0 = c0;
+            q.c0h = q.c0l = 0;
+            if (fx_st) fx_coef(c0, fxl.s, q.c0h, q.c0l);
             if (j == 0) {
                 q.s1 = sigma1 / e;
                 q.s2 = 0.0;
@@ -1166,6 +1429,30 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
         }
     }
 
+    nlfx::Tables fT{};
+    int fsm = 0, fgx = 1;
+    if (fx_nl) {  // attributes set before any capture
+        fT = nonlocal_fx_tables(nl, *fxt);
+        fsm = (int)nlfx::smem_bytes(fT);
+        const int groups = (maxcol + FG - 1) / FG;
+        fgx = std::min(groups, std::max(1, 152 * 8 / (fxt->nrange * nblk)));
+        auto attr = [&](auto k9, auto k18) {
+            return nl.max_np <= 9
+                       ? cudaFuncSetAttribute(k9, cudaFuncAttributeMaxDynamicSharedMemorySize, fsm)
+                       : cudaFuncSetAttribute(k18, cudaFuncAttributeMaxDynamicSharedMemorySize, fsm);
+        };
+        SGPU_CUDA_TRY(attr(k_nl_fx_zb<false, true, 9>, k_nl_fx_zb<false, true, 18>));
+        SGPU_CUDA_TRY(attr(k_nl_fx_zb<true, false, 9>, k_nl_fx_zb<true, false, 18>));
+        SGPU_CUDA_TRY(attr(k_nl_fx_zb<true, true, 9>, k_nl_fx_zb<true, true, 18>));
+    }
+    const BBlock<double2> *dB128 = reinterpret_cast<const BBlock<double2> *>(dB);
+    // the sums of the partial projections into one of the two buffers
+    auto fx_reduce = [&](bool second) {
+        k_fx_reduce_zb<<<dim3((2 * maxcol + 127) / 128, nl.ntot, nblk), 128, 0, st>>>(
+            dB128, fxt->sum_ptr, fxt->sum_idx, ctx->dV, nl.gamma64, second);
+        ctx->launches++;
+    };
+
     auto issue = [&]() -> int {
         int cur = route ? 2 : 1, prev = 0;  // buffer ids: 0 X, 1 Y, 2 scratch
         for (int j = 0; j < m; j++) {
@@ -1180,7 +1467,15 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
                 prev = cur;
                 cur = dst;
             }
-            if (has_nl) {
+            if (fx_nl && j == 0) {  // later degrees are projected as their apply finishes them
+                ProfScope ps(ctx, SGPU_KERNEL_NL_PROJECT, st);
+                auto kern = nl.max_np <= 9 ? k_nl_fx_zb<false, true, 9> : k_nl_fx_zb<false, true, 18>;
+                kern<<<dim3(nblk * fgx, fxt->nrange), 32 * nlfx::kWarps, fsm, st>>>(fT, dB128, dC, m, j, in,
+                                                                                   false, fgx);
+                ctx->launches++;
+                fx_reduce(false);
+            }
+            if (has_nl && !fx_nl) {
                 SGPU_CUDA_TRY(cudaMemsetAsync(alpha, 0, abytes, st));
                 ProfScope ps(ctx, SGPU_KERNEL_NL_PROJECT, st);
                 const dim3 pg(nl.nimg, (unsigned)hg.size());
@@ -1204,7 +1499,19 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
                         nl.ip_displ, nl.gamma64, ctx->dV);
                 ctx->launches++;
             }
-            for (long w0 = 0; w0 < totcols; w0 += maxw) {
+            for (long w0 = 0; fx_st && w0 < totcols; w0 += 65535 / fxl.g.nslab) {
+                const long nw = std::min<long>(65535 / fxl.g.nslab, totcols - w0);
+                ProfScope ps(ctx, SGPU_KERNEL_STENCIL, st);
+                const dim3 grid(fxl.tilesx, fxl.tilesy, (unsigned)(nw * fxl.g.nslab));
+                auto kern = fxl.ns <= 2 ? (fxl.cube ? k_stencil_fxzb<2, true> : k_stencil_fxzb<2, false>)
+                            : fxl.ns == 3 ? (fxl.cube ? k_stencil_fxzb<3, true> : k_stencil_fxzb<3, false>)
+                                          : (fxl.cube ? k_stencil_fxzb<4, true> : k_stencil_fxzb<4, false>);
+                kern<<<grid, fxl.threads, fxl.smem, st>>>(dB128, dC, dW + w0, fxl.g, ctx->veff64,
+                                                          ctx->veff_key ? ctx->veff_fx : nullptr, Nd, m,
+                                                          j, in, out, zsel);
+                ctx->launches++;
+            }
+            for (long w0 = 0; !fx_st && w0 < totcols; w0 += maxw) {
                 const long nw = std::min(maxw, totcols - w0);
                 ProfScope ps(ctx, SGPU_KERNEL_STENCIL, st);
                 if constexpr (sizeof(CT) == 8) {
@@ -1222,7 +1529,16 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
                                                                zsel);
                 ctx->launches++;
             }
-            if (has_nl) {
+            if (fx_nl) {
+                ProfScope ps(ctx, SGPU_KERNEL_NL_APPLY, st);
+                const bool more = j + 1 < m, second = j & 1;
+                auto kern = more ? (nl.max_np <= 9 ? k_nl_fx_zb<true, true, 9> : k_nl_fx_zb<true, true, 18>)
+                                 : (nl.max_np <= 9 ? k_nl_fx_zb<true, false, 9> : k_nl_fx_zb<true, false, 18>);
+                kern<<<dim3(nblk * fgx, fxt->nrange), 32 * nlfx::kWarps, fsm, st>>>(fT, dB128, dC, m, j, out,
+                                                                                   second, fgx);
+                ctx->launches++;
+                if (more) fx_reduce(!second);
+            } else if (has_nl) {
                 ProfScope ps(ctx, SGPU_KERNEL_NL_APPLY, st);
                 constexpr int CB = zapply_cb<CT>();
                 const size_t stage = sizeof(CT) * (size_t)nl.max_chunk_rows * zstage_ld<CT, CB>();
@@ -1263,7 +1579,19 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
     if (ctx->prof_on) return issue();  // per-launch events need plain launches
     std::vector<long> key = {(long)sizeof(CT), nblk, m, (long)(uintptr_t)tb, (long)(uintptr_t)W,
                              (long)(uintptr_t)alpha, (long)hg.size(), nslab, (long)pairs,
-                             (long)(uintptr_t)ctx->veff64, (long)(uintptr_t)ctx->veff32};
+                             (long)(uintptr_t)ctx->veff64, (long)(uintptr_t)ctx->veff32,
+                             (long)fx_st, (long)fx_nl, (long)(uintptr_t)alpha2, (long)(uintptr_t)part,
+                             (long)(uintptr_t)(fx_nl ? fxt->chi : nullptr), fgx,
+                             (long)(uintptr_t)ctx->veff_fx, (long)(ctx->veff_key != 0)};
+    if (fx_st) {  // the launch's numbers: they move with the coefficients and the potential's size
+        key.push_back(fxl.s);
+        key.push_back(fxl.g.dv);
+        key.push_back(fxl.g.KW);
+        key.push_back(fxl.g.nslab * 4096L + fxl.g.TX * 64 + fxl.g.TY);
+        for (int a = 0; a < 3; a++)
+            for (int r = 0; r < kMaxFDn; r++)
+                key.push_back(((long)fxl.g.wh[a][r] << 32) ^ (unsigned)fxl.g.wl[a][r]);
+    }
     for (int b = 0; b < nblk; b++) {
         key.push_back(blk[b].ncol);
         key.push_back((long)(uintptr_t)blk[b].X);

@@ -1114,11 +1114,10 @@ void nonlocal_free(Nonlocal &nl)
                     nl.rng_pt0,  nl.rng_ent0, nl.rng_item0, nl.item_e0, nl.item_row,
                     nl.item_wsplit,
                     nl.pe_lp,    nl.pe_chi32, nl.tc_pt0, nl.tc_pts, nl.tc_row0, nl.tc_rows,
-                    nl.tc_ent0,  nl.tc_ent,   nl.tc_chi,   nl.fx_pt0, nl.fx_pts, nl.fx_item0,
-                    nl.fx_ent0,  nl.fx_items, nl.fx_wsplit, nl.fx_lp, nl.fx_chi,  nl.fx_er,
-                    nl.fx_row0,  nl.fx_sum_ptr, nl.fx_sum_idx, nl.fx_rows};
+                    nl.tc_ent0,  nl.tc_ent,   nl.tc_chi, nl.fx_er};
     for (void *p : ptrs)
         if (p) cudaFree(p);
+    nonlocal_fx_free(nl);
     nl = Nonlocal();
 }
 

@@ -67,26 +67,27 @@ int launch(sgpu_ctx *ctx, int ncol, const double *alpha, double scale, double *o
            const double *x, long ld, double *alpha_next, long lda, cudaStream_t st)
 {
     const Nonlocal &nl = ctx->nl;
-    const nlfx::Tables T = nonlocal_fx_tables(nl);
+    const int groups = (ncol + nlfx::kLanes - 1) / nlfx::kLanes;
+    const NlFx &X = nonlocal_fx_pick(nl, groups);
+    const nlfx::Tables T = nonlocal_fx_tables(nl, X);
     const size_t smem = nlfx::smem_bytes(T);
     auto kern = nl.max_np <= 9 ? k_nl_fx<APPLY, PROJ, 9> : k_nl_fx<APPLY, PROJ, 18>;
     SGPU_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)smem));
-    const int groups = (ncol + nlfx::kLanes - 1) / nlfx::kLanes;
     const long ldp = (long)groups * nlfx::kLanes;
     double *part = nullptr;
     if (PROJ)
-        SGPU_TRY(ws_get(ctx, WS_NLPART, sizeof(double) * (size_t)nl.fx_nrows * ldp, (void **)&part));
+        SGPU_TRY(ws_get(ctx, WS_NLPART, sizeof(double) * (size_t)X.nrows * ldp, (void **)&part));
     {
         ProfScope ps(ctx, APPLY ? SGPU_KERNEL_NL_APPLY : SGPU_KERNEL_NL_PROJECT, st);
-        for (int r0 = 0; r0 < nl.fx_nrange; r0 += 65535) {
+        for (int r0 = 0; r0 < X.nrange; r0 += 65535) {
             nlfx::Tables R = T;
             R.pt0 += r0;
             R.item0 += r0;
             R.row0 += r0;
             // blocks of few ranges split the column groups, so that there are at least 8 per SM
-            const int gx = std::min(groups, std::max(1, 152 * 8 / nl.fx_nrange));
-            const dim3 grid(gx, std::min(65535, nl.fx_nrange - r0));
+            const int gx = std::min(groups, std::max(1, 152 * 8 / X.nrange));
+            const dim3 grid(gx, std::min(65535, X.nrange - r0));
             kern<<<grid, 32 * nlfx::kWarps, smem, st>>>(R, ncol, alpha, scale, out, x, ld, part,
                                                         lda, ldp);
         }
@@ -96,7 +97,7 @@ int launch(sgpu_ctx *ctx, int ncol, const double *alpha, double scale, double *o
         ProfScope ps(ctx, SGPU_KERNEL_NL_PROJECT, st);
         const int bx = ncol <= 64 ? 32 : 128;
         k_fx_reduce<<<dim3((ncol + bx - 1) / bx, nl.ntot), bx, 0, st>>>(
-            nl.fx_sum_ptr, nl.fx_sum_idx, part, ldp, ncol, ctx->dV, nl.gamma64, alpha_next, lda);
+            X.sum_ptr, X.sum_idx, part, ldp, ncol, ctx->dV, nl.gamma64, alpha_next, lda);
         SGPU_CUDA_TRY(cudaGetLastError());
     }
     return SGPU_OK;
@@ -104,14 +105,33 @@ int launch(sgpu_ctx *ctx, int ncol, const double *alpha, double scale, double *o
 
 }  // namespace
 
-nlfx::Tables nonlocal_fx_tables(const Nonlocal &nl)
+nlfx::Tables nonlocal_fx_tables(const Nonlocal &nl, const NlFx &x)
 {
-    return {nl.fx_pt0, nl.fx_pts, nl.fx_item0, nl.fx_items, nl.fx_ent0, nl.fx_wsplit, nl.fx_lp,
-            nl.fx_chi, nl.fx_rows, nl.fx_row0, nl.fx_jp, nl.fx_max_rows, nl.fx_max_ent,
-            nl.fx_max_items};
+    return {x.pt0, x.pts, x.item0, x.items, x.ent0, x.wsplit, x.lp, x.chi, x.rows, x.row0, nl.fx_jp,
+            x.max_rows, x.max_ent, x.max_items};
 }
 
-bool nonlocal_fx_ready(const sgpu_ctx *ctx) { return ctx->has_nl && ctx->nl.fx_nrange > 0; }
+// The large ranges when they and the column groups make two blocks per SM, else the small ones:
+// 32-point ranges hold few entries per atom, so the rows' and columns' conversions weigh more
+// (26^3, 32 columns: 28 large ranges leave most SMs idle; 34^3, 20 blocks of 64 complex columns:
+// 80 large ranges against 310 small ones)
+const NlFx &nonlocal_fx_pick(const Nonlocal &nl, long groups)
+{
+    return nl.fx[1].nrange > 0 && nl.fx[0].nrange * groups < 304 ? nl.fx[1] : nl.fx[0];
+}
+
+bool nonlocal_fx_ready(const sgpu_ctx *ctx) { return ctx->has_nl && ctx->nl.fx[0].nrange > 0; }
+
+void nonlocal_fx_free(Nonlocal &nl)
+{
+    for (NlFx &x : nl.fx) {
+        void *ptrs[] = {x.pt0, x.pts, x.item0, x.ent0, x.wsplit, x.items, x.rows, x.lp, x.chi, x.row0,
+                        x.sum_ptr, x.sum_idx};
+        for (void *p : ptrs)
+            if (p) cudaFree(p);
+        x = NlFx();
+    }
+}
 
 int launch_nonlocal_fx_project(sgpu_ctx *ctx, int ncol, const double *x, long ldx, double *alpha,
                                long lda, cudaStream_t st)
@@ -129,38 +149,14 @@ int launch_nonlocal_fx_apply(sgpu_ctx *ctx, int ncol, const double *alpha, long 
 
 // Range tables. A range takes covered points in the order of 32 x 4 x 4 blocks of the grid until it
 // holds `cap` of them or the next point's images would take its rows past kRows or its Chi digits
-// past kChiBytes; cap is the
-// largest of 128, 64 and 32 that still gives two blocks per SM for one column group, so small
-// cells spread over the chip. No tables (and the FP64 kernels stay) for more than 18 projectors
-// per atom, for a point under more than kPtRows projector rows (the 64-bit sums hold that many)
-// and for Chi values outside 1e-40 .. 1e40.
-int nonlocal_fx_build(Nonlocal &nl, const std::vector<int> &ord, const std::vector<int> &covpts,
-                      const std::vector<int> &covptr, const std::vector<long> &ent_chi,
-                      const std::vector<int4> &ent_meta, const double *chi)
+// past kChiBytes. No tables (and the FP64 kernels stay) for more than 18 projectors per atom, for a
+// point under more than kPtRows projector rows (the 64-bit sums hold that many) and for Chi
+// values outside 1e-40 .. 1e40.
+static int build_ranges(Nonlocal &nl, NlFx &x, int cap, const std::vector<int> &er,
+                        const std::vector<int> &ord, const std::vector<int> &covpts,
+                        const std::vector<int> &covptr, const std::vector<long> &ent_chi,
+                        const std::vector<int4> &ent_meta)
 {
-    nl.fx_nrange = 0;
-    if (nl.max_np > 18 || nl.max_np < 1 || nl.ncov == 0) return SGPU_OK;
-    // exponent of each projector row's largest Chi value
-    std::vector<int> er(nl.ntot, 0);
-    {
-        std::vector<double> mx(nl.ntot, 0.0);
-        for (long e = 0; e < nl.nent; e++) {
-            const int4 m = ent_meta[e];
-            for (int j = 0; j < m.y; j++) {
-                const double v = std::fabs(chi[ent_chi[e] + (long)j * m.z]);
-                if (!(v < 1e40)) return SGPU_OK;  // NaN too
-                mx[m.x + j] = std::max(mx[m.x + j], v);
-            }
-        }
-        for (int i = 0; i < nl.ntot; i++) {
-            if (mx[i] == 0.0) continue;
-            if (mx[i] < 1e-40) return SGPU_OK;
-            std::frexp(mx[i], &er[i]);
-        }
-    }
-    int cap = nlfx::kPts;
-    while (cap > 32 && nl.ncov < cap * 304) cap /= 2;
-
     std::vector<int> pt0(1, 0), pts, item0(1, 0), ent0(1, 0), row0(1, 0), wsplit;
     std::vector<int4> items, rowinfo;
     std::vector<unsigned char> lp;
@@ -172,10 +168,9 @@ int nonlocal_fx_build(Nonlocal &nl, const std::vector<int> &ord, const std::vect
     rows.reserve(nl.nent);
     std::vector<int> slot(nl.nimg, -1);                 // image -> item of the current range
     std::vector<std::vector<std::pair<int, int>>> bucket;  // per item: (point, entry)
-    nl.fx_jp = nl.max_np <= 9 ? 10 : 18;
     const int max_ent = nlfx::kChiBytes / (8 * nl.fx_jp);
     int k = 0;
-    nl.fx_max_rows = nl.fx_max_ent = nl.fx_max_items = 0;
+    x.max_rows = x.max_ent = x.max_items = 0;
     while (k < nl.ncov) {
         const int q0 = k;
         int nrow = 0, nitem = 0, nent = 0;
@@ -205,9 +200,9 @@ int nonlocal_fx_build(Nonlocal &nl, const std::vector<int> &ord, const std::vect
             k++;
         }
         if (k == q0) return SGPU_OK;
-        nl.fx_max_rows = std::max(nl.fx_max_rows, nrow);
-        nl.fx_max_ent = std::max(nl.fx_max_ent, nent);
-        nl.fx_max_items = std::max(nl.fx_max_items, nitem);
+        x.max_rows = std::max(x.max_rows, nrow);
+        x.max_ent = std::max(x.max_ent, nent);
+        x.max_items = std::max(x.max_items, nitem);
         // owner warps of the apply: runs of points with about equal entry counts
         int wb[nlfx::kWarps + 1];
         {
@@ -250,8 +245,8 @@ int nonlocal_fx_build(Nonlocal &nl, const std::vector<int> &ord, const std::vect
         row0.push_back(row0.back() + nrow);
     }
     // per projector row, its rows of the partial buffer in range order
-    nl.fx_nrows = row0.back();
-    std::vector<int> sum_ptr(nl.ntot + 1, 0), sum_idx(nl.fx_nrows);
+    x.nrows = row0.back();
+    std::vector<int> sum_ptr(nl.ntot + 1, 0), sum_idx(x.nrows);
     for (const int4 &I : items)
         for (int j = 0; j < I.z; j++) sum_ptr[I.y + j + 1]++;
     for (int i = 0; i < nl.ntot; i++) sum_ptr[i + 1] += sum_ptr[i];
@@ -275,28 +270,27 @@ int nonlocal_fx_build(Nonlocal &nl, const std::vector<int> &ord, const std::vect
     };
     long2 *dsrc = nullptr;
     int2 *drows = nullptr;
-    up(&nl.fx_pt0, pt0);
-    up(&nl.fx_pts, pts);
-    up(&nl.fx_item0, item0);
-    up(&nl.fx_items, items);
-    up(&nl.fx_ent0, ent0);
-    up(&nl.fx_wsplit, wsplit);
-    up(&nl.fx_lp, lp);
-    up(&nl.fx_er, er);
-    up(&nl.fx_rows, rowinfo);
-    up(&nl.fx_row0, row0);
-    up(&nl.fx_sum_ptr, sum_ptr);
-    up(&nl.fx_sum_idx, sum_idx);
+    up(&x.pt0, pt0);
+    up(&x.pts, pts);
+    up(&x.item0, item0);
+    up(&x.items, items);
+    up(&x.ent0, ent0);
+    up(&x.wsplit, wsplit);
+    up(&x.lp, lp);
+    up(&x.rows, rowinfo);
+    up(&x.row0, row0);
+    up(&x.sum_ptr, sum_ptr);
+    up(&x.sum_idx, sum_idx);
     up(&dsrc, src);
     up(&drows, rows);
     const size_t cbytes = sizeof(int2) * (size_t)nl.nent * nl.fx_jp;
-    if (rc == SGPU_OK && cudaMalloc((void **)&nl.fx_chi, cbytes) != cudaSuccess) {
+    if (rc == SGPU_OK && cudaMalloc((void **)&x.chi, cbytes) != cudaSuccess) {
         set_error("set_nonlocal: device allocation of the Chi digits failed");
         rc = SGPU_ERR_CUDA;
     }
     if (rc == SGPU_OK) {
         k_fx_chi<<<152 * 8, 256>>>(dsrc, drows, nl.nent, nl.fx_jp, nl.chi64, nl.fx_er,
-                                   reinterpret_cast<int2 *>(nl.fx_chi));
+                                   reinterpret_cast<int2 *>(x.chi));
         if (cudaDeviceSynchronize() != cudaSuccess) {
             set_error("set_nonlocal: the Chi digit kernel failed");
             rc = SGPU_ERR_CUDA;
@@ -304,8 +298,43 @@ int nonlocal_fx_build(Nonlocal &nl, const std::vector<int> &ord, const std::vect
     }
     if (dsrc) cudaFree(dsrc);
     if (drows) cudaFree(drows);
-    if (rc == SGPU_OK) nl.fx_nrange = (int)pt0.size() - 1;
+    if (rc == SGPU_OK) x.nrange = (int)pt0.size() - 1;
     return rc;
+}
+
+
+int nonlocal_fx_build(Nonlocal &nl, const std::vector<int> &ord, const std::vector<int> &covpts,
+                      const std::vector<int> &covptr, const std::vector<long> &ent_chi,
+                      const std::vector<int4> &ent_meta, const double *chi)
+{
+    if (nl.max_np > 18 || nl.max_np < 1 || nl.ncov == 0) return SGPU_OK;
+    // exponent of each projector row's largest Chi value
+    std::vector<int> er(nl.ntot, 0);
+    {
+        std::vector<double> mx(nl.ntot, 0.0);
+        for (long e = 0; e < nl.nent; e++) {
+            const int4 m = ent_meta[e];
+            for (int j = 0; j < m.y; j++) {
+                const double v = std::fabs(chi[ent_chi[e] + (long)j * m.z]);
+                if (!(v < 1e40)) return SGPU_OK;  // NaN too
+                mx[m.x + j] = std::max(mx[m.x + j], v);
+            }
+        }
+        for (int i = 0; i < nl.ntot; i++) {
+            if (mx[i] == 0.0) continue;
+            if (mx[i] < 1e-40) return SGPU_OK;
+            std::frexp(mx[i], &er[i]);
+        }
+    }
+    SGPU_CUDA_TRY(cudaMalloc((void **)&nl.fx_er, sizeof(int) * er.size()));
+    SGPU_CUDA_TRY(cudaMemcpy(nl.fx_er, er.data(), sizeof(int) * er.size(), cudaMemcpyHostToDevice));
+    nl.fx_jp = nl.max_np <= 9 ? 10 : 18;
+    SGPU_TRY(build_ranges(nl, nl.fx[0], nlfx::kPts, er, ord, covpts, covptr, ent_chi, ent_meta));
+    // small ranges where one column group in large ones leaves SMs without a block
+    if (nl.fx[0].nrange > 0 && nl.fx[0].nrange < 304)
+        SGPU_TRY(build_ranges(nl, nl.fx[1], nl.fx[0].nrange < 152 ? 32 : 64, er, ord, covpts, covptr,
+                              ent_chi, ent_meta));
+    return SGPU_OK;
 }
 
 }  // namespace sgpu

@@ -375,5 +375,6 @@ __device__ __forceinline__ void block(const Tables &T, int r, int g0, int gstep,
 
 }  // namespace nlfx
 
-nlfx::Tables nonlocal_fx_tables(const Nonlocal &nl);
+nlfx::Tables nonlocal_fx_tables(const Nonlocal &nl, const NlFx &x);
+const NlFx &nonlocal_fx_pick(const Nonlocal &nl, long groups);
 }  // namespace sgpu

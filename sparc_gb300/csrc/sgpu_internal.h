@@ -55,6 +55,18 @@ void set_error(const std::string &msg);
 //    alpha = Chiᵀ x, parallel over (image, point chunk);
 //  * point order (a CSR over covered grid points): for the owner-computes apply
 //    Hx[p] += sum over entries (image, i) of Chi_img[i, :] alpha_atom.
+// FP64 apply and projection in block fixed point (nonlocal_fx.cuh): the tables of one range size;
+// nrange 0: none
+struct NlFx {
+    int nrange = 0, max_rows = 0, max_ent = 0, max_items = 0, nrows = 0;
+    int *pt0 = nullptr, *pts = nullptr, *item0 = nullptr, *ent0 = nullptr, *wsplit = nullptr;
+    int4 *items = nullptr, *rows = nullptr;
+    unsigned char *lp = nullptr;
+    int4 *chi = nullptr;
+    int *row0 = nullptr;
+    int *sum_ptr = nullptr, *sum_idx = nullptr;  // projector row -> its partial rows
+};
+
 struct Nonlocal {
     int natom = 0, nimg = 0, ntot = 0, max_np = 0;
     long nchi = 0, npos = 0;
@@ -107,16 +119,9 @@ struct Nonlocal {
     int *tc_ent0 = nullptr;     // tc_nrange + 1: first merged entry of each range
     int *tc_ent = nullptr;      // point | row offset << 7 | projector count << 14
     float *tc_chi = nullptr;    // Chi values of the merged entries, range_jp per entry
-    // FP64 apply and projection in block fixed point (nonlocal_fx.cuh); fx_nrange 0: no tables
-    int fx_nrange = 0, fx_jp = 0, fx_max_rows = 0, fx_max_ent = 0, fx_max_items = 0,
-        fx_nrows = 0;
-    int *fx_pt0 = nullptr, *fx_pts = nullptr, *fx_item0 = nullptr, *fx_ent0 = nullptr;
-    int4 *fx_items = nullptr, *fx_rows = nullptr;
-    int *fx_wsplit = nullptr;
-    unsigned char *fx_lp = nullptr;
-    int4 *fx_chi = nullptr;
-    int *fx_er = nullptr, *fx_row0 = nullptr;
-    int *fx_sum_ptr = nullptr, *fx_sum_idx = nullptr;  // projector row -> its partial rows
+    NlFx fx[2];                 // fixed-point tables: large ranges, and small ones (or none)
+    int *fx_er = nullptr;       // exponent of each projector row's largest Chi value
+    int fx_jp = 0;
 };
 
 // A potential as fixed-point digits (fixed64.cuh) for the FP64 stencil; key: the exponent key of its
@@ -322,6 +327,7 @@ std::vector<int> compact_order(int Nx, int Ny, const std::vector<int> &covpts);
 // written, not added to), and the apply into out with, when alpha_next is given, the projection
 // of the finished out
 bool nonlocal_fx_ready(const sgpu_ctx *ctx);
+void nonlocal_fx_free(Nonlocal &nl);
 int nonlocal_fx_build(Nonlocal &nl, const std::vector<int> &ord, const std::vector<int> &covpts,
                       const std::vector<int> &covptr, const std::vector<long> &ent_chi,
                       const std::vector<int4> &ent_meta, const double *chi);

@@ -40,6 +40,7 @@ struct StencilFxParams {
     long ldx, ldo, ldz;
     int Nx, Ny, Nz, nslab, zlen;
     int TX, TY, hx, hy;      // tile; halo entries of the x sides (12 TY) and of the y sides
+    int s;                   // unit of the coefficient digits: 2^-s
     int KW;                  // T 2^(KW + E) is the stencil sum (E the block exponent)
     int dv;                  // the potential's products count 2^-dv of the stencil's
     int c0h, c0l;            // digits of c0 and of a w_r
@@ -404,6 +405,7 @@ inline bool fx_setup(StencilFxParams &p, int FDn, unsigned vkey)
         eS = std::max(eS, ev + 3);
     }
     const int s = 2 * fx::kDigit + 1 - eS;          // S 2^s < 2^59: digits below 2^30
+    p.s = s;
     fx_coef(p.c0, s, p.c0h, p.c0l);
     for (int d = 0; d < 3; d++)
         for (int r = 0; r < FDn; r++) fx_coef(p.w[d][r], s, p.wh[d][r], p.wl[d][r]);

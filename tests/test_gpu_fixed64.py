@@ -172,3 +172,71 @@ def test_nonlocal_nonfinite_columns(gpu_available):
     assert np.all(np.isnan(y[5][covered])) and not np.any(np.isfinite(y[7][covered]))
     assert np.all(y[36] == 0.0) and np.all(y[:, ~covered] == 0.0)
     ctx.close()
+
+
+def _kpt_case(N, h, natom, seed):
+    rng = np.random.default_rng(seed)
+    c = fd_d2_coeffs(6, h)
+    grid = dict(Nx=N[0], Ny=N[1], Nz=N[2], FDn=6, cx=c, cy=c, cz=c, dV=h ** 3)
+    nl = synthetic_nonlocal(rng, N, h, natom=natom, rc=1.6)
+    L = np.array(N) * h
+    # two images per atom at most matter here: give every image a copy of the cell
+    coords = rng.uniform(0, 1, (len(nl["img_atom"]), 3)) * L + rng.integers(-1, 2, (len(nl["img_atom"]), 3)) * L
+    ctx = sg.Context(*N, 6, c, c, c, h ** 3)
+    v = rng.normal(size=N[0] * N[1] * N[2])
+    ctx.set_veff(np.concatenate([v, -0.5 * v]), nspin=2)
+    ctx.set_nonlocal(nl["ip_displ"], nl["gamma"], nl["img_atom"], nl["img_ndc"], nl["grid_pos"],
+                     nl["chi"])
+    ctx.set_kpoint_geometry(L, coords)
+    S = 1.5 * (abs(c[0]) + 2 * np.abs(c[1:]).sum()) + np.abs(v).max()
+    return ctx, Oracle(grid, nl), rng, L, coords, v, S
+
+
+@pytest.mark.parametrize("N", [(17, 14, 20), (6, 12, 9), (34, 13, 12), (25, 24, 31)])
+def test_bloch_columns(gpu_available, N):
+    """Tiles with halos across the cell faces, Bloch vectors with zero, half and other components,
+    column counts around the group of 16, both spins, one block and batched, a non-finite column.
+    One apply is off by at most the oracle's own rounding: 80 units of 2^-53 (complex factors
+    double the real kernel's 40) of the sum of coefficients, plus as much for the projectors."""
+    import torch
+    ctx, o, rng, L, co, v, S = _kpt_case(N, 0.45, 3, sum(N))
+    Nd = N[0] * N[1] * N[2]
+    ks = [2 * np.pi / L * np.array(q) for q in ((0, 0, 0), (0.5, 0, -0.25), (0.1, 0.3, 0.2))]
+    for k in ks:
+        for ncol in (1, 15, 17):
+            x = rng.uniform(-1, 1, (ncol, Nd)) + 1j * rng.uniform(-1, 1, (ncol, Nd))
+            y = np.zeros_like(x)
+            ctx.Hamiltonian_vectors_mult_kpt(k, -7.0, x, y, spin=1)
+            ref = o.hamiltonian_kpt(k, L, co, -0.5 * v, -7.0, x)
+            vnl = np.abs(o.vnl_kpt(k, L, co, x)).max()
+            assert np.abs(y - ref).max() <= 80 * 2.0 ** -53 * (1.5 * (S + 7.0) + 200 * vnl)
+    blocks, x0 = [], []
+    for i, k in enumerate(ks):
+        for spin in (0, 1):
+            ncol = (3, 16, 20)[i]
+            x = torch.complex(torch.from_numpy(rng.uniform(-1, 1, (ncol, Nd))),
+                              torch.from_numpy(rng.uniform(-1, 1, (ncol, Nd)))).cuda()
+            if i == 1 and spin == 0:
+                x[4, 7] = float("nan")
+            x0.append(x.clone())
+            blocks.append(dict(spin=spin, k=[float(q) for q in k], X=x, Y=torch.empty_like(x),
+                               a=0.3 * S, b=2.5 * S, a0=-2.0 * S))
+    for rep in range(2):  # the second call replays the captured launches on new numbers
+        for b, x in zip(blocks, x0):
+            b["X"].copy_(x)
+        ctx.ChebyshevFiltering_batched(blocks, 5)
+        for i, (b, x) in enumerate(zip(blocks, x0)):
+            X, Y = x.cpu().numpy().copy(), np.zeros((x.shape[0], Nd), dtype=np.complex128)
+            ctx.ChebyshevFiltering_kpt(np.array(b["k"]), X, Y, 5, b["a"], b["b"], b["a0"],
+                                       spin=b["spin"])
+            y, xx = b["Y"].cpu().numpy(), b["X"].cpu().numpy()
+            ok = [n for n in range(x.shape[0]) if not (i == 2 and n == 4)]
+            assert np.isfinite(y[ok]).all()
+            assert np.abs(y - Y)[ok].max() <= 1e-12 * np.abs(Y[ok]).max()
+            assert np.abs(xx - X)[ok].max() <= 1e-12 * np.abs(X[ok]).max()
+            if i == 2:
+                assert np.isnan(y[4]).any()
+        if rep == 0:
+            for b in blocks:  # other bounds: the same shapes and buffers
+                b["b"] *= 1.1
+    ctx.close()

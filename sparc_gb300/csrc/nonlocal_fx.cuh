@@ -69,7 +69,8 @@ inline size_t smem_bytes(const Tables &T)
 {
     return sizeof(long long) * kPts * kPitch + 8 * (size_t)kLanes * T.max_rows +
            8 * (size_t)T.max_ent * T.jp + align16(T.max_ent) + 16 * (size_t)T.max_rows +
-           16 * (size_t)T.max_items + align16(4 * (size_t)T.max_items * (kWarps + 2));
+           16 * (size_t)T.max_items +
+           align16(4 * ((size_t)T.max_items + 1 + (size_t)T.max_items * (kWarps + 1)));
 }
 
 // raw sum in units of 2^57. A product is below 2^113, so 128 of them end below 2^63 units (what an

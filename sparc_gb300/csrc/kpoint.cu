@@ -590,40 +590,28 @@ __global__ void __launch_bounds__(32 * nlfx::kWarps, 2)
                                          reinterpret_cast<double *>(part), lda, ldp, phase,
                                          nlfxz_smem);
 }
-// alpha row = dV Gamma times the sum of its partial rows, in their order; one component a thread
-__device__ __forceinline__ void fx_reduce_row(const int *__restrict__ ptr, const int *__restrict__ idx,
-                                              const double *__restrict__ part, long ldp, int c, int row,
-                                              double f, double *__restrict__ alpha, long lda)
-{
-    double s[4] = {0.0, 0.0, 0.0, 0.0};
-    const int e1 = ptr[row + 1];
-    int e = ptr[row];
-    for (; e + 4 <= e1; e += 4)
-#pragma unroll
-        for (int u = 0; u < 4; u++) s[u] += __ldg(part + (long)idx[e + u] * ldp + c);
-    for (; e < e1; e++) s[0] += __ldg(part + (long)idx[e] * ldp + c);
-    alpha[(long)row * lda + c] = f * ((s[0] + s[1]) + (s[2] + s[3]));
-}
-__global__ void k_fx_reduce_zb(const BBlock<double2> *__restrict__ blocks, const int *__restrict__ ptr,
-                               const int *__restrict__ idx, double dV,
-                               const double *__restrict__ gamma, bool second)
+// alpha rows from the partial projections (nlfx::reduce_row on the interleaved components)
+__global__ void __launch_bounds__(256)
+    k_fx_reduce_zb(const BBlock<double2> *__restrict__ blocks, const int *__restrict__ ptr,
+                   const int *__restrict__ idx, double dV, const double *__restrict__ gamma,
+                   bool second)
 {
     const BBlock<double2> &B = blocks[blockIdx.z];
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < 2 * B.ncol)
-        fx_reduce_row(ptr, idx, reinterpret_cast<const double *>(B.part), 2 * B.ldp, c, blockIdx.y,
-                      dV * gamma[blockIdx.y],
-                      reinterpret_cast<double *>(second ? B.alpha2 : B.alpha), 2L * B.ncol);
+    const int row = blockIdx.y;
+    if ((int)blockIdx.x * 32 >= 2 * B.ncol) return;
+    nlfx::reduce_row(ptr[row], ptr[row + 1], idx, reinterpret_cast<const double *>(B.part), 2 * B.ldp,
+                     blockIdx.x * 32, 2 * B.ncol, dV * gamma[row],
+                     reinterpret_cast<double *>(second ? B.alpha2 : B.alpha) + 2L * B.ncol * row);
 }
-__global__ void k_fx_reduce_z(const double2 *__restrict__ part, long ldp, const int *__restrict__ ptr,
-                              const int *__restrict__ idx, double dV,
-                              const double *__restrict__ gamma, int ncol, double2 *__restrict__ alpha,
-                              long lda)
+__global__ void __launch_bounds__(256)
+    k_fx_reduce_z(const double2 *__restrict__ part, long ldp, const int *__restrict__ ptr,
+                  const int *__restrict__ idx, double dV, const double *__restrict__ gamma, int ncol,
+                  double2 *__restrict__ alpha, long lda)
 {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < 2 * ncol)
-        fx_reduce_row(ptr, idx, reinterpret_cast<const double *>(part), 2 * ldp, c, blockIdx.y,
-                      dV * gamma[blockIdx.y], reinterpret_cast<double *>(alpha), 2 * lda);
+    const int row = blockIdx.y;
+    nlfx::reduce_row(ptr[row], ptr[row + 1], idx, reinterpret_cast<const double *>(part), 2 * ldp,
+                     blockIdx.x * 32, 2 * ncol, dV * gamma[row],
+                     reinterpret_cast<double *>(alpha) + 2 * lda * row);
 }
 
 template <int R>
@@ -1097,7 +1085,7 @@ static int nonlocal_z(sgpu_ctx *ctx, int ncol, const CT *x, long ldx, CT *out, l
                     ProfScope ps(ctx, SGPU_KERNEL_NL_PROJECT, st);
                     project<<<grid, 32 * nlfx::kWarps, sm, st>>>(T, ncol, nullptr, 0.0,
                         const_cast<CT *>(x), ldx, part, lda, ldp, ks->img_phase);
-                    k_fx_reduce_z<<<dim3((2 * ncol + 127) / 128, nl.ntot), 128, 0, st>>>(
+                    k_fx_reduce_z<<<dim3((2 * ncol + 31) / 32, nl.ntot), 256, 0, st>>>(
                         part, ldp, X.sum_ptr, X.sum_idx, ctx->dV, nl.gamma64, ncol, alpha, lda);
                 }
                 ProfScope ps(ctx, SGPU_KERNEL_NL_APPLY, st);
@@ -1448,7 +1436,7 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
     const BBlock<double2> *dB128 = reinterpret_cast<const BBlock<double2> *>(dB);
     // the sums of the partial projections into one of the two buffers
     auto fx_reduce = [&](bool second) {
-        k_fx_reduce_zb<<<dim3((2 * maxcol + 127) / 128, nl.ntot, nblk), 128, 0, st>>>(
+        k_fx_reduce_zb<<<dim3((2 * maxcol + 31) / 32, nl.ntot, nblk), 256, 0, st>>>(
             dB128, fxt->sum_ptr, fxt->sum_idx, ctx->dV, nl.gamma64, second);
         ctx->launches++;
     };

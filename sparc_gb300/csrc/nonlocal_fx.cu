@@ -21,23 +21,15 @@ __global__ void __launch_bounds__(32 * nlfx::kWarps, 2)
                                           out, x, ld, part, lda, ldp, nullptr, smem_nlfx);
 }
 
-// alpha[row] = dV Gamma[row] times the sum of the row's partial projections, in the order of ptr/idx;
-// n: doubles per row
-__global__ void k_fx_reduce(const int *__restrict__ ptr, const int *__restrict__ idx,
-                            const double *__restrict__ part, long ldp, int n, double dV,
-                            const double *__restrict__ gamma, double *__restrict__ alpha, long lda)
+// alpha[row] = dV Gamma[row] times the sum of the row's partial projections (nlfx::reduce_row)
+__global__ void __launch_bounds__(256)
+    k_fx_reduce(const int *__restrict__ ptr, const int *__restrict__ idx,
+                const double *__restrict__ part, long ldp, int n, double dV,
+                const double *__restrict__ gamma, double *__restrict__ alpha, long lda)
 {
     const int row = blockIdx.y;
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n) return;
-    const int e1 = ptr[row + 1];
-    double s[4] = {0.0, 0.0, 0.0, 0.0};
-    int e = ptr[row];
-    for (; e + 4 <= e1; e += 4)
-#pragma unroll
-        for (int u = 0; u < 4; u++) s[u] += __ldg(part + (long)idx[e + u] * ldp + c);
-    for (; e < e1; e++) s[0] += __ldg(part + (long)idx[e] * ldp + c);
-    alpha[(long)row * lda + c] = dV * gamma[row] * ((s[0] + s[1]) + (s[2] + s[3]));
+    nlfx::reduce_row(ptr[row], ptr[row + 1], idx, part, ldp, blockIdx.x * 32, n,
+                     dV * __ldg(gamma + row), alpha + (long)row * lda);
 }
 
 // Chi digits of the entries: value j of entry e is chi[src[e].x + j * src[e].y] scaled by its row's
@@ -95,8 +87,7 @@ int launch(sgpu_ctx *ctx, int ncol, const double *alpha, double scale, double *o
     }
     if (PROJ) {
         ProfScope ps(ctx, SGPU_KERNEL_NL_PROJECT, st);
-        const int bx = ncol <= 64 ? 32 : 128;
-        k_fx_reduce<<<dim3((ncol + bx - 1) / bx, nl.ntot), bx, 0, st>>>(
+        k_fx_reduce<<<dim3((ncol + 31) / 32, nl.ntot), 256, 0, st>>>(
             X.sum_ptr, X.sum_idx, part, ldp, ncol, ctx->dV, nl.gamma64, alpha_next, lda);
         SGPU_CUDA_TRY(cudaGetLastError());
     }

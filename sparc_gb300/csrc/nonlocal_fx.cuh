@@ -374,6 +374,35 @@ __device__ __forceinline__ void block(const Tables &T, int r, int g0, int gstep,
     }
 }
 
+// out[c] = f times the sum over e in [e0, e1) of part[idx[e]][c] for the 32 doubles c from c0 (below
+// n): the block's eight warps take every eighth row, and their sums are added in warp order, so
+// the result is fixed by the tables alone. One thread per column instead waits for its rows one
+// after another (26^3: 15 us for 144 rows).
+__device__ __forceinline__ void reduce_row(int e0, int e1, const int *__restrict__ idx,
+                                           const double *__restrict__ part, long ldp, int c0, int n,
+                                           double f, double *__restrict__ out)
+{
+    __shared__ double sh[kWarps][32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = c0 + lane;
+    double s0 = 0.0, s1 = 0.0;
+    if (c < n) {
+        int e = e0 + warp;
+        for (; e + kWarps < e1; e += 2 * kWarps) {
+            s0 += __ldg(part + (long)__ldg(idx + e) * ldp + c);
+            s1 += __ldg(part + (long)__ldg(idx + e + kWarps) * ldp + c);
+        }
+        if (e < e1) s0 += __ldg(part + (long)__ldg(idx + e) * ldp + c);
+    }
+    sh[warp][lane] = s0 + s1;
+    __syncthreads();
+    if (warp == 0 && c < n) {
+        double s = sh[0][lane];
+#pragma unroll
+        for (int w = 1; w < kWarps; w++) s += sh[w][lane];
+        out[c] = f * s;
+    }
+}
+
 }  // namespace nlfx
 
 nlfx::Tables nonlocal_fx_tables(const Nonlocal &nl, const NlFx &x);

@@ -130,6 +130,43 @@ __global__ void __launch_bounds__(BX *BY)
     }
 }
 
+// FP64 kernel for the smallest launches: a point per thread, its 37 values straight from L1, the
+// arithmetic of k_stencil_orth. Nothing waits for a barrier or a previous plane, so a launch takes
+// a few microseconds as long as the FP64 pipe's 42 instructions per point do (0.6 us per 10^4
+// points and columns): 14^3 x 8 in 7.4 us where the fixed-point slabs take 11.2.
+__global__ void __launch_bounds__(128) k_stencil_point(const StencilParams<double> p)
+{
+    constexpr int R = kMaxFDn;
+    const int NxNy = p.Nx * p.Ny, n = NxNy * p.Nz;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int col = blockIdx.y;
+    const double *__restrict__ x = p.x + (long)col * p.ldx;
+    const int k = i / NxNy, jx = i - k * NxNy, j = jx / p.Nx, ix = jx - j * p.Nx;
+    const double xi = __ldg(x + i);
+    const double v = p.v ? __ldg(p.v + i) : 0.0;
+    const double z = p.z ? p.z[(long)col * p.ldz + i] : 0.0;
+    double rx = p.c0 * xi, ry = 0.0, rz = 0.0;
+#pragma unroll
+    for (int q = 1; q <= R; q++) {
+        const int xm = i - q + (ix < q ? p.Nx : 0), xp = i + q - (ix + q >= p.Nx ? p.Nx : 0);
+        const int ym = i - q * p.Nx + (j < q ? NxNy : 0), yp = i + q * p.Nx - (j + q >= p.Ny ? NxNy : 0);
+        const int zm = i - q * NxNy + (k < q ? n : 0), zp = i + q * NxNy - (k + q >= p.Nz ? n : 0);
+        rx = fma(__ldg(x + xm) + __ldg(x + xp), p.wx[q], rx);
+        ry = fma(__ldg(x + ym) + __ldg(x + yp), p.wy[q], ry);
+        rz = fma(__ldg(x + zm) + __ldg(x + zp), p.wz[q], rz);
+    }
+    double res = rx + (ry + rz);
+    if (p.v) res += p.bv * (v * xi);
+    double o = p.s1 * res;
+    if (p.z) o += p.s2 * z;
+    p.out[(long)col * p.ldo + i] = o;
+}
+// Largest points x columns for it. Both kernels per call of the filter, point against slabs: 14^3 x 1
+// 7.4 and 9.6 us, 20^3 x 6 9 and 11, 46^3 x 1 13 and 15; 26^3 x 5, 20^3 x 12 and 14^3 x 32 (88000 to
+// 96000) 13 and 12 to 13; 61x45x53 x 1 (145000) 17 and 14, 20^3 x 24 (192000) 21 and 15.
+constexpr long kPointMax = 100000;
+
 // FP32 kernel: each thread owns two neighbouring x-points. Shared-memory reads are paired
 // (8-byte), the neighbour pair sums use Blackwell's packed f32x2 add, and the weighted sums
 // run as three independent FMA chains (x, y, z) whose weights come straight from the kernel
@@ -1156,6 +1193,12 @@ int launch_stencil(sgpu_ctx *ctx, int ncol, double a, double bv, double c, const
     if (!z || s2 == 0.0) p.z = nullptr;
 
     if constexpr (sizeof(T) == 8) {
+        if (ctx->Nd * ncol <= kPointMax) {
+            ProfScope ps(ctx, SGPU_KERNEL_STENCIL, st);
+            k_stencil_point<<<dim3((unsigned)((ctx->Nd + 127) / 128), ncol), 128, 0, st>>>(p);
+            SGPU_CUDA_TRY(cudaGetLastError());
+            return SGPU_OK;
+        }
         bool done = false;
         if (fixed) SGPU_TRY(launch_stencil_fx(ctx, ncol, p, pot, &done, st));
         if (done) return SGPU_OK;

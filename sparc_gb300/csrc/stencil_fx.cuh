@@ -354,8 +354,9 @@ inline void fx_coef(double w, int s, int &h, int &l)
 // Tile edges and z slabs of a launch, by the time that a model of the kernel gives. A plane of a
 // resident block costs 2.8 clocks per point and SM, plus 0.17 of a point per halo value
 // (measured at 96^3: 16x16 tiles 3.34, 32x16 3.53, 32x32 4.17 clocks per point), a block alone
-// on its SM 1.35 and two 1.1 of that (their barriers are exposed), and at least 900 clocks (the
-// latency of one step); a slab starts with the 13 planes of its queue, about 5 planes' time.
+// on its SM 1.35 and two 1.1 of that (their barriers are exposed), and at least 2700 clocks (the
+// latency of one step, from 14^3 and 26^3 launches); a slab starts with the 13 planes of its
+// queue, about 5 planes' time.
 // Many columns: whole columns in the tiles that pad least; few: enough slabs and small tiles to
 // fill the SMs.
 inline void fx_plan(int Nx, int Ny, int Nz, int ncol, int nsm, int &TX, int &TY, int &nslab)
@@ -379,7 +380,7 @@ inline void fx_plan(int Nx, int Ny, int Nz, int ncol, int nsm, int &TX, int &TY,
                 const double waves = std::ceil(nblk / ((double)nsm * fit));
                 const double res = std::min<double>(fit, std::ceil(nblk / nsm));
                 const double work = res * (2.0 * thr + 0.17 * halo) * (res < 4 ? f[(int)res] : 1.0);
-                const double t = waves * (5.0 + (Nz + ns - 1) / ns) * std::max(900.0, 2.8 * work);
+                const double t = waves * (5.0 + (Nz + ns - 1) / ns) * std::max(2700.0, 2.8 * work);
                 if (t < 0.999 * best) { best = t; TX = tx; TY = ty; nslab = ns; }
             }
         }

@@ -325,7 +325,7 @@ inline bool fxz_plan(int Nx, int Ny, int Nz, long ncol, int nsm, int &TX, int &T
                 const double waves = std::ceil(nblk / ((double)nsm * fit));
                 const double res = std::min<double>(fit, std::ceil(nblk / nsm));
                 const double work = res * 2.0 * (thr + 0.17 * halo) * (res < 4 ? f[(int)res] : 1.0);
-                const double t = waves * (5.0 + (Nz + ns - 1) / ns) * std::max(900.0, 2.8 * work);
+                const double t = waves * (5.0 + (Nz + ns - 1) / ns) * std::max(2700.0, 2.8 * work);
                 // as good: the wider tile (rows are read along x; 34^3: 17 x 9 tiles 2.86 ms per
                 // degree, 9 x 17 3.00)
                 if (t < 0.999 * best || (t < 1.001 * best && tx > TX)) {

@@ -45,6 +45,31 @@ def test_stencil_fields(gpu_available, N, h):
     ctx.close()
 
 
+@pytest.mark.parametrize("N", [(14, 14, 14), (6, 7, 9), (31, 17, 23), (45, 33, 12), (34, 12, 70),
+                               (77, 20, 13)])
+@pytest.mark.parametrize("h", [(0.4, 0.4, 0.4), (0.4, 0.37, 0.45)])
+def test_stencil_fields_many_columns(gpu_available, N, h):
+    """The same fields and bound in calls of at least 120000 points and columns, above the sizes
+    that the point-per-thread kernel takes: the fields' columns in turn."""
+    rng = np.random.default_rng(sum(N))
+    c = [fd_d2_coeffs(6, x) for x in h]
+    grid = dict(Nx=N[0], Ny=N[1], Nz=N[2], FDn=6, cx=c[0], cy=c[1], cz=c[2], dV=float(np.prod(h)))
+    ctx = sg.Context(*N, 6, *c, grid["dV"])
+    o = Oracle(grid, None)
+    Nd = N[0] * N[1] * N[2]
+    v = rng.normal(size=Nd)
+    S = 0.5 * sum(abs(w[0]) + 2 * np.abs(w[1:]).sum() for w in c) + 3.1 + np.abs(v).max()
+    cols = np.concatenate(list(_fields(N, rng).values()))
+    x = np.ascontiguousarray(np.resize(cols, (max(len(cols), -(-120000 // Nd)), Nd)))
+    y = np.full_like(x, np.nan)
+    ctx.Lap_plus_diag_vec_mult_orth(-0.5, 1.0, -3.1, v, x, y)
+    ref = o.lap_plus_diag(-0.5, 1.0, -3.1, v, cols)
+    for n in range(x.shape[0]):
+        tol = 40 * 2.0 ** -53 * S * np.abs(x[n]).max()
+        assert np.abs(y[n] - ref[n % len(cols)]).max() <= tol
+    ctx.close()
+
+
 @pytest.mark.parametrize("scale", [1.0, 1e3, 1e9, 0.0])
 def test_stencil_potential_range(gpu_available, scale):
     """A potential of the stencil's own size, one far above it (the FP64 kernel takes over) and
@@ -75,8 +100,10 @@ def test_stencil_potential_range(gpu_available, scale):
     ctx.close()
 
 
-def test_stencil_nonfinite(gpu_available):
-    """An infinity and a NaN reach exactly the points whose stencil touches them."""
+@pytest.mark.parametrize("reps", [1, 4])
+def test_stencil_nonfinite(gpu_available, reps):
+    """An infinity and a NaN reach exactly the points whose stencil touches them; below and above
+    the sizes of the point-per-thread kernel."""
     N, h = (33, 21, 30), 0.4
     rng = np.random.default_rng(6)
     c = fd_d2_coeffs(6, h)
@@ -87,9 +114,10 @@ def test_stencil_nonfinite(gpu_available):
     x[0, Nd // 3] = np.nan
     x[1, Nd // 2] = np.inf
     x[2, 7] = -np.inf
+    x = np.tile(x, (reps, 1))
     y = np.zeros_like(x)
     ctx.Lap_vec_mult(0.3, x, y)
-    ref = Oracle(grid, None).lap_plus_diag(1.0, 0.0, 0.3, None, x)
+    ref = np.tile(Oracle(grid, None).lap_plus_diag(1.0, 0.0, 0.3, None, x[:3]), (reps, 1))
     fin = np.isfinite(ref)
     assert np.array_equal(np.isfinite(y), fin) and np.array_equal(np.isnan(y), np.isnan(ref))
     S = 3 * (abs(c[0]) + 2 * np.abs(c[1:]).sum()) + 0.3

@@ -108,6 +108,19 @@ __device__ __forceinline__ void mma_bf16(unsigned tmem_d, unsigned long long ade
         : "memory");
 }
 
+// instruction descriptor with n columns (kIdesc is the 128-column one)
+__device__ __forceinline__ void mma_bf16_n(unsigned tmem_d, unsigned long long adesc,
+                                           unsigned long long bdesc, int n, unsigned accumulate)
+{
+    const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(n >> 3) << 17) |
+                           ((unsigned)(TM >> 4) << 24);
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
 // arrive once on the barrier when every tcgen05.mma issued so far by this thread has completed
 __device__ __forceinline__ void mma_commit(unsigned bar)
 {
@@ -309,19 +322,38 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_tc_gemm(const TcParams p)
                         const unsigned a0 = sbase + st * S::stage_bytes;
                         const unsigned b0 = a0 + NS * TILE_BYTES;
                         const bool chunk_first = k == c * CHUNK_STEPS;
+                        if constexpr (NS == 3) {
+                            // the levels lie side by side in tensor memory and B's slices in
+                            // shared memory: two slices are one 256-column product on two levels
 #pragma unroll
-                        for (int i = 0; i < NS; i++) {
+                            for (int kk = 0; kk < 2; kk++) {
+                                const unsigned fresh = chunk_first && kk == 0 ? 0u : 1u;
+                                auto mma = [&](int i, int j, int nj, unsigned accum) {
+                                    mma_bf16_n(tmem + (i + j) * TN,
+                                               smem_desc(a0 + i * TILE_BYTES + kk * 256),
+                                               smem_desc(b0 + j * TILE_BYTES + kk * 256), nj * TN,
+                                               accum);
+                                };
+                                mma(0, 0, 2, fresh);
+                                mma(0, 2, 1, fresh);
+                                mma(1, 0, 2, 1u);
+                                mma(2, 0, 1, 1u);
+                            }
+                        } else {
 #pragma unroll
-                            for (int j = 0; i + j < NS; j++) {
-                                const int acc = min(i + j, 3);
-                                const bool acc_first = i == 0 && j <= 3;
+                            for (int i = 0; i < NS; i++) {
 #pragma unroll
-                                for (int kk = 0; kk < 2; kk++) {
-                                    const unsigned accum =
-                                        (chunk_first && acc_first && kk == 0) ? 0u : 1u;
-                                    mma_bf16(tmem + acc * TN,
-                                             smem_desc(a0 + i * TILE_BYTES + kk * 256),
-                                             smem_desc(b0 + j * TILE_BYTES + kk * 256), accum);
+                                for (int j = 0; i + j < NS; j++) {
+                                    const int acc = min(i + j, 3);
+                                    const bool acc_first = i == 0 && j <= 3;
+#pragma unroll
+                                    for (int kk = 0; kk < 2; kk++) {
+                                        const unsigned accum =
+                                            (chunk_first && acc_first && kk == 0) ? 0u : 1u;
+                                        mma_bf16(tmem + acc * TN,
+                                                 smem_desc(a0 + i * TILE_BYTES + kk * 256),
+                                                 smem_desc(b0 + j * TILE_BYTES + kk * 256), accum);
+                                    }
                                 }
                             }
                         }
@@ -464,21 +496,74 @@ __device__ __forceinline__ Bits bits_of(float x)
     return r;
 }
 
-// slices of x 2^(-e) (|x 2^-e| < 1) as exact BF16 numbers S_i 2^(-7(i+1)), i < NS
-template <int NS>
-__device__ __forceinline__ void split7(Bits x, int e, __nv_bfloat16 *out)
+// 7-bit digits of x 2^-e (|x 2^-e| < 1) as numbers d_i 2^(-7(i+1)), i < NS, of the fixed-point
+// integer V, each rounded to nearest (with eight slices nothing depends on which of two forms a
+// digit takes: there a bias of 64 per digit makes them plain bit fields). A digit becomes a float
+// by placing it below the exponent of 1.5 2^23 units: one add, no conversion instruction (with
+// integer conversions and 64-bit digits throughout the split of a 456533 x 520 FP32 operand took
+// 1.40 ms against 0.36 for its bytes).
+template <int NS, typename VT>
+__device__ __forceinline__ void digits7(VT V, float (&d)[NS])
 {
-    const int sh = x.p - e + 7 * NS;  // U = round(m 2^sh)
+    VT bias = 0;
+#pragma unroll
+    for (int i = 0; i + 1 < NS; i++) bias = (bias << 7) + 64;
+    if (NS == 8) V += bias;
+#pragma unroll
+    for (int i = 0; i < NS; i++) {
+        // unit 2^(-7(i+1)): the float 1.5 2^23 units has its last bit there
+        const int base = ((127 + 23 - 7 * (i + 1)) << 23) | 0x400000;
+        const int sh = 7 * (NS - 1 - i);
+        int f;
+        if (NS == 8) {
+            f = i == 0 ? (int)(V >> sh) : (int)((V >> sh) & 127) - 64;
+        } else {
+            const VT S = sh ? (V + ((VT)1 << (sh ? sh - 1 : 0))) >> sh : V;
+            V -= S << sh;
+            f = (int)S;
+        }
+        d[i] = __fsub_rn(__int_as_float(base + f), __int_as_float(base));
+    }
+}
+template <int NS>
+__device__ __forceinline__ void split7(Bits x, int e, float (&d)[NS])
+{
+    const int sh = x.p - e + 7 * NS;  // V = round(m 2^sh)
     long long V;
     if (sh >= 0) V = x.m << min(sh, 62);
     else if (sh > -62) V = (x.m + (1ll << (-sh - 1))) >> (-sh);
     else V = 0;
+    digits7<NS>(V, d);
+}
+// a value of a K-vector with scale e (after eb more binary digits): the FP32, three-slice form in
+// 32-bit integers (24 bits of significand, 21 of fixed point)
+template <int NS, typename T>
+__device__ __forceinline__ void split_value(T x, int e, float (&d)[NS])
+{
+    if constexpr (sizeof(T) == 4 && NS == 3) {
+        const unsigned b = __float_as_uint(x);
+        const int be = (int)((b >> 23) & 0xff);
+        const int m = (int)(b & 0x7fffffu) | (be ? 0x800000 : 0);
+        const int s = e - (be ? be : 1) + 150 - 21;  // V = m 2^-s, s >= 2 unless x = 0
+        const int sm = (int)b < 0 ? -m : m;
+        digits7<3>(m && s < 26 ? (sm + (1 << (s - 1))) >> s : 0, d);
+    } else {
+        split7<NS>(bits_of(x), e, d);
+    }
+}
+// the slices of eight consecutive K values, `slice` elements apart
+template <int NS>
+__device__ __forceinline__ void put8(const float (&sl)[8][NS], __nv_bfloat16 *dst, long slice)
+{
 #pragma unroll
     for (int i = 0; i < NS; i++) {
-        const int d = 7 * (NS - 1 - i);
-        const long long S = d ? (V + (1ll << (d - 1))) >> d : V;
-        V -= S << d;
-        out[i] = __float2bfloat16_rn(__ll2float_rn(S) * __int_as_float((127 - 7 * (i + 1)) << 23));
+        unsigned w[4];
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+            const __nv_bfloat162 b = __floats2bfloat162_rn(sl[2 * t][i], sl[2 * t + 1][i]);
+            w[t] = *reinterpret_cast<const unsigned *>(&b);
+        }
+        *reinterpret_cast<uint4 *>(dst + i * slice) = make_uint4(w[0], w[1], w[2], w[3]);
     }
 }
 
@@ -493,6 +578,21 @@ __device__ __forceinline__ int tile_off(int r, int k)
 // (max |x| < 2^e); 0 for a zero row
 __device__ __forceinline__ int scale_of(int fe_max) { return fe_max < -(1 << 27) ? 0 : fe_max; }
 
+// a key ordered as |x| is (up to the low word of a double; zero for zero only), and the frexp
+// exponent of its values
+__device__ __forceinline__ unsigned magnitude_key(float x) { return __float_as_uint(x) & 0x7fffffffu; }
+__device__ __forceinline__ unsigned magnitude_key(double x)
+{
+    const unsigned h = (unsigned)__double2hiint(x) & 0x7fffffffu;
+    return h | (__double2loint(x) != 0 && h == 0u ? 1u : 0u);
+}
+template <typename T>
+__device__ __forceinline__ int key_exponent(unsigned key)
+{
+    if (sizeof(T) == 4) return key >> 23 ? (int)(key >> 23) - 126 : -126;
+    return key >> 20 ? (int)(key >> 20) - 1022 : -1022;
+}
+
 // scale of each column of X (rows x cols, column-major), the entries of row r first scaled by
 // 2^(ksign * ek[r]) when ek is given: one block per column
 template <typename T>
@@ -501,8 +601,15 @@ __global__ void k_colmax_exp(const T *__restrict__ X, long ld, long rows, const 
 {
     const T *x = X + (long)blockIdx.x * ld;
     int mx = -(1 << 28);
-    for (long r = threadIdx.x; r < rows; r += blockDim.x)
-        mx = max(mx, bits_of(x[r]).fe + (ek ? ksign * ek[r] : 0));
+    if (ek) {
+        for (long r = threadIdx.x; r < rows; r += blockDim.x)
+            mx = max(mx, bits_of(x[r]).fe + ksign * ek[r]);
+    } else {  // the largest magnitude by its bit pattern, its exponent once
+        unsigned key = 0u;
+#pragma unroll 8
+        for (long r = threadIdx.x; r < rows; r += blockDim.x) key = max(key, magnitude_key(x[r]));
+        if (key) mx = key_exponent<T>(key);
+    }
     __shared__ int red[32];
     for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
@@ -544,23 +651,16 @@ __global__ void __launch_bounds__(256) k_split_cols(const T *__restrict__ X, lon
         const int r = u >> 2, g = u & 3;
         const int n = rb * TM + r;
         const long k0 = (long)s * TK + g * 8;
-        __nv_bfloat16 sl[8][NS];
+        float sl[8][NS];
         const int en = n < ncols ? e[n] : 0;
 #pragma unroll
         for (int t = 0; t < 8; t++) {
             const long k = k0 + t;
             const bool in = n < ncols && k < krows;
-            const Bits v = bits_of(in ? X[(long)n * ld + k] : T(0));
-            split7<NS>(v, en - (ek && in ? ksign * ek[k] : 0), sl[t]);
+            split_value<NS>(in ? X[(long)n * ld + k] : T(0), en - (ek && in ? ksign * ek[k] : 0),
+                            sl[t]);
         }
-#pragma unroll
-        for (int i = 0; i < NS; i++) {
-            __align__(16) __nv_bfloat16 w[8];
-#pragma unroll
-            for (int t = 0; t < 8; t++) w[t] = sl[t][i];
-            *reinterpret_cast<uint4 *>(tiles + i * TILE_ELEMS + tile_off(r, g * 8)) =
-                *reinterpret_cast<const uint4 *>(w);
-        }
+        put8<NS>(sl, tiles + tile_off(r, g * 8), TILE_ELEMS);
     }
 }
 
@@ -579,22 +679,14 @@ __global__ void __launch_bounds__(256) k_split_rows(const T *__restrict__ X, lon
         const int g = u >> 7, r = u & 127;  // a warp: 32 consecutive rows, one K group
         const long m = (long)rb * TM + r;
         const int em = m < rows ? e[m] : 0;
-        __nv_bfloat16 sl[8][NS];
+        float sl[8][NS];
 #pragma unroll
         for (int t = 0; t < 8; t++) {
             const int k = s * TK + g * 8 + t;
             const bool in = m < rows && k < kcols;
-            const Bits v = bits_of(in ? X[(long)k * ld + m] : T(0));
-            split7<NS>(v, em + (in ? ec[k] : 0), sl[t]);
+            split_value<NS>(in ? X[(long)k * ld + m] : T(0), em + (in ? ec[k] : 0), sl[t]);
         }
-#pragma unroll
-        for (int i = 0; i < NS; i++) {
-            __align__(16) __nv_bfloat16 w[8];
-#pragma unroll
-            for (int t = 0; t < 8; t++) w[t] = sl[t][i];
-            *reinterpret_cast<uint4 *>(tiles + i * TILE_ELEMS + tile_off(r, g * 8)) =
-                *reinterpret_cast<const uint4 *>(w);
-        }
+        put8<NS>(sl, tiles + tile_off(r, g * 8), TILE_ELEMS);
     }
 }
 
@@ -815,19 +907,6 @@ struct TcxParams {
     long ldc;
     int *status;
 };
-
-// instruction descriptor with n columns (kIdesc is the 128-column one)
-__device__ __forceinline__ void mma_bf16_n(unsigned tmem_d, unsigned long long adesc,
-                                           unsigned long long bdesc, int n, unsigned accumulate)
-{
-    const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(n >> 3) << 17) |
-                           ((unsigned)(TM >> 4) << 24);
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
 
 // Gram work item -> (row tile, column tile): the 128 x 64 tiles that touch the upper triangle
 __device__ __forceinline__ void upper_tile(int t, int ntiles, int &mt, int &nt)
@@ -1070,42 +1149,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_tc_gemm_x(const TcxParams p, in
                      : "memory");
 }
 
-// Eight balanced 7-bit digits of x 2^-e (|x 2^-e| < 1) as BF16 numbers d_i 2^(-7(i+1)). A bias of 64
-// per digit makes them plain bit fields; a digit becomes a float by placing it below the
-// exponent of 1.5 2^23 ulps (one add, no conversion instruction).
-__device__ __forceinline__ void split8x(Bits x, int e, float (&d)[XS])
-{
-    const int sh = x.p - e + 7 * XS;
-    long long V;
-    if (sh >= 0) V = x.m << min(sh, 62);
-    else if (sh > -62) V = (x.m + (1ll << (-sh - 1))) >> (-sh);
-    else V = 0;
-    constexpr long long bias = 64ll * (1ll + (1ll << 7) + (1ll << 14) + (1ll << 21) + (1ll << 28) +
-                                       (1ll << 35) + (1ll << 42));
-    V += bias;
-#pragma unroll
-    for (int i = 0; i < XS; i++) {
-        // unit 2^(-7(i+1)): the float 1.5 2^23 units has its last bit there
-        const int base = ((127 + 23 - 7 * (i + 1)) << 23) | 0x400000;
-        const int f = i == 0 ? (int)(V >> (7 * (XS - 1)))
-                             : (int)((V >> (7 * (XS - 1 - i))) & 127) - 64;
-        d[i] = __fsub_rn(__int_as_float(base + f), __int_as_float(base));
-    }
-}
-__device__ __forceinline__ void put8x(const float (&sl)[8][XS], __nv_bfloat16 *dst, long slice)
-{
-#pragma unroll
-    for (int i = 0; i < XS; i++) {
-        unsigned w[4];
-#pragma unroll
-        for (int t = 0; t < 4; t++) {
-            const __nv_bfloat162 b = __floats2bfloat162_rn(sl[2 * t][i], sl[2 * t + 1][i]);
-            w[t] = *reinterpret_cast<const unsigned *>(&b);
-        }
-        *reinterpret_cast<uint4 *>(dst + i * slice) = make_uint4(w[0], w[1], w[2], w[3]);
-    }
-}
-
 // as k_split_cols: tile row = column n of X, K = rows k0 .. of X; slice-major layout
 __global__ void __launch_bounds__(256) k_split_cols_x(const double *__restrict__ X, long ld,
                                                       long krows, int ncols,
@@ -1126,10 +1169,10 @@ __global__ void __launch_bounds__(256) k_split_cols_x(const double *__restrict__
         for (int t = 0; t < 8; t++) {
             const long k = k0 + t;
             const bool in = n < ncols && k < krows;
-            split8x(bits_of(in ? X[(long)n * ld + k] : 0.0), en - (ek && in ? ksign * ek[k] : 0),
-                    sl[t]);
+            split_value<XS>(in ? X[(long)n * ld + k] : 0.0, en - (ek && in ? ksign * ek[k] : 0),
+                            sl[t]);
         }
-        put8x(sl, base + tile_off(r, g * 8), slice);
+        put8<XS>(sl, base + tile_off(r, g * 8), slice);
     }
 }
 // as k_split_rows: tile row = grid point, K = columns of X scaled by 2^-ec
@@ -1151,9 +1194,9 @@ __global__ void __launch_bounds__(256) k_split_rows_x(const double *__restrict__
         for (int t = 0; t < 8; t++) {
             const int k = s * TK + g * 8 + t;
             const bool in = m < rows && k < kcols;
-            split8x(bits_of(in ? X[(long)k * ld + m] : 0.0), em + (in ? ec[k] : 0), sl[t]);
+            split_value<XS>(in ? X[(long)k * ld + m] : 0.0, em + (in ? ec[k] : 0), sl[t]);
         }
-        put8x(sl, base + tile_off(r, g * 8), slice);
+        put8<XS>(sl, base + tile_off(r, g * 8), slice);
     }
 }
 

@@ -3,9 +3,10 @@
 // side, and the Bloch factor of a value's unwrapped position applied in FP64 before it becomes
 // digits (only to values from outside the cell).
 //
-// What bounds it: as there, and eight FP64 instructions per point (output scale, recurrence term and
-// the factors of halo values from outside the cell). 34^3, 20 blocks of 64 columns: 12.6 ms per
-// degree in k_stencil_zb<double2>, 2.9 here.
+// What bounds it: latency at the 15 warps that 128 registers leave (46 % of the issue slots busy, the
+// FP64 pipe, which has the output scale, the recurrence term and the factors, 37 %; with the
+// factors as selects on every value it was the bound at 75 %, and 2.9 ms). 34^3, 20 blocks of 64
+// columns: 12.6 ms per degree in k_stencil_zb<double2>, 1.87 here.
 #pragma once
 
 #include "stencil_fx.cuh"
@@ -34,6 +35,19 @@ struct FxZCol {                // one column
 __device__ __forceinline__ double2 fxz_mul(double2 a, double2 b)
 {
     return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
+}
+
+// v times the factor f[i] in the warps where some lane's i is not one, the index of a factor of one.
+// A loop, so that the branch stays: a conditional product becomes predicated instructions, which
+// hold the FP64 pipe (16 clocks an instruction) also where every lane is off.
+__device__ __forceinline__ double2 fxz_turn(double2 v, const double2 *f, int i, int one)
+{
+    bool turn = i != one;
+    while (__any_sync(0xffffffffu, turn)) {
+        v = fxz_mul(v, f[i]);
+        turn = false;
+    }
+    return v;
 }
 
 // planes k .. ze-1 of a thread's point in FP64, straight from global memory
@@ -90,7 +104,7 @@ __device__ __forceinline__ void stencil_fxz(const FxZConst &p, const FxZCol &c, 
 {
     constexpr int R = kMaxFDn, P = kFxZPitch;
     __shared__ unsigned s_key;
-    __shared__ double2 s_f[9];                      // factors of the shifts (dx, dy), index 3 dy' + dx'
+    __shared__ double2 s_f[27];                     // factors of the shifts, index 9 dz' + 3 dy' + dx'
     const int t = threadIdx.x, nthr = blockDim.x;
     const int ty = min(t / p.TX, p.TY - 1), tx = t % p.TX;
     const bool own = t < p.TX * p.TY;               // threads beyond the tile only load halos
@@ -99,7 +113,9 @@ __device__ __forceinline__ void stencil_fxz(const FxZConst &p, const FxZCol &c, 
     const int x0 = blockIdx.x * p.TX, y0 = blockIdx.y * p.TY;
     const int zs = slab * p.zlen, ze = min(zs + p.zlen, p.Nz);
     if (zs >= ze) return;
-    if (t < 9) s_f[t] = fxz_mul(c.bf[t % 3], c.bf[3 + t / 3]);
+    if (t < 27)
+        s_f[t] = t == 13 ? make_double2(1.0, 0.0)
+                         : fxz_mul(fxz_mul(c.bf[t % 3], c.bf[3 + t / 3 % 3]), c.bf[6 + t / 9]);
     const int i = x0 + tx, j = y0 + ty;
     const bool act = own && i < p.Nx && j < p.Ny;
     const unsigned plane = 16u * (unsigned)p.Nx * (unsigned)p.Ny;
@@ -107,7 +123,7 @@ __device__ __forceinline__ void stencil_fxz(const FxZConst &p, const FxZCol &c, 
     // checked that no position is a whole period or more away)
     auto place = [&](int px, int py, int &f) -> unsigned {
         const int dx = px < 0 ? 0 : px >= p.Nx ? 2 : 1, dy = py < 0 ? 0 : py >= p.Ny ? 2 : 1;
-        f = 3 * dy + dx;
+        f = 9 + 3 * dy + dx;
         return 16u * (unsigned)(px - (dx - 1) * p.Nx + (py - (dy - 1) * p.Ny) * p.Nx);
     };
     int of;
@@ -120,10 +136,12 @@ __device__ __forceinline__ void stencil_fxz(const FxZConst &p, const FxZCol &c, 
         const int e = t + u * nthr;
         ho[u] = 0u;
         hs[u] = -1;
-        hf[u] = 4;
+        hf[u] = 13;
         if (e < p.hx) {
-            const int row = e / (2 * R), q = e - row * 2 * R;
-            const int dx = q < R ? q - R : p.TX + q - R;
+            // all of the left side, then the right one: most warps hold values of one side, and
+            // a warp without values from outside the cell skips the factors
+            const int side = e / (R * p.TY), q = e - side * R * p.TY, row = q / R;
+            const int dx = q - row * R + (side ? p.TX : -R);
             ho[u] = place(x0 + dx, y0 + row, hf[u]);
             hs[u] = (row + R) * P + R + dx;
         } else if (e < p.hx + p.hy) {
@@ -137,10 +155,10 @@ __device__ __forceinline__ void stencil_fxz(const FxZConst &p, const FxZCol &c, 
     __syncthreads();
     // a factor of one (a zero Bloch component) costs nothing
     auto is_one = [](double2 f) { return f.x == 1.0 && f.y == 0.0; };
-    if (is_one(s_f[of])) of = 4;
+    if (is_one(s_f[of])) of = 13;
 #pragma unroll
     for (int u = 0; u < NS; u++)
-        if (is_one(s_f[hf[u]])) hf[u] = 4;
+        if (is_one(s_f[hf[u]])) hf[u] = 13;
     const bool turn_z = !is_one(c.bf[8]);
     auto ld = [&](const double2 *base, unsigned off) {
         return __ldg(reinterpret_cast<const double2 *>(reinterpret_cast<const char *>(base) + off));
@@ -150,21 +168,23 @@ __device__ __forceinline__ void stencil_fxz(const FxZConst &p, const FxZCol &c, 
     int2 vv = make_int2(0, 0);
     int E = fx::kMinExp, k = zs, kc = 0;            // kc: unwrapped plane of the next centre to load
     bool over = false;
-    auto centre = [&](int kk) {                     // this thread's value at unwrapped plane kk
+    int cf = 13;                                    // factor of the centre loaded ahead
+    auto centre = [&](int kk, int &f) {             // this thread's value at unwrapped plane kk
         const int dz = kk < 0 ? 0 : kk >= p.Nz ? 2 : 1;
-        double2 v = ld(c.x, plane * (unsigned)(kk - (dz - 1) * p.Nz) + o);
-        if (dz != 1 && turn_z) v = fxz_mul(v, c.bf[6 + dz]);
-        return of == 4 ? v : fxz_mul(v, s_f[of]);
+        f = turn_z ? of + 9 * (dz - 1) : of;
+        return ld(c.x, plane * (unsigned)(kk - (dz - 1) * p.Nz) + o);
     };
     auto load_next = [&](int kh) {                  // centre of plane kc (advanced), halo of plane kh
-        cc = kc < 2 * p.Nz ? centre(kc) : make_double2(0.0, 0.0);
+        cc = kc < 2 * p.Nz ? centre(kc, cf) : make_double2(0.0, 0.0);
         kc++;
         const unsigned ph = plane * (unsigned)kh;
 #pragma unroll
-        for (int u = 0; u < NS; u++) {
-            h[u] = ld(c.x, ph + ho[u]);
-            if (hf[u] != 4) h[u] = fxz_mul(h[u], s_f[hf[u]]);
-        }
+        for (int u = 0; u < NS; u++) h[u] = ld(c.x, ph + ho[u]);
+    };
+    auto turn_loaded = [&]() {                      // a step after the loads were issued
+        cc = fxz_turn(cc, s_f, cf, 13);
+#pragma unroll
+        for (int u = 0; u < NS; u++) h[u] = fxz_turn(h[u], s_f, hf[u], 13);
     };
     auto load_vz = [&](int kk) {
         const unsigned pk = plane * (unsigned)kk + o;
@@ -236,17 +256,13 @@ __device__ __forceinline__ void stencil_fxz(const FxZConst &p, const FxZCol &c, 
         }
         const int K = p.KW + E;
         double yr = fx::to_double(Tr, K), yi = fx::to_double(Ti, K);
-        if (c.z) {
-            yr = fma(c.s1, yr, c.s2 * z.x);
-            yi = fma(c.s1, yi, c.s2 * z.y);
-        } else if (c.s1 != 1.0) {
-            yr *= c.s1;
-            yi *= c.s1;
-        }
+        yr = fma(c.s1, yr, c.s2 * z.x);  // z is zero without a recurrence term
+        yi = fma(c.s1, yi, c.s2 * z.y);
         if (act)
             *reinterpret_cast<double2 *>(reinterpret_cast<char *>(c.out) + (plane * (unsigned)k + o)) =
                 make_double2(yr, yi);
         k++;
+        if (go_on && k + 1 < ze) turn_loaded();
         over = (key_of_loaded() >> 20) > (unsigned)E;
         return go_on;
     };
@@ -259,12 +275,15 @@ __device__ __forceinline__ void stencil_fxz(const FxZConst &p, const FxZCol &c, 
         unsigned key = 0u;
 #pragma unroll
         for (int m = 0; m <= 2 * R; m++) {
-            w[m] = centre(k - R + m);
+            int f;
+            w[m] = centre(k - R + m, f);
+            w[m] = fxz_turn(w[m], s_f, f, 13);
             key = max(key, key2(w[m]));
         }
         if (act) load_vz(k);
         kc = k + R + 1;
         load_next(k);  // the halo of plane k (the centre that comes with it is loaded again)
+        turn_loaded();
         key = __reduce_max_sync(0xffffffffu, max(key, key_of_loaded()));
         __syncthreads();
         if ((t & 31) == 0) atomicMax(&s_key, key);
@@ -284,6 +303,7 @@ __device__ __forceinline__ void stencil_fxz(const FxZConst &p, const FxZCol &c, 
         if (k + 1 < ze) {
             kc = k + R + 1;
             load_next(k + 1);
+            turn_loaded();
             over = (key_of_loaded() >> 20) > (unsigned)E;
         }
         while (true) {
@@ -326,8 +346,8 @@ inline bool fxz_plan(int Nx, int Ny, int Nz, long ncol, int nsm, int &TX, int &T
                 const double res = std::min<double>(fit, std::ceil(nblk / nsm));
                 const double work = res * 2.0 * (thr + 0.17 * halo) * (res < 4 ? f[(int)res] : 1.0);
                 const double t = waves * (5.0 + (Nz + ns - 1) / ns) * std::max(2700.0, 2.8 * work);
-                // as good: the wider tile (rows are read along x; 34^3: 17 x 9 tiles 2.86 ms per
-                // degree, 9 x 17 3.00)
+                // as good: the wider tile (rows are read along x; 34^3: 17 x 9 tiles 1.87 ms per
+                // degree, 9 x 17 2.05)
                 if (t < 0.999 * best || (t < 1.001 * best && tx > TX)) {
                     best = t; TX = tx; TY = ty; nslab = ns;
                 }

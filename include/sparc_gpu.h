@@ -625,10 +625,10 @@ int sgpu_set_gemm_emulation(sgpu_ctx *ctx, int mode);
  * reference (which calls cblas_dgemm). */
 int sgpu_set_rr_products(sgpu_ctx *ctx, int mode);
 
-/* complex64 stencil form: 1 (default) two x-neighbouring points per thread with packed reads
- * and a per-k table of Bloch factors (used where Nx and the leading dimensions are even and
- * the blocks 16-byte aligned); 0 the one-point-per-thread kernel. Both compute the same
- * operation sequence per point up to the rounding of the Bloch factors. */
+/* complex64 stencil form: 1 (default) tiles with packed FP32 arithmetic and a per-k table of
+ * Bloch factors; 0 the general kernel, which also serves grids whose tiles would reach a whole
+ * period away. Both compute the same operation sequence per point up to the rounding of the
+ * Bloch factors. */
 int sgpu_set_zstencil_pairs(sgpu_ctx *ctx, int on);
 
 /* Rayleigh-Ritz step of sgpu_CheFSI_batched / sgpu_scf_kpt: 1 (default) batches blocks of one

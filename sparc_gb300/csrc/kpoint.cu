@@ -179,51 +179,6 @@ __device__ __forceinline__ void stencil_z_body(const StencilZParams<CT> &p, int 
     }
 }
 
-constexpr int kPairMaxThreads = 320;
-
-template <int R>
-__global__ void __launch_bounds__(kPairMaxThreads)
-    k_stencil_z_c64(const __grid_constant__ ZPairConst g, const ZPairParams p)
-{
-    stencil_c64_pairs<R>(g, p, blockIdx.z / g.nslab, blockIdx.z % g.nslab);
-}
-
-// Tile of the pair kernel: BX (even, points) with the least padding of Nx, then BY with
-// the least padding of Ny among the heights that keep the block within kPairMaxThreads.
-static void zpair_tile(int Nx, int Ny, int R, int *bx2, int *by)
-{
-    int best = 1 << 30;
-    *bx2 = 16;
-    for (int t = std::min(32, std::max(4, (Nx + 1) / 2)); t >= 4; t--) {
-        const int waste = (Nx + 2 * t - 1) / (2 * t) * (2 * t) - Nx;
-        if (waste < best) { best = waste; *bx2 = t; }
-    }
-    best = 1 << 30;
-    *by = R;
-    for (int t = std::max(R, kPairMaxThreads / *bx2); t >= R; t--) {
-        if (*bx2 * t > kPairMaxThreads) continue;
-        const int waste = (Ny + t - 1) / t * t - Ny;
-        if (waste < best) { best = waste; *by = t; }
-    }
-}
-
-// The pair kernel applies when every fetch is within one period of the cell and the pairs are
-// 16-byte aligned.
-static bool zpair_ok(int Nx, int Ny, int Nz, int R, int bx2, int by)
-{
-    const int BX = 2 * bx2;
-    const int tx = (Nx + BX - 1) / BX, ty = (Ny + by - 1) / by;
-    const ZRing z = zring_shape(bx2, by, R, kPairAhead);
-    return Nx % 2 == 0 && R % 2 == 0 && R < Nx && R < Ny && R < Nz &&
-           tx * BX + R <= 2 * Nx && ty * by + R <= 2 * Ny &&
-           z.ncopy <= kPairCopies * bx2 * by && z.bytes <= 200 * 1024;
-}
-
-static size_t zpair_smem(int bx2, int by, int R)
-{
-    return zring_shape(bx2, by, R, kPairAhead).bytes;
-}
-
 // Threads per block of the complex stencil: complex128 (FP64-pipe bound, more registers per
 // point) at most 256, complex64 at most 512.
 template <typename CT>
@@ -562,6 +517,46 @@ __global__ void __launch_bounds__(kFxZThreads, 1)
     c.bf = b.bf;
     stencil_fxz<NS, CUBE>(g, c, slab, fxz_smem);
 }
+// complex64, the columns of all blocks and those of one
+template <int NS>
+__global__ void __launch_bounds__(kZTileThreads, kZTileResident / kZTileThreads)
+    k_stencil_ztb(const BBlock<float2> *__restrict__ blocks, const BCoef *__restrict__ coef,
+                  const int2 *__restrict__ work, const __grid_constant__ ZTileConst g,
+                  const float *__restrict__ veff32, long Nd, int m, int deg, int in_sel, int out_sel,
+                  int z_sel)
+{
+    extern __shared__ __align__(16) unsigned char zt_smem[];
+    const int w = blockIdx.z / g.nslab, slab = blockIdx.z % g.nslab;
+    const int2 bc = work[w];
+    const BBlock<float2> &B = blocks[bc.x];
+    const BCoef &cf = coef[(long)bc.x * m + deg];
+    ZTileCol c;
+    c.x = B.buf[in_sel] + (long)bc.y * B.ld[in_sel];
+    c.out = B.buf[out_sel] + (long)bc.y * B.ld[out_sel];
+    c.z = z_sel >= 0 ? B.buf[z_sel] + (long)bc.y * B.ld[z_sel] : nullptr;
+    c.v = veff32 ? veff32 + (long)B.spin * Nd : nullptr;
+    c.c0 = (float)cf.c0; c.s1 = (float)cf.s1; c.s2 = (float)cf.s2;
+    c.bf = B.bf;
+    stencil_c64_tile<NS>(g, c, slab, zt_smem);
+}
+struct ZTileOne {
+    ZTileCol c;            // column 0
+    long ldx, ldo, ldz;
+    double2 bf[9];
+};
+template <int NS>
+__global__ void __launch_bounds__(kZTileThreads, kZTileResident / kZTileThreads)
+    k_stencil_zt(const __grid_constant__ ZTileConst g, const __grid_constant__ ZTileOne b)
+{
+    extern __shared__ __align__(16) unsigned char zt_smem[];
+    const int col = blockIdx.z / g.nslab, slab = blockIdx.z % g.nslab;
+    ZTileCol c = b.c;
+    c.x += (long)col * b.ldx;
+    c.out += (long)col * b.ldo;
+    if (c.z) c.z += (long)col * b.ldz;
+    c.bf = b.bf;
+    stencil_c64_tile<NS>(g, c, slab, zt_smem);
+}
 // complex128 nonlocal products in block fixed point: grid (block and column-group phase, range)
 template <bool APPLY, bool PROJ, int MAXJ>
 __global__ void __launch_bounds__(32 * nlfx::kWarps, 2)
@@ -612,28 +607,6 @@ __global__ void __launch_bounds__(256)
     nlfx::reduce_row(ptr[row], ptr[row + 1], idx, reinterpret_cast<const double *>(part), 2 * ldp,
                      blockIdx.x * 32, 2 * ncol, dV * gamma[row],
                      reinterpret_cast<double *>(alpha) + 2 * lda * row);
-}
-
-template <int R>
-__global__ void __launch_bounds__(kPairMaxThreads)
-    k_stencil_zb_c64(const BBlock<float2> *__restrict__ blocks, const BCoef *__restrict__ coef,
-                     const int2 *__restrict__ work, const __grid_constant__ ZPairConst g,
-                     const float *__restrict__ veff32, long Nd, int m, int deg, int in_sel,
-                     int out_sel, int z_sel)
-{
-    const int w = blockIdx.z / g.nslab, slab = blockIdx.z % g.nslab;
-    const int2 bc = work[w];
-    const BBlock<float2> &B = blocks[bc.x];
-    const BCoef cf = coef[(long)bc.x * m + deg];
-    ZPairParams p;
-    p.x = B.buf[in_sel]; p.ldx = B.ld[in_sel];
-    p.out = B.buf[out_sel]; p.ldo = B.ld[out_sel];
-    p.z = z_sel >= 0 ? B.buf[z_sel] : nullptr; p.ldz = z_sel >= 0 ? B.ld[z_sel] : 0;
-    p.v32 = veff32 + (long)B.spin * Nd;
-    p.c0 = (float)cf.c0; p.s1 = (float)cf.s1; p.s2 = (float)cf.s2;
-#pragma unroll
-    for (int i = 0; i < 9; i++) p.bf[i] = make_float2((float)B.bf[i].x, (float)B.bf[i].y);
-    stencil_c64_pairs<R>(g, p, bc.y, slab);
 }
 
 // grid (image, column group); cg[y] = (block, first column)
@@ -881,7 +854,7 @@ static bool fxz_launch(const sgpu_ctx *ctx, const double (&w)[3][kMaxFDn], doubl
     L->s = d.s;
     FxZConst &g = L->g;
     g.Nx = ctx->Nx; g.Ny = ctx->Ny; g.Nz = ctx->Nz;
-    if (!fxz_plan(g.Nx, g.Ny, g.Nz, ncol, 152, g.TX, g.TY, g.nslab)) return false;
+    if (!fxz_plan(kFxZModel, g.Nx, g.Ny, g.Nz, ncol, 152, g.TX, g.TY, g.nslab)) return false;
     g.zlen = (g.Nz + g.nslab - 1) / g.nslab;
     g.hx = 2 * kMaxFDn * g.TY;
     g.hy = 2 * kMaxFDn * g.TX;
@@ -891,6 +864,42 @@ static bool fxz_launch(const sgpu_ctx *ctx, const double (&w)[3][kMaxFDn], doubl
     L->tilesy = (g.Ny + g.TY - 1) / g.TY;
     L->smem = 2 * sizeof(int4) * (size_t)kFxZPitch * (g.TY + 2 * kMaxFDn);
     L->cube = std::equal(w[0], w[0] + kMaxFDn, w[1]) && std::equal(w[0], w[0] + kMaxFDn, w[2]);
+    return true;
+}
+
+struct ZTileLaunch {
+    ZTileConst g{};
+    int ns, threads, tilesx, tilesy;
+    size_t smem;
+};
+// A step of the SM's resident blocks takes 1350 clocks and about one more per thread, half as many
+// again with a third halo value per thread (34^3 from 128 to 384 threads per block).
+constexpr FxZModel kZTileModel = {40, kZTileThreads, kZTileResident, 0.95, 0.0, 1.5, 0.0, 1350.0};
+// a cx, a cy, a cz are the launch's weights. False where the tiles do not fit the grid: there, and
+// with the option off, the one-point kernel, which also takes a scaled potential (per degree of a
+// batched filter 14^3 x 6 columns 11 us against 20 and more, 31 x 45 x 27 x 32 25 against 91,
+// 34^3 x 1280 0.59 ms against 1.41).
+static bool ztile_launch(const sgpu_ctx *ctx, double a, long ncol, ZTileLaunch *L)
+{
+    if (!ctx->zpair_on || ctx->Nd >= (1L << 27)) return false;
+    ZTileConst &g = L->g;
+    for (int r = 0; r <= kMaxFDn; r++) {
+        g.wx[r] = (float)(ctx->cx[r] * a);
+        g.wy[r] = (float)(ctx->cy[r] * a);
+        g.wz[r] = (float)(ctx->cz[r] * a);
+    }
+    g.Nx = ctx->Nx; g.Ny = ctx->Ny; g.Nz = ctx->Nz;
+    if (!fxz_plan(kZTileModel, g.Nx, g.Ny, g.Nz, ncol, 152, g.TX, g.TY, g.nslab)) return false;
+    g.zlen = (g.Nz + g.nslab - 1) / g.nslab;
+    g.hx = 2 * kMaxFDn * g.TY;
+    g.hy = 2 * kMaxFDn * g.TX;
+    // rows 16 entries longer than the tile: a warp's points lie in consecutive banks across rows
+    g.P = g.TX + 16;
+    L->threads = fxz_threads(g.TX, g.TY);
+    L->ns = (g.hx + g.hy + L->threads - 1) / L->threads;
+    L->tilesx = (g.Nx + g.TX - 1) / g.TX;
+    L->tilesy = (g.Ny + g.TY - 1) / g.TY;
+    L->smem = 2 * sizeof(float2) * (size_t)g.P * (g.TY + 2 * kMaxFDn);
     return true;
 }
 
@@ -976,54 +985,29 @@ static int stencil_z(sgpu_ctx *ctx, const double *k, int ncol, double a, double 
             return SGPU_OK;
         }
     }
-    if constexpr (sizeof(CT) == 8) {  // complex64: the pair kernel where it applies
-        int PX2, PY;
-        zpair_tile(ctx->Nx, ctx->Ny, R, &PX2, &PY);
-        bool ok = ctx->zpair_on && zpair_ok(ctx->Nx, ctx->Ny, ctx->Nz, R, PX2, PY) &&
-                  ldx % 2 == 0 && ldo % 2 == 0 && (!p.z || ldz % 2 == 0) &&
-                  (uintptr_t)x % 16 == 0 && (uintptr_t)out % 16 == 0 &&
-                  (!p.z || (uintptr_t)z % 16 == 0) && (!p.v32 || ctx->Nd % 2 == 0);
-        if (ok) {
-            ZPairParams zp;
-            ZPairConst zg;
-            zp.x = x; zp.out = out; zp.z = p.z; zp.v32 = p.v32;
-            zp.ldx = ldx; zp.ldo = ldo; zp.ldz = ldz;
-            zg.Nx = ctx->Nx; zg.Ny = ctx->Ny; zg.Nz = ctx->Nz;
-            for (int r = 0; r <= R; r++) {
-                zg.wx[r] = (float)p.wx[r]; zg.wy[r] = (float)p.wy[r]; zg.wz[r] = (float)p.wz[r];
-            }
-            // the potential scale bv multiplies the FP32 potential as in the generic kernel
-            zp.c0 = (float)p.c0; zp.s1 = (float)p.s1; zp.s2 = (float)p.s2;
+    if constexpr (sizeof(CT) == 8) {
+        ZTileLaunch L;
+        if ((!p.v32 || bv == 1.0) && ztile_launch(ctx, a, ncol, &L)) {
+            ZTileOne b{};
+            b.c.x = x; b.c.out = out; b.c.z = p.z; b.c.v = p.v32;
+            b.c.c0 = (float)c0; b.c.s1 = (float)s1; b.c.s2 = (float)s2;
+            b.ldx = ldx; b.ldo = ldo; b.ldz = ldz;
             const double kL[3] = {p.k.kLx, p.k.kLy, p.k.kLz};
-            for (int a = 0; a < 3; a++)
-                for (int d = -1; d <= 1; d++)
-                    zp.bf[3 * a + d + 1] = make_float2((float)std::cos(d * kL[a]),
-                                                       (float)std::sin(d * kL[a]));
-            if (p.v32 && bv != 1.0) ok = false;  // the pair kernel takes bv = 1
-            if (ok) {
-                const size_t psm = zpair_smem(PX2, PY, R);
-                SGPU_CUDA_TRY(cudaFuncSetAttribute(k_stencil_z_c64<R>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)psm));
-                const int ptx = (ctx->Nx + 2 * PX2 - 1) / (2 * PX2), pty = (ctx->Ny + PY - 1) / PY;
-                int nslab = 1;
-                while ((long)ptx * pty * ncol * nslab < 152L * 8 && ctx->Nz / (nslab * 2) >= 8)
-                    nslab *= 2;
-                zg.zlen = (ctx->Nz + nslab - 1) / nslab;
-                zg.nslab = nslab;
-                const int maxz = 65535 / nslab;
-                for (int c0i = 0; c0i < ncol; c0i += maxz) {
-                    const int nc = std::min(maxz, ncol - c0i);
-                    ZPairParams q = zp;
-                    q.x = x + (long)c0i * ldx;
-                    q.out = out + (long)c0i * ldo;
-                    if (q.z) q.z = zp.z + (long)c0i * ldz;
-                    ProfScope ps(ctx, SGPU_KERNEL_STENCIL, st);
-                    k_stencil_z_c64<R><<<dim3(ptx, pty, nc * nslab), dim3(PX2, PY), psm, st>>>(zg, q);
-                }
-                SGPU_CUDA_TRY(cudaGetLastError());
-                return SGPU_OK;
+            for (int q = 0; q < 9; q++)
+                b.bf[q] = make_double2(std::cos((q % 3 - 1) * kL[q / 3]), std::sin((q % 3 - 1) * kL[q / 3]));
+            const int maxz = 65535 / L.g.nslab;
+            for (int c0i = 0; c0i < ncol; c0i += maxz) {
+                const int nc = std::min(maxz, ncol - c0i);
+                ZTileOne q = b;
+                q.c.x = x + (long)c0i * ldx;
+                q.c.out = out + (long)c0i * ldo;
+                if (q.c.z) q.c.z = p.z + (long)c0i * ldz;
+                ProfScope ps(ctx, SGPU_KERNEL_STENCIL, st);
+                auto kern = L.ns <= 2 ? k_stencil_zt<2> : L.ns == 3 ? k_stencil_zt<3> : k_stencil_zt<4>;
+                kern<<<dim3(L.tilesx, L.tilesy, nc * L.g.nslab), L.threads, L.smem, st>>>(L.g, q);
             }
+            SGPU_CUDA_TRY(cudaGetLastError());
+            return SGPU_OK;
         }
     }
     int BX, BY;
@@ -1237,6 +1221,8 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
     constexpr bool Z128 = sizeof(CT) == 16;
     constexpr int FG = nlfx::kLanes / 2;
     FxZLaunch fxl;
+    ZTileLaunch ztl;
+    const bool zt = !Z128 && ztile_launch(ctx, -0.5, totcols, &ztl);
     bool fx_st = false, fx_nl = false;
     const NlFx *fxt = nullptr;
     CT *alpha2 = nullptr, *part = nullptr;
@@ -1371,36 +1357,12 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
     size_t zsm = zstencil_smem<CT>(BX, BY, R);  // attribute set before any capture
     SGPU_CUDA_TRY(cudaFuncSetAttribute(k_stencil_zb<CT, R>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsm));
-    // complex64: the pair kernel when its alignment and one-period conditions hold
-    bool pairs = false;
-    int PX2 = 0, PY = 0;
-    if constexpr (sizeof(CT) == 8) {
-        zpair_tile(ctx->Nx, ctx->Ny, R, &PX2, &PY);
-        pairs = ctx->zpair_on && zpair_ok(ctx->Nx, ctx->Ny, ctx->Nz, R, PX2, PY) &&
-                (uintptr_t)W % 16 == 0 && Nd % 2 == 0;
-        for (int b = 0; b < nblk && pairs; b++)
-            pairs = blk[b].ldi % 2 == 0 && blk[b].ldo % 2 == 0 &&
-                    (uintptr_t)blk[b].X % 16 == 0 && (uintptr_t)blk[b].Y % 16 == 0;
-        if (pairs) {
-            BX = 2 * PX2;
-            BY = PY;
-            zsm = zpair_smem(PX2, PY, R);
-            SGPU_CUDA_TRY(cudaFuncSetAttribute(k_stencil_zb_c64<R>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)zsm));
-        }
-    }
     const int tilesx = (ctx->Nx + BX - 1) / BX, tilesy = (ctx->Ny + BY - 1) / BY;
     int nslab = 1;
     while ((long)tilesx * tilesy * totcols * nslab < 152L * 8 && ctx->Nz / (nslab * 2) >= 8)
         nslab *= 2;
     cs.nslab = nslab;
     cs.zlen = (ctx->Nz + nslab - 1) / nslab;
-    ZPairConst pg;  // launch-wide data of the complex64 pair kernel
-    for (int r = 0; r <= R; r++) {
-        pg.wx[r] = (float)cs.wx[r]; pg.wy[r] = (float)cs.wy[r]; pg.wz[r] = (float)cs.wz[r];
-    }
-    pg.Nx = cs.Nx; pg.Ny = cs.Ny; pg.Nz = cs.Nz; pg.nslab = cs.nslab; pg.zlen = cs.zlen;
     const long maxw = 65535 / nslab;
     const size_t abytes = has_nl ? sizeof(CT) * (size_t)nl.ntot * totcols : 0;
     int maxcol = 0;
@@ -1499,19 +1461,21 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
                                                           j, in, out, zsel);
                 ctx->launches++;
             }
-            for (long w0 = 0; !fx_st && w0 < totcols; w0 += maxw) {
+            if constexpr (sizeof(CT) == 8) {
+                for (long w0 = 0; zt && w0 < totcols; w0 += 65535 / ztl.g.nslab) {
+                    const long nw = std::min<long>(65535 / ztl.g.nslab, totcols - w0);
+                    ProfScope ps(ctx, SGPU_KERNEL_STENCIL, st);
+                    auto kern = ztl.ns <= 2 ? k_stencil_ztb<2>
+                                            : ztl.ns == 3 ? k_stencil_ztb<3> : k_stencil_ztb<4>;
+                    kern<<<dim3(ztl.tilesx, ztl.tilesy, (unsigned)(nw * ztl.g.nslab)), ztl.threads,
+                           ztl.smem, st>>>(reinterpret_cast<const BBlock<float2> *>(dB), dC, dW + w0,
+                                           ztl.g, ctx->veff32, Nd, m, j, in, out, zsel);
+                    ctx->launches++;
+                }
+            }
+            for (long w0 = 0; !fx_st && !zt && w0 < totcols; w0 += maxw) {
                 const long nw = std::min(maxw, totcols - w0);
                 ProfScope ps(ctx, SGPU_KERNEL_STENCIL, st);
-                if constexpr (sizeof(CT) == 8) {
-                    if (pairs) {
-                        k_stencil_zb_c64<R><<<dim3(tilesx, tilesy, (unsigned)(nw * nslab)),
-                                              dim3(PX2, PY), zsm, st>>>(
-                            reinterpret_cast<const BBlock<float2> *>(dB), dC, dW + w0, pg,
-                            ctx->veff32, Nd, m, j, in, out, zsel);
-                        ctx->launches++;
-                        continue;
-                    }
-                }
                 k_stencil_zb<CT, R><<<dim3(tilesx, tilesy, (unsigned)(nw * nslab)),
                                       dim3(BX, BY), zsm, st>>>(dB, dC, dW + w0, cs, j, in, out,
                                                                zsel);
@@ -1566,7 +1530,7 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
 
     if (ctx->prof_on) return issue();  // per-launch events need plain launches
     std::vector<long> key = {(long)sizeof(CT), nblk, m, (long)(uintptr_t)tb, (long)(uintptr_t)W,
-                             (long)(uintptr_t)alpha, (long)hg.size(), nslab, (long)pairs,
+                             (long)(uintptr_t)alpha, (long)hg.size(), nslab, (long)zt,
                              (long)(uintptr_t)ctx->veff64, (long)(uintptr_t)ctx->veff32,
                              (long)fx_st, (long)fx_nl, (long)(uintptr_t)alpha2, (long)(uintptr_t)part,
                              (long)(uintptr_t)(fx_nl ? fxt->chi : nullptr), fgx,
@@ -1579,6 +1543,15 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
         for (int a = 0; a < 3; a++)
             for (int r = 0; r < kMaxFDn; r++)
                 key.push_back(((long)fxl.g.wh[a][r] << 32) ^ (unsigned)fxl.g.wl[a][r]);
+    }
+    if (zt) {
+        key.push_back(ztl.g.nslab * 4096L + ztl.g.TX * 64 + ztl.g.TY);
+        for (const float *w : {ztl.g.wx, ztl.g.wy, ztl.g.wz})
+            for (int r = 0; r <= kMaxFDn; r++) {
+                int bits;
+                std::memcpy(&bits, w + r, sizeof(bits));
+                key.push_back(bits);
+            }
     }
     for (int b = 0; b < nblk; b++) {
         key.push_back(blk[b].ncol);

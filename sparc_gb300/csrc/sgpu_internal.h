@@ -217,8 +217,8 @@ struct sgpu_ctx {
                         // the mixed SCF's FP64 phase (six slices) and plain FP64 calls (eight
                         // slices, full FP64 accuracy), 2 six slices for plain FP64 calls too;
                         // 0 cuBLAS
-    int zpair_on = 1;   // complex64 stencil: the two-points-per-thread kernel (1) or the
-                        // one-point kernel (0) (sgpu_set_zstencil_pairs)
+    int zpair_on = 1;   // complex64 stencil: the tile kernel with tabulated factors (1) or the
+                        // general kernel (0) (sgpu_set_zstencil_pairs)
     double tune_fused_ms = 0.0;  // last timing of the fused apply + projection (chosen form)
     double tune_fused_cpl_ms[2] = {0, 0};  // last timings of the 2- and 4-column forms
     double tune_fused_tc_ms = 0.0;         // last timing of the tensor-core form

@@ -317,6 +317,15 @@ __device__ __forceinline__ void stencil_fxz(const FxZConst &p, const FxZCol &c, 
 
 // ---- host side
 
+// what fxz_plan weighs: largest tile edge, block and resident threads of an SM; of a step, the
+// clocks per thread and per halo value, the factor on them where a thread has more than two
+// halo values, the least that they come to, and what is added
+struct FxZModel {
+    int tile, threads, resident;
+    double point, halo, more, least, add;
+};
+constexpr FxZModel kFxZModel = {kFxZTile, kFxZThreads, 512, 5.6, 0.95, 1.0, 2700.0, 0.0};
+
 inline int fxz_threads(int TX, int TY)
 {
     const int halo = 2 * kMaxFDn * (TX + TY);
@@ -325,27 +334,29 @@ inline int fxz_threads(int TX, int TY)
 
 // Tile and slabs: the model of fx_plan with a complex point in the place of a point pair. False
 // when a tile's halo would reach a whole period away (grids under a dozen points a side).
-inline bool fxz_plan(int Nx, int Ny, int Nz, long ncol, int nsm, int &TX, int &TY, int &nslab)
+inline bool fxz_plan(const FxZModel &md, int Nx, int Ny, int Nz, long ncol, int nsm, int &TX, int &TY,
+                     int &nslab)
 {
     double best = 1e300;
     TX = TY = 0;
-    for (int ex = 4; ex <= kFxZTile; ex++) {
+    for (int ex = 4; ex <= md.tile; ex++) {
         const int nx = (Nx + ex - 1) / ex, tx = (Nx + nx - 1) / nx;
         if ((tx != ex && ex != 4) || nx * tx + kMaxFDn > 2 * Nx) continue;
-        for (int ey = 4; ey <= kFxZTile; ey++) {
+        for (int ey = 4; ey <= md.tile; ey++) {
             const int ny = (Ny + ey - 1) / ey, ty = (Ny + ny - 1) / ny;
             if ((ty != ey && ey != 4) || ny * ty + kMaxFDn > 2 * Ny) continue;
             const double halo = 2.0 * kMaxFDn * (tx + ty);
             const int thr = fxz_threads(tx, ty);
-            if (thr > kFxZThreads) continue;
-            const int fit = std::min(512 / thr, 8);
+            if (thr > md.threads) continue;
+            const int fit = std::min(md.resident / thr, 8);
             static const double f[4] = {1.35, 1.35, 1.1, 1.04};
             for (int ns = 1; ns <= std::max(1, Nz / 3); ns *= 2) {
                 const double nblk = (double)nx * ny * ncol * ns;
                 const double waves = std::ceil(nblk / ((double)nsm * fit));
                 const double res = std::min<double>(fit, std::ceil(nblk / nsm));
-                const double work = res * 2.0 * (thr + 0.17 * halo) * (res < 4 ? f[(int)res] : 1.0);
-                const double t = waves * (5.0 + (Nz + ns - 1) / ns) * std::max(2700.0, 2.8 * work);
+                const double work = res * (md.point * thr + md.halo * halo) *
+                                    (res < 4 ? f[(int)res] : 1.0) * (halo > 2 * thr ? md.more : 1.0);
+                const double t = waves * (5.0 + (Nz + ns - 1) / ns) * (std::max(md.least, work) + md.add);
                 // as good: the wider tile (rows are read along x; 34^3: 17 x 9 tiles 1.87 ms per
                 // degree, 9 x 17 2.05)
                 if (t < 0.999 * best || (t < 1.001 * best && tx > TX)) {

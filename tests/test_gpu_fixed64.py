@@ -268,3 +268,47 @@ def test_bloch_columns(gpu_available, N):
             for b in blocks:  # other bounds: the same shapes and buffers
                 b["b"] *= 1.1
     ctx.close()
+
+
+@pytest.mark.parametrize("ncol", [1, 40])
+@pytest.mark.parametrize("N", [(17, 14, 20), (6, 12, 9), (34, 13, 12), (25, 24, 31), (41, 7, 6)])
+def test_complex64_tiles(gpu_available, N, ncol):
+    """Two degrees of the complex64 filter against complex128. Bound: 40 units of 2^-24 (37 terms in
+    chains of six, the factor and the roundings of values and weights take fewer) of the sum of
+    |coefficient| times the largest value, for each application."""
+    h, a, b, a0 = 0.4, 0.5, 40.0, -0.8
+    rng = np.random.default_rng(sum(N) + ncol)
+    c = fd_d2_coeffs(6, h)
+    ctx = sg.Context(*N, 6, c, c, c, h ** 3)
+    Nd = N[0] * N[1] * N[2]
+    v = rng.normal(size=Nd)
+    ctx.set_veff(v)
+    L = np.array(N) * h
+    ctx.set_kpoint_geometry(L, np.zeros((0, 3)))
+    x = rng.uniform(-1, 1, (ncol, Nd)) + 1j * rng.uniform(-1, 1, (ncol, Nd))
+    e, cen = 0.5 * (b - a), 0.5 * (b + a)
+    s1 = e / (a0 - cen)
+    s2 = 1.0 / (2.0 / s1 - s1)
+    S = 1.5 * (abs(c[0]) + 2 * np.abs(c[1:]).sum()) + np.abs(v).max() + cen
+    u = 40 * 2.0 ** -24 * np.sqrt(2.0)
+    for k in ((0.0, 0.0, 0.0), (0.0, np.pi / L[1], 0.0), (0.3, -0.2, 0.1)):
+        y, ref = np.zeros_like(x), np.zeros_like(x)
+        ctx.ChebyshevFiltering_kpt(list(k), x.copy(), y, 2, a, b, a0, precision=sg.SGPU_PREC_FP32)
+        ctx.ChebyshevFiltering_kpt(list(k), x.copy(), ref, 2, a, b, a0)
+        m0 = np.sqrt(2.0)
+        m1 = abs(s1 / e) * S * m0                      # bound of the first iterate
+        e1 = u * m1
+        e2 = abs(2 * s2 / e) * S * (e1 + u * m1) + 3 * 2.0 ** -24 * abs(s1 * s2) * m0
+        assert np.abs(y - ref).max() <= e2, k
+    # an infinity spreads as it does in the general kernel
+    x[0, Nd // 2] = np.inf
+    x[-1, 3] = np.nan
+    out = []
+    for on in (True, False):
+        ctx.set_zstencil_pairs(on)
+        y = np.zeros_like(x)
+        ctx.ChebyshevFiltering_kpt([0.3, -0.2, 0.1], x.copy(), y, 2, a, b, a0,
+                                   precision=sg.SGPU_PREC_FP32)
+        out.append(np.isfinite(y))
+    assert np.array_equal(out[0], out[1])
+    ctx.close()

@@ -438,7 +438,7 @@ struct BBlock {
 
 struct BCoef {
     double c0, s1, s2;      // centre weight (with the shift), output and recurrence scales
-    int c0h, c0l;           // digits of c0 (fixed-point form)
+    int c0h, c0l, c0r;           // digits of c0 (fixed-point form)
 };
 
 struct BConst {
@@ -493,7 +493,7 @@ __global__ void __launch_bounds__(kFxZThreads, 1)
     c.z = z_sel >= 0 ? B.buf[z_sel] + (long)bc.y * B.ld[z_sel] : nullptr;
     c.v = veff ? veff + (long)B.spin * Nd : nullptr;
     c.vd = veff_fx ? veff_fx + (long)B.spin * Nd : nullptr;
-    c.c0h = cf.c0h; c.c0l = cf.c0l;
+    c.c0h = cf.c0h; c.c0l = cf.c0l; c.c0r = cf.c0r;
     c.c0 = cf.c0; c.s1 = cf.s1; c.s2 = cf.s2;
     c.bf = B.bf;
     stencil_fxz<NS, CUBE>(g, c, slab, fxz_smem);
@@ -961,7 +961,7 @@ static int stencil_z(sgpu_ctx *ctx, const double *k, int ncol, double a, double 
             b.c.x = x; b.c.out = out; b.c.z = p.z;
             b.c.v = p.v;
             b.c.vd = p.v && pot->key ? pot->vd : nullptr;
-            fx_coef(c0, L.s, b.c.c0h, b.c.c0l);
+            fx_coef(c0, L.s, b.c.c0h, b.c.c0l, b.c.c0r);
             b.c.c0 = c0; b.c.s1 = s1; b.c.s2 = s2;
             b.ldx = ldx; b.ldo = ldo; b.ldz = ldz;
             const double kL[3] = {p.k.kLx, p.k.kLy, p.k.kLz};
@@ -1287,7 +1287,7 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
             BCoef &q = hc[(size_t)b * m + j];
             q.c0 = c0;
             q.c0h = q.c0l = 0;
-            if (fx_st) fx_coef(c0, fxl.s, q.c0h, q.c0l);
+            if (fx_st) fx_coef(c0, fxl.s, q.c0h, q.c0l, q.c0r);
             if (j == 0) {
                 q.s1 = sigma1 / e;
                 q.s2 = 0.0;
@@ -1541,8 +1541,10 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
         key.push_back(fxl.g.KW);
         key.push_back(fxl.g.nslab * 4096L + fxl.g.TX * 64 + fxl.g.TY);
         for (int a = 0; a < 3; a++)
-            for (int r = 0; r < kMaxFDn; r++)
+            for (int r = 0; r < kMaxFDn; r++) {
                 key.push_back(((long)fxl.g.wh[a][r] << 32) ^ (unsigned)fxl.g.wl[a][r]);
+                key.push_back(fxl.g.wr[a][r]);
+            }
     }
     if (zt) {
         key.push_back(ztl.g.nslab * 4096L + ztl.g.TX * 64 + ztl.g.TY);

@@ -16,9 +16,10 @@
 //
 // What bounds it: instruction issue (61 % of the slots busy, 60 % of the integer multiply pipe, 59 %
 // of the shared-memory wavefronts, HBM 29 %). Per point about 36 integer adds, 24 wide
-// multiply-adds (60 with three spacings), 20 instructions per converted value (2.5 of them on a
-// 16 x 16 tile) and 40 for the way back, against 42 FP64 instructions at two lanes per clock in
-// k_stencil_orth. 96^3, 512 columns: 37.3 -> 4.75 ms per launch.
+// multiply-adds and 7 high products (60 and 19 with three spacings), 21 instructions per converted
+// value (2.5 of them on a 16 x 16 tile) and 40 for the way back, against 42 FP64 instructions at
+// two lanes per clock in k_stencil_orth. 96^3, 512 columns: 37.3 -> 5.29 ms per launch (4.75 with
+// coefficients of two digits, whose rounding cost a filter its accuracy).
 #pragma once
 
 #include <algorithm>
@@ -43,8 +44,8 @@ struct StencilFxParams {
     int s;                   // unit of the coefficient digits: 2^-s
     int KW;                  // T 2^(KW + E) is the stencil sum (E the block exponent)
     int dv;                  // the potential's products count 2^-dv of the stencil's
-    int c0h, c0l;            // digits of c0 and of a w_r
-    int wh[3][kMaxFDn], wl[3][kMaxFDn];
+    int c0h, c0l, c0r;       // digits of c0 and of a w_r
+    int wh[3][kMaxFDn], wl[3][kMaxFDn], wr[3][kMaxFDn];
     double s2;
     // FP64 path of a block whose values the fixed-point range does not cover
     double c0, bv, s1;
@@ -221,38 +222,40 @@ __global__ void __launch_bounds__(kFxThreads, 1) k_stencil_fx(const StencilFxPar
         auto ph = [&](int m) { return (m & 1) ? L[m >> 1].z : L[m >> 1].x; };
         auto pl = [&](int m) { return (m & 1) ? L[m >> 1].w : L[m >> 1].y; };
         long long hh0 = 0, mid0 = 0, hh1 = 0, mid1 = 0;
-        fx::mac(hh0, mid0, cen.x, cen.y, p.c0h, p.c0l);
-        fx::mac(hh1, mid1, cen.z, cen.w, p.c0h, p.c0l);
+        int lo0 = 0, lo1 = 0;
+        fx::mac(hh0, mid0, lo0, cen.x, cen.y, p.c0h, p.c0l, p.c0r);
+        fx::mac(hh1, mid1, lo1, cen.z, cen.w, p.c0h, p.c0l, p.c0r);
 #pragma unroll
         for (int r = 1; r <= R; r++) {
             const int4 a = S.q[U + R - r], b = S.q[U + R + r];
             const int4 c = *reinterpret_cast<const int4 *>(buf + sc - r * P);
             const int4 d = *reinterpret_cast<const int4 *>(buf + sc + r * P);
-            const int wh = p.wh[0][r - 1], wl = p.wl[0][r - 1];
+            const int wh = p.wh[0][r - 1], wl = p.wl[0][r - 1], wr = p.wr[0][r - 1];
             if constexpr (CUBE) {
-                fx::mac(hh0, mid0, a.x + b.x + c.x + d.x + ph(R - r) + ph(R + r),
-                        a.y + b.y + c.y + d.y + pl(R - r) + pl(R + r), wh, wl);
-                fx::mac(hh1, mid1, a.z + b.z + c.z + d.z + ph(R + 1 - r) + ph(R + 1 + r),
-                        a.w + b.w + c.w + d.w + pl(R + 1 - r) + pl(R + 1 + r), wh, wl);
+                fx::mac(hh0, mid0, lo0, a.x + b.x + c.x + d.x + ph(R - r) + ph(R + r),
+                        a.y + b.y + c.y + d.y + pl(R - r) + pl(R + r), wh, wl, wr);
+                fx::mac(hh1, mid1, lo1, a.z + b.z + c.z + d.z + ph(R + 1 - r) + ph(R + 1 + r),
+                        a.w + b.w + c.w + d.w + pl(R + 1 - r) + pl(R + 1 + r), wh, wl, wr);
             } else {
-                const int uh = p.wh[1][r - 1], ul = p.wl[1][r - 1];
-                const int th = p.wh[2][r - 1], tl = p.wl[2][r - 1];
-                fx::mac(hh0, mid0, a.x + b.x, a.y + b.y, th, tl);
-                fx::mac(hh1, mid1, a.z + b.z, a.w + b.w, th, tl);
-                fx::mac(hh0, mid0, c.x + d.x, c.y + d.y, uh, ul);
-                fx::mac(hh1, mid1, c.z + d.z, c.w + d.w, uh, ul);
-                fx::mac(hh0, mid0, ph(R - r) + ph(R + r), pl(R - r) + pl(R + r), wh, wl);
-                fx::mac(hh1, mid1, ph(R + 1 - r) + ph(R + 1 + r), pl(R + 1 - r) + pl(R + 1 + r),
-                        wh, wl);
+                const int uh = p.wh[1][r - 1], ul = p.wl[1][r - 1], ur = p.wr[1][r - 1];
+                const int th = p.wh[2][r - 1], tl = p.wl[2][r - 1], tr = p.wr[2][r - 1];
+                fx::mac(hh0, mid0, lo0, a.x + b.x, a.y + b.y, th, tl, tr);
+                fx::mac(hh1, mid1, lo1, a.z + b.z, a.w + b.w, th, tl, tr);
+                fx::mac(hh0, mid0, lo0, c.x + d.x, c.y + d.y, uh, ul, ur);
+                fx::mac(hh1, mid1, lo1, c.z + d.z, c.w + d.w, uh, ul, ur);
+                fx::mac(hh0, mid0, lo0, ph(R - r) + ph(R + r), pl(R - r) + pl(R + r), wh, wl, wr);
+                fx::mac(hh1, mid1, lo1, ph(R + 1 - r) + ph(R + 1 + r), pl(R + 1 - r) + pl(R + 1 + r),
+                        wh, wl, wr);
             }
         }
-        long long T0 = fx::total(hh0, mid0), T1 = fx::total(hh1, mid1);
+        long long T0 = fx::total(hh0, mid0, lo0), T1 = fx::total(hh1, mid1, lo1);
         if (p.vd) {
             long long a0 = 0, b0 = 0, a1 = 0, b1 = 0;
             fx::mac(a0, b0, cen.x, cen.y, v0.x, v0.y);
             fx::mac(a1, b1, cen.z, cen.w, v1.x, v1.y);
-            T0 += fx::total(a0, b0) >> p.dv;
-            T1 += fx::total(a1, b1) >> p.dv;
+            const long long half = (1ll << p.dv) >> 1;
+            T0 += (fx::total(a0, b0) + half) >> p.dv;
+            T1 += (fx::total(a1, b1) + half) >> p.dv;
         }
         const int K = p.KW + S.E;
         double y0v = fx::to_double(T0, K), y1v = fx::to_double(T1, K);
@@ -342,10 +345,12 @@ inline int fx_threads(int TX, int TY)
     return std::max((TX / 2 * TY + 31) / 32 * 32, (halo / 4 + 31) / 32 * 32);
 }
 
-// digits of w 2^s, rounded to nearest
-inline void fx_coef(double w, int s, int &h, int &l)
+// digits of w 2^s = h 2^29 + l + r 2^-30, rounded to nearest
+inline void fx_coef(double w, int s, int &h, int &l, int &r)
 {
-    const long long W = std::llrint(std::ldexp(w, s));
+    const double u = std::ldexp(w, s);
+    const long long W = std::llrint(u);
+    r = (int)std::llrint(std::ldexp(u - (double)W, 30));
     const long long H = (W + (1ll << (fx::kDigit - 1))) >> fx::kDigit;
     h = (int)H;
     l = (int)(W - H * (1ll << fx::kDigit));
@@ -407,11 +412,12 @@ inline bool fx_setup(StencilFxParams &p, int FDn, unsigned vkey)
     }
     const int s = 2 * fx::kDigit + 1 - eS;          // S 2^s < 2^59: digits below 2^30
     p.s = s;
-    fx_coef(p.c0, s, p.c0h, p.c0l);
+    fx_coef(p.c0, s, p.c0h, p.c0l, p.c0r);
     for (int d = 0; d < 3; d++)
-        for (int r = 0; r < FDn; r++) fx_coef(p.w[d][r], s, p.wh[d][r], p.wl[d][r]);
+        for (int r = 0; r < FDn; r++)
+            fx_coef(p.w[d][r], s, p.wh[d][r], p.wl[d][r], p.wr[d][r]);
     // a potential value is V 2^(ev + 1 - kBits): its products are shifted to the unit 2^-s
-    if (vkey != 0u) p.dv = std::min(fx::kBits - 1 - ev - s, 63);
+    if (vkey != 0u) p.dv = std::min(fx::kBits - 1 - ev - s, 62);
     // T counts 2^(kDigit + kDrop) quanta x units; the quantum is 2^(E - 1023 + 1 - kBits)
     p.KW = fx::kDigit + fx::kDrop - s - 1023 + 1 - fx::kBits;
     return true;

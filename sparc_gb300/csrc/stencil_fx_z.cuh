@@ -6,7 +6,7 @@
 // What bounds it: latency at the 15 warps that 128 registers leave (46 % of the issue slots busy, the
 // FP64 pipe, which has the output scale, the recurrence term and the factors, 37 %; with the
 // factors as selects on every value it was the bound at 75 %, and 2.9 ms). 34^3, 20 blocks of 64
-// columns: 12.6 ms per degree in k_stencil_zb<double2>, 1.87 here.
+// columns: 12.6 ms per degree in k_stencil_zb<double2>, 2.03 here.
 #pragma once
 
 #include "stencil_fx.cuh"
@@ -18,7 +18,7 @@ struct FxZConst {              // one launch: all its columns
     int Nx, Ny, Nz, nslab, zlen;
     int TX, TY, hx, hy;
     int KW, dv;
-    int wh[3][kMaxFDn], wl[3][kMaxFDn];
+    int wh[3][kMaxFDn], wl[3][kMaxFDn], wr[3][kMaxFDn];
     double w[3][kMaxFDn];      // FP64 path
 };
 
@@ -27,7 +27,7 @@ struct FxZCol {                // one column
     double2 *out;
     const int2 *vd;            // digits of the potential, or null
     const double *v;
-    int c0h, c0l;
+    int c0h, c0l, c0r;
     double c0, s1, s2;
     const double2 *bf;         // e^{i d k_a L_a}, index 3 a + d + 1
 };
@@ -222,37 +222,39 @@ __device__ __forceinline__ void stencil_fxz(const FxZConst &p, const FxZCol &c, 
         }
         const int4 cen = q[U + R];
         long long hr = 0, mr = 0, hi = 0, mi = 0;
-        fx::mac(hr, mr, cen.x, cen.y, c.c0h, c.c0l);
-        fx::mac(hi, mi, cen.z, cen.w, c.c0h, c.c0l);
+        int lr = 0, li = 0;
+        fx::mac(hr, mr, lr, cen.x, cen.y, c.c0h, c.c0l, c.c0r);
+        fx::mac(hi, mi, li, cen.z, cen.w, c.c0h, c.c0l, c.c0r);
 #pragma unroll
         for (int r = 1; r <= R; r++) {
             const int4 a = q[U + R - r], b = q[U + R + r];
             const int4 d = buf[sc - r * P], e = buf[sc + r * P];
             const int4 f = buf[sc - r], g = buf[sc + r];
-            const int wh = p.wh[0][r - 1], wl = p.wl[0][r - 1];
+            const int wh = p.wh[0][r - 1], wl = p.wl[0][r - 1], wr = p.wr[0][r - 1];
             if constexpr (CUBE) {
-                fx::mac(hr, mr, a.x + b.x + d.x + e.x + f.x + g.x, a.y + b.y + d.y + e.y + f.y + g.y,
-                        wh, wl);
-                fx::mac(hi, mi, a.z + b.z + d.z + e.z + f.z + g.z, a.w + b.w + d.w + e.w + f.w + g.w,
-                        wh, wl);
+                fx::mac(hr, mr, lr, a.x + b.x + d.x + e.x + f.x + g.x, a.y + b.y + d.y + e.y + f.y + g.y,
+                        wh, wl, wr);
+                fx::mac(hi, mi, li, a.z + b.z + d.z + e.z + f.z + g.z, a.w + b.w + d.w + e.w + f.w + g.w,
+                        wh, wl, wr);
             } else {
-                const int uh = p.wh[1][r - 1], ul = p.wl[1][r - 1];
-                const int th = p.wh[2][r - 1], tl = p.wl[2][r - 1];
-                fx::mac(hr, mr, a.x + b.x, a.y + b.y, th, tl);
-                fx::mac(hi, mi, a.z + b.z, a.w + b.w, th, tl);
-                fx::mac(hr, mr, d.x + e.x, d.y + e.y, uh, ul);
-                fx::mac(hi, mi, d.z + e.z, d.w + e.w, uh, ul);
-                fx::mac(hr, mr, f.x + g.x, f.y + g.y, wh, wl);
-                fx::mac(hi, mi, f.z + g.z, f.w + g.w, wh, wl);
+                const int uh = p.wh[1][r - 1], ul = p.wl[1][r - 1], ur = p.wr[1][r - 1];
+                const int th = p.wh[2][r - 1], tl = p.wl[2][r - 1], tr = p.wr[2][r - 1];
+                fx::mac(hr, mr, lr, a.x + b.x, a.y + b.y, th, tl, tr);
+                fx::mac(hi, mi, li, a.z + b.z, a.w + b.w, th, tl, tr);
+                fx::mac(hr, mr, lr, d.x + e.x, d.y + e.y, uh, ul, ur);
+                fx::mac(hi, mi, li, d.z + e.z, d.w + e.w, uh, ul, ur);
+                fx::mac(hr, mr, lr, f.x + g.x, f.y + g.y, wh, wl, wr);
+                fx::mac(hi, mi, li, f.z + g.z, f.w + g.w, wh, wl, wr);
             }
         }
-        long long Tr = fx::total(hr, mr), Ti = fx::total(hi, mi);
+        long long Tr = fx::total(hr, mr, lr), Ti = fx::total(hi, mi, li);
         if (c.vd) {
             long long a0 = 0, b0 = 0, a1 = 0, b1 = 0;
             fx::mac(a0, b0, cen.x, cen.y, v.x, v.y);
             fx::mac(a1, b1, cen.z, cen.w, v.x, v.y);
-            Tr += fx::total(a0, b0) >> p.dv;
-            Ti += fx::total(a1, b1) >> p.dv;
+            const long long half = (1ll << p.dv) >> 1;
+            Tr += (fx::total(a0, b0) + half) >> p.dv;
+            Ti += (fx::total(a1, b1) + half) >> p.dv;
         }
         const int K = p.KW + E;
         double yr = fx::to_double(Tr, K), yi = fx::to_double(Ti, K);
@@ -357,8 +359,8 @@ inline bool fxz_plan(const FxZModel &md, int Nx, int Ny, int Nz, long ncol, int 
                 const double work = res * (md.point * thr + md.halo * halo) *
                                     (res < 4 ? f[(int)res] : 1.0) * (halo > 2 * thr ? md.more : 1.0);
                 const double t = waves * (5.0 + (Nz + ns - 1) / ns) * (std::max(md.least, work) + md.add);
-                // as good: the wider tile (rows are read along x; 34^3: 17 x 9 tiles 1.87 ms per
-                // degree, 9 x 17 2.05)
+                // as good: the wider tile (rows are read along x; 34^3: 17 x 9 tiles take
+                // 9 % less than 9 x 17)
                 if (t < 0.999 * best || (t < 1.001 * best && tx > TX)) {
                     best = t; TX = tx; TY = ty; nslab = ns;
                 }
@@ -377,6 +379,7 @@ inline void fxz_const(FxZConst &g, const StencilFxParams &d)
         for (int r = 0; r < kMaxFDn; r++) {
             g.wh[a][r] = d.wh[a][r];
             g.wl[a][r] = d.wl[a][r];
+            g.wr[a][r] = d.wr[a][r];
             g.w[a][r] = d.w[a][r];
         }
 }

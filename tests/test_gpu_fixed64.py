@@ -312,3 +312,42 @@ def test_complex64_tiles(gpu_available, N, ncol):
         out.append(np.isfinite(y))
     assert np.array_equal(out[0], out[1])
     ctx.close()
+
+
+def test_filter_against_extended_precision(gpu_available):
+    """What repeats in every application (rounded coefficients, values cut one way) adds up over the
+    degrees of a filter: one column of a degree-20 filter, in norm, within two roundings of 2^-53."""
+    N, h, m, a, b, a0 = (26, 22, 31), 0.4, 20, 0.5, 50.0, -1.0
+    rng = np.random.default_rng(11)
+    c = fd_d2_coeffs(6, h)
+    ctx = sg.Context(*N, 6, c, c, c, h ** 3)
+    Nd = N[0] * N[1] * N[2]
+    v = rng.normal(size=Nd)
+    ctx.set_veff(v)
+    x = rng.uniform(-1, 1, (6, Nd))
+    y = np.zeros_like(x)
+    ctx.ChebyshevFiltering(x.copy(), y, m, a, b, a0)
+    ctx.close()
+    ld = np.longdouble
+    e, cen = 0.5 * (b - a), 0.5 * (b + a)
+    c0 = (c[0] * -0.5 + c[0] * -0.5) + c[0] * -0.5 - cen  # the scalars as doubles
+    shape = N[::-1]
+
+    def apply(u):
+        r = (ld(c0) + v.astype(ld).reshape(shape)) * u
+        for ax in range(3):
+            for q in range(1, 7):
+                r = r + ld(c[q] * -0.5) * (np.roll(u, q, ax) + np.roll(u, -q, ax))
+        return r
+
+    sigma = e / (a0 - cen)
+    gamma = 2.0 / sigma
+    prev = x[0].astype(ld).reshape(shape)
+    cur = apply(prev) * ld(sigma / e)
+    for _ in range(1, m):
+        s2 = 1.0 / (gamma - sigma)
+        prev, cur = cur, apply(cur) * ld(2.0 * s2 / e) - ld(sigma * s2) * prev
+        sigma = s2
+    cur = cur.reshape(-1)
+    err = np.sqrt(((y[0] - cur) ** 2).sum() / (cur ** 2).sum())
+    assert err <= 2 * 2.0 ** -53

@@ -223,6 +223,7 @@ int sgpu_set_grid_coeffs(sgpu_ctx *ctx, const double *cx, const double *cy, cons
     SGPU_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     for (int p = 0; p <= ctx->FDn; p++) { ctx->cx[p] = cx[p]; ctx->cy[p] = cy[p]; ctx->cz[p] = cz[p]; }
     ctx->dV = dV;
+    ctx->set_count++;
     return SGPU_OK;
 }
 
@@ -303,6 +304,7 @@ int sgpu_set_nonlocal(sgpu_ctx *ctx, int n_atom, const int *IP_displ, const doub
         set_error("sgpu_set_nonlocal: bad sizes or null arrays");
         return SGPU_ERR_ARG;
     }
+    ctx->set_count++;
     if (n_atom == 0 || n_img == 0) {
         nonlocal_free(ctx->nl);
         ctx->has_nl = false;

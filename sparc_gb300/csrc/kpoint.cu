@@ -1529,12 +1529,14 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
     };
 
     if (ctx->prof_on) return issue();  // per-launch events need plain launches
-    std::vector<long> key = {(long)sizeof(CT), nblk, m, (long)(uintptr_t)tb, (long)(uintptr_t)W,
+    // what the captured launches hold: buffers and workspaces, shapes, and, through set_count, the
+    // nonlocal tables (their pointers, sizes and grid extents), the grid's weights and dV: freed
+    // tables commonly come back at the same address with other sizes
+    std::vector<long> key = {ctx->set_count, (long)sizeof(CT), nblk, m, (long)(uintptr_t)tb, (long)(uintptr_t)W,
                              (long)(uintptr_t)alpha, (long)hg.size(), nslab, (long)zt,
                              (long)(uintptr_t)ctx->veff64, (long)(uintptr_t)ctx->veff32,
                              (long)fx_st, (long)fx_nl, (long)(uintptr_t)alpha2, (long)(uintptr_t)part,
-                             (long)(uintptr_t)(fx_nl ? fxt->chi : nullptr), fgx,
-                             (long)(uintptr_t)ctx->veff_fx, (long)(ctx->veff_key != 0)};
+                             fx_nl ? fxt - nl.fx : -1L, fgx, (long)(uintptr_t)ctx->veff_fx, (long)(ctx->veff_key != 0)};
     if (fx_st) {  // the launch's numbers: they move with the coefficients and the potential's size
         key.push_back(fxl.s);
         key.push_back(fxl.g.dv);
@@ -1557,6 +1559,7 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
     }
     for (int b = 0; b < nblk; b++) {
         key.push_back(blk[b].ncol);
+        key.push_back(blk[b].ldi);
         key.push_back((long)(uintptr_t)blk[b].X);
         key.push_back((long)(uintptr_t)blk[b].Y);
     }

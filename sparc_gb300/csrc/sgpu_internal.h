@@ -185,6 +185,8 @@ struct sgpu_ctx {
     unsigned veff_key = 0;
     sgpu::Nonlocal nl;
     bool has_nl = false;
+    long set_count = 0;        // calls that changed the nonlocal set or the grid's numbers; captured
+                               // launches hold those by value and pointer and are dropped with them
     cublasHandle_t cublas = nullptr;
     cusolverDnHandle_t cusolver = nullptr;
     cusolverDnParams_t xparams = nullptr;   // 64-bit cuSOLVER API parameters (batched syev)

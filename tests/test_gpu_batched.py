@@ -115,3 +115,45 @@ def test_complex64_pair_stencil_matches_one_point_kernel(gpu_available):
     ctx.set_zstencil_pairs(True)
     for a, b in zip(outs[True], outs[False]):
         assert rel_err(a, b) < 2e-6
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+def test_batched_follows_a_new_nonlocal_set(gpu_available, precision):
+    """Projectors replaced between two batched filters on the same blocks (as many images, but other
+    points, values, Gamma and counts; then other finite-difference weights and volume element): the
+    second filter uses the new ones, as the per-block call does."""
+    import torch
+    from sparc_gb300.synthetic import fd_d2_coeffs, synthetic_nonlocal
+    N, h, ncol = (18, 16, 20), 0.42, 9
+    Nd, L = N[0] * N[1] * N[2], np.array(N) * h
+    rng = np.random.default_rng(21)
+    c = fd_d2_coeffs(6, h)
+    ctx = sg.Context(*N, 6, c, c, c, h ** 3)
+    ctx.set_veff(rng.normal(0.0, 0.3, Nd))
+    natom = 5
+    coords = rng.uniform(0, 1, (natom, 3)) * L
+    k = np.array([0.2, -0.1, 0.3])
+    x0 = torch.complex(torch.from_numpy(rng.uniform(-1, 1, (ncol, Nd))),
+                       torch.from_numpy(rng.uniform(-1, 1, (ncol, Nd))))
+    cdt = torch.complex128 if precision == 64 else torch.complex64
+    X = x0.to(cdt).cuda()
+    Y = torch.empty_like(X)
+    tol = 1e-12 if precision == 64 else 1e-5
+    kset = False
+    for rc, lmax, hh in ((1.9, 2, h), (1.1, 2, h), (2.3, 1, h), (1.9, 2, h), (1.9, 2, 0.4)):
+        nl = synthetic_nonlocal(rng, N, h, natom=natom, rc=rc, lmax=lmax)
+        ctx.set_nonlocal(nl["ip_displ"], nl["gamma"], nl["img_atom"], nl["img_ndc"],
+                         nl["grid_pos"], nl["chi"])
+        w = fd_d2_coeffs(6, hh)
+        ctx.set_grid_coeffs(w, w, w, hh ** 3)
+        if not kset:
+            ctx.set_kpoint_geometry(L, coords)
+            kset = True
+        for _ in range(2):
+            X.copy_(x0.to(cdt))
+            ctx.ChebyshevFiltering_batched([dict(spin=0, k=k, X=X, Y=Y, a=0.5, b=40.0, a0=-0.8)], 4,
+                                           precision=precision)
+        Xr, Yr = x0.numpy().copy(), np.zeros((ncol, Nd), dtype=np.complex128)
+        ctx.ChebyshevFiltering_kpt(k, Xr, Yr, 4, 0.5, 40.0, -0.8, precision=precision)
+        assert rel_err(Y.cpu().numpy().astype(np.complex128), Yr) < tol, (rc, lmax, hh)
+    ctx.close()

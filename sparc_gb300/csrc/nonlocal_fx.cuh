@@ -118,6 +118,9 @@ __device__ __forceinline__ void block(const Tables &T, int r, int g0, int gstep,
     const int q0 = T.row0[r], nrow = T.row0[r + 1] - q0;
     const int b0 = T.ent0[i0], nent = T.ent0[i0 + nit] - b0;
     const int ngroup = (ncol + NC - 1) / NC;
+    // a batched launch has as many blocks per range as its widest member needs; the others leave
+    // before they have copies in flight (the wait for those is in the first group)
+    if (g0 >= ngroup) return;
 
     // ---- the range's tables and Chi digits
     {

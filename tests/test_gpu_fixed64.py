@@ -270,6 +270,25 @@ def test_bloch_columns(gpu_available, N):
     ctx.close()
 
 
+def test_bloch_blocks_of_uneven_widths(gpu_available):
+    """One column beside many: most thread blocks of the narrow member have no column group. Every
+    column is the one of the single call to the rounding of four degrees."""
+    import torch
+    ctx, o, rng, L, co, v, S = _kpt_case((17, 14, 20), 0.45, 3, 8)
+    Nd = 17 * 14 * 20
+    k = 2 * np.pi / L * np.array((0.1, 0.3, 0.2))
+    xs = [torch.complex(torch.from_numpy(rng.uniform(-1, 1, (n, Nd))),
+                        torch.from_numpy(rng.uniform(-1, 1, (n, Nd)))) for n in (1, 90, 17, 2)]
+    blocks = [dict(spin=0, k=[float(q) for q in k], X=x.cuda(), Y=torch.empty_like(x, device="cuda"),
+                   a=0.3 * S, b=2.5 * S, a0=-2.0 * S) for x in xs]
+    ctx.ChebyshevFiltering_batched(blocks, 4)
+    for b, x in zip(blocks, xs):
+        X, Y = x.numpy().copy(), np.zeros(x.shape, dtype=np.complex128)
+        ctx.ChebyshevFiltering_kpt(k, X, Y, 4, b["a"], b["b"], b["a0"])
+        assert np.abs(b["Y"].cpu().numpy() - Y).max() <= 1e-12 * np.abs(Y).max()
+    ctx.close()
+
+
 @pytest.mark.parametrize("ncol", [1, 40])
 @pytest.mark.parametrize("N", [(17, 14, 20), (6, 12, 9), (34, 13, 12), (25, 24, 31), (41, 7, 6)])
 def test_complex64_tiles(gpu_available, N, ncol):

@@ -531,6 +531,13 @@ int sgpu_kernel_status(sgpu_ctx *ctx, int *status);
  * bound works) and leaves it cleared. No copy is in flight and nothing faults. */
 int sgpu_check_wait_bound(sgpu_ctx *ctx, int *status);
 
+/* Failures made on the host, for tests of what a call does about them; mask 0 ends them. 1: device
+ * scratch that a call can do without cannot be allocated; 2: the fixed-point tables of set_veff
+ * and set_nonlocal cannot be; 4: a bounded wait of the FP64 Rayleigh-Ritz products is reported as
+ * run out, with part of their output unwritten. A call then takes the form that needs none of
+ * these, with the same result. */
+int sgpu_inject_failure(sgpu_ctx *ctx, int mask);
+
 /* Measures this GPU's FP64 FMA rate (TFLOP/s, an FMA counted as two flops) with one
  * arithmetic-only kernel timed by CUDA events on the context stream: the ceiling of the FP64
  * stencil and nonlocal kernels, which on this part are bound by the FP64 pipe rather than by

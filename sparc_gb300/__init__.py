@@ -44,7 +44,7 @@ EXPORTED = [
     "sgpu_kernel_status", "sgpu_check_wait_bound", "sgpu_set_nonlocal_fuse",
     "sgpu_get_nonlocal_fuse", "sgpu_get_nonlocal_fuse_tc", "sgpu_ChebyshevFiltering_y", "sgpu_Project_Hamiltonian_f32",
     "sgpu_Subspace_Rotation_f32", "sgpu_set_gemm_emulation", "sgpu_measure_fp64_rate",
-    "sgpu_set_rr_products", "sgpu_set_eig_solver", "sgpu_Project_Hamiltonian_kpt",
+    "sgpu_set_rr_products", "sgpu_set_eig_solver", "sgpu_inject_failure", "sgpu_Project_Hamiltonian_kpt",
     "sgpu_Solve_Generalized_EigenProblem_kpt", "sgpu_Subspace_Rotation_kpt", "sgpu_CheFSI_batched",
 ]
 
@@ -780,6 +780,11 @@ class Context:
         st = ctypes.c_int()
         _check(lib().sgpu_check_wait_bound(self._h, ctypes.byref(st)))
         return int(st.value)
+
+    def inject_failure(self, mask):
+        """Failures made on the host, for tests (sgpu_inject_failure): 1 optional scratch, 2 the
+        fixed-point tables, 4 a wait of the FP64 Rayleigh-Ritz products; 0 none."""
+        _check(lib().sgpu_inject_failure(self._h, int(mask)))
 
     def last_filter_ms(self):
         ms = ctypes.c_float()

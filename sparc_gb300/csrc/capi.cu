@@ -14,6 +14,28 @@ static thread_local std::string g_err;
 
 void set_error(const std::string &msg) { g_err = msg; }
 
+// scratch of forms that have a slower twin without it: the first to go when memory is short
+static bool ws_optional(int slot)
+{
+    return slot == WS_SPLIT_A || slot == WS_SPLIT_B || slot == WS_FXPOT || slot == WS_NLPART;
+}
+
+// Gives back the optional scratch that no call in progress holds: a request for one of the
+// Rayleigh-Ritz slots comes from a call that may hold the others. Nothing else asks for a slot
+// between getting one of these and its last launch.
+int ws_release(sgpu_ctx *ctx, int asking)
+{
+    const bool rr = asking == WS_SPLIT_A || asking == WS_SPLIT_B || asking == WS_TC_PART;
+    for (int s : {(int)WS_NLPART, (int)WS_FXPOT, (int)WS_SPLIT_A, (int)WS_SPLIT_B}) {
+        Workspace &w = ctx->ws[s];
+        if (s == asking || !w.ptr || (rr && (s == WS_SPLIT_A || s == WS_SPLIT_B))) continue;
+        SGPU_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+        cudaFree(w.ptr);
+        w = Workspace();
+    }
+    return SGPU_OK;
+}
+
 int ws_get(sgpu_ctx *ctx, int slot, size_t bytes, void **out)
 {
     Workspace &w = ctx->ws[slot];
@@ -25,8 +47,15 @@ int ws_get(sgpu_ctx *ctx, int slot, size_t bytes, void **out)
             w.bytes = 0;
         }
         size_t nb = bytes + bytes / 8 + 256;
+        if ((ctx->inject & 1) && ws_optional(slot)) nb = (size_t)1 << 60;
         cudaError_t e = cudaMalloc(&w.ptr, nb);
         if (e != cudaSuccess) {
+            cudaGetLastError();  // the callers' launch checks must not meet it
+            SGPU_TRY(ws_release(ctx, slot));
+            e = cudaMalloc(&w.ptr, nb);
+        }
+        if (e != cudaSuccess) {
+            cudaGetLastError();
             set_error(std::string("device workspace allocation of ") + std::to_string(nb) +
                       " bytes failed: " + cudaGetErrorString(e));
             w.ptr = nullptr;
@@ -280,7 +309,7 @@ int sgpu_set_veff(sgpu_ctx *ctx, int nspin, const double *veff)
         ctx->nspin_veff = 0;
         SGPU_CUDA_TRY(cudaMalloc(&ctx->veff64, n * sizeof(double)));
         SGPU_CUDA_TRY(cudaMalloc(&ctx->veff32, n * sizeof(float)));
-        SGPU_CUDA_TRY(cudaMalloc(&ctx->veff_fx, (n + 1) * sizeof(int2)));
+        SGPU_CUDA_TRY(cudaMalloc(&ctx->veff_fx, ctx->inject & 2 ? (size_t)1 << 60 : (n + 1) * sizeof(int2)));
         ctx->nspin_veff = nspin;
     }
     SGPU_CUDA_TRY(cudaMemcpyAsync(ctx->veff64, veff, n * sizeof(double), cudaMemcpyDefault,
@@ -665,6 +694,17 @@ int sgpu_check_wait_bound(sgpu_ctx *ctx, int *status)
     if (rc != SGPU_OK) return rc;
     set_error("sgpu_check_wait_bound: the bounded wait did not report running out");
     return SGPU_ERR_STATE;
+}
+
+int sgpu_inject_failure(sgpu_ctx *ctx, int mask)
+{
+    SGPU_TRY(check_ctx(ctx));
+    if (mask & ~7) {
+        set_error("sgpu_inject_failure: unknown failure");
+        return SGPU_ERR_ARG;
+    }
+    ctx->inject = mask;
+    return SGPU_OK;
 }
 
 int sgpu_measure_fp64_rate(sgpu_ctx *ctx, double *tflops)

@@ -143,7 +143,7 @@ int launch_nonlocal_fx_apply(sgpu_ctx *ctx, int ncol, const double *alpha, long 
 // past kChiBytes. No tables (and the FP64 kernels stay) for more than 18 projectors per atom, for a
 // point under more than kPtRows projector rows (the 64-bit sums hold that many) and for Chi
 // values outside 1e-40 .. 1e40.
-static int build_ranges(Nonlocal &nl, NlFx &x, int cap, const std::vector<int> &er,
+static int build_ranges(Nonlocal &nl, NlFx &x, int cap, bool fail, const std::vector<int> &er,
                         const std::vector<int> &ord, const std::vector<int> &covpts,
                         const std::vector<int> &covptr, const std::vector<long> &ent_chi,
                         const std::vector<int4> &ent_meta)
@@ -252,7 +252,8 @@ static int build_ranges(Nonlocal &nl, NlFx &x, int cap, const std::vector<int> &
     auto up = [&](auto **dst, const auto &v) {
         using T = std::remove_reference_t<decltype(v[0])>;
         if (rc != SGPU_OK) return;
-        if (cudaMalloc((void **)dst, sizeof(T) * std::max<size_t>(v.size(), 1)) != cudaSuccess ||
+        const size_t n = fail ? (size_t)1 << 60 : sizeof(T) * std::max<size_t>(v.size(), 1);
+        if (cudaMalloc((void **)dst, n) != cudaSuccess ||
             (!v.empty() && cudaMemcpy((void *)*dst, v.data(), sizeof(T) * v.size(),
                                       cudaMemcpyHostToDevice) != cudaSuccess)) {
             set_error("set_nonlocal: device allocation of the fixed-point range tables failed");
@@ -296,7 +297,7 @@ static int build_ranges(Nonlocal &nl, NlFx &x, int cap, const std::vector<int> &
 
 int nonlocal_fx_build(Nonlocal &nl, const std::vector<int> &ord, const std::vector<int> &covpts,
                       const std::vector<int> &covptr, const std::vector<long> &ent_chi,
-                      const std::vector<int4> &ent_meta, const double *chi)
+                      const std::vector<int4> &ent_meta, const double *chi, bool fail)
 {
     if (nl.max_np > 18 || nl.max_np < 1 || nl.ncov == 0) return SGPU_OK;
     // exponent of each projector row's largest Chi value
@@ -320,10 +321,10 @@ int nonlocal_fx_build(Nonlocal &nl, const std::vector<int> &ord, const std::vect
     SGPU_CUDA_TRY(cudaMalloc((void **)&nl.fx_er, sizeof(int) * er.size()));
     SGPU_CUDA_TRY(cudaMemcpy(nl.fx_er, er.data(), sizeof(int) * er.size(), cudaMemcpyHostToDevice));
     nl.fx_jp = nl.max_np <= 9 ? 10 : 18;
-    SGPU_TRY(build_ranges(nl, nl.fx[0], nlfx::kPts, er, ord, covpts, covptr, ent_chi, ent_meta));
+    SGPU_TRY(build_ranges(nl, nl.fx[0], nlfx::kPts, fail, er, ord, covpts, covptr, ent_chi, ent_meta));
     // small ranges where one column group in large ones leaves SMs without a block
     if (nl.fx[0].nrange > 0 && nl.fx[0].nrange < 304)
-        SGPU_TRY(build_ranges(nl, nl.fx[1], nl.fx[0].nrange < 152 ? 32 : 64, er, ord, covpts, covptr,
+        SGPU_TRY(build_ranges(nl, nl.fx[1], nl.fx[0].nrange < 152 ? 32 : 64, fail, er, ord, covpts, covptr,
                               ent_chi, ent_meta));
     return SGPU_OK;
 }

@@ -1217,6 +1217,10 @@ int launch_gemm_x(sgpu_ctx *ctx, const TcxParams &p, cudaStream_t st)
                                        (int)XSMEM));
     ProfScope ps(ctx, SGPU_KERNEL_OTHER, st);
     k_tc_gemm_x<<<std::max(1, std::min(ntot, nsm)), NTHREADS, XSMEM, st>>>(p, nupper);
+    if (ctx->inject & 4) {  // a wait that ran out: a column left unwritten, the status word set
+        SGPU_CUDA_TRY(cudaMemsetAsync(p.C, 0xff, sizeof(double) * p.M, st));
+        SGPU_CUDA_TRY(cudaMemsetAsync(p.status, STATUS_TC_WAIT, 1, st));
+    }
     SGPU_CUDA_TRY(cudaGetLastError());
     return SGPU_OK;
 }

@@ -185,6 +185,7 @@ struct sgpu_ctx {
     unsigned veff_key = 0;
     sgpu::Nonlocal nl;
     bool has_nl = false;
+    int inject = 0;            // failures that a test asks for (sgpu_inject_failure)
     long set_count = 0;        // calls that changed the nonlocal set or the grid's numbers; captured
                                // launches hold those by value and pointer and are dropped with them
     cublasHandle_t cublas = nullptr;
@@ -254,6 +255,9 @@ enum WsSlot {
 
 // grow-only device scratch
 int ws_get(sgpu_ctx *ctx, int slot, size_t bytes, void **out);
+// gives back scratch that calls can do without, except what a request for slot `asking` may hold
+// (-1: none in use)
+int ws_release(sgpu_ctx *ctx, int asking);
 int fp64_fma_rate(sgpu_ctx *ctx, double *tflops);
 
 // profiling: returns an event pair recorded around a launch of `kind` (or nulls when off)
@@ -332,7 +336,7 @@ bool nonlocal_fx_ready(const sgpu_ctx *ctx);
 void nonlocal_fx_free(Nonlocal &nl);
 int nonlocal_fx_build(Nonlocal &nl, const std::vector<int> &ord, const std::vector<int> &covpts,
                       const std::vector<int> &covptr, const std::vector<long> &ent_chi,
-                      const std::vector<int4> &ent_meta, const double *chi);
+                      const std::vector<int4> &ent_meta, const double *chi, bool fail);
 int launch_nonlocal_fx_project(sgpu_ctx *ctx, int ncol, const double *x, long ldx, double *alpha,
                                long lda, cudaStream_t st);
 int launch_nonlocal_fx_apply(sgpu_ctx *ctx, int ncol, const double *alpha, long lda, double scale,

@@ -82,6 +82,7 @@ int project_f64(sgpu_ctx *ctx, int ncol, const double *Y, long ldy, const double
         const int rc = tc_project_x(ctx, ncol, Y, ldy, HY, ldh, Hp, Mp, &done, st);
         if (rc != SGPU_OK && rc != SGPU_ERR_NOMEM) return rc;
         if (done) return SGPU_OK;
+        if (rc == SGPU_ERR_NOMEM) SGPU_TRY(ws_release(ctx, -1));  // the slices that did fit
     }
     SGPU_TRY(ensure_handles(ctx));
     SGPU_CUBLAS_TRY(cublasSetStream(ctx->cublas, st));
@@ -419,6 +420,7 @@ int rotate_f64(sgpu_ctx *ctx, int ncol, const double *Y, long ldy, const double 
         const int rc = tc_rotate_x(ctx, ncol, Y, ldy, Q, X, ldx, &done, st);
         if (rc != SGPU_OK && rc != SGPU_ERR_NOMEM) return rc;
         if (done) return SGPU_OK;
+        if (rc == SGPU_ERR_NOMEM) SGPU_TRY(ws_release(ctx, -1));
     }
     SGPU_TRY(ensure_handles(ctx));
     SGPU_CUBLAS_TRY(cublasSetStream(ctx->cublas, st));

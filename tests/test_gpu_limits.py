@@ -1,0 +1,71 @@
+"""What a call does when device scratch, a table or a kernel's bounded wait fails (failures made on
+the host, sgpu_inject_failure), and at the edges of what the fixed-point FP64 kernels take."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import sparc_gb300 as sg
+from oracle.oracle import Oracle
+from sparc_gb300.synthetic import fd_d2_coeffs, synthetic_nonlocal
+
+pytestmark = pytest.mark.gpu
+
+SCRATCH, TABLES, RR_WAIT = 1, 2, 4
+
+
+def _system(N, h, natom=6, rc=2.2, nspin=1, seed=1):
+    """A context with a potential and projectors, and the arrays they were made from."""
+    rng = np.random.default_rng(seed)
+    c = fd_d2_coeffs(6, h)
+    Nd = N[0] * N[1] * N[2]
+    nl = synthetic_nonlocal(rng, N, h, natom=natom, rc=rc) if natom else None
+    ctx = sg.Context(*N, 6, c, c, c, h ** 3)
+    v = rng.normal(0.0, 0.4, nspin * Nd)
+    _set(ctx, v, nl, nspin)
+    return ctx, v, nl, dict(Nx=N[0], Ny=N[1], Nz=N[2], FDn=6, cx=c, cy=c, cz=c, dV=h ** 3), rng
+
+
+def _set(ctx, v, nl, nspin=1):
+    ctx.set_veff(v, nspin=nspin)
+    if nl:
+        ctx.set_nonlocal(nl["ip_displ"], nl["gamma"], nl["img_atom"], nl["img_ndc"],
+                         nl["grid_pos"], nl["chi"])
+
+
+def _close(a, b, tol=1e-12):
+    """Equal to the rounding of two FP64 routes, relative to the largest value."""
+    assert np.isfinite(b).all()
+    assert np.abs(a - b).max() <= tol * np.abs(b).max()
+
+
+def test_failed_allocation_is_not_met_again(gpu_available):
+    """A block that no device holds is refused for want of memory; the next call is not affected by
+    the allocation that failed."""
+    N, h = (30, 28, 26), 0.4
+    ctx, v, nl, grid, rng = _system(N, h)
+    Nd = ctx.Nd
+    x = rng.uniform(-1, 1, (8, Nd))
+    y = np.zeros_like(x)
+    rc = sg.lib().sgpu_Lap_vec_mult(ctx._h, 2 ** 31 - 1, ctypes.c_double(0.1), sg._ptr(x), Nd,
+                                    sg._ptr(y), Nd)
+    assert rc == 3, sg.lib().sgpu_last_error().decode()
+    ctx.Lap_vec_mult(0.1, x, y)
+    _close(y, Oracle(grid, None).lap_plus_diag(1.0, 0.0, 0.1, None, x))
+    ctx.close()
+
+
+def test_rr_products_without_scratch(gpu_available):
+    """No room for the slices: the FP64 GEMMs."""
+    ctx, v, nl, grid, rng = _system((30, 28, 26), 0.4, natom=0)
+    ncol = 70
+    Y = rng.uniform(-1, 1, (ncol, ctx.Nd))
+    Q = rng.normal(size=(ncol, ncol))
+    ctx.inject_failure(SCRATCH)
+    HY, Hp, Mp, X = np.zeros_like(Y), np.zeros_like(Q), np.zeros_like(Q), np.zeros_like(Y)
+    ctx.Project_Hamiltonian(Y, HY, Hp, Mp)
+    ctx.Subspace_Rotation(Y, Q, X)
+    _close(Mp, Y @ Y.T)
+    _close(Hp, Y @ HY.T)
+    _close(X, Q @ Y)
+    ctx.close()

@@ -1270,18 +1270,20 @@ int tc_rotate(sgpu_ctx *ctx, int ncol, const T *Y, long ldy, const double *Q, in
     return rotate_impl<T, 3>(ctx, ncol, Y, ldy, Q, ldq, X, ldx, st);
 }
 
-// Whether the last products met an infinity or a NaN (synchronises the stream)
-static int x_nonfinite(const int *flag, bool *bad, cudaStream_t st)
+// Whether the last products are to be kept (synchronises the stream): no infinity or NaN was met
+// (flag[0]; the FP64 GEMM gives the right ones) and no block gave up a bounded wait and left tiles
+// unwritten (flag[1], which stands in for the context's status word: the GEMM forms them again)
+static int x_complete(const int *flag, bool *ok, cudaStream_t st)
 {
-    int h = 0;
-    SGPU_CUDA_TRY(cudaMemcpyAsync(&h, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+    int h[2] = {0, 0};
+    SGPU_CUDA_TRY(cudaMemcpyAsync(h, flag, sizeof(h), cudaMemcpyDeviceToHost, st));
     SGPU_CUDA_TRY(cudaStreamSynchronize(st));
-    *bad = h != 0;
+    *ok = h[0] == 0 && h[1] == 0;
     return SGPU_OK;
 }
 
 // Hp = Yᵀ HY and Mp = Yᵀ Y to full FP64 accuracy. *done false, with nothing written that a caller
-// would keep: an entry is not finite (the FP64 GEMM gives the right infinities and NaN).
+// would keep: the FP64 GEMM is to form them (x_complete).
 int tc_project_x(sgpu_ctx *ctx, int ncol, const double *Y, long ldy, const double *HY, long ldh,
                  double *Hp, double *Mp, bool *done, cudaStream_t st)
 {
@@ -1304,7 +1306,7 @@ int tc_project_x(sgpu_ctx *ctx, int ncol, const double *Y, long ldy, const doubl
     const size_t psz = (size_t)ncol * ncol;
     SGPU_TRY(ws_get(ctx, WS_TC_PART, sizeof(double) * 2 * npass * ksplit * psz, (void **)&part));
     int *ey = reinterpret_cast<int *>(wa + step_bytes * per), *eh = ey + ncol, *flag = eh + ncol;
-    SGPU_CUDA_TRY(cudaMemsetAsync(flag, 0, sizeof(int), st));
+    SGPU_CUDA_TRY(cudaMemsetAsync(flag, 0, 2 * sizeof(int), st));
     SGPU_TRY(x_col_scales(ctx, Y, ldy, Nd, ncol, nullptr, 0, ey, flag, st));
     SGPU_TRY(x_col_scales(ctx, HY, ldh, Nd, ncol, nullptr, 0, eh, flag, st));
     __nv_bfloat16 *ty = reinterpret_cast<__nv_bfloat16 *>(wa);
@@ -1332,7 +1334,7 @@ int tc_project_x(sgpu_ctx *ctx, int ncol, const double *Y, long ldy, const doubl
             p.eA = ey;
             p.eB = w ? eh : ey;
             p.C = part + ((size_t)w * npass + ps) * ksplit * psz;
-            p.status = ctx->kstatus;
+            p.status = flag + 1;
             SGPU_TRY(launch_gemm_x(ctx, p, st));
         }
     }
@@ -1343,10 +1345,7 @@ int tc_project_x(sgpu_ctx *ctx, int ncol, const double *Y, long ldy, const doubl
                                                               ncol);
         SGPU_CUDA_TRY(cudaGetLastError());
     }
-    bool bad = false;
-    SGPU_TRY(x_nonfinite(flag, &bad, st));
-    *done = !bad;
-    return SGPU_OK;
+    return x_complete(flag, done, st);
 }
 
 // X = Y Q to full FP64 accuracy (Q ncol x ncol, ld ncol); *done as above
@@ -1368,11 +1367,11 @@ int tc_rotate_x(sgpu_ctx *ctx, int ncol, const double *Y, long ldy, const double
     int *ec = reinterpret_cast<int *>(wb + qbytes), *eq = ec + ncol, *flag = eq + ncol;
     __nv_bfloat16 *ta = reinterpret_cast<__nv_bfloat16 *>(wa);
     __nv_bfloat16 *tq = reinterpret_cast<__nv_bfloat16 *>(wb);
-    SGPU_CUDA_TRY(cudaMemsetAsync(flag, 0, sizeof(int), st));
+    SGPU_CUDA_TRY(cudaMemsetAsync(flag, 0, 2 * sizeof(int), st));
     // column balance of Y; row c of Q gets the inverse power of two
     SGPU_TRY(x_col_scales(ctx, Y, ldy, Nd, ncol, nullptr, 0, ec, flag, st));
     SGPU_TRY(x_col_scales(ctx, Q, ncol, ncol, ncol, nullptr, 0, eq, flag, st));
-    SGPU_TRY(x_col_scales(ctx, Q, ncol, ncol, ncol, ec, 1, eq, flag + 1, st));
+    SGPU_TRY(x_col_scales(ctx, Q, ncol, ncol, ncol, ec, 1, eq, flag + 2, st));
     {
         ProfScope sc(ctx, SGPU_KERNEL_OTHER, st);
         k_split_cols_x<<<(unsigned)(ksteps * nqb), 256, 0, st>>>(Q, ncol, ncol, ncol, eq, ec, 1, nqb,
@@ -1405,13 +1404,10 @@ int tc_rotate_x(sgpu_ctx *ctx, int ncol, const double *Y, long ldy, const double
         p.eB = eq;
         p.C = X + m0;
         p.ldc = ldx;
-        p.status = ctx->kstatus;
+        p.status = flag + 1;
         SGPU_TRY(launch_gemm_x(ctx, p, st));
     }
-    bool bad = false;
-    SGPU_TRY(x_nonfinite(flag, &bad, st));
-    *done = !bad;
-    return SGPU_OK;
+    return x_complete(flag, done, st);
 }
 
 template int tc_project<double>(sgpu_ctx *, int, const double *, long, const double *, long,

@@ -309,7 +309,8 @@ int sgpu_Project_Hamiltonian(sgpu_ctx *ctx, int spin, const double *Y, int ldi, 
     SGPU_TRY(unstage_vec(ctx, dHp, Hp, n2));
     SGPU_TRY(unstage_vec(ctx, dMp, Mp, n2));
     SGPU_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    return SGPU_OK;
+    // the six-slice kernels report a wait that ran out in the context's status word
+    return ctx->rr_tc == 2 ? kernel_status_check(ctx) : SGPU_OK;
 }
 
 int sgpu_Project_Hamiltonian_std(sgpu_ctx *ctx, int spin, double *Y, int ldi, double *HY,
@@ -437,7 +438,7 @@ int sgpu_Subspace_Rotation(sgpu_ctx *ctx, const double *Y, int ldi, const double
                                         sizeof(double) * ctx->Nd, ncol, cudaMemcpyDeviceToHost,
                                         ctx->stream));
     SGPU_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    return SGPU_OK;
+    return ctx->rr_tc == 2 ? kernel_status_check(ctx) : SGPU_OK;
 }
 
 // FP32 orbital blocks (device): the Rayleigh-Ritz products of the mixed SCF's FP32 phase, Hp

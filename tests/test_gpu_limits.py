@@ -69,3 +69,22 @@ def test_rr_products_without_scratch(gpu_available):
     _close(Hp, Y @ HY.T)
     _close(X, Q @ Y)
     ctx.close()
+
+
+@pytest.mark.parametrize("ncol", [7, 70])
+def test_rr_products_after_a_wait_ran_out(gpu_available, ncol):
+    """A block that gave up a wait leaves tiles unwritten: the products are formed again by the FP64
+    GEMMs, and nothing is left in the status word."""
+    ctx, v, nl, grid, rng = _system((30, 28, 26), 0.4, natom=0)
+    Y = rng.uniform(-1, 1, (ncol, ctx.Nd))
+    Q = rng.normal(size=(ncol, ncol))
+    ctx.inject_failure(RR_WAIT)
+    HY, Hp, Mp, X = np.zeros_like(Y), np.zeros_like(Q), np.zeros_like(Q), np.zeros_like(Y)
+    ctx.Project_Hamiltonian(Y, HY, Hp, Mp)
+    ctx.Subspace_Rotation(Y, Q, X)
+    _close(Mp, Y @ Y.T)
+    _close(Hp, Y @ HY.T)
+    _close(X, Q @ Y)
+    ctx.inject_failure(0)
+    assert ctx.kernel_status() == 0
+    ctx.close()

@@ -402,7 +402,8 @@ inline bool fx_setup(StencilFxParams &p, int FDn, unsigned vkey)
     double S = std::fabs(p.c0);
     for (int d = 0; d < 3; d++)
         for (int r = 0; r < FDn; r++) S += 2.0 * std::fabs(p.w[d][r]);
-    if (!(S > 1e-60 && S < 1e60) || !(std::fabs(p.s1) < 1e60)) return false;
+    // a sum's last unit is 2^(eS + E - 60) biased: at least 2^29 for the smallest S and E taken here
+    if (!(S > 1e-50 && S < 1e60) || !(std::fabs(p.s1) < 1e60)) return false;
     p.dv = 0;
     int eS = std::ilogb(S) + 1;                     // S < 2^eS
     const int ev = (int)(vkey >> 20) - 1023;        // |bv v| < 2^(ev + 1)

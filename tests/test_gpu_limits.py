@@ -88,3 +88,24 @@ def test_rr_products_after_a_wait_ran_out(gpu_available, ncol):
     ctx.inject_failure(0)
     assert ctx.kernel_status() == 0
     ctx.close()
+
+
+def test_smallest_coefficients_and_values(gpu_available):
+    """Coefficients that add up to 2e-60 and values of 1.5e-231 beside others 2^-55 of it: results
+    down to the smallest exponents, within the bound of the 37-term sum."""
+    N, h = (50, 48, 46), 0.4
+    Nd = N[0] * N[1] * N[2]
+    c = fd_d2_coeffs(6, h)
+    S0 = 3 * (abs(c[0]) + 2 * np.abs(c[1:]).sum())
+    c = c * (2e-60 / S0)
+    ctx = sg.Context(*N, 6, c, c, c, h ** 3)
+    grid = dict(Nx=N[0], Ny=N[1], Nz=N[2], FDn=6, cx=c, cy=c, cz=c, dV=h ** 3)
+    rng = np.random.default_rng(3)
+    x = rng.choice([-1.0, 1.0], size=(1, Nd)) * 1.5e-231 * 2.0 ** -55
+    x[0, rng.integers(0, Nd, 200)] = 1.5e-231
+    y = np.zeros_like(x)
+    ctx.Lap_vec_mult(0.0, x, y)
+    ref = Oracle(grid, None).lap_plus_diag(1.0, 0.0, 0.0, None, x)
+    assert np.isfinite(y).all()
+    assert np.abs(y - ref).max() <= 40 * 2.0 ** -53 * 2e-60 * 1.5e-231 + 40 * 5e-324
+    ctx.close()

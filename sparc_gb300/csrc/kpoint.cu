@@ -592,10 +592,10 @@ __global__ void __launch_bounds__(256)
                    bool second)
 {
     const BBlock<double2> &B = blocks[blockIdx.z];
-    const int row = blockIdx.y;
-    if ((int)blockIdx.x * 32 >= 2 * B.ncol) return;
+    const int row = blockIdx.x;
+    if ((int)blockIdx.y * 32 >= 2 * B.ncol) return;
     nlfx::reduce_row(ptr[row], ptr[row + 1], idx, reinterpret_cast<const double *>(B.part), 2 * B.ldp,
-                     blockIdx.x * 32, 2 * B.ncol, dV * gamma[row],
+                     blockIdx.y * 32, 2 * B.ncol, dV * gamma[row],
                      reinterpret_cast<double *>(second ? B.alpha2 : B.alpha) + 2L * B.ncol * row);
 }
 __global__ void __launch_bounds__(256)
@@ -603,9 +603,9 @@ __global__ void __launch_bounds__(256)
                   const int *__restrict__ idx, double dV, const double *__restrict__ gamma, int ncol,
                   double2 *__restrict__ alpha, long lda)
 {
-    const int row = blockIdx.y;
+    const int row = blockIdx.x;
     nlfx::reduce_row(ptr[row], ptr[row + 1], idx, reinterpret_cast<const double *>(part), 2 * ldp,
-                     blockIdx.x * 32, 2 * ncol, dV * gamma[row],
+                     blockIdx.y * 32, 2 * ncol, dV * gamma[row],
                      reinterpret_cast<double *>(alpha) + 2 * lda * row);
 }
 
@@ -1069,7 +1069,7 @@ static int nonlocal_z(sgpu_ctx *ctx, int ncol, const CT *x, long ldx, CT *out, l
                     ProfScope ps(ctx, SGPU_KERNEL_NL_PROJECT, st);
                     project<<<grid, 32 * nlfx::kWarps, sm, st>>>(T, ncol, nullptr, 0.0,
                         const_cast<CT *>(x), ldx, part, lda, ldp, ks->img_phase);
-                    k_fx_reduce_z<<<dim3((2 * ncol + 31) / 32, nl.ntot), 256, 0, st>>>(
+                    k_fx_reduce_z<<<dim3(nl.ntot, (2 * ncol + 31) / 32), 256, 0, st>>>(
                         part, ldp, X.sum_ptr, X.sum_idx, ctx->dV, nl.gamma64, ncol, alpha, lda);
                 }
                 ProfScope ps(ctx, SGPU_KERNEL_NL_APPLY, st);
@@ -1398,7 +1398,7 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
     const BBlock<double2> *dB128 = reinterpret_cast<const BBlock<double2> *>(dB);
     // the sums of the partial projections into one of the two buffers
     auto fx_reduce = [&](bool second) {
-        k_fx_reduce_zb<<<dim3((2 * maxcol + 31) / 32, nl.ntot, nblk), 256, 0, st>>>(
+        k_fx_reduce_zb<<<dim3(nl.ntot, (2 * maxcol + 31) / 32, nblk), 256, 0, st>>>(
             dB128, fxt->sum_ptr, fxt->sum_idx, ctx->dV, nl.gamma64, second);
         ctx->launches++;
     };

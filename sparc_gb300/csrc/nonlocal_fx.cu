@@ -27,8 +27,8 @@ __global__ void __launch_bounds__(256)
                 const double *__restrict__ part, long ldp, int n, double dV,
                 const double *__restrict__ gamma, double *__restrict__ alpha, long lda)
 {
-    const int row = blockIdx.y;
-    nlfx::reduce_row(ptr[row], ptr[row + 1], idx, part, ldp, blockIdx.x * 32, n,
+    const int row = blockIdx.x;  // x: more rows than a y dimension holds are in use
+    nlfx::reduce_row(ptr[row], ptr[row + 1], idx, part, ldp, blockIdx.y * 32, n,
                      dV * __ldg(gamma + row), alpha + (long)row * lda);
 }
 
@@ -87,7 +87,7 @@ int launch(sgpu_ctx *ctx, int ncol, const double *alpha, double scale, double *o
     }
     if (PROJ) {
         ProfScope ps(ctx, SGPU_KERNEL_NL_PROJECT, st);
-        k_fx_reduce<<<dim3((ncol + 31) / 32, nl.ntot), 256, 0, st>>>(
+        k_fx_reduce<<<dim3(nl.ntot, (ncol + 31) / 32), 256, 0, st>>>(
             X.sum_ptr, X.sum_idx, part, ldp, ncol, ctx->dV, nl.gamma64, alpha_next, lda);
         SGPU_CUDA_TRY(cudaGetLastError());
     }

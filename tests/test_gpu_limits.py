@@ -109,3 +109,40 @@ def test_smallest_coefficients_and_values(gpu_available):
     assert np.isfinite(y).all()
     assert np.abs(y - ref).max() <= 40 * 2.0 ** -53 * 2e-60 * 1.5e-231 + 40 * 5e-324
     ctx.close()
+
+
+def test_more_projector_rows_than_a_grid_dimension(gpu_available):
+    """7300 atoms of nine projectors, five points each: 65700 rows, real and complex."""
+    import torch
+    N, h, natom, npt = (40, 40, 40), 0.4, 7300, 5
+    Nd = N[0] * N[1] * N[2]
+    rng = np.random.default_rng(2)
+    nl = dict(ip_displ=np.arange(natom + 1, dtype=np.int32) * 9,
+              gamma=rng.uniform(-2, 2, 9 * natom), img_atom=np.arange(natom, dtype=np.int32),
+              img_ndc=np.full(natom, npt, dtype=np.int32),
+              grid_pos=np.concatenate([np.sort(rng.choice(Nd, npt, replace=False))
+                                       for _ in range(natom)]).astype(np.int32),
+              chi=rng.uniform(-1, 1, 9 * npt * natom))
+    c = fd_d2_coeffs(6, h)
+    grid = dict(Nx=N[0], Ny=N[1], Nz=N[2], FDn=6, cx=c, cy=c, cz=c, dV=h ** 3)
+    ctx = sg.Context(*N, 6, c, c, c, h ** 3)
+    v = rng.normal(0.0, 0.4, Nd)
+    _set(ctx, v, nl)
+    L = np.array(N) * h
+    coords = rng.uniform(0, 1, (natom, 3)) * L
+    ctx.set_kpoint_geometry(L, coords)
+    o = Oracle(grid, nl)
+    x = rng.uniform(-1, 1, (3, Nd))
+    y = np.zeros_like(x)
+    ctx.Vnl_vec_mult(x, y)
+    _close(y, o.vnl(x))
+    z = x + 1j * rng.uniform(-1, 1, (3, Nd))
+    k = np.array([0.2, -0.1, 0.3])
+    w = np.zeros_like(z)
+    ctx.Vnl_vec_mult_kpt(k, z, w)
+    _close(w, o.vnl_kpt(k, L, coords, z))
+    X = torch.from_numpy(z).cuda()
+    Y = torch.empty_like(X)
+    ctx.ChebyshevFiltering_batched([dict(spin=0, k=k, X=X, Y=Y, a=0.5, b=40.0, a0=-0.8)], 2)
+    _close(Y.cpu().numpy(), o.chebyshev_kpt(k, L, coords, v, 2, 0.5, 40.0, -0.8, z)[1])
+    ctx.close()

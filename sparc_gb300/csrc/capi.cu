@@ -699,7 +699,7 @@ int sgpu_check_wait_bound(sgpu_ctx *ctx, int *status)
 int sgpu_inject_failure(sgpu_ctx *ctx, int mask)
 {
     SGPU_TRY(check_ctx(ctx));
-    if (mask & ~7) {
+    if (mask & ~15) {
         set_error("sgpu_inject_failure: unknown failure");
         return SGPU_ERR_ARG;
     }

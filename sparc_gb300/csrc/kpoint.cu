@@ -945,16 +945,20 @@ static int stencil_z(sgpu_ctx *ctx, const double *k, int ncol, double a, double 
             w[2][r] = p.wz[r + 1];
         }
         // (the kernel's own FP64 path takes bv = 1)
-        const bool can = !p.v || bv == 1.0;
+        bool can = !p.v || bv == 1.0;
         FxPot own{};
         if (can && p.v && !pot) {  // a caller's potential: its digits for this call
             char *ws = nullptr;
-            SGPU_TRY(ws_get(ctx, WS_FXPOT, sizeof(int2) * (size_t)ctx->Nd + 16, (void **)&ws));
-            SGPU_TRY(fx_potential(ctx, p.v, bv, ctx->Nd, reinterpret_cast<int2 *>(ws + 16),
-                                  reinterpret_cast<unsigned *>(ws), &own.key, st));
-            SGPU_CUDA_TRY(cudaStreamSynchronize(st));
-            own.vd = reinterpret_cast<int2 *>(ws + 16);
-            pot = &own;
+            const int rc = ws_get(ctx, WS_FXPOT, sizeof(int2) * (size_t)ctx->Nd + 16, (void **)&ws);
+            can = rc != SGPU_ERR_NOMEM;
+            if (can) {
+                SGPU_TRY(rc);
+                SGPU_TRY(fx_potential(ctx, p.v, bv, ctx->Nd, reinterpret_cast<int2 *>(ws + 16),
+                                      reinterpret_cast<unsigned *>(ws), &own.key, st));
+                SGPU_CUDA_TRY(cudaStreamSynchronize(st));
+                own.vd = reinterpret_cast<int2 *>(ws + 16);
+                pot = &own;
+            }
         }
         if (can && fxz_launch(ctx, w, c0, p.v ? pot->key : 0u, ncol, &L)) {
             FxZOne b{};
@@ -1052,29 +1056,37 @@ static int nonlocal_z(sgpu_ctx *ctx, int ncol, const CT *x, long ldx, CT *out, l
     SGPU_TRY(ws_get(ctx, WS_ALPHA, sizeof(CT) * (size_t)nl.ntot * lda, (void **)&alpha));
     if constexpr (sizeof(CT) == 16)
         if (nonlocal_fx_ready(ctx)) {
-            const int groups = (ncol + nlfx::kLanes / 2 - 1) / (nlfx::kLanes / 2);
+            constexpr int FG = nlfx::kLanes / 2;
+            const int groups = (ncol + FG - 1) / FG;
             const NlFx &X = nonlocal_fx_pick(nl, groups);
             const nlfx::Tables T = nonlocal_fx_tables(nl, X);
-            const long ldp = (long)groups * (nlfx::kLanes / 2);
             const int sm = (int)nlfx::smem_bytes(T);
             CT *part = nullptr;
-            SGPU_TRY(ws_get(ctx, WS_NLPART, sizeof(CT) * (size_t)X.nrows * ldp, (void **)&part));
-            auto project = nl.max_np <= 9 ? k_nl_fx_z<false, true, 9> : k_nl_fx_z<false, true, 18>;
-            auto apply = nl.max_np <= 9 ? k_nl_fx_z<true, false, 9> : k_nl_fx_z<true, false, 18>;
-            if (X.nrange <= 65535) {
-                const dim3 grid(std::min(groups, std::max(1, 152 * 8 / X.nrange)), X.nrange);
+            int chunk = groups;
+            const int rc = X.nrange > 65535
+                               ? SGPU_ERR_NOMEM
+                               : nonlocal_fx_part(ctx, sizeof(CT) * (size_t)X.nrows * FG, groups, &chunk,
+                                                  (void **)&part);
+            if (rc != SGPU_ERR_NOMEM) {
+                SGPU_TRY(rc);
+                auto project = nl.max_np <= 9 ? k_nl_fx_z<false, true, 9> : k_nl_fx_z<false, true, 18>;
+                auto apply = nl.max_np <= 9 ? k_nl_fx_z<true, false, 9> : k_nl_fx_z<true, false, 18>;
                 SGPU_CUDA_TRY(cudaFuncSetAttribute(project, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
                 SGPU_CUDA_TRY(cudaFuncSetAttribute(apply, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-                {
+                const long ldp = (long)chunk * FG;
+                auto gx = [&](int gn) { return std::min(gn, std::max(1, 152 * 8 / X.nrange)); };
+                for (int g0 = 0; g0 < groups; g0 += chunk) {
+                    const int c0 = g0 * FG, gn = std::min(chunk, groups - g0);
+                    const int n = std::min(ncol - c0, gn * FG);
                     ProfScope ps(ctx, SGPU_KERNEL_NL_PROJECT, st);
-                    project<<<grid, 32 * nlfx::kWarps, sm, st>>>(T, ncol, nullptr, 0.0,
-                        const_cast<CT *>(x), ldx, part, lda, ldp, ks->img_phase);
-                    k_fx_reduce_z<<<dim3(nl.ntot, (2 * ncol + 31) / 32), 256, 0, st>>>(
-                        part, ldp, X.sum_ptr, X.sum_idx, ctx->dV, nl.gamma64, ncol, alpha, lda);
+                    project<<<dim3(gx(gn), X.nrange), 32 * nlfx::kWarps, sm, st>>>(T, n, nullptr, 0.0,
+                        const_cast<CT *>(x) + (long)c0 * ldx, ldx, part, lda, ldp, ks->img_phase);
+                    k_fx_reduce_z<<<dim3(nl.ntot, (2 * n + 31) / 32), 256, 0, st>>>(
+                        part, ldp, X.sum_ptr, X.sum_idx, ctx->dV, nl.gamma64, n, alpha + c0, lda);
                 }
                 ProfScope ps(ctx, SGPU_KERNEL_NL_APPLY, st);
-                apply<<<grid, 32 * nlfx::kWarps, sm, st>>>(T, ncol, alpha, scale, out, ldo, nullptr, lda,
-                                                           ldp, ks->img_phase);
+                apply<<<dim3(gx(groups), X.nrange), 32 * nlfx::kWarps, sm, st>>>(T, ncol, alpha, scale, out,
+                    ldo, nullptr, lda, ldp, ks->img_phase);
                 SGPU_CUDA_TRY(cudaGetLastError());
                 return SGPU_OK;
             }
@@ -1226,7 +1238,7 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
     bool fx_st = false, fx_nl = false;
     const NlFx *fxt = nullptr;
     CT *alpha2 = nullptr, *part = nullptr;
-    std::vector<long> partoff(nblk + 1, 0);
+    std::vector<long> partoff(nblk, 0);
     if (Z128) {
         double w[3][kMaxFDn], c0max = 0.0;
         for (int r = 0; r < kMaxFDn; r++) {
@@ -1241,13 +1253,36 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
         fx_nl = has_nl && nonlocal_fx_ready(ctx);
     }
     if (fx_nl) {
-        for (int b = 0; b < nblk; b++) partoff[b + 1] = partoff[b] + (blk[b].ncol + FG - 1) / FG * FG;
-        fxt = &nonlocal_fx_pick(nl, partoff[nblk] / FG);
-        fx_nl = fxt->nrange <= 65535;
+        long groups = 0;
+        int widest = 0;
+        for (int b = 0; b < nblk; b++) {
+            groups += (blk[b].ncol + FG - 1) / FG;
+            widest = std::max(widest, blk[b].ncol);
+        }
+        fxt = &nonlocal_fx_pick(nl, groups);
+        fx_nl = fxt->nrange <= 65535 && widest <= (1 << 20);  // grid dimensions of the launches
     }
+    // Members take turns with the partial rows where those of all take more than scratch_max: members
+    // turn[t] .. turn[t + 1] - 1 are launched together. No room: the FP64 kernels.
+    std::vector<int> turn;
     if (fx_nl) {
-        SGPU_TRY(ws_get(ctx, WS_ALPHA2, sizeof(CT) * (size_t)nl.ntot * totcols, (void **)&alpha2));
-        SGPU_TRY(ws_get(ctx, WS_NLPART, sizeof(CT) * (size_t)fxt->nrows * partoff[nblk], (void **)&part));
+        const size_t colbytes = sizeof(CT) * (size_t)fxt->nrows;
+        long most = 0, here = 0;
+        for (int b = 0; b < nblk; b++) {
+            const long w = (blk[b].ncol + FG - 1) / FG * FG;
+            if (b == 0 || (here + w) * colbytes > scratch_max(ctx)) {
+                turn.push_back(b);
+                here = 0;
+            }
+            partoff[b] = here;
+            here += w;
+            most = std::max(most, here);
+        }
+        turn.push_back(nblk);
+        int rc = ws_get(ctx, WS_ALPHA2, sizeof(CT) * (size_t)nl.ntot * totcols, (void **)&alpha2);
+        if (rc == SGPU_OK) rc = ws_get(ctx, WS_NLPART, colbytes * most, (void **)&part);
+        if (rc != SGPU_OK && rc != SGPU_ERR_NOMEM) return rc;
+        fx_nl = rc == SGPU_OK;
     }
 
     // host copies of the tables: blocks | coef | work | column groups | phases
@@ -1274,7 +1309,7 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
         B.spin = f.spin;
         B.alpha2 = fx_nl ? alpha2 + (size_t)nl.ntot * coloff[b] : nullptr;
         B.part = fx_nl ? part + (size_t)fxt->nrows * partoff[b] : nullptr;
-        B.ldp = partoff[b + 1] - partoff[b];
+        B.ldp = (f.ncol + FG - 1) / FG * FG;
         // recurrence scalars of ChebyshevFiltering_kpt (src/eigenSolverKpt.c:458-550)
         const double e = 0.5 * (f.b - f.a), c = 0.5 * (f.b + f.a);
         double sigma = e / (f.a0 - c);
@@ -1385,7 +1420,7 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
         fT = nonlocal_fx_tables(nl, *fxt);
         fsm = (int)nlfx::smem_bytes(fT);
         const int groups = (maxcol + FG - 1) / FG;
-        fgx = std::min(groups, std::max(1, 152 * 8 / (fxt->nrange * nblk)));
+        fgx = std::min(groups, std::max(1, (int)(152L * 8 / ((long)fxt->nrange * nblk))));
         auto attr = [&](auto k9, auto k18) {
             return nl.max_np <= 9
                        ? cudaFuncSetAttribute(k9, cudaFuncAttributeMaxDynamicSharedMemorySize, fsm)
@@ -1396,11 +1431,22 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
         SGPU_CUDA_TRY(attr(k_nl_fx_zb<true, true, 9>, k_nl_fx_zb<true, true, 18>));
     }
     const BBlock<double2> *dB128 = reinterpret_cast<const BBlock<double2> *>(dB);
-    // the sums of the partial projections into one of the two buffers
-    auto fx_reduce = [&](bool second) {
-        k_fx_reduce_zb<<<dim3(nl.ntot, (2 * maxcol + 31) / 32, nblk), 256, 0, st>>>(
-            dB128, fxt->sum_ptr, fxt->sum_idx, ctx->dV, nl.gamma64, second);
-        ctx->launches++;
+    // one of the fused form's kernels on buffer `sel`, member group by member group; `sums` of them
+    // adds up the partial projections into one of the two buffers
+    auto fx_launch = [&](auto kern, int j, int sel, bool second, int kind, bool sums, bool into) {
+        for (size_t t = 0; t + 1 < turn.size(); t++) {
+            const int b0 = turn[t], nb = turn[t + 1] - b0;
+            {
+                ProfScope ps(ctx, kind, st);
+                kern<<<dim3(nb * fgx, fxt->nrange), 32 * nlfx::kWarps, fsm, st>>>(
+                    fT, dB128 + b0, dC + (long)b0 * m, m, j, sel, second, fgx);
+                ctx->launches++;
+            }
+            if (!sums) continue;
+            ProfScope ps(ctx, SGPU_KERNEL_NL_PROJECT, st);
+            k_fx_reduce_zb<<<dim3(nl.ntot, (2 * maxcol + 31) / 32, nb), 256, 0, st>>>(
+                dB128 + b0, fxt->sum_ptr, fxt->sum_idx, ctx->dV, nl.gamma64, into);
+        }
     };
 
     auto issue = [&]() -> int {
@@ -1417,14 +1463,9 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
                 prev = cur;
                 cur = dst;
             }
-            if (fx_nl && j == 0) {  // later degrees are projected as their apply finishes them
-                ProfScope ps(ctx, SGPU_KERNEL_NL_PROJECT, st);
-                auto kern = nl.max_np <= 9 ? k_nl_fx_zb<false, true, 9> : k_nl_fx_zb<false, true, 18>;
-                kern<<<dim3(nblk * fgx, fxt->nrange), 32 * nlfx::kWarps, fsm, st>>>(fT, dB128, dC, m, j, in,
-                                                                                   false, fgx);
-                ctx->launches++;
-                fx_reduce(false);
-            }
+            if (fx_nl && j == 0)  // later degrees are projected as their apply finishes them
+                fx_launch(nl.max_np <= 9 ? k_nl_fx_zb<false, true, 9> : k_nl_fx_zb<false, true, 18>, j, in,
+                          false, SGPU_KERNEL_NL_PROJECT, true, false);
             if (has_nl && !fx_nl) {
                 SGPU_CUDA_TRY(cudaMemsetAsync(alpha, 0, abytes, st));
                 ProfScope ps(ctx, SGPU_KERNEL_NL_PROJECT, st);
@@ -1482,14 +1523,10 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
                 ctx->launches++;
             }
             if (fx_nl) {
-                ProfScope ps(ctx, SGPU_KERNEL_NL_APPLY, st);
                 const bool more = j + 1 < m, second = j & 1;
                 auto kern = more ? (nl.max_np <= 9 ? k_nl_fx_zb<true, true, 9> : k_nl_fx_zb<true, true, 18>)
                                  : (nl.max_np <= 9 ? k_nl_fx_zb<true, false, 9> : k_nl_fx_zb<true, false, 18>);
-                kern<<<dim3(nblk * fgx, fxt->nrange), 32 * nlfx::kWarps, fsm, st>>>(fT, dB128, dC, m, j, out,
-                                                                                   second, fgx);
-                ctx->launches++;
-                if (more) fx_reduce(!second);
+                fx_launch(kern, j, out, second, SGPU_KERNEL_NL_APPLY, more, !second);
             } else if (has_nl) {
                 ProfScope ps(ctx, SGPU_KERNEL_NL_APPLY, st);
                 constexpr int CB = zapply_cb<CT>();

@@ -66,32 +66,47 @@ int launch(sgpu_ctx *ctx, int ncol, const double *alpha, double scale, double *o
     auto kern = nl.max_np <= 9 ? k_nl_fx<APPLY, PROJ, 9> : k_nl_fx<APPLY, PROJ, 18>;
     SGPU_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)smem));
-    const long ldp = (long)groups * nlfx::kLanes;
     double *part = nullptr;
+    int chunk = groups;
     if (PROJ)
-        SGPU_TRY(ws_get(ctx, WS_NLPART, sizeof(double) * (size_t)X.nrows * ldp, (void **)&part));
-    {
-        ProfScope ps(ctx, APPLY ? SGPU_KERNEL_NL_APPLY : SGPU_KERNEL_NL_PROJECT, st);
-        for (int r0 = 0; r0 < X.nrange; r0 += 65535) {
-            nlfx::Tables R = T;
-            R.pt0 += r0;
-            R.item0 += r0;
-            R.row0 += r0;
-            // blocks of few ranges split the column groups, so that there are at least 8 per SM
-            const int gx = std::min(groups, std::max(1, 152 * 8 / X.nrange));
-            const dim3 grid(gx, std::min(65535, X.nrange - r0));
-            kern<<<grid, 32 * nlfx::kWarps, smem, st>>>(R, ncol, alpha, scale, out, x, ld, part,
-                                                        lda, ldp);
+        SGPU_TRY(nonlocal_fx_part(ctx, sizeof(double) * (size_t)X.nrows * nlfx::kLanes, groups, &chunk,
+                                  (void **)&part));
+    const long ldp = (long)chunk * nlfx::kLanes;
+    for (int g0 = 0; g0 < groups; g0 += chunk) {
+        const int c0 = g0 * nlfx::kLanes, gn = std::min(chunk, groups - g0);
+        const int n = std::min(ncol - c0, gn * nlfx::kLanes);
+        {
+            ProfScope ps(ctx, APPLY ? SGPU_KERNEL_NL_APPLY : SGPU_KERNEL_NL_PROJECT, st);
+            for (int r0 = 0; r0 < X.nrange; r0 += 65535) {
+                nlfx::Tables R = T;
+                R.pt0 += r0;
+                R.item0 += r0;
+                R.row0 += r0;
+                // blocks of few ranges split the column groups, so that there are at least 8 per SM
+                const int gx = std::min(gn, std::max(1, 152 * 8 / X.nrange));
+                const dim3 grid(gx, std::min(65535, X.nrange - r0));
+                kern<<<grid, 32 * nlfx::kWarps, smem, st>>>(
+                    R, n, APPLY ? alpha + c0 : nullptr, scale, APPLY ? out + (long)c0 * ld : nullptr,
+                    APPLY ? nullptr : x + (long)c0 * ld, ld, part, lda, ldp);
+            }
+            SGPU_CUDA_TRY(cudaGetLastError());
         }
-        SGPU_CUDA_TRY(cudaGetLastError());
-    }
-    if (PROJ) {
-        ProfScope ps(ctx, SGPU_KERNEL_NL_PROJECT, st);
-        k_fx_reduce<<<dim3(nl.ntot, (ncol + 31) / 32), 256, 0, st>>>(
-            X.sum_ptr, X.sum_idx, part, ldp, ncol, ctx->dV, nl.gamma64, alpha_next, lda);
-        SGPU_CUDA_TRY(cudaGetLastError());
+        if (PROJ) {
+            ProfScope ps(ctx, SGPU_KERNEL_NL_PROJECT, st);
+            k_fx_reduce<<<dim3(nl.ntot, gn), 256, 0, st>>>(X.sum_ptr, X.sum_idx, part, ldp, n, ctx->dV,
+                                                           nl.gamma64, alpha_next + c0, lda);
+            SGPU_CUDA_TRY(cudaGetLastError());
+        }
     }
     return SGPU_OK;
+}
+
+// the projection in FP64, which adds up in alpha itself and needs no partial rows
+int project_fp64(sgpu_ctx *ctx, int ncol, const double *x, long ldx, double *alpha, long lda,
+                 cudaStream_t st)
+{
+    SGPU_CUDA_TRY(cudaMemsetAsync(alpha, 0, sizeof(double) * (size_t)ctx->nl.ntot * lda, st));
+    return launch_nonlocal_project<double>(ctx, ncol, x, ldx, alpha, lda, st, false);
 }
 
 }  // namespace
@@ -124,18 +139,33 @@ void nonlocal_fx_free(Nonlocal &nl)
     }
 }
 
+int nonlocal_fx_part(sgpu_ctx *ctx, size_t group_bytes, int groups, int *chunk, void **part)
+{
+    int c = (int)std::min<size_t>(std::min(groups, 32768), std::max<size_t>(1, scratch_max(ctx) / group_bytes));
+    for (;; c = (c + 1) / 2) {
+        const int rc = ws_get(ctx, WS_NLPART, group_bytes * c, part);
+        *chunk = c;
+        if (rc != SGPU_ERR_NOMEM || c == 1) return rc;
+    }
+}
+
 int launch_nonlocal_fx_project(sgpu_ctx *ctx, int ncol, const double *x, long ldx, double *alpha,
                                long lda, cudaStream_t st)
 {
-    return launch<false, true>(ctx, ncol, nullptr, 0.0, nullptr, x, ldx, alpha, lda, st);
+    const int rc = launch<false, true>(ctx, ncol, nullptr, 0.0, nullptr, x, ldx, alpha, lda, st);
+    return rc == SGPU_ERR_NOMEM ? project_fp64(ctx, ncol, x, ldx, alpha, lda, st) : rc;
 }
 
 int launch_nonlocal_fx_apply(sgpu_ctx *ctx, int ncol, const double *alpha, long lda, double scale,
                              double *out, long ldo, double *alpha_next, cudaStream_t st)
 {
-    if (alpha_next)
-        return launch<true, true>(ctx, ncol, alpha, scale, out, nullptr, ldo, alpha_next, lda, st);
-    return launch<true, false>(ctx, ncol, alpha, scale, out, nullptr, ldo, nullptr, lda, st);
+    if (alpha_next) {  // the partial rows are sought before anything is launched
+        const int rc =
+            launch<true, true>(ctx, ncol, alpha, scale, out, nullptr, ldo, alpha_next, lda, st);
+        if (rc != SGPU_ERR_NOMEM) return rc;
+    }
+    SGPU_TRY((launch<true, false>(ctx, ncol, alpha, scale, out, nullptr, ldo, nullptr, lda, st)));
+    return alpha_next ? project_fp64(ctx, ncol, out, ldo, alpha_next, lda, st) : SGPU_OK;
 }
 
 // Range tables. A range takes covered points in the order of 32 x 4 x 4 blocks of the grid until it

@@ -410,4 +410,8 @@ __device__ __forceinline__ void reduce_row(int e0, int e1, const int *__restrict
 
 nlfx::Tables nonlocal_fx_tables(const Nonlocal &nl, const NlFx &x);
 const NlFx &nonlocal_fx_pick(const Nonlocal &nl, long groups);
+// The partial rows (WS_NLPART) of `groups` column groups of group_bytes each, or of as many at a time
+// as scratch_max and the device's free memory hold (*chunk); SGPU_ERR_NOMEM: not even one, and the
+// caller takes the FP64 kernels, which need none
+int nonlocal_fx_part(sgpu_ctx *ctx, size_t group_bytes, int groups, int *chunk, void **part);
 }  // namespace sgpu

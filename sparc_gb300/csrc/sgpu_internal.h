@@ -255,6 +255,8 @@ enum WsSlot {
 
 // grow-only device scratch
 int ws_get(sgpu_ctx *ctx, int slot, size_t bytes, void **out);
+// bytes that one operand's scratch takes at most: calls that need more work in several passes
+inline size_t scratch_max(const sgpu_ctx *ctx) { return ctx->inject & 8 ? (size_t)1 << 20 : (size_t)2 << 30; }
 // gives back scratch that calls can do without, except what a request for slot `asking` may hold
 // (-1: none in use)
 int ws_release(sgpu_ctx *ctx, int asking);

@@ -1078,7 +1078,8 @@ int launch_bulk(const StencilParams<float> &q, dim3 grid, cudaStream_t st)
     return SGPU_OK;
 }
 
-// FP64 stencil in block fixed point; *done false when the coefficients are out of its range
+// FP64 stencil in block fixed point; *done false when the coefficients are out of its range or there
+// is no room for the digits of a caller's potential
 int launch_stencil_fx(sgpu_ctx *ctx, int ncol, const StencilParams<double> &q, const FxPot *pot,
                       bool *done, cudaStream_t st)
 {
@@ -1098,7 +1099,9 @@ int launch_stencil_fx(sgpu_ctx *ctx, int ncol, const StencilParams<double> &q, c
     FxPot own{};
     if (q.v && !pot) {  // a caller's potential: its digits for this call
         char *w = nullptr;
-        SGPU_TRY(ws_get(ctx, WS_FXPOT, sizeof(int2) * (size_t)ctx->Nd + 16, (void **)&w));
+        const int rc = ws_get(ctx, WS_FXPOT, sizeof(int2) * (size_t)ctx->Nd + 16, (void **)&w);
+        if (rc == SGPU_ERR_NOMEM) return SGPU_OK;
+        SGPU_TRY(rc);
         SGPU_TRY(fx_potential(ctx, q.v, q.bv, ctx->Nd, reinterpret_cast<int2 *>(w + 16),
                               reinterpret_cast<unsigned *>(w), &own.key, st));
         SGPU_CUDA_TRY(cudaStreamSynchronize(st));

@@ -11,7 +11,7 @@ from sparc_gb300.synthetic import fd_d2_coeffs, synthetic_nonlocal
 
 pytestmark = pytest.mark.gpu
 
-SCRATCH, TABLES, RR_WAIT = 1, 2, 4
+SCRATCH, TABLES, RR_WAIT, SMALL = 1, 2, 4, 8
 
 
 def _system(N, h, natom=6, rc=2.2, nspin=1, seed=1):
@@ -145,4 +145,47 @@ def test_more_projector_rows_than_a_grid_dimension(gpu_available):
     Y = torch.empty_like(X)
     ctx.ChebyshevFiltering_batched([dict(spin=0, k=k, X=X, Y=Y, a=0.5, b=40.0, a0=-0.8)], 2)
     _close(Y.cpu().numpy(), o.chebyshev_kpt(k, L, coords, v, 2, 0.5, 40.0, -0.8, z)[1])
+    ctx.close()
+
+
+def test_nonlocal_and_stencil_without_scratch(gpu_available):
+    """No room for the partial projections or a caller's potential as digits: the FP64 kernels, in
+    every call that uses either, real and complex, single and batched. Room for some column groups'
+    partial projections: those take turns."""
+    import torch
+    N, h = (30, 28, 26), 0.4
+    ctx, v, nl, grid, rng = _system(N, h)
+    o, Nd, ncol = Oracle(grid, nl), ctx.Nd, 165
+    L = np.array(N) * h
+    coords = rng.uniform(0, 1, (len(nl["img_atom"]), 3)) * L
+    ctx.set_kpoint_geometry(L, coords)
+    x = rng.uniform(-1, 1, (ncol, Nd))
+    z = x[:90] + 1j * rng.uniform(-1, 1, (90, Nd))
+    k = np.array([0.2, -0.1, 0.3])
+    zt = torch.from_numpy(z).cuda()
+    for mask in (SCRATCH, SMALL, 0):
+        ctx.inject_failure(mask)
+        y = np.zeros_like(x)
+        ctx.Vnl_vec_mult(x, y)
+        _close(y, o.vnl(x))
+        ctx.Lap_plus_diag_vec_mult_orth(-0.5, 1.0, 0.3, v, x, y)
+        _close(y, o.lap_plus_diag(-0.5, 1.0, 0.3, v, x))
+        ctx.Hamiltonian_vectors_mult(0.3, x, y)
+        _close(y, o.hamiltonian(v, 0.3, x))
+        X, Y = x.copy(), np.zeros_like(x)
+        ctx.ChebyshevFiltering(X, Y, 5, 0.5, 40.0, -0.8)
+        Xo, Yo = o.chebyshev(v, 5, 0.5, 40.0, -0.8, x)
+        _close(Y, Yo)
+        _close(X, Xo)
+        w = np.zeros_like(z)
+        ctx.Hamiltonian_vectors_mult_kpt(k, 0.3, z, w)
+        _close(w, o.hamiltonian_kpt(k, L, coords, v, 0.3, z))
+        Xo, Yo = o.chebyshev_kpt(k, L, coords, v, 5, 0.5, 40.0, -0.8, z)
+        cuts = [0, 3, 40, 41, 90]
+        blocks = [dict(spin=0, k=k, X=zt[i:j].clone(), Y=torch.empty_like(zt[i:j]), a=0.5, b=40.0,
+                       a0=-0.8) for i, j in zip(cuts, cuts[1:])]
+        ctx.ChebyshevFiltering_batched(blocks, 5)
+        for blk, i, j in zip(blocks, cuts, cuts[1:]):
+            _close(blk["Y"].cpu().numpy(), Yo[i:j])
+            _close(blk["X"].cpu().numpy(), Xo[i:j])
     ctx.close()

@@ -309,16 +309,22 @@ int sgpu_set_veff(sgpu_ctx *ctx, int nspin, const double *veff)
         ctx->nspin_veff = 0;
         SGPU_CUDA_TRY(cudaMalloc(&ctx->veff64, n * sizeof(double)));
         SGPU_CUDA_TRY(cudaMalloc(&ctx->veff32, n * sizeof(float)));
-        SGPU_CUDA_TRY(cudaMalloc(&ctx->veff_fx, ctx->inject & 2 ? (size_t)1 << 60 : (n + 1) * sizeof(int2)));
+        // without room for the digits the FP64 kernels read veff64
+        if (cudaMalloc(&ctx->veff_fx, ctx->inject & 2 ? (size_t)1 << 60 : (n + 1) * sizeof(int2)) !=
+            cudaSuccess) {
+            cudaGetLastError();
+            ctx->veff_fx = nullptr;
+        }
         ctx->nspin_veff = nspin;
     }
     SGPU_CUDA_TRY(cudaMemcpyAsync(ctx->veff64, veff, n * sizeof(double), cudaMemcpyDefault,
                                   ctx->stream));
     SGPU_TRY(convert_cols<double, float>(ctx->veff64, (long)n, ctx->veff32, (long)n, (long)n, 1,
                                          ctx->stream));
-    SGPU_TRY(fx_potential(ctx, ctx->veff64, 1.0, (long)n, ctx->veff_fx,
-                          reinterpret_cast<unsigned *>(ctx->veff_fx + n), &ctx->veff_key,
-                          ctx->stream));
+    if (ctx->veff_fx)
+        SGPU_TRY(fx_potential(ctx, ctx->veff64, 1.0, (long)n, ctx->veff_fx,
+                              reinterpret_cast<unsigned *>(ctx->veff_fx + n), &ctx->veff_key,
+                              ctx->stream));
     SGPU_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     return SGPU_OK;
 }

@@ -51,7 +51,7 @@ int hamiltonian_dev(sgpu_ctx *ctx, int spin, int ncol, double c, const T *x, lon
         SGPU_TRY(launch_nonlocal_project<T>(ctx, ncol, x, ldx, a, lda, st));
         alpha = a;
     }
-    const FxPot pot{ctx->veff_fx + (long)spin * ctx->Nd, ctx->veff_key};
+    const FxPot pot = fx_pot(ctx, spin);
     SGPU_TRY(launch_stencil<T>(ctx, ncol, -0.5, 1.0, c, veff_of<T>(ctx, spin), x, ldx, hx, ldh,
                                s1, s2, z, ldz, st, &pot));
     if (!alpha) return SGPU_OK;

@@ -960,7 +960,7 @@ static int stencil_z(sgpu_ctx *ctx, const double *k, int ncol, double a, double 
                 pot = &own;
             }
         }
-        if (can && fxz_launch(ctx, w, c0, p.v ? pot->key : 0u, ncol, &L)) {
+        if (can && (!p.v || pot->vd) && fxz_launch(ctx, w, c0, p.v ? pot->key : 0u, ncol, &L)) {
             FxZOne b{};
             b.c.x = x; b.c.out = out; b.c.z = p.z;
             b.c.v = p.v;
@@ -1156,7 +1156,7 @@ int hamiltonian_z(sgpu_ctx *ctx, int spin, const double *k, int ncol, double c, 
     const bool f64 = sizeof(CT) == 16;
     const double *v = f64 ? ctx->veff64 + (long)spin * ctx->Nd : nullptr;
     const float *v32 = f64 ? nullptr : ctx->veff32 + (long)spin * ctx->Nd;
-    const FxPot pot{ctx->veff_fx + (long)spin * ctx->Nd, ctx->veff_key};
+    const FxPot pot = fx_pot(ctx, spin);
     SGPU_TRY(stencil_z<CT>(ctx, k, ncol, -0.5, 1.0, c, v, v32, x, ldx, hx, ldh, s1, s2, z, ldz, st, &pot));
     SGPU_TRY(nonlocal_z<CT>(ctx, ncol, x, ldx, hx, ldh, s1, st));
     return SGPU_OK;
@@ -1249,7 +1249,7 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
         for (int b = 0; b < nblk; b++)
             c0max = std::max(c0max, std::fabs(-0.5 * (ctx->cx[0] + ctx->cy[0] + ctx->cz[0]) -
                                               0.5 * (blk[b].a + blk[b].b)));
-        fx_st = fxz_launch(ctx, w, c0max * 1.0000001, ctx->veff_key, totcols, &fxl);
+        fx_st = ctx->veff_fx && fxz_launch(ctx, w, c0max * 1.0000001, ctx->veff_key, totcols, &fxl);
         fx_nl = has_nl && nonlocal_fx_ready(ctx);
     }
     if (fx_nl) {

@@ -1354,7 +1354,14 @@ int nonlocal_upload(sgpu_ctx *ctx, int natom, const int *ip_displ, const double 
 #undef UP
     const std::vector<int> ord = compact_order(ctx->Nx, ctx->Ny, covpts);
     if (rc == SGPU_OK) rc = nonlocal_tc_build(nl, ord, covpts, covptr, ent_chi, ent_meta, chi);
-    if (rc == SGPU_OK) rc = nonlocal_fx_build(nl, ord, covpts, covptr, ent_chi, ent_meta, chi, ctx->inject & 2);
+    if (rc == SGPU_OK) {
+        rc = nonlocal_fx_build(nl, ord, covpts, covptr, ent_chi, ent_meta, chi, ctx->inject & 2);
+        if (rc == SGPU_ERR_NOMEM) {  // the FP64 kernels need none of these tables
+            cudaGetLastError();
+            nonlocal_fx_free(nl);
+            rc = SGPU_OK;
+        }
+    }
     if (rc != SGPU_OK) {
         nonlocal_free(nl);
         return rc;

@@ -172,7 +172,7 @@ int launch_nonlocal_fx_apply(sgpu_ctx *ctx, int ncol, const double *alpha, long 
 // holds `cap` of them or the next point's images would take its rows past kRows or its Chi digits
 // past kChiBytes. No tables (and the FP64 kernels stay) for more than 18 projectors per atom, for a
 // point under more than kPtRows projector rows (the 64-bit sums hold that many) and for Chi
-// values outside 1e-40 .. 1e40.
+// values outside 1e-40 .. 1e40. SGPU_ERR_NOMEM: no room for them.
 static int build_ranges(Nonlocal &nl, NlFx &x, int cap, bool fail, const std::vector<int> &er,
                         const std::vector<int> &ord, const std::vector<int> &covpts,
                         const std::vector<int> &covptr, const std::vector<long> &ent_chi,
@@ -283,10 +283,11 @@ static int build_ranges(Nonlocal &nl, NlFx &x, int cap, bool fail, const std::ve
         using T = std::remove_reference_t<decltype(v[0])>;
         if (rc != SGPU_OK) return;
         const size_t n = fail ? (size_t)1 << 60 : sizeof(T) * std::max<size_t>(v.size(), 1);
-        if (cudaMalloc((void **)dst, n) != cudaSuccess ||
-            (!v.empty() && cudaMemcpy((void *)*dst, v.data(), sizeof(T) * v.size(),
-                                      cudaMemcpyHostToDevice) != cudaSuccess)) {
-            set_error("set_nonlocal: device allocation of the fixed-point range tables failed");
+        if (cudaMalloc((void **)dst, n) != cudaSuccess) {
+            rc = SGPU_ERR_NOMEM;
+        } else if (!v.empty() && cudaMemcpy((void *)*dst, v.data(), sizeof(T) * v.size(),
+                                            cudaMemcpyHostToDevice) != cudaSuccess) {
+            set_error("set_nonlocal: copy of the fixed-point range tables failed");
             rc = SGPU_ERR_CUDA;
         }
     };
@@ -306,10 +307,8 @@ static int build_ranges(Nonlocal &nl, NlFx &x, int cap, bool fail, const std::ve
     up(&dsrc, src);
     up(&drows, rows);
     const size_t cbytes = sizeof(int2) * (size_t)nl.nent * nl.fx_jp;
-    if (rc == SGPU_OK && cudaMalloc((void **)&x.chi, cbytes) != cudaSuccess) {
-        set_error("set_nonlocal: device allocation of the Chi digits failed");
-        rc = SGPU_ERR_CUDA;
-    }
+    if (rc == SGPU_OK && cudaMalloc((void **)&x.chi, cbytes) != cudaSuccess)
+        rc = SGPU_ERR_NOMEM;
     if (rc == SGPU_OK) {
         k_fx_chi<<<152 * 8, 256>>>(dsrc, drows, nl.nent, nl.fx_jp, nl.chi64, nl.fx_er,
                                    reinterpret_cast<int2 *>(x.chi));
@@ -348,7 +347,7 @@ int nonlocal_fx_build(Nonlocal &nl, const std::vector<int> &ord, const std::vect
             std::frexp(mx[i], &er[i]);
         }
     }
-    SGPU_CUDA_TRY(cudaMalloc((void **)&nl.fx_er, sizeof(int) * er.size()));
+    if (cudaMalloc((void **)&nl.fx_er, sizeof(int) * er.size()) != cudaSuccess) return SGPU_ERR_NOMEM;
     SGPU_CUDA_TRY(cudaMemcpy(nl.fx_er, er.data(), sizeof(int) * er.size(), cudaMemcpyHostToDevice));
     nl.fx_jp = nl.max_np <= 9 ? 10 : 18;
     SGPU_TRY(build_ranges(nl, nl.fx[0], nlfx::kPts, fail, er, ord, covpts, covptr, ent_chi, ent_meta));

@@ -125,7 +125,7 @@ struct Nonlocal {
 };
 
 // A potential as fixed-point digits (fixed64.cuh) for the FP64 stencil; key: the exponent key of its
-// largest magnitude, which sets the digits' scale (0: all zero)
+// largest magnitude, which sets the digits' scale (0: all zero). vd null: no digits
 struct FxPot {
     const int2 *vd = nullptr;
     unsigned key = 0;
@@ -181,7 +181,7 @@ struct sgpu_ctx {
     int nspin_veff = 0;
     double *veff64 = nullptr;  // Nd * nspin
     float *veff32 = nullptr;
-    int2 *veff_fx = nullptr;   // digits of veff64 (all spins at one scale), key after them
+    int2 *veff_fx = nullptr;   // digits of veff64 (all spins at one scale), key after them; or null
     unsigned veff_key = 0;
     sgpu::Nonlocal nl;
     bool has_nl = false;
@@ -280,6 +280,11 @@ int wait_bound_check(sgpu_ctx *ctx);
 
 // memory-kind query: true when p is device (or managed) memory this context can use directly
 bool is_device_ptr(const void *p);
+
+inline FxPot fx_pot(const sgpu_ctx *ctx, int spin)
+{
+    return {ctx->veff_fx ? ctx->veff_fx + (long)spin * ctx->Nd : nullptr, ctx->veff_key};
+}
 
 // ---- stencil (stencil.cu)
 // out[:, n] = s1 * ( a*Lap + bv*diag(v) + c*I ) x[:, n]  +  s2 * z[:, n]

@@ -1079,7 +1079,7 @@ int launch_bulk(const StencilParams<float> &q, dim3 grid, cudaStream_t st)
 }
 
 // FP64 stencil in block fixed point; *done false when the coefficients are out of its range or there
-// is no room for the digits of a caller's potential
+// was no room for the digits of the potential
 int launch_stencil_fx(sgpu_ctx *ctx, int ncol, const StencilParams<double> &q, const FxPot *pot,
                       bool *done, cudaStream_t st)
 {
@@ -1108,6 +1108,7 @@ int launch_stencil_fx(sgpu_ctx *ctx, int ncol, const StencilParams<double> &q, c
         own.vd = reinterpret_cast<int2 *>(w + 16);
         pot = &own;
     }
+    if (q.v && !pot->vd) return SGPU_OK;
     const unsigned vkey = q.v ? pot->key : 0u;
     p.vd = vkey ? pot->vd : nullptr;
     if (!fx_setup(p, R, vkey)) return SGPU_OK;

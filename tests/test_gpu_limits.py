@@ -189,3 +189,38 @@ def test_nonlocal_and_stencil_without_scratch(gpu_available):
             _close(blk["Y"].cpu().numpy(), Yo[i:j])
             _close(blk["X"].cpu().numpy(), Xo[i:j])
     ctx.close()
+
+
+def test_sets_without_tables(gpu_available):
+    """No room for the fixed-point tables of the potential or the projectors: both sets are accepted
+    as before and the FP64 kernels serve them; a later set has its tables again."""
+    import torch
+    N, h = (30, 28, 26), 0.4
+    ctx, v, nl, grid, rng = _system(N, h)
+    o, Nd, ncol = Oracle(grid, nl), ctx.Nd, 11
+    L = np.array(N) * h
+    coords = rng.uniform(0, 1, (len(nl["img_atom"]), 3)) * L
+    ctx.set_kpoint_geometry(L, coords)
+    x = rng.uniform(-1, 1, (ncol, Nd))
+    z = x + 1j * rng.uniform(-1, 1, (ncol, Nd))
+    k = np.array([0.2, -0.1, 0.3])
+    zt = torch.from_numpy(z).cuda()
+    for mask in (TABLES, 0):
+        ctx.inject_failure(mask)
+        _set(ctx, np.concatenate([v, -0.5 * v]), nl, 2)
+        for spin, s in ((0, 1.0), (1, -0.5)):
+            y = np.zeros_like(x)
+            ctx.Hamiltonian_vectors_mult(0.3, x, y, spin=spin)
+            _close(y, o.hamiltonian(s * v, 0.3, x))
+            X, Y = x.copy(), np.zeros_like(x)
+            ctx.ChebyshevFiltering(X, Y, 4, 0.5, 40.0, -0.8, spin=spin)
+            _close(Y, o.chebyshev(s * v, 4, 0.5, 40.0, -0.8, x)[1])
+            w = np.zeros_like(z)
+            ctx.Hamiltonian_vectors_mult_kpt(k, 0.3, z, w, spin=spin)
+            _close(w, o.hamiltonian_kpt(k, L, coords, s * v, 0.3, z))
+            Xb, Yb = zt.clone(), torch.empty_like(zt)
+            ctx.ChebyshevFiltering_batched([dict(spin=spin, k=k, X=Xb, Y=Yb, a=0.5, b=40.0,
+                                                 a0=-0.8)], 4)
+            _close(Yb.cpu().numpy(), o.chebyshev_kpt(k, L, coords, s * v, 4, 0.5, 40.0, -0.8, z)[1])
+        _set(ctx, v, nl, 1)
+    ctx.close()

@@ -690,16 +690,16 @@ __global__ void __launch_bounds__(256) k_split_rows(const T *__restrict__ X, lon
     }
 }
 
-// C = sum of the K-range partial sums (fixed order), ld ldc
+// C (+)= sum of the K-range partial sums (fixed order), ld ldc
 __global__ void k_reduce_parts(const double *__restrict__ part, int ksplit, int n, double *C,
-                               int ldc)
+                               int ldc, bool add = false)
 {
     const long total = (long)n * n;
     for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < total;
          t += (long)gridDim.x * blockDim.x) {
-        double v = 0.0;
-        for (int s = 0; s < ksplit; s++) v += part[(long)s * total + t];
         const long j = t / n, i = t - j * n;
+        double v = add ? C[j * ldc + i] : 0.0;
+        for (int s = 0; s < ksplit; s++) v += part[(long)s * total + t];
         C[j * ldc + i] = v;
     }
 }
@@ -1226,8 +1226,7 @@ int launch_gemm_x(sgpu_ctx *ctx, const TcxParams &p, cudaStream_t st)
 }
 
 // Workspaces are bounded: the products run over ranges of grid points whose slices of one operand
-// take at most this many bytes
-constexpr size_t kXOperand = (size_t)2 << 30;
+// take at most scratch_max bytes, and each range's sums are added to the result before the next
 
 int x_row_blocks(int ncol)  // 128-row blocks that cover the 128- and the 64-row tiles
 {
@@ -1294,7 +1293,7 @@ int tc_project_x(sgpu_ctx *ctx, int ncol, const double *Y, long ldy, const doubl
     const int nupper = upper_tiles(mt, nt);
     const size_t step_bytes = sizeof(__nv_bfloat16) * (size_t)XS * nrb * (TM / 8) * XG;
     const int steps = (int)((Nd + TK - 1) / TK);
-    const int per = (int)std::max<size_t>(CHUNK_STEPS, std::min<size_t>(steps, kXOperand / step_bytes));
+    const int per = (int)std::max<size_t>(CHUNK_STEPS, std::min<size_t>(steps, scratch_max(ctx) / step_bytes));
     const int npass = (steps + per - 1) / per;
     int ksplit = std::max(1, 152 / nupper);
     ksplit = std::min(ksplit, std::max(1, per / CHUNK_STEPS));
@@ -1304,7 +1303,7 @@ int tc_project_x(sgpu_ctx *ctx, int ncol, const double *Y, long ldy, const doubl
     SGPU_TRY(ws_get(ctx, WS_SPLIT_A, step_bytes * per + ebytes, (void **)&wa));
     SGPU_TRY(ws_get(ctx, WS_SPLIT_B, step_bytes * per, (void **)&wb));
     const size_t psz = (size_t)ncol * ncol;
-    SGPU_TRY(ws_get(ctx, WS_TC_PART, sizeof(double) * 2 * npass * ksplit * psz, (void **)&part));
+    SGPU_TRY(ws_get(ctx, WS_TC_PART, sizeof(double) * ksplit * psz, (void **)&part));
     int *ey = reinterpret_cast<int *>(wa + step_bytes * per), *eh = ey + ncol, *flag = eh + ncol;
     SGPU_CUDA_TRY(cudaMemsetAsync(flag, 0, 2 * sizeof(int), st));
     SGPU_TRY(x_col_scales(ctx, Y, ldy, Nd, ncol, nullptr, 0, ey, flag, st));
@@ -1333,17 +1332,14 @@ int tc_project_x(sgpu_ctx *ctx, int ncol, const double *Y, long ldy, const doubl
             p.M = p.N = ncol;
             p.eA = ey;
             p.eB = w ? eh : ey;
-            p.C = part + ((size_t)w * npass + ps) * ksplit * psz;
+            p.C = part;
             p.status = flag + 1;
             SGPU_TRY(launch_gemm_x(ctx, p, st));
+            ProfScope sc(ctx, SGPU_KERNEL_OTHER, st);
+            k_reduce_parts<<<blocks_for((long)psz), 256, 0, st>>>(part, ksplit, ncol, w ? Hp : Mp, ncol,
+                                                                  ps > 0);
+            SGPU_CUDA_TRY(cudaGetLastError());
         }
-    }
-    for (int w = 0; w < 2; w++) {
-        ProfScope sc(ctx, SGPU_KERNEL_OTHER, st);
-        k_reduce_parts<<<blocks_for((long)psz), 256, 0, st>>>(part + (size_t)w * npass * ksplit * psz,
-                                                              npass * ksplit, ncol, w ? Hp : Mp,
-                                                              ncol);
-        SGPU_CUDA_TRY(cudaGetLastError());
     }
     return x_complete(flag, done, st);
 }
@@ -1357,7 +1353,7 @@ int tc_rotate_x(sgpu_ctx *ctx, int ncol, const double *Y, long ldy, const double
     const int ksteps = (ncol + TK - 1) / TK, nqb = x_row_blocks(ncol);
     const size_t blk_bytes = sizeof(__nv_bfloat16) * (size_t)ksteps * XS * (TM / 8) * XG;
     const long blocks = (Nd + TM - 1) / TM;
-    const long per = std::max<long>(1, std::min<long>(blocks, (long)(kXOperand / blk_bytes)));
+    const long per = std::max<long>(1, std::min<long>(blocks, (long)(scratch_max(ctx) / blk_bytes)));
     char *wa = nullptr, *wb = nullptr;
     const size_t qbytes = sizeof(__nv_bfloat16) * (size_t)ksteps * XS * nqb * (TM / 8) * XG;
     SGPU_TRY(ws_get(ctx, WS_SPLIT_A, blk_bytes * per + sizeof(int) * ((size_t)per * TM + 64),

@@ -224,3 +224,27 @@ def test_sets_without_tables(gpu_available):
             _close(Yb.cpu().numpy(), o.chebyshev_kpt(k, L, coords, s * v, 4, 0.5, 40.0, -0.8, z)[1])
         _set(ctx, v, nl, 1)
     ctx.close()
+
+
+def test_rr_products_in_many_passes(gpu_available):
+    """Slices held to 1 MB: 43 ranges of 512 points, whose sums take no more room than one range's."""
+    import torch
+    N, ncol = (30, 28, 26), 200
+    ctx, v, nl, grid, rng = _system(N, 0.4, natom=0)
+    Y = torch.from_numpy(rng.uniform(-1, 1, (ncol, ctx.Nd))).cuda()
+    Q = torch.from_numpy(rng.normal(size=(ncol, ncol))).cuda()
+    HY, X, Hp, Mp = torch.empty_like(Y), torch.empty_like(Y), torch.empty_like(Q), torch.empty_like(Q)
+    ctx.inject_failure(SMALL)
+    ctx.Project_Hamiltonian(Y[:64], HY[:64], Hp[:64, :64].contiguous(), Mp[:64, :64].contiguous())
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    ctx.Project_Hamiltonian(Y, HY, Hp, Mp)
+    ctx.Subspace_Rotation(Y, Q, X)
+    torch.cuda.synchronize()
+    # two operands of 2 MB (the least range), one set of 200 x 200 sums, an eighth of slack each
+    assert free - torch.cuda.mem_get_info()[0] < 16 << 20
+    y, hy = Y.cpu().numpy(), HY.cpu().numpy()
+    _close(Mp.cpu().numpy(), y @ y.T)
+    _close(Hp.cpu().numpy(), y @ hy.T)
+    _close(X.cpu().numpy(), Q.cpu().numpy() @ y)
+    ctx.close()

@@ -4,22 +4,26 @@
 // point (the scale s1 and the recurrence term).
 //
 // A block owns a TX x TY tile of an xy-plane for one column and marches along z; a thread owns
-// two x-neighbouring points. Digits of the planes k-6 .. k+7 sit in a register queue (14 slots,
-// the z-loop unrolled by 14 so the queue rotates by renaming), digits of the current plane and
-// its halo in one of two shared-memory buffers, one barrier per plane. In the step of plane k
-// the block converts plane k+1's halo and plane k+7's centre, which the previous step loaded,
-// and loads the next ones; the largest exponent of what was loaded goes through shared memory
-// one step ahead, so every thread knows before it converts whether the block scale still covers
-// it. A larger value restarts the march at that plane with a new scale (the window's largest
-// value, so the scale follows the data along z); values that the fixed-point range does not
-// cover (infinities, NaN, extreme exponents) send the rest of the slab through the FP64 path.
+// two x-neighbouring points. Digits of the planes k-6 .. k+8 sit in a register queue (15 slots,
+// shifted by two every second plane), digits of the current plane and its halo in one of two
+// shared-memory buffers, one barrier per plane. In the step of plane k the block converts plane
+// k+1's halo and plane k+7's centre, which the previous step loaded, and loads the next ones; the
+// largest exponent of what was loaded goes through the barrier one step ahead, so every thread
+// knows before it converts whether the block scale still covers it. A larger value restarts the
+// march at that plane with a new scale, the window's largest value, and so does a window without a
+// value within 2^-4 of the scale: the scale follows the data along z both ways. (With a scale that
+// only grew, a column that falls off into a vacuum was rounded to 2^-57 of its largest value
+// everywhere: after 85 planes of exp(-0.35) that is 1e-5 of the values there.) Values that the
+// fixed-point range does not cover (infinities, NaN, extreme exponents) send the rest of the slab through the
+// FP64 path.
 //
 // What bounds it: instruction issue (61 % of the slots busy, 60 % of the integer multiply pipe, 59 %
 // of the shared-memory wavefronts, HBM 29 %). Per point about 36 integer adds, 24 wide
 // multiply-adds and 7 high products (60 and 19 with three spacings), 21 instructions per converted
 // value (2.5 of them on a 16 x 16 tile) and 40 for the way back, against 42 FP64 instructions at
-// two lanes per clock in k_stencil_orth. 96^3, 512 columns: 37.3 -> 5.29 ms per launch (4.75 with
-// coefficients of two digits, whose rounding cost a filter its accuracy).
+// two lanes per clock in k_stencil_orth. 96^3, 512 columns: 37.3 -> 5.44 ms per launch (5.29 without
+// the lowering of the scale; 4.75 with coefficients of two digits as well, whose rounding cost a
+// filter its accuracy; the shares above were taken at 4.75).
 #pragma once
 
 #include <algorithm>
@@ -55,7 +59,7 @@ struct StencilFxParams {
 constexpr int kFxTile = 32;                        // largest tile edge
 constexpr int kFxPitch = kFxTile + 2 * kMaxFDn;    // shared-memory row (points), 8 bytes each
 constexpr int kFxThreads = 512;
-constexpr int kFxUnroll = 2; static_assert(kFxUnroll == 2 || kFxUnroll == 4, "step pairs");                      // planes between two shifts of the queue
+constexpr int kFxUnroll = 2;                       // planes between two shifts of the queue
 
 // planes k .. ze-1 of a block's tile in FP64, straight from global memory
 __device__ __noinline__ void stencil_fx_slow(const StencilFxParams &p, const double *xc,
@@ -106,8 +110,16 @@ struct FxState {
     int E, k;
     unsigned pk;               // byte offset of plane k
     unsigned pc;               // byte offset of the next centre plane to load (wrapped)
-    bool over;                 // a value loaded ahead exceeds the block scale
+    bool over;                 // the scale has to change: a value loaded ahead exceeds it, or none is near
 };
+
+// A block's scale is lowered when its window holds no value within 2^-kFxNear of it any more. Every
+// second plane a thread that has just loaded such a value notes the plane in one of two slots, in
+// turn, and all read the slot of two planes before: more than kFxQuiet planes without a note there
+// restart the march, with the scale of a window that has left the noted planes behind. (A note of
+// every plane, in the steps themselves, took 5.67 ms where this takes 5.44 and none 5.29.)
+constexpr unsigned kFxNear = 4;
+constexpr int kFxQuiet = 14;
 
 // NS: halo values per thread. CUBE: equal weights in the three directions, so the six neighbours
 // at one distance are added before the multiplication (24 wide multiply-adds per point, not 60).
@@ -117,6 +129,7 @@ __global__ void __launch_bounds__(kFxThreads, 1) k_stencil_fx(const StencilFxPar
     constexpr int R = kMaxFDn, P = kFxPitch;
     extern __shared__ __align__(16) unsigned char fx_smem[];
     __shared__ unsigned s_key;
+    __shared__ int s_near[2];
     const int t = threadIdx.x, nthr = blockDim.x;
     const int TXP = p.TX >> 1;
     const int ty = min(t / TXP, p.TY - 1), tx = t % TXP;
@@ -269,15 +282,16 @@ __global__ void __launch_bounds__(kFxThreads, 1) k_stencil_fx(const StencilFxPar
         char *ob = reinterpret_cast<char *>(oc);
         if (act0) *reinterpret_cast<double *>(ob + (pk + o0)) = y0v;
         if (act1) *reinterpret_cast<double *>(ob + (pk + o1)) = y1v;
+        // what was loaded in this step against the scale
+        S.over = (key_of_loaded() >> 20) > (unsigned)S.E;
         S.k++;
         S.pk = pk + plane;
-        S.over = (key_of_loaded() >> 20) > (unsigned)S.E;
         return go_on;
     };
 
     while (S.k < ze) {
         // ---- (re)start at plane k: centres of planes k-6 .. k+6, halo of plane k, scale
-        __syncthreads();  // the previous march's readers of the buffers and of s_key are done
+        __syncthreads();  // the previous march's readers of the buffers, of s_key and s_near are done
         if (t == 0) s_key = 0u;
         double w0[2 * R + 1], w1[2 * R + 1];
         unsigned key = 0u;
@@ -311,6 +325,7 @@ __global__ void __launch_bounds__(kFxThreads, 1) k_stencil_fx(const StencilFxPar
             return;
         }
         S.E = max(S.E, fx::kMinExp);
+        if (t < 2) s_near[t] = S.E == fx::kMinExp ? 1 << 30 : S.k;
 #pragma unroll
         for (int m = 0; m <= 2 * R; m++) {
             const int2 a = fx::to_digits(w0[m], S.E), b = fx::to_digits(w1[m], S.E);
@@ -326,12 +341,10 @@ __global__ void __launch_bounds__(kFxThreads, 1) k_stencil_fx(const StencilFxPar
         while (true) {
             if (!step(std::integral_constant<int, 0>{}, s0, s0 + bufsz)) break;
             if (!step(std::integral_constant<int, 1>{}, s0 + bufsz, s0)) break;
-            if constexpr (kFxUnroll == 4) {
-                if (!step(std::integral_constant<int, 2>{}, s0, s0 + bufsz)) break;
-                if (!step(std::integral_constant<int, 3>{}, s0 + bufsz, s0)) break;
-            }
 #pragma unroll
             for (int m = 0; m <= 2 * R; m++) S.q[m] = S.q[m + kFxUnroll];
+            S.over |= S.k - s_near[((S.k >> 1) & 1) ^ 1] > kFxQuiet;
+            if ((key_of_loaded() >> 20) + kFxNear >= (unsigned)S.E) s_near[(S.k >> 1) & 1] = S.k;
         }
     }
 }

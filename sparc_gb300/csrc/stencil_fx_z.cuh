@@ -6,7 +6,7 @@
 // What bounds it: latency at the 15 warps that 128 registers leave (46 % of the issue slots busy, the
 // FP64 pipe, which has the output scale, the recurrence term and the factors, 37 %; with the
 // factors as selects on every value it was the bound at 75 %, and 2.9 ms). 34^3, 20 blocks of 64
-// columns: 12.6 ms per degree in k_stencil_zb<double2>, 2.03 here.
+// columns: 12.6 ms per degree in k_stencil_zb<double2>, 2.05 here.
 #pragma once
 
 #include "stencil_fx.cuh"
@@ -104,6 +104,7 @@ __device__ __forceinline__ void stencil_fxz(const FxZConst &p, const FxZCol &c, 
 {
     constexpr int R = kMaxFDn, P = kFxZPitch;
     __shared__ unsigned s_key;
+    __shared__ int s_near[2];                       // as in stencil_fx.cuh
     __shared__ double2 s_f[27];                     // factors of the shifts, index 9 dz' + 3 dy' + dx'
     const int t = threadIdx.x, nthr = blockDim.x;
     const int ty = min(t / p.TX, p.TY - 1), tx = t % p.TX;
@@ -297,6 +298,7 @@ __device__ __forceinline__ void stencil_fxz(const FxZConst &p, const FxZCol &c, 
             return;
         }
         E = max(E, fx::kMinExp);
+        if (t < 2) s_near[t] = E == fx::kMinExp ? 1 << 30 : k;
 #pragma unroll
         for (int m = 0; m <= 2 * R; m++) q[m] = dig(w[m]);
         if (own) s0[sc] = q[R];
@@ -313,6 +315,8 @@ __device__ __forceinline__ void stencil_fxz(const FxZConst &p, const FxZCol &c, 
             if (!step(std::integral_constant<int, 1>{}, s0 + bufsz, s0)) break;
 #pragma unroll
             for (int m = 0; m <= 2 * R; m++) q[m] = q[m + kFxUnroll];
+            over |= k - s_near[((k >> 1) & 1) ^ 1] > kFxQuiet;
+            if ((key_of_loaded() >> 20) + kFxNear >= (unsigned)E) s_near[(k >> 1) & 1] = k;
         }
     }
 }

@@ -248,3 +248,45 @@ def test_rr_products_in_many_passes(gpu_available):
     _close(Hp.cpu().numpy(), y @ hy.T)
     _close(X.cpu().numpy(), Q.cpu().numpy() @ y)
     ctx.close()
+
+
+@pytest.mark.parametrize("N", [(18, 14, 170), (33, 30, 130)])
+@pytest.mark.parametrize("ncol", [4, 300])
+@pytest.mark.parametrize("bloch", [False, True])
+def test_columns_that_decay(gpu_available, N, ncol, bloch):
+    """A slab's states fall off into the vacuum, here by exp(-0.35) a plane and by 1e-10 and more in
+    all, and rise again behind it. A block's scale is below 2^5 of the largest value that it loaded in
+    its last 14 steps, planes at most 14 away, and values are rounded to 2^-57 of the scale: a
+    result is off by at most 40 units of 2^-53 of the sum of |coefficient| (as many again for the
+    parts of a complex value) times the largest value of the planes up to 16 away."""
+    h, dz = 0.4, 16
+    rng = np.random.default_rng(sum(N) + ncol)
+    c = fd_d2_coeffs(6, h)
+    Nd, per = N[0] * N[1] * N[2], N[0] * N[1]
+    ctx = sg.Context(*N, 6, c, c, c, h ** 3)
+    z = np.arange(N[2])
+    d = np.minimum((z - 20) % N[2], (20 - z) % N[2])
+    prof = np.exp(-0.35 * d)
+    some = rng.choice(ncol, 3)
+    x = rng.uniform(-1, 1, (ncol, Nd)) * np.repeat(prof, per)
+    S = 1.5 * (abs(c[0]) + 2 * np.abs(c[1:]).sum()) + 0.7
+    near = np.max([np.roll(prof, s) for s in range(-dz, dz + 1)], axis=0)
+    tol = 40 * 2.0 ** -53 * S * np.repeat(near, per)
+    ld = np.longdouble
+    if bloch:
+        ctx.set_kpoint_geometry(np.array(N) * h, np.zeros((0, 3)))
+        x = x + 1j * rng.uniform(-1, 1, (ncol, Nd)) * np.repeat(prof, per)
+        y = np.zeros_like(x)
+        ctx.Lap_plus_diag_vec_mult_orth_kpt(np.zeros(3), -0.5, 0.0, 0.7, None, x, y)
+        tol = 2 * tol
+    else:
+        y = np.zeros_like(x)
+        ctx.Lap_plus_diag_vec_mult_orth(-0.5, 0.0, 0.7, None, x, y)
+    for n in some:
+        u = x[n].reshape(N[::-1]).astype(np.clongdouble if bloch else ld)
+        r = (ld(-0.5) * 3 * ld(c[0]) + ld(0.7)) * u
+        for ax in range(3):
+            for q in range(1, 7):
+                r = r + ld(-0.5) * ld(c[q]) * (np.roll(u, q, ax) + np.roll(u, -q, ax))
+        assert np.all(np.abs(y[n] - r.reshape(-1)) <= tol)
+    ctx.close()

@@ -104,3 +104,69 @@ def test_nonfinite_blocks_follow_the_fp64_gemm(gpu_available):
     ref = (Q @ np.nan_to_num(Y, nan=0.0, posinf=0.0))[:, pts]
     assert np.abs(X[:, pts] - ref).max() <= 1e-12 * np.abs(ref).max()
     ctx.close()
+
+
+def _exact_dot(a, b):
+    """The dot product of two FP64 vectors, rounded once: every product split into two exact parts
+    (Veltkamp, Dekker), all parts added by math.fsum."""
+    import math
+
+    def split(x):
+        c = 134217729.0 * x
+        hi = c - (c - x)
+        return hi, x - hi
+
+    p = a * b
+    (ah, al), (bh, bl) = split(a), split(b)
+    e = ((ah * bh - p) + ah * bl + al * bh) + al * bl
+    return math.fsum(np.concatenate([p, e]))
+
+
+def test_products_of_a_large_block_are_closer_than_the_fp64_gemm(gpu_available):
+    """77^3 points, 520 columns over four decades: Gram entries and rotated values against exact dot
+    products. The eight-slice form is off by less than DSYRK and DGEMM are, at worst and on
+    average, and by at most 4 units of 2^-53 of the factors' norms."""
+    import torch
+    N, ncol = (77, 77, 77), 520
+    ctx = _ctx(N)
+    Nd = 77 ** 3
+    g = torch.Generator(device="cuda")
+    g.manual_seed(8)
+    Y = torch.rand((ncol, Nd), generator=g, device="cuda", dtype=torch.float64) - 0.5
+    s = 10.0 ** (4 * torch.rand((ncol, 1), generator=g, device="cuda", dtype=torch.float64) - 2)
+    Y *= s
+    Q = (torch.rand((ncol, ncol), generator=g, device="cuda", dtype=torch.float64) - 0.5) / s.T
+    HY, X = torch.empty_like(Y), torch.empty_like(Y)
+    Hp, Mp = torch.empty_like(Q), torch.empty_like(Q)
+    rng = np.random.default_rng(9)
+    pairs = [(i, i) for i in rng.integers(0, ncol, 6)] + [tuple(p) for p in rng.integers(0, ncol, (14, 2))]
+    spots = [(int(n), int(p)) for n, p in zip(rng.integers(0, ncol, 200), rng.integers(0, Nd, 200))]
+    err, exact = {}, None
+    for mode in (1, 0):
+        ctx.set_rr_products(mode)
+        ctx.Project_Hamiltonian(Y, HY, Hp, Mp)
+        ctx.Subspace_Rotation(Y, Q, X)
+        if exact is None:
+            y = {i: Y[i].cpu().numpy() for p in pairs for i in p}
+            h = {i: HY[i].cpu().numpy() for p in pairs for i in p}
+            yp = {p: Y[:, p].cpu().numpy() for _, p in spots}
+            q = Q.cpu().numpy()
+            exact = ([_exact_dot(y[i], y[j]) for i, j in pairs],
+                     [_exact_dot(y[min(p)], h[max(p)]) for p in pairs],
+                     [_exact_dot(q[n], yp[p]) for n, p in spots])
+            norm = ([np.linalg.norm(y[i]) * np.linalg.norm(y[j]) for i, j in pairs],
+                    [np.linalg.norm(y[min(p)]) * np.linalg.norm(h[max(p)]) for p in pairs],
+                    [np.linalg.norm(q[n] * s[:, 0].cpu().numpy()) *
+                     np.linalg.norm(yp[p] / s[:, 0].cpu().numpy()) for n, p in spots])
+        m, hp = Mp.cpu().numpy(), Hp.cpu().numpy()
+        # the upper triangle of Yᵀ HY: row the smaller, column the larger index (column-major)
+        val = ([m[i, j] for i, j in pairs], [hp[max(p), min(p)] for p in pairs],
+               [float(X[n, p]) for n, p in spots])
+        err[mode] = [np.abs(np.array(v) - np.array(x)) / np.array(w)
+                     for v, x, w in zip(val, exact, norm)]
+    ctx.close()
+    print("errors (worst, mean) of Mp, Hp, X:",
+          {k: [(float(e.max()), float(e.mean())) for e in v] for k, v in err.items()})
+    for tc, gemm in zip(err[1], err[0]):
+        assert tc.max() <= gemm.max() and tc.mean() <= gemm.mean()
+        assert tc.max() <= 4 * 2.0 ** -53

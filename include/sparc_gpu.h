@@ -624,13 +624,32 @@ int sgpu_set_gemm_emulation(sgpu_ctx *ctx, int mode);
  * mixed SCF's FP32 phase) and FP64-accurate (6 slices, 21 products) for the mixed SCF's FP64
  * phase after the switch; plain FP64 calls (sgpu_Project_Hamiltonian,
  * sgpu_Subspace_Rotation, the plain FP64 SCF) use 8 slices (36 products; every level summed
- * apart, closer to the exact products than cuBLAS DSYRK/DGEMM), except rotations of fewer than
- * 48 columns and blocks with infinities or NaN, which go to cuBLAS.
+ * apart): values to 56 bits of the largest of their column (of their row, for the rotation),
+ * closer to the exact products than cuBLAS DSYRK/DGEMM in the norms of the factors (77^3 x 520:
+ * 3e-16 and 4e-14 at worst). Rotations of fewer than 48 columns, blocks with infinities or NaN
+ * and calls without room for the slices go to cuBLAS.
  * mode 2: the 6-slice products for the plain FP64 calls too.
  * mode 0: cuBLAS everywhere (sgpu_set_gemm_emulation then picks the FP32-block form).
  * The Gram products compute the upper triangle and mirror it. No counterpart in the
  * reference (which calls cblas_dgemm). */
 int sgpu_set_rr_products(sgpu_ctx *ctx, int mode);
+
+/* FP64 and complex128 stencil and nonlocal products: 1 (default) in block fixed point, several
+ * times faster on this part; 0 in FP64 arithmetic throughout. Fixed point rounds to 57 bits of the
+ * largest value of a block: for the stencil the values of a tile of at most 32 x 32 points and of
+ * the planes that its stencil reaches, and the potential and the coefficients against the sum of
+ * the coefficients; for the nonlocal products a column's values and projections over a range of
+ * 128 neighbouring points, and a projector row's Chi values. In the norm of such a block a product
+ * is at least as accurate as in FP64. A value 2^-k of its block's largest keeps 57 - k bits, so a
+ * column that falls off within a few points may be off by more than in FP64 far from its centre:
+ * filters of degree 20 with projectors, in the norm of a column, are at 0.6 to 0.9 of the error of
+ * the FP64 kernels for uniform and for smooth columns, at 1.0 to 2.0 for columns that fall off by
+ * exp(-0.9 r) (Bohr) from a point. Tiles and ranges depend on the number of columns, and with
+ * them the last bits of a column. Potentials above 16 times the largest power of two in the sum
+ * of the coefficients (a launch then takes 7 times as long), more than 18 projectors per atom and
+ * values outside about 1e-230 .. 1e230 take the FP64 kernels with either. The Rayleigh-Ritz
+ * products have sgpu_set_rr_products. */
+int sgpu_set_fixed_point(sgpu_ctx *ctx, int on);
 
 /* complex64 stencil form: 1 (default) tiles with packed FP32 arithmetic and a per-k table of
  * Bloch factors; 0 the general kernel, which also serves grids whose tiles would reach a whole

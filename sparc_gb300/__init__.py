@@ -44,7 +44,7 @@ EXPORTED = [
     "sgpu_kernel_status", "sgpu_check_wait_bound", "sgpu_set_nonlocal_fuse",
     "sgpu_get_nonlocal_fuse", "sgpu_get_nonlocal_fuse_tc", "sgpu_ChebyshevFiltering_y", "sgpu_Project_Hamiltonian_f32",
     "sgpu_Subspace_Rotation_f32", "sgpu_set_gemm_emulation", "sgpu_measure_fp64_rate",
-    "sgpu_set_rr_products", "sgpu_set_eig_solver", "sgpu_inject_failure", "sgpu_Project_Hamiltonian_kpt",
+    "sgpu_set_rr_products", "sgpu_set_eig_solver", "sgpu_inject_failure", "sgpu_set_fixed_point", "sgpu_Project_Hamiltonian_kpt",
     "sgpu_Solve_Generalized_EigenProblem_kpt", "sgpu_Subspace_Rotation_kpt", "sgpu_CheFSI_batched",
 ]
 
@@ -780,6 +780,11 @@ class Context:
         st = ctypes.c_int()
         _check(lib().sgpu_check_wait_bound(self._h, ctypes.byref(st)))
         return int(st.value)
+
+    def set_fixed_point(self, on):
+        """FP64 and complex128 stencil and nonlocal products in block fixed point (True, the
+        default) or in FP64 arithmetic throughout (sgpu_set_fixed_point)."""
+        _check(lib().sgpu_set_fixed_point(self._h, int(bool(on))))
 
     def inject_failure(self, mask):
         """Failures made on the host, for tests (sgpu_inject_failure): 1 optional scratch, 2 the

@@ -702,6 +702,17 @@ int sgpu_check_wait_bound(sgpu_ctx *ctx, int *status)
     return SGPU_ERR_STATE;
 }
 
+int sgpu_set_fixed_point(sgpu_ctx *ctx, int on)
+{
+    SGPU_TRY(check_ctx(ctx));
+    if (on != 0 && on != 1) {
+        set_error("sgpu_set_fixed_point: on must be 0 or 1");
+        return SGPU_ERR_ARG;
+    }
+    ctx->fx_on = on;
+    return SGPU_OK;
+}
+
 int sgpu_inject_failure(sgpu_ctx *ctx, int mask)
 {
     SGPU_TRY(check_ctx(ctx));

@@ -844,7 +844,7 @@ struct FxZLaunch {
 static bool fxz_launch(const sgpu_ctx *ctx, const double (&w)[3][kMaxFDn], double c0, unsigned vkey,
                        long ncol, FxZLaunch *L)
 {
-    if (ctx->Nd >= (1L << 27)) return false;
+    if (!ctx->fx_on || ctx->Nd >= (1L << 27)) return false;
     StencilFxParams d{};
     d.c0 = c0;
     d.s1 = 1.0;
@@ -945,7 +945,7 @@ static int stencil_z(sgpu_ctx *ctx, const double *k, int ncol, double a, double 
             w[2][r] = p.wz[r + 1];
         }
         // (the kernel's own FP64 path takes bv = 1)
-        bool can = !p.v || bv == 1.0;
+        bool can = ctx->fx_on && (!p.v || bv == 1.0);
         FxPot own{};
         if (can && p.v && !pot) {  // a caller's potential: its digits for this call
             char *ws = nullptr;

@@ -126,7 +126,10 @@ const NlFx &nonlocal_fx_pick(const Nonlocal &nl, long groups)
     return nl.fx[1].nrange > 0 && nl.fx[0].nrange * groups < 304 ? nl.fx[1] : nl.fx[0];
 }
 
-bool nonlocal_fx_ready(const sgpu_ctx *ctx) { return ctx->has_nl && ctx->nl.fx[0].nrange > 0; }
+bool nonlocal_fx_ready(const sgpu_ctx *ctx)
+{
+    return ctx->fx_on && ctx->has_nl && ctx->nl.fx[0].nrange > 0;
+}
 
 void nonlocal_fx_free(Nonlocal &nl)
 {

@@ -185,6 +185,8 @@ struct sgpu_ctx {
     unsigned veff_key = 0;
     sgpu::Nonlocal nl;
     bool has_nl = false;
+    int fx_on = 1;             // FP64 stencil and nonlocal products in block fixed point
+                               // (sgpu_set_fixed_point)
     int inject = 0;            // failures that a test asks for (sgpu_inject_failure)
     long set_count = 0;        // calls that changed the nonlocal set or the grid's numbers; captured
                                // launches hold those by value and pointer and are dropped with them

@@ -1204,7 +1204,7 @@ int launch_stencil(sgpu_ctx *ctx, int ncol, double a, double bv, double c, const
             return SGPU_OK;
         }
         bool done = false;
-        if (fixed) SGPU_TRY(launch_stencil_fx(ctx, ncol, p, pot, &done, st));
+        if (fixed && ctx->fx_on) SGPU_TRY(launch_stencil_fx(ctx, ncol, p, pot, &done, st));
         if (done) return SGPU_OK;
     }
 

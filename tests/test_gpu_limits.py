@@ -290,3 +290,37 @@ def test_columns_that_decay(gpu_available, N, ncol, bloch):
                 r = r + ld(-0.5) * ld(c[q]) * (np.roll(u, q, ax) + np.roll(u, -q, ax))
         assert np.all(np.abs(y[n] - r.reshape(-1)) <= tol)
     ctx.close()
+
+
+@pytest.mark.parametrize("ncol", [3, 300])
+def test_fp64_arithmetic_on_request(gpu_available, ncol):
+    """set_fixed_point(False): every point is as accurate as the values that its own stencil or
+    projectors touch, 40 units of 2^-53 of the sum of |coefficient| times the largest value of six
+    planes around, and n units of the products' magnitudes at the point itself (n: points of a
+    sphere and rows over a point). Columns fall off along z."""
+    N, h = (18, 14, 90), 0.4
+    ctx, v, nl, grid, rng = _system(N, h, natom=7, rc=2.2)
+    ctx.set_fixed_point(False)
+    Nd, per, c = ctx.Nd, N[0] * N[1], grid["cx"]
+    z = np.arange(N[2])
+    prof = np.exp(-0.35 * np.minimum((z - 20) % N[2], (20 - z) % N[2]))
+    near = np.repeat(np.max([np.roll(prof, s) for s in range(-6, 7)], axis=0), per)
+    x = rng.uniform(-1, 1, (ncol, Nd)) * np.repeat(prof, per)
+    S = 1.5 * (abs(c[0]) + 2 * np.abs(c[1:]).sum()) + 0.7
+    y = np.zeros_like(x)
+    ctx.Lap_plus_diag_vec_mult_orth(-0.5, 0.0, 0.7, None, x, y)
+    some = rng.choice(ncol, 2)
+    lap = Oracle(grid, None).lap_plus_diag(-0.5, 0.0, 0.7, None, x[some])
+    assert np.all(np.abs(y[some] - lap) <= 40 * 2.0 ** -53 * S * near)
+    ctx.set_kpoint_geometry(np.array(N) * h, np.zeros((len(nl["img_atom"]), 3)))
+    w = np.zeros_like(x, dtype=complex)
+    ctx.Lap_plus_diag_vec_mult_orth_kpt(np.zeros(3), -0.5, 0.0, 0.7, None, x.astype(complex), w)
+    assert np.all(np.abs(w[some] - lap) <= 80 * 2.0 ** -53 * S * near)
+    y[:] = 0.0
+    ctx.Vnl_vec_mult(x, y)
+    size = Oracle(grid, dict(nl, chi=np.abs(nl["chi"]), gamma=np.abs(nl["gamma"]))).vnl(np.abs(x[some]))
+    n = nl["img_ndc"].max() + np.bincount(nl["grid_pos"], minlength=Nd).max() * 9
+    assert np.all(np.abs(y[some] - Oracle(grid, nl).vnl(x[some])) <= n * 2.0 ** -53 * size)
+    with pytest.raises(sg.SgpuError):
+        sg._check(sg.lib().sgpu_set_fixed_point(ctx._h, 2))
+    ctx.close()

@@ -2,7 +2,8 @@
 // (the kernel body is in nonlocal_fx.cuh).
 #include <algorithm>
 #include <cmath>
-#include <type_traits>
+#include <cstring>
+#include <string>
 #include <vector>
 
 #include "nonlocal_fx.cuh"
@@ -134,10 +135,7 @@ bool nonlocal_fx_ready(const sgpu_ctx *ctx)
 void nonlocal_fx_free(Nonlocal &nl)
 {
     for (NlFx &x : nl.fx) {
-        void *ptrs[] = {x.pt0, x.pts, x.item0, x.ent0, x.wsplit, x.items, x.rows, x.lp, x.chi, x.row0,
-                        x.sum_ptr, x.sum_idx};
-        for (void *p : ptrs)
-            if (p) cudaFree(p);
+        if (x.mem) cudaFree(x.mem);
         x = NlFx();
     }
 }
@@ -281,49 +279,71 @@ static int build_ranges(Nonlocal &nl, NlFx &x, int cap, bool fail, const std::ve
                 for (int j = 0; j < items[i].z; j++)
                     sum_idx[at[items[i].y + j]++] = row0[r] + items[i].x + j;
     }
-    int rc = SGPU_OK;
-    auto up = [&](auto **dst, const auto &v) {
-        using T = std::remove_reference_t<decltype(v[0])>;
-        if (rc != SGPU_OK) return;
-        const size_t n = fail ? (size_t)1 << 60 : sizeof(T) * std::max<size_t>(v.size(), 1);
-        if (cudaMalloc((void **)dst, n) != cudaSuccess) {
-            rc = SGPU_ERR_NOMEM;
-        } else if (!v.empty() && cudaMemcpy((void *)*dst, v.data(), sizeof(T) * v.size(),
-                                            cudaMemcpyHostToDevice) != cudaSuccess) {
-            set_error("set_nonlocal: copy of the fixed-point range tables failed");
-            rc = SGPU_ERR_CUDA;
-        }
+    // one allocation for the tables, another for what the Chi kernel reads
+    struct Put {
+        void **dst;
+        const void *src;
+        size_t at, bytes;
+    };
+    std::vector<Put> put;
+    size_t size = 0, tsize = 0;
+    auto table = [&](auto **dst, const auto &v, size_t &to) {
+        const size_t at = (to + 255) / 256 * 256;
+        to = at + sizeof(v[0]) * v.size();
+        put.push_back({(void **)dst, v.data(), at, to - at});
     };
     long2 *dsrc = nullptr;
     int2 *drows = nullptr;
-    up(&x.pt0, pt0);
-    up(&x.pts, pts);
-    up(&x.item0, item0);
-    up(&x.items, items);
-    up(&x.ent0, ent0);
-    up(&x.wsplit, wsplit);
-    up(&x.lp, lp);
-    up(&x.rows, rowinfo);
-    up(&x.row0, row0);
-    up(&x.sum_ptr, sum_ptr);
-    up(&x.sum_idx, sum_idx);
-    up(&dsrc, src);
-    up(&drows, rows);
-    const size_t cbytes = sizeof(int2) * (size_t)nl.nent * nl.fx_jp;
-    if (rc == SGPU_OK && cudaMalloc((void **)&x.chi, cbytes) != cudaSuccess)
+    table(&dsrc, src, tsize);
+    table(&drows, rows, tsize);
+    table(&x.pt0, pt0, size);
+    table(&x.pts, pts, size);
+    table(&x.item0, item0, size);
+    table(&x.items, items, size);
+    table(&x.ent0, ent0, size);
+    table(&x.wsplit, wsplit, size);
+    table(&x.lp, lp, size);
+    table(&x.rows, rowinfo, size);
+    table(&x.row0, row0, size);
+    table(&x.sum_ptr, sum_ptr, size);
+    table(&x.sum_idx, sum_idx, size);
+    const size_t ochi = (size + 255) / 256 * 256;
+    const size_t bytes = ochi + sizeof(int2) * (size_t)nl.nent * nl.fx_jp;
+    char *base = nullptr, *temp = nullptr;
+    int rc = SGPU_OK;
+    if (cudaMalloc(&base, fail ? (size_t)1 << 60 : bytes) != cudaSuccess ||
+        cudaMalloc(&temp, tsize) != cudaSuccess) {
         rc = SGPU_ERR_NOMEM;
-    if (rc == SGPU_OK) {
-        k_fx_chi<<<152 * 8, 256>>>(dsrc, drows, nl.nent, nl.fx_jp, nl.chi64, nl.fx_er,
-                                   reinterpret_cast<int2 *>(x.chi));
-        if (cudaDeviceSynchronize() != cudaSuccess) {
-            set_error("set_nonlocal: the Chi digit kernel failed");
+    } else {
+        // small tables in one copy (a copy takes about 10 us), large ones from where they are
+        cudaError_t e = cudaSuccess;
+        std::vector<char> host(size < ((size_t)4 << 20) ? size : 0);
+        for (size_t p = 0; p < put.size() && e == cudaSuccess; p++) {
+            const Put &q = put[p];
+            *q.dst = (p < 2 ? temp : base) + q.at;
+            if (p >= 2 && !host.empty()) std::memcpy(host.data() + q.at, q.src, q.bytes);
+            else e = cudaMemcpy(*q.dst, q.src, q.bytes, cudaMemcpyHostToDevice);
+        }
+        if (e == cudaSuccess && !host.empty()) e = cudaMemcpy(base, host.data(), size, cudaMemcpyHostToDevice);
+        x.chi = reinterpret_cast<int4 *>(base + ochi);
+        if (e == cudaSuccess) {
+            k_fx_chi<<<152 * 8, 256>>>(dsrc, drows, nl.nent, nl.fx_jp, nl.chi64, nl.fx_er,
+                                       reinterpret_cast<int2 *>(x.chi));
+            e = cudaDeviceSynchronize();
+        }
+        if (e != cudaSuccess) {
+            set_error(std::string("set_nonlocal: the fixed-point tables: ") + cudaGetErrorString(e));
             rc = SGPU_ERR_CUDA;
         }
     }
-    if (dsrc) cudaFree(dsrc);
-    if (drows) cudaFree(drows);
-    if (rc == SGPU_OK) x.nrange = (int)pt0.size() - 1;
-    return rc;
+    if (temp) cudaFree(temp);
+    if (rc != SGPU_OK) {
+        if (base) cudaFree(base);
+        return rc;
+    }
+    x.mem = base;
+    x.nrange = (int)pt0.size() - 1;
+    return SGPU_OK;
 }
 
 

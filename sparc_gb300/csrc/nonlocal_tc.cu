@@ -434,18 +434,20 @@ int launch_nonlocal_apply_project_tc(sgpu_ctx *ctx, int ncol, const float *alpha
 constexpr int kTcBx = 32, kTcBy = 4, kTcBz = 4;
 std::vector<int> compact_order(int Nx, int Ny, const std::vector<int> &covpts)
 {
+    // covpts ascend, and so do a block's points in its own (z, y, x) order: counting by block keeps it
     const long nbx = (Nx + kTcBx - 1) / kTcBx, nby = (Ny + kTcBy - 1) / kTcBy;
-    std::vector<std::pair<long long, int>> key(covpts.size());
-    for (size_t c = 0; c < covpts.size(); c++) {
-        const long g = covpts[c];
+    auto block = [&](long g) {
         const long x = g % Nx, y = (g / Nx) % Ny, z = g / ((long)Nx * Ny);
-        const long blk = ((z / kTcBz) * nby + y / kTcBy) * nbx + x / kTcBx;
-        const long in = ((z % kTcBz) * kTcBy + y % kTcBy) * kTcBx + x % kTcBx;
-        key[c] = {(long long)blk * (kTcBx * kTcBy * kTcBz) + in, (int)c};
+        return ((z / kTcBz) * nby + y / kTcBy) * nbx + x / kTcBx;
+    };
+    std::vector<int> blk(covpts.size()), ord(covpts.size()), at(1, 0);
+    for (size_t c = 0; c < covpts.size(); c++) {
+        blk[c] = (int)block(covpts[c]);
+        if (blk[c] + 2 > (int)at.size()) at.resize(blk[c] + 2, 0);
+        at[blk[c] + 1]++;
     }
-    std::sort(key.begin(), key.end());
-    std::vector<int> ord(covpts.size());
-    for (size_t c = 0; c < ord.size(); c++) ord[c] = key[c].second;
+    for (size_t b = 1; b < at.size(); b++) at[b] += at[b - 1];
+    for (size_t c = 0; c < covpts.size(); c++) ord[at[blk[c]]++] = (int)c;
     return ord;
 }
 int nonlocal_tc_build(Nonlocal &nl, const std::vector<int> &ord, const std::vector<int> &covpts,

@@ -65,6 +65,7 @@ struct NlFx {
     int4 *chi = nullptr;
     int *row0 = nullptr;
     int *sum_ptr = nullptr, *sum_idx = nullptr;  // projector row -> its partial rows
+    void *mem = nullptr;  // the one allocation that holds them all
 };
 
 struct Nonlocal {

@@ -1060,7 +1060,7 @@ static int nonlocal_z(sgpu_ctx *ctx, int ncol, const CT *x, long ldx, CT *out, l
             const int groups = (ncol + FG - 1) / FG;
             const NlFx &X = nonlocal_fx_pick(nl, groups);
             const nlfx::Tables T = nonlocal_fx_tables(nl, X);
-            const int sm = (int)nlfx::smem_bytes(T);
+            const int sm = (int)T.L.bytes;
             CT *part = nullptr;
             int chunk = groups;
             const int rc = X.nrange > 65535
@@ -1418,7 +1418,7 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
     int fsm = 0, fgx = 1;
     if (fx_nl) {  // attributes set before any capture
         fT = nonlocal_fx_tables(nl, *fxt);
-        fsm = (int)nlfx::smem_bytes(fT);
+        fsm = (int)fT.L.bytes;
         const int groups = (maxcol + FG - 1) / FG;
         fgx = std::min(groups, std::max(1, (int)(152L * 8 / ((long)fxt->nrange * nblk))));
         auto attr = [&](auto k9, auto k18) {

@@ -22,7 +22,7 @@
 //            memory, and the range's sums go to a partial buffer that k_fx_reduce adds up per
 //            projector row in a fixed order (the result does not depend on scheduling)
 // With both, the finished output tile is projected for the next filter degree without reading it
-// again. Chi digits are read at warp-uniform addresses through L1. A column whose values the
+// again. Chi digits are read at warp-uniform addresses of shared memory. A column whose values the
 // fixed-point range does not cover (infinities, NaN, extreme exponents) sends the block's sums
 // through FP64 arithmetic.
 //
@@ -34,19 +34,15 @@
 #pragma once
 
 #include "fixed64.cuh"
+#include "nonlocal_fx_layout.h"
 #include "sgpu_internal.h"
 
 namespace sgpu {
 namespace nlfx {
 
-constexpr int kPts = 128;      // covered points per range at most: 128 products of an item and of
-                               // a point's rows fit the 64-bit sums in units of 2^57
 constexpr int kPtRows = 128;   // projector rows over one point at most
 constexpr int kRows = 128;     // projector rows per range (items' rows added up) at most
 constexpr int kChiBytes = 32 * 1024;  // Chi digits per range at most (two blocks per SM)
-constexpr int kLanes = 32;     // real columns per group
-constexpr int kWarps = 8;
-constexpr int kPitch = kLanes + 1;  // tile row, 8-byte elements
 constexpr int kChiBits = 56;   // |Chi digit value| < 2^kChiBits
 
 struct Tables {
@@ -60,18 +56,9 @@ struct Tables {
     const int4 *chi;    // entry: jp / 2 pairs of digits (h, l, h, l)
     const int4 *rows;   // row of a range: (alpha row, image, er), |Chi| of the row < 2^er
     const int *row0;    // nrange + 1: first row of each range (rows, partial buffer)
-    int jp, max_rows, max_ent, max_items;
+    int jp;
+    Layout L;           // shared memory for the largest of the ranges
 };
-
-inline __host__ __device__ size_t align16(size_t b) { return (b + 15) / 16 * 16; }
-// shared memory: tile, alpha digits / projection sums, Chi digits, points, row and item tables
-inline size_t smem_bytes(const Tables &T)
-{
-    return sizeof(long long) * kPts * kPitch + 8 * (size_t)kLanes * T.max_rows +
-           8 * (size_t)T.max_ent * T.jp + align16(T.max_ent) + 16 * (size_t)T.max_rows +
-           16 * (size_t)T.max_items +
-           align16(4 * ((size_t)T.max_items + 1 + (size_t)T.max_items * (kWarps + 1)));
-}
 
 // raw sum in units of 2^57. A product is below 2^113, so 128 of them end below 2^63 units (what an
 // intermediate sum wraps, a later one wraps back); mid alone must not wrap: 64 products at most
@@ -101,15 +88,15 @@ __device__ __forceinline__ void block(const Tables &T, int r, int g0, int gstep,
     constexpr int CW = NC / kWarps;                 // columns per warp
     constexpr int NV = kPts / 32;                   // points per lane
     constexpr int NA = kRows / kWarps;              // alpha rows per warp
-    long long *tile = reinterpret_cast<long long *>(smem);       // [kPts][kPitch]
-    int2 *al = reinterpret_cast<int2 *>(tile + kPts * kPitch);   // [rows][kLanes]
-    int4 *chi = reinterpret_cast<int4 *>(al + T.max_rows * kLanes);
     const int hp = T.jp >> 1;                                    // digit pairs per entry
-    unsigned char *lps = reinterpret_cast<unsigned char *>(chi + T.max_ent * hp);
-    int4 *rows = reinterpret_cast<int4 *>(lps + align16(T.max_ent));
-    int4 *items = rows + T.max_rows;
-    int *ent0 = reinterpret_cast<int *>(items + T.max_items);    // [items + 1], then wsplit
-    int *wsplit = ent0 + T.max_items + 1;
+    long long *tile = reinterpret_cast<long long *>(smem);       // [kPts][kPitch]
+    int2 *al = reinterpret_cast<int2 *>(smem + T.L.al);            // [rows][kLanes]
+    int4 *chi = reinterpret_cast<int4 *>(smem + T.L.chi);
+    unsigned char *lps = smem + T.L.lps;
+    int4 *rows = reinterpret_cast<int4 *>(smem + T.L.rows);
+    int4 *items = reinterpret_cast<int4 *>(smem + T.L.items);
+    int *ent0 = reinterpret_cast<int *>(smem + T.L.ent0);
+    int *wsplit = reinterpret_cast<int *>(smem + T.L.wsplit);
     __shared__ unsigned s_key[kLanes];
     __shared__ int s_bad, s_E[kLanes];
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;

@@ -184,13 +184,13 @@ __device__ __forceinline__ void stencil_z_body(const StencilZParams<CT> &p, int 
 template <typename CT>
 __host__ __device__ constexpr int zstencil_threads() { return sizeof(CT) == 16 ? 256 : 512; }
 
-// Tile of the complex stencil for an Nx x Ny plane: the widest x extent in [16, 64] with the
-// least padding, then the tallest y extent in [R, maxt / bx] with the least padding.
+// Tile of the complex stencil for an Nx x Ny plane: the widest x extent in [16, 64] of which R rows
+// make at most maxt threads with the least padding, then the tallest y extent in [R, maxt / bx] with the least padding.
 static void zstencil_tile(int Nx, int Ny, int R, int maxt, int *bx, int *by)
 {
     int best = 1 << 30;
     *bx = 32;
-    for (int t = std::min(64, std::max(16, Nx)); t >= 16; t--) {
+    for (int t = std::min({64, maxt / R, std::max(16, Nx)}); t >= 16; t--) {
         const int waste = (Nx + t - 1) / t * t - Nx;
         if (waste < best) { best = waste; *bx = t; }
     }

@@ -324,3 +324,33 @@ def test_fp64_arithmetic_on_request(gpu_available, ncol):
     with pytest.raises(sg.SgpuError):
         sg._check(sg.lib().sgpu_set_fixed_point(ctx._h, 2))
     ctx.close()
+
+
+@pytest.mark.parametrize("N", [(47, 14, 12), (96, 9, 12), (64, 13, 7)])
+def test_general_complex_kernel_on_wide_planes(gpu_available, N):
+    """Planes of 43 points and more along x, where the best tile of the general complex128 stencil
+    once had more threads than its blocks may have; alone and batched."""
+    import torch
+    h = 0.4
+    rng = np.random.default_rng(sum(N))
+    c = fd_d2_coeffs(6, h)
+    Nd, L = N[0] * N[1] * N[2], np.array(N) * h
+    ctx = sg.Context(*N, 6, c, c, c, h ** 3)
+    v = rng.normal(0.0, 0.4, Nd)
+    ctx.set_veff(v)
+    ctx.set_kpoint_geometry(L, np.zeros((0, 3)))
+    ctx.set_fixed_point(False)
+    o = Oracle(dict(Nx=N[0], Ny=N[1], Nz=N[2], FDn=6, cx=c, cy=c, cz=c, dV=h ** 3), None)
+    k = np.array([0.2, -0.1, 0.3])
+    z = rng.uniform(-1, 1, (3, Nd)) + 1j * rng.uniform(-1, 1, (3, Nd))
+    w = np.zeros_like(z)
+    ctx.Hamiltonian_vectors_mult_kpt(k, 0.3, z, w)
+    _close(w, o.lap_plus_diag_kpt(k, L, -0.5, 1.0, 0.3, v, z))
+    X = torch.from_numpy(z).cuda()
+    Y = torch.empty_like(X)
+    ctx.ChebyshevFiltering_batched([dict(spin=0, k=k, X=X, Y=Y, a=0.5, b=40.0, a0=-0.8)], 4)
+    Xf, Yf = z.copy(), np.zeros_like(z)
+    ctx.set_fixed_point(True)
+    ctx.ChebyshevFiltering_kpt(k, Xf, Yf, 4, 0.5, 40.0, -0.8)
+    _close(Y.cpu().numpy(), Yf)
+    ctx.close()

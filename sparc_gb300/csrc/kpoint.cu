@@ -1017,8 +1017,7 @@ static int stencil_z(sgpu_ctx *ctx, const double *k, int ncol, double a, double 
     int BX, BY;
     zstencil_tile(ctx->Nx, ctx->Ny, R, zstencil_threads<CT>(), &BX, &BY);
     const size_t zsm = zstencil_smem<CT>(BX, BY, R);
-    SGPU_CUDA_TRY(cudaFuncSetAttribute(k_stencil_z<CT, R>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsm));
+    SGPU_CUDA_TRY(allow_smem(k_stencil_z<CT, R>));
     const int tilesx = (ctx->Nx + BX - 1) / BX, tilesy = (ctx->Ny + BY - 1) / BY;
     long blocks1 = (long)tilesx * tilesy * ncol;
     int nslab = 1;
@@ -1071,8 +1070,8 @@ static int nonlocal_z(sgpu_ctx *ctx, int ncol, const CT *x, long ldx, CT *out, l
                 SGPU_TRY(rc);
                 auto project = nl.max_np <= 9 ? k_nl_fx_z<false, true, 9> : k_nl_fx_z<false, true, 18>;
                 auto apply = nl.max_np <= 9 ? k_nl_fx_z<true, false, 9> : k_nl_fx_z<true, false, 18>;
-                SGPU_CUDA_TRY(cudaFuncSetAttribute(project, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-                SGPU_CUDA_TRY(cudaFuncSetAttribute(apply, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+                SGPU_CUDA_TRY(allow_smem(project));
+                SGPU_CUDA_TRY(allow_smem(apply));
                 const long ldp = (long)chunk * FG;
                 auto gx = [&](int gn) { return std::min(gn, std::max(1, 152 * 8 / X.nrange)); };
                 for (int g0 = 0; g0 < groups; g0 += chunk) {
@@ -1115,8 +1114,7 @@ static int nonlocal_z(sgpu_ctx *ctx, int ncol, const CT *x, long ldx, CT *out, l
         if (nl.nchunk > 0 && stage <= kZStageMax) {
             const dim3 sg(nl.nchunk, (ncol + CB - 1) / CB);
             auto launch = [&](auto kern) -> int {
-                SGPU_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)std::max<size_t>(stage, 16)));
+                SGPU_CUDA_TRY(allow_smem(kern));
                 kern<<<sg, kApplyChunkZ, std::max<size_t>(stage, 16), st>>>(
                     nl.ncov, nl.cov_pt, nl.cov_ptr, nl.ent_chi, nl.ent_meta, nl.ent_slot,
                     nl.chunk_row_ptr, nl.chunk_rows, chi_z<CT>(nl), ks->img_phase, ncol, alpha,
@@ -1390,8 +1388,7 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
     int BX, BY;
     zstencil_tile(ctx->Nx, ctx->Ny, R, zstencil_threads<CT>(), &BX, &BY);
     size_t zsm = zstencil_smem<CT>(BX, BY, R);  // attribute set before any capture
-    SGPU_CUDA_TRY(cudaFuncSetAttribute(k_stencil_zb<CT, R>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsm));
+    SGPU_CUDA_TRY(allow_smem(k_stencil_zb<CT, R>));
     const int tilesx = (ctx->Nx + BX - 1) / BX, tilesy = (ctx->Ny + BY - 1) / BY;
     int nslab = 1;
     while ((long)tilesx * tilesy * totcols * nslab < 152L * 8 && ctx->Nz / (nslab * 2) >= 8)
@@ -1407,10 +1404,8 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
             sizeof(CT) * (size_t)nl.max_chunk_rows * zstage_ld<CT, zapply_cb<CT>()>();
         if (nl.nchunk > 0 && stage <= kZStageMax) {
             const int sm = (int)std::max<size_t>(stage, 16);
-            SGPU_CUDA_TRY(cudaFuncSetAttribute(k_nl_apply_zb_staged<CT, 9>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-            SGPU_CUDA_TRY(cudaFuncSetAttribute(k_nl_apply_zb_staged<CT, 18>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+            SGPU_CUDA_TRY(allow_smem(k_nl_apply_zb_staged<CT, 9>));
+            SGPU_CUDA_TRY(allow_smem(k_nl_apply_zb_staged<CT, 18>));
         }
     }
 
@@ -1423,8 +1418,8 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
         fgx = std::min(groups, std::max(1, (int)(152L * 8 / ((long)fxt->nrange * nblk))));
         auto attr = [&](auto k9, auto k18) {
             return nl.max_np <= 9
-                       ? cudaFuncSetAttribute(k9, cudaFuncAttributeMaxDynamicSharedMemorySize, fsm)
-                       : cudaFuncSetAttribute(k18, cudaFuncAttributeMaxDynamicSharedMemorySize, fsm);
+                       ? allow_smem(k9)
+                       : allow_smem(k18);
         };
         SGPU_CUDA_TRY(attr(k_nl_fx_zb<false, true, 9>, k_nl_fx_zb<false, true, 18>));
         SGPU_CUDA_TRY(attr(k_nl_fx_zb<true, false, 9>, k_nl_fx_zb<true, false, 18>));

@@ -859,8 +859,7 @@ static int project_launch(sgpu_ctx *ctx, int ncol, const T *x, long ldx, T *alph
     const size_t xs_elems = std::max((size_t)NC * (PCH + 1), (size_t)HALVES * MAXJ * NC);
     const size_t smem = sizeof(T) * ((size_t)MAXJP * kSegPts + xs_elems) + sizeof(int) * kSegPts;
     auto kern = k_nl_project<T, PCH, NC, MAXJ>;
-    SGPU_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem));
+    SGPU_CUDA_TRY(allow_smem(kern));
     const Nonlocal &nl = ctx->nl;
     ProfScope ps(ctx, SGPU_KERNEL_NL_PROJECT, st);
     kern<<<nl.nseg, kProjThreads, smem, st>>>(
@@ -877,8 +876,7 @@ static int project_range_launch(sgpu_ctx *ctx, int ncol, const float *x, long ld
     const size_t smem = sizeof(float) * ((size_t)kRangePts * 66 + (size_t)nl.max_range_ent * nl.range_jp) +
                         sizeof(int) * ((size_t)nl.max_range_ent + kRangePts);
     auto kern = k_nl_project_range<MAXJ>;
-    SGPU_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem));
+    SGPU_CUDA_TRY(allow_smem(kern));
     ProfScope ps(ctx, SGPU_KERNEL_NL_PROJECT, st);
     kern<<<nl.nrange, 256, smem, st>>>(nl.rng_pt0, nl.rng_ent0, nl.rng_item0, nl.item_e0,
                                        nl.item_row, nl.pe_lp, nl.pe_chi32, nl.cov_pt, nl.gamma32,
@@ -957,8 +955,7 @@ int launch_nonlocal_apply(sgpu_ctx *ctx, int ncol, const T *alpha, long lda, dou
 #define SGPU_STAGED(NPM)                                                                     \
     {                                                                                        \
         auto kern = k_nl_apply_staged<T, SCB, NPM>;                                          \
-        SGPU_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
-                                           (int)std::max<size_t>(stage, 16)));               \
+        SGPU_CUDA_TRY(allow_smem(kern));                                                     \
         kern<<<sg, kApplyChunk, std::max<size_t>(stage, 16), st>>>(                          \
             nl.ncov, nl.cov_pt, nl.cov_ptr, nl.ent_chi, nl.ent_meta, nl.ent_slot,            \
             nl.chunk_row_ptr, nl.chunk_rows, chi_of<T>(nl), ncol, alpha, lda, (T)scale, out, \
@@ -983,8 +980,7 @@ int launch_nonlocal_apply(sgpu_ctx *ctx, int ncol, const T *alpha, long lda, dou
 #define SGPU_RAPPLY(MJ)                                                                      \
     {                                                                                        \
         auto kern = k_nl_apply_range<MJ>;                                                    \
-        SGPU_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
-                                           (int)rsm));                                       \
+        SGPU_CUDA_TRY(allow_smem(kern));                                                     \
         kern<<<nl.nrange, 256, rsm, st>>>(nl.rng_pt0, nl.rng_ent0, nl.rng_item0, nl.item_wsplit, \
                                           nl.item_row, nl.pe_lp, nl.pe_chi32, nl.cov_pt,     \
                                           ncol, alpha, lda, (float)scale, out, ldo);         \
@@ -1001,9 +997,7 @@ int launch_nonlocal_apply(sgpu_ctx *ctx, int ncol, const T *alpha, long lda, dou
         }
         const size_t dsm = sizeof(float) * (size_t)nl.max_chunk_rows * (64 + kApplyChunk);
         if (ctx->nl_apply_variant == 3 && nl.nchunk > 0 && dsm <= kApplyDenseMax) {
-            SGPU_CUDA_TRY(cudaFuncSetAttribute(k_nl_apply_dense,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)std::max<size_t>(dsm, 16)));
+            SGPU_CUDA_TRY(allow_smem(k_nl_apply_dense));
             const dim3 dg(nl.nchunk, (ncol + 63) / 64);
             ProfScope ps(ctx, SGPU_KERNEL_NL_APPLY, st);
             k_nl_apply_dense<<<dg, 256, std::max<size_t>(dsm, 16), st>>>(
@@ -1072,8 +1066,7 @@ int launch_nonlocal_apply_project(sgpu_ctx *ctx, int ncol, const float *alpha, l
 #define SGPU_FAPPLY(MJ, CPL)                                                                 \
     {                                                                                        \
         auto kern = k_nl_apply_project_range<MJ, CPL>;                                       \
-        SGPU_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
-                                           (int)rsm));                                       \
+        SGPU_CUDA_TRY(allow_smem(kern));                                                     \
         kern<<<nl.nrange, 256, rsm, st>>>(nl.rng_pt0, nl.rng_ent0, nl.rng_item0, nl.item_e0, \
                                           nl.item_wsplit, nl.item_row, nl.pe_lp, nl.pe_chi32, \
                                           nl.cov_pt, nl.gamma32, ncol, alpha, lda,           \

@@ -65,8 +65,7 @@ int launch(sgpu_ctx *ctx, int ncol, const double *alpha, double scale, double *o
     const nlfx::Tables T = nonlocal_fx_tables(nl, X);
     const size_t smem = T.L.bytes;
     auto kern = nl.max_np <= 9 ? k_nl_fx<APPLY, PROJ, 9> : k_nl_fx<APPLY, PROJ, 18>;
-    SGPU_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem));
+    SGPU_CUDA_TRY(allow_smem(kern));
     double *part = nullptr;
     int chunk = groups;
     if (PROJ)

@@ -411,8 +411,7 @@ int launch_nonlocal_apply_project_tc(sgpu_ctx *ctx, int ncol, const float *alpha
     TcTables T{nl.tc_pt0, nl.tc_row0, nl.tc_rows, nl.tc_ent0, nl.tc_ent, nl.tc_chi,
                nl.range_jp, nl.tc_pts, nl.gamma32};
     ProfScope ps(ctx, SGPU_KERNEL_NL_APPLY, st);
-    SGPU_CUDA_TRY(cudaFuncSetAttribute(k_nl_apply_project_tc,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
+    SGPU_CUDA_TRY(allow_smem(k_nl_apply_project_tc));
     k_nl_apply_project_tc<<<nl.tc_nrange, kTcThreads, kTcSmem, st>>>(
         T, ncol, alpha, lda, (float)scale, out, ldo, alpha_next, (float)ctx->dV, ctx->kstatus);
     SGPU_CUDA_TRY(cudaGetLastError());

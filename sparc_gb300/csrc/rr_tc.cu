@@ -712,8 +712,7 @@ int launch_gemm(sgpu_ctx *ctx, const TcParams &p, int ntiles, cudaStream_t st)
     SGPU_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device));
     const int nblocks = std::max(1, std::min(ntiles, nsm));  // persistent: one CTA per SM
     auto kern = k_tc_gemm<NS>;
-    SGPU_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem));
+    SGPU_CUDA_TRY(allow_smem(kern));
     ProfScope ps(ctx, SGPU_KERNEL_OTHER, st);
     kern<<<nblocks, NTHREADS, smem, st>>>(p);
     SGPU_CUDA_TRY(cudaGetLastError());
@@ -1213,8 +1212,7 @@ int launch_gemm_x(sgpu_ctx *ctx, const TcxParams &p, cudaStream_t st)
     SGPU_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device));
     const int nupper = upper_tiles(p.mtiles, p.ntiles);
     const int ntot = p.mode == 0 ? nupper * p.ksplit : p.mtiles * p.ntiles;
-    SGPU_CUDA_TRY(cudaFuncSetAttribute(k_tc_gemm_x, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)XSMEM));
+    SGPU_CUDA_TRY(allow_smem(k_tc_gemm_x));
     ProfScope ps(ctx, SGPU_KERNEL_OTHER, st);
     k_tc_gemm_x<<<std::max(1, std::min(ntot, nsm)), NTHREADS, XSMEM, st>>>(p, nupper);
     if (ctx->inject & 4) {  // a wait that ran out: a column left unwritten, the status word set

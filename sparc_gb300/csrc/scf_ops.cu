@@ -611,8 +611,7 @@ static int anderson_gamma(sgpu_ctx *ctx, long n, int m, const double *F, const d
     // at 77^3 as single dots, 2 launches here
     if (m == kGramM) {
         const size_t sm = sizeof(double) * 256 * kGramPairs;
-        SGPU_CUDA_TRY(cudaFuncSetAttribute(k_gram_partial<kGramM>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        SGPU_CUDA_TRY(allow_smem(k_gram_partial<kGramM>));
         k_gram_partial<kGramM><<<kRedBlocks, 256, sm, st>>>(F, f, n, part);
         k_gram_sum<<<kGramPairs, 256, 0, st>>>(part, kRedBlocks, m, ftf, ftb);
         ctx->launches += 2;

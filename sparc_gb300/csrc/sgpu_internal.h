@@ -23,6 +23,20 @@ constexpr int kRangeItemEnt = 96;    // entries per work item of the range proje
 constexpr int kRangeWarps = 8;       // warps per range block
 static_assert(kRangePts % kRangeWarps == 0, "whole tile rows per warp");
 
+// Lets a kernel be launched with any dynamic shared memory that an SM has for it. The attribute belongs
+// to the process: set to each launch's own size, another thread's smaller size (another context, another
+// grid) could come between it and the launch, which then failed.
+template <typename K>
+inline cudaError_t allow_smem(K *kern)
+{
+    constexpr int kBlockMax = 227 * 1024;  // static and dynamic, sm_103
+    cudaFuncAttributes a{};
+    const cudaError_t e = cudaFuncGetAttributes(&a, (const void *)kern);
+    const int most = kBlockMax - (int)a.sharedSizeBytes;
+    if (e != cudaSuccess || a.maxDynamicSharedSizeBytes >= most) return e;
+    return cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
+
 // thread-local error text, returned by sgpu_last_error()
 void set_error(const std::string &msg);
 

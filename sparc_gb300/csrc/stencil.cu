@@ -777,8 +777,7 @@ int launch_ring(const StencilParams<float> &q, dim3 grid, cudaStream_t st)
 {
     constexpr size_t smem = RingShape<R, BX, BY, D, EW, VG>::smem_bytes;
     auto kern = k_stencil_f32_ring<R, BX, BY, MINB, EW, D, VG>;
-    SGPU_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem));
+    SGPU_CUDA_TRY(allow_smem(kern));
     kern<<<grid, dim3(BX / 2, BY / 2), smem, st>>>(q);
     return SGPU_OK;
 }
@@ -1072,8 +1071,7 @@ int launch_bulk(const StencilParams<float> &q, dim3 grid, cudaStream_t st)
 {
     constexpr size_t smem = BulkShape<R, BX, BY, D>::smem_bytes;
     auto kern = k_stencil_f32_bulk<R, BX, BY, MINB, D>;
-    SGPU_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem));
+    SGPU_CUDA_TRY(allow_smem(kern));
     kern<<<grid, dim3(BX / 2, BY / 2), smem, st>>>(q);
     return SGPU_OK;
 }

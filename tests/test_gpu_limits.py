@@ -354,3 +354,34 @@ def test_general_complex_kernel_on_wide_planes(gpu_available, N):
     ctx.ChebyshevFiltering_kpt(k, Xf, Yf, 4, 0.5, 40.0, -0.8)
     _close(Y.cpu().numpy(), Yf)
     ctx.close()
+
+
+def test_two_threads_with_ranges_of_different_size(gpu_available):
+    """Two contexts, each used by a thread of its own, whose launches of one kernel ask for different
+    amounts of shared memory: neither's calls are disturbed."""
+    import threading
+
+    import torch
+    work, bad = [], []
+    for N, natom, rc in (((24, 22, 20), 1, 1.0), ((30, 28, 26), 30, 3.0)):
+        ctx, v, nl, grid, rng = _system(N, 0.4, natom=natom, rc=rc)
+        x = torch.from_numpy(rng.uniform(-1, 1, (4, ctx.Nd))).cuda()
+        work.append((ctx, x, torch.zeros_like(x), Oracle(grid, nl)))
+
+    def run(ctx, x, y):
+        for _ in range(3000):
+            try:
+                y.zero_()
+                ctx.Vnl_vec_mult(x, y)
+            except sg.SgpuError as e:
+                bad.append(str(e))
+
+    threads = [threading.Thread(target=run, args=w[:3]) for w in work]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad, bad[:3]
+    for ctx, x, y, o in work:
+        _close(y.cpu().numpy(), o.vnl(x.cpu().numpy()))
+        ctx.close()

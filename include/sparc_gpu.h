@@ -534,7 +534,8 @@ int sgpu_check_wait_bound(sgpu_ctx *ctx, int *status);
 /* Failures made on the host, for tests of what a call does about them; mask 0 ends them. 1: device
  * scratch that a call can do without cannot be allocated; 2: the fixed-point tables of set_veff
  * and set_nonlocal cannot be; 4: a bounded wait of the FP64 Rayleigh-Ritz products is reported as
- * run out, with part of their output unwritten; 8: an operand's scratch is held to 1 MB. A call then takes the form that needs none of
+ * run out, with part of their output unwritten; 8: an operand's scratch is held to 1 MB;
+ * 16: the first try of every other allocation fails, as on a device that the scratch fills. A call then takes the form that needs none of
  * these, with the same result. */
 int sgpu_inject_failure(sgpu_ctx *ctx, int mask);
 

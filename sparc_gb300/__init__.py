@@ -788,8 +788,8 @@ class Context:
 
     def inject_failure(self, mask):
         """Failures made on the host, for tests (sgpu_inject_failure): 1 optional scratch, 2 the
-        fixed-point tables, 4 a wait of the FP64 Rayleigh-Ritz products, 8 scratch held to 1 MB;
-        0 none."""
+        fixed-point tables, 4 a wait of the FP64 Rayleigh-Ritz products, 8 scratch held to 1 MB,
+        16 the first try of other allocations; 0 none."""
         _check(lib().sgpu_inject_failure(self._h, int(mask)))
 
     def last_filter_ms(self):

@@ -29,7 +29,7 @@ static int tune_stencil(sgpu_ctx *ctx, int ncol, int *best, double *ms)
     }
     const long Nd = ctx->Nd;
     float *buf = nullptr;
-    SGPU_CUDA_TRY(cudaMallocAsync(&buf, sizeof(float) * (size_t)Nd * ncol * 2, st));
+    SGPU_CUDA_TRY(dev_alloc_async(ctx, &buf, sizeof(float) * (size_t)Nd * ncol * 2, st));
     float *X = buf, *Y = buf + (size_t)Nd * ncol;
     int rc = SGPU_OK;
     if (cudaMemsetAsync(buf, 0, sizeof(float) * (size_t)Nd * ncol * 2, st) != cudaSuccess)
@@ -70,7 +70,7 @@ static int tune_stencil(sgpu_ctx *ctx, int ncol, int *best, double *ms)
     if (rc == SGPU_OK && ctx->has_nl && ctx->nl.ntot > 0 && ctx->nl.ncov > 0) {
         const long lda = nonlocal_alpha_ld(ncol, 4);
         float *alpha = nullptr;
-        if (cudaMallocAsync(&alpha, sizeof(float) * (size_t)ctx->nl.ntot * lda, st) != cudaSuccess ||
+        if (dev_alloc_async(ctx, &alpha, sizeof(float) * (size_t)ctx->nl.ntot * lda, st) != cudaSuccess ||
             cudaMemsetAsync(alpha, 0, sizeof(float) * (size_t)ctx->nl.ntot * lda, st) != cudaSuccess) {
             rc = SGPU_ERR_CUDA;
         } else {
@@ -128,7 +128,7 @@ static int tune_stencil(sgpu_ctx *ctx, int ncol, int *best, double *ms)
             float *anext = nullptr;
             const size_t abytes = sizeof(float) * (size_t)ctx->nl.ntot * lda;
             if (rc == SGPU_OK && ctx->nl.nrange > 0) {
-                if (cudaMallocAsync(&anext, abytes, st) != cudaSuccess) rc = SGPU_ERR_CUDA;
+                if (dev_alloc_async(ctx, &anext, abytes, st) != cudaSuccess) rc = SGPU_ERR_CUDA;
                 float fbest = 1e30f;
                 int cbest = 2;
                 ctx->tune_fused_tc_ms = 0.0;

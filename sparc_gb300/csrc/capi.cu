@@ -67,6 +67,30 @@ int ws_get(sgpu_ctx *ctx, int slot, size_t bytes, void **out)
     return SGPU_OK;
 }
 
+cudaError_t dev_alloc(sgpu_ctx *ctx, void **p, size_t bytes)
+{
+    *p = nullptr;
+    cudaError_t e = cudaMalloc(p, ctx->inject & 16 ? (size_t)1 << 60 : bytes);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    if (ws_release(ctx, -1) != SGPU_OK) return e;
+    e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
+}
+
+cudaError_t dev_alloc_async(sgpu_ctx *ctx, void **p, size_t bytes, cudaStream_t st)
+{
+    *p = nullptr;
+    cudaError_t e = cudaMallocAsync(p, ctx->inject & 16 ? (size_t)1 << 60 : bytes, st);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    if (ws_release(ctx, -1) != SGPU_OK) return e;
+    e = cudaMallocAsync(p, bytes, st);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
+}
+
 int kernel_status_check(sgpu_ctx *ctx, int *status)
 {
     int h = 0;
@@ -307,8 +331,8 @@ int sgpu_set_veff(sgpu_ctx *ctx, int nspin, const double *veff)
         ctx->veff32 = nullptr;
         ctx->veff_fx = nullptr;
         ctx->nspin_veff = 0;
-        SGPU_CUDA_TRY(cudaMalloc(&ctx->veff64, n * sizeof(double)));
-        SGPU_CUDA_TRY(cudaMalloc(&ctx->veff32, n * sizeof(float)));
+        SGPU_CUDA_TRY(dev_alloc(ctx, &ctx->veff64, n * sizeof(double)));
+        SGPU_CUDA_TRY(dev_alloc(ctx, &ctx->veff32, n * sizeof(float)));
         // without room for the digits the FP64 kernels read veff64
         if (cudaMalloc(&ctx->veff_fx, ctx->inject & 2 ? (size_t)1 << 60 : (n + 1) * sizeof(int2)) !=
             cudaSuccess) {
@@ -716,7 +740,7 @@ int sgpu_set_fixed_point(sgpu_ctx *ctx, int on)
 int sgpu_inject_failure(sgpu_ctx *ctx, int mask)
 {
     SGPU_TRY(check_ctx(ctx));
-    if (mask & ~15) {
+    if (mask & ~31) {
         set_error("sgpu_inject_failure: unknown failure");
         return SGPU_ERR_ARG;
     }

@@ -149,7 +149,7 @@ int sgpu_Calculate_nonlocal_forces(sgpu_ctx *ctx, int ncol, const double *X, int
     const size_t n = 4 * asz + (size_t)Nd * ncol + ncol + nl.ntot + 3 * (size_t)nl.natom +
                      (dev_x ? 0 : (size_t)Nd * ncol);
     double *buf = nullptr;
-    SGPU_CUDA_TRY(cudaMallocAsync(&buf, sizeof(double) * n, st));
+    SGPU_CUDA_TRY(dev_alloc_async(ctx, &buf, sizeof(double) * n, st));
     double *alpha = buf, *dX = alpha + 4 * asz, *docc = dX + (size_t)Nd * ncol,
            *ones = docc + ncol, *dF = ones + nl.ntot, *xs = dF + 3 * nl.natom;
     const double *xd = X;
@@ -219,7 +219,7 @@ int sgpu_Gradient_vectors_dir(sgpu_ctx *ctx, int ncol, const double *cell, const
     const bool dx_ = is_device_ptr(x), dy_ = is_device_ptr(Dx);
     double *buf = nullptr;
     const size_t n = (dx_ ? 0 : (size_t)Nd * ncol) + (dy_ ? 0 : (size_t)Nd * ncol);
-    if (n) SGPU_CUDA_TRY(cudaMallocAsync(&buf, sizeof(double) * n, st));
+    if (n) SGPU_CUDA_TRY(dev_alloc_async(ctx, &buf, sizeof(double) * n, st));
     const double *xd = x;
     double *yd = Dx;
     long lx = ldi, ly = ldo;

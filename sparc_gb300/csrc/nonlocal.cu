@@ -1116,9 +1116,9 @@ void nonlocal_free(Nonlocal &nl)
 
 namespace {
 template <typename T>
-int upload(T **dst, const T *src, size_t n)
+int upload(sgpu_ctx *ctx, T **dst, const T *src, size_t n)
 {
-    SGPU_CUDA_TRY(cudaMalloc((void **)dst, sizeof(T) * (n > 0 ? n : 1)));
+    SGPU_CUDA_TRY(dev_alloc(ctx, dst, sizeof(T) * (n > 0 ? n : 1)));
     if (n > 0) SGPU_CUDA_TRY(cudaMemcpy(*dst, src, sizeof(T) * n, cudaMemcpyHostToDevice));
     return SGPU_OK;
 }
@@ -1316,7 +1316,7 @@ int nonlocal_upload(sgpu_ctx *ctx, int natom, const int *ip_displ, const double 
 
     int rc = SGPU_OK;
 #define UP(dst, src, n)                                                                      \
-    if (rc == SGPU_OK) rc = upload(&nl.dst, src, n)
+    if (rc == SGPU_OK) rc = upload(ctx, &nl.dst, src, n)
     UP(ip_displ, ip_displ, (size_t)natom + 1);
     UP(img_atom, img_atom, (size_t)nimg);
     UP(img_ndc, img_ndc, (size_t)nimg);
@@ -1346,9 +1346,9 @@ int nonlocal_upload(sgpu_ctx *ctx, int natom, const int *ip_displ, const double 
     UP(pe_chi32, pe_chi.data(), pe_chi.size());
 #undef UP
     const std::vector<int> ord = compact_order(ctx->Nx, ctx->Ny, covpts);
-    if (rc == SGPU_OK) rc = nonlocal_tc_build(nl, ord, covpts, covptr, ent_chi, ent_meta, chi);
+    if (rc == SGPU_OK) rc = nonlocal_tc_build(ctx, nl, ord, covpts, covptr, ent_chi, ent_meta, chi);
     if (rc == SGPU_OK) {
-        rc = nonlocal_fx_build(nl, ord, covpts, covptr, ent_chi, ent_meta, chi, ctx->inject & 2);
+        rc = nonlocal_fx_build(ctx, nl, ord, covpts, covptr, ent_chi, ent_meta, chi);
         if (rc == SGPU_ERR_NOMEM) {  // the FP64 kernels need none of these tables
             cudaGetLastError();
             nonlocal_fx_free(nl);

@@ -173,7 +173,7 @@ int launch_nonlocal_fx_apply(sgpu_ctx *ctx, int ncol, const double *alpha, long 
 // past kChiBytes. No tables (and the FP64 kernels stay) for more than 18 projectors per atom, for a
 // point under more than kPtRows projector rows (the 64-bit sums hold that many) and for Chi
 // values outside 1e-40 .. 1e40. SGPU_ERR_NOMEM: no room for them.
-static int build_ranges(Nonlocal &nl, NlFx &x, int cap, bool fail, const std::vector<int> &er,
+static int build_ranges(sgpu_ctx *ctx, Nonlocal &nl, NlFx &x, int cap, const std::vector<int> &er,
                         const std::vector<int> &ord, const std::vector<int> &covpts,
                         const std::vector<int> &covptr, const std::vector<long> &ent_chi,
                         const std::vector<int4> &ent_meta)
@@ -310,8 +310,8 @@ static int build_ranges(Nonlocal &nl, NlFx &x, int cap, bool fail, const std::ve
     const size_t bytes = ochi + sizeof(int2) * (size_t)nl.nent * nl.fx_jp;
     char *base = nullptr, *temp = nullptr;
     int rc = SGPU_OK;
-    if (cudaMalloc(&base, fail ? (size_t)1 << 60 : bytes) != cudaSuccess ||
-        cudaMalloc(&temp, tsize) != cudaSuccess) {
+    if (dev_alloc(ctx, &base, ctx->inject & 2 ? (size_t)1 << 60 : bytes) != cudaSuccess ||
+        dev_alloc(ctx, &temp, tsize) != cudaSuccess) {
         rc = SGPU_ERR_NOMEM;
     } else {
         // small tables in one copy (a copy takes about 10 us), large ones from where they are
@@ -346,9 +346,9 @@ static int build_ranges(Nonlocal &nl, NlFx &x, int cap, bool fail, const std::ve
 }
 
 
-int nonlocal_fx_build(Nonlocal &nl, const std::vector<int> &ord, const std::vector<int> &covpts,
+int nonlocal_fx_build(sgpu_ctx *ctx, Nonlocal &nl, const std::vector<int> &ord, const std::vector<int> &covpts,
                       const std::vector<int> &covptr, const std::vector<long> &ent_chi,
-                      const std::vector<int4> &ent_meta, const double *chi, bool fail)
+                      const std::vector<int4> &ent_meta, const double *chi)
 {
     if (nl.max_np > 18 || nl.max_np < 1 || nl.ncov == 0) return SGPU_OK;
     // exponent of each projector row's largest Chi value
@@ -369,13 +369,13 @@ int nonlocal_fx_build(Nonlocal &nl, const std::vector<int> &ord, const std::vect
             std::frexp(mx[i], &er[i]);
         }
     }
-    if (cudaMalloc((void **)&nl.fx_er, sizeof(int) * er.size()) != cudaSuccess) return SGPU_ERR_NOMEM;
+    if (dev_alloc(ctx, &nl.fx_er, sizeof(int) * er.size()) != cudaSuccess) return SGPU_ERR_NOMEM;
     SGPU_CUDA_TRY(cudaMemcpy(nl.fx_er, er.data(), sizeof(int) * er.size(), cudaMemcpyHostToDevice));
     nl.fx_jp = nl.max_np <= 9 ? 10 : 18;
-    SGPU_TRY(build_ranges(nl, nl.fx[0], nlfx::kPts, fail, er, ord, covpts, covptr, ent_chi, ent_meta));
+    SGPU_TRY(build_ranges(ctx, nl, nl.fx[0], nlfx::kPts, er, ord, covpts, covptr, ent_chi, ent_meta));
     // small ranges where one column group in large ones leaves SMs without a block
     if (nl.fx[0].nrange > 0 && nl.fx[0].nrange < 304)
-        SGPU_TRY(build_ranges(nl, nl.fx[1], nl.fx[0].nrange < 152 ? 32 : 64, fail, er, ord, covpts, covptr,
+        SGPU_TRY(build_ranges(ctx, nl, nl.fx[1], nl.fx[0].nrange < 152 ? 32 : 64, er, ord, covpts, covptr,
                               ent_chi, ent_meta));
     return SGPU_OK;
 }

@@ -449,7 +449,7 @@ std::vector<int> compact_order(int Nx, int Ny, const std::vector<int> &covpts)
     for (size_t c = 0; c < covpts.size(); c++) ord[at[blk[c]]++] = (int)c;
     return ord;
 }
-int nonlocal_tc_build(Nonlocal &nl, const std::vector<int> &ord, const std::vector<int> &covpts,
+int nonlocal_tc_build(sgpu_ctx *ctx, Nonlocal &nl, const std::vector<int> &ord, const std::vector<int> &covpts,
                       const std::vector<int> &covptr, const std::vector<long> &ent_chi,
                       const std::vector<int4> &ent_meta, const double *chi)
 {
@@ -519,7 +519,7 @@ int nonlocal_tc_build(Nonlocal &nl, const std::vector<int> &ord, const std::vect
     auto up = [&](auto **dst, const auto &v) {
         using T = std::remove_reference_t<decltype(v[0])>;
         if (rc != SGPU_OK) return;
-        if (cudaMalloc((void **)dst, sizeof(T) * std::max<size_t>(v.size(), 1)) != cudaSuccess ||
+        if (dev_alloc(ctx, dst, sizeof(T) * std::max<size_t>(v.size(), 1)) != cudaSuccess ||
             (!v.empty() && cudaMemcpy(*dst, v.data(), sizeof(T) * v.size(),
                                       cudaMemcpyHostToDevice) != cudaSuccess)) {
             set_error("set_nonlocal: device allocation of the tensor-core range tables failed");

@@ -737,7 +737,7 @@ int sgpu_scf(sgpu_ctx *ctx, const sgpu_scf_params *prm, const double *b, const d
 
     // persistent device vectors of the SCF (SPARC_OBJ fields of the same role)
     double *vec = nullptr;
-    SGPU_CUDA_TRY(cudaMalloc(&vec, sizeof(double) * (size_t)N * 8 + sizeof(double) * 4 * (size_t)Ns * Ns + 4096));
+    SGPU_CUDA_TRY(dev_alloc(ctx, &vec, sizeof(double) * (size_t)N * 8 + sizeof(double) * 4 * (size_t)Ns * Ns + 4096));
     struct Guard { double *p; ~Guard() { if (p) cudaFree(p); } } guard{vec};
     double *d_b = vec, *d_core = vec + N, *d_rho = vec + 2 * N, *d_phi = vec + 3 * N;
     double *d_vxc = vec + 4 * N, *d_exc = vec + 5 * N, *d_veff = vec + 6 * N, *d_rhoout = vec + 7 * N;
@@ -753,13 +753,13 @@ int sgpu_scf(sgpu_ctx *ctx, const sgpu_scf_params *prm, const double *b, const d
     // orbital blocks: FP64 X, Y always; FP32 pair while in mixed mode
     double *X64 = nullptr, *Y64 = nullptr;
     float *X32 = nullptr, *Y32 = nullptr;
-    SGPU_CUDA_TRY(cudaMalloc(&X64, sizeof(double) * (size_t)nb));
+    SGPU_CUDA_TRY(dev_alloc(ctx, &X64, sizeof(double) * (size_t)nb));
     struct G2 { double *p; ~G2() { if (p) cudaFree(p); } } gx{X64};
-    SGPU_CUDA_TRY(cudaMalloc(&Y64, sizeof(double) * (size_t)nb));
+    SGPU_CUDA_TRY(dev_alloc(ctx, &Y64, sizeof(double) * (size_t)nb));
     struct G3 { double *p; ~G3() { if (p) cudaFree(p); } } gy{Y64};
     bool mixed = prm->precision == SGPU_PREC_FP32;
     if (mixed) {
-        SGPU_CUDA_TRY(cudaMalloc(&X32, sizeof(float) * (size_t)nb * 2));
+        SGPU_CUDA_TRY(dev_alloc(ctx, &X32, sizeof(float) * (size_t)nb * 2));
         Y32 = X32 + nb;
     }
     struct G4 { float *p; ~G4() { if (p) cudaFree(p); } } g32{X32};

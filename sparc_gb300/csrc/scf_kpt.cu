@@ -121,7 +121,7 @@ int sgpu_scf_kpt(sgpu_ctx *ctx, const sgpu_scf_params *prm, int nkpt, const doub
     // persistent device vectors: in3 / out3 = [total, up, down] input and output densities
     // (only the total without spin), g = the mixed vector ([total, magz] with spin)
     DevFree gv;
-    SGPU_CUDA_TRY(cudaMalloc(&gv.p, sizeof(double) * ((size_t)N * 16 + (size_t)nblk * Ns) + 256));
+    SGPU_CUDA_TRY(dev_alloc(ctx, &gv.p, sizeof(double) * ((size_t)N * 16 + (size_t)nblk * Ns) + 256));
     double *vec = static_cast<double *>(gv.p);
     double *d_b = vec, *d_core = vec + N, *d_phi = vec + 2 * N, *d_exc = vec + 3 * N;
     double *d_in3 = vec + 4 * N, *d_out3 = vec + 7 * N, *d_g = vec + 10 * N;
@@ -149,11 +149,11 @@ int sgpu_scf_kpt(sgpu_ctx *ctx, const sgpu_scf_params *prm, int nkpt, const doub
     bool mixed = prm->precision == SGPU_PREC_FP32;
     DevFree g64, g32;
     const long ncplx = nb * nblk;
-    SGPU_CUDA_TRY(cudaMalloc(&g64.p, sizeof(double2) * (size_t)ncplx * 2));
+    SGPU_CUDA_TRY(dev_alloc(ctx, &g64.p, sizeof(double2) * (size_t)ncplx * 2));
     double2 *X64 = static_cast<double2 *>(g64.p), *Y64 = X64 + ncplx;
     float2 *X32 = nullptr, *Y32 = nullptr;
     if (mixed) {
-        SGPU_CUDA_TRY(cudaMalloc(&g32.p, sizeof(float2) * (size_t)ncplx * 2));
+        SGPU_CUDA_TRY(dev_alloc(ctx, &g32.p, sizeof(float2) * (size_t)ncplx * 2));
         X32 = static_cast<float2 *>(g32.p);
         Y32 = X32 + ncplx;
     }

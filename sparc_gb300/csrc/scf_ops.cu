@@ -799,7 +799,7 @@ int mixing_init(sgpu_ctx *ctx, const MixParams &prm, const double *x0)
         ctx->mix = ms;
         ms->m = prm.m;
         ms->prm.nspden = prm.nspden;
-        if (cudaMalloc(&ms->buf, sizeof(double) * (size_t)N * (8 + 2 * prm.m)) != cudaSuccess) {
+        if (dev_alloc(ctx, &ms->buf, sizeof(double) * (size_t)N * (8 + 2 * prm.m)) != cudaSuccess) {
             set_error("mixing: device allocation failed");
             delete ms;
             ctx->mix = nullptr;

@@ -277,6 +277,20 @@ inline size_t scratch_max(const sgpu_ctx *ctx) { return ctx->inject & 8 ? (size_
 // gives back scratch that calls can do without, except what a request for slot `asking` may hold
 // (-1: none in use)
 int ws_release(sgpu_ctx *ctx, int asking);
+// cudaMalloc and cudaMallocAsync that take that scratch back before they give up: for allocations made
+// while no call holds any of it
+cudaError_t dev_alloc(sgpu_ctx *ctx, void **p, size_t bytes);
+cudaError_t dev_alloc_async(sgpu_ctx *ctx, void **p, size_t bytes, cudaStream_t st);
+template <typename T>
+cudaError_t dev_alloc(sgpu_ctx *ctx, T **p, size_t bytes)
+{
+    return dev_alloc(ctx, reinterpret_cast<void **>(p), bytes);
+}
+template <typename T>
+cudaError_t dev_alloc_async(sgpu_ctx *ctx, T **p, size_t bytes, cudaStream_t st)
+{
+    return dev_alloc_async(ctx, reinterpret_cast<void **>(p), bytes, st);
+}
 int fp64_fma_rate(sgpu_ctx *ctx, double *tflops);
 
 // profiling: returns an event pair recorded around a launch of `kind` (or nulls when off)
@@ -348,7 +362,7 @@ int launch_nonlocal_apply_project_tc(sgpu_ctx *ctx, int ncol, const float *alpha
                                      cudaStream_t st);
 bool nonlocal_tc_ready(const sgpu_ctx *ctx);
 // builds the tensor-core range tables from the point CSR of nonlocal_upload
-int nonlocal_tc_build(Nonlocal &nl, const std::vector<int> &ord, const std::vector<int> &covpts,
+int nonlocal_tc_build(sgpu_ctx *ctx, Nonlocal &nl, const std::vector<int> &ord, const std::vector<int> &covpts,
                       const std::vector<int> &covptr, const std::vector<long> &ent_chi,
                       const std::vector<int4> &ent_meta, const double *chi);
 // covered points in the order of compact blocks of the grid (nonlocal_tc.cu)
@@ -358,9 +372,9 @@ std::vector<int> compact_order(int Nx, int Ny, const std::vector<int> &covpts);
 // of the finished out
 bool nonlocal_fx_ready(const sgpu_ctx *ctx);
 void nonlocal_fx_free(Nonlocal &nl);
-int nonlocal_fx_build(Nonlocal &nl, const std::vector<int> &ord, const std::vector<int> &covpts,
+int nonlocal_fx_build(sgpu_ctx *ctx, Nonlocal &nl, const std::vector<int> &ord, const std::vector<int> &covpts,
                       const std::vector<int> &covptr, const std::vector<long> &ent_chi,
-                      const std::vector<int4> &ent_meta, const double *chi, bool fail);
+                      const std::vector<int4> &ent_meta, const double *chi);
 int launch_nonlocal_fx_project(sgpu_ctx *ctx, int ncol, const double *x, long ldx, double *alpha,
                                long lda, cudaStream_t st);
 int launch_nonlocal_fx_apply(sgpu_ctx *ctx, int ncol, const double *alpha, long lda, double scale,

@@ -11,7 +11,7 @@ from sparc_gb300.synthetic import fd_d2_coeffs, synthetic_nonlocal
 
 pytestmark = pytest.mark.gpu
 
-SCRATCH, TABLES, RR_WAIT, SMALL = 1, 2, 4, 8
+SCRATCH, TABLES, RR_WAIT, SMALL, FIRST_TRY = 1, 2, 4, 8, 16
 
 
 def _system(N, h, natom=6, rc=2.2, nspin=1, seed=1):
@@ -385,3 +385,25 @@ def test_two_threads_with_ranges_of_different_size(gpu_available):
     for ctx, x, y, o in work:
         _close(y.cpu().numpy(), o.vnl(x.cpu().numpy()))
         ctx.close()
+
+
+def test_other_allocations_take_scratch_back(gpu_available):
+    """Allocations that fail while optional scratch is held (sets, forces, tuning) are tried again
+    without it; the calls' results stay."""
+    ctx, v, nl, grid, rng = _system((30, 28, 26), 0.4)
+    o, cell, ncol = Oracle(grid, nl), np.array((30, 28, 26)) * 0.4, 64
+    x = rng.uniform(-1, 1, (ncol, ctx.Nd))
+    occ = rng.uniform(0, 1, ncol)
+    h, s = np.zeros_like(x), [np.zeros((ncol, ncol)) for _ in range(2)]
+    ctx.Project_Hamiltonian(x, h, *s)  # slices and partial projections are kept from here on
+    forces = ctx.Calculate_nonlocal_forces(cell, x, occ)
+    ctx.Project_Hamiltonian(x, h, *s)
+    ctx.inject_failure(FIRST_TRY)
+    _close(ctx.Calculate_nonlocal_forces(cell, x, occ), forces, 1e-11)
+    ctx.autotune(ncol=16)
+    _set(ctx, np.concatenate([v, 0.5 * v]), nl, 2)
+    ctx.inject_failure(0)
+    y = np.zeros_like(x)
+    ctx.Hamiltonian_vectors_mult(0.2, x, y, spin=1)
+    _close(y, o.hamiltonian(0.5 * v, 0.2, x))
+    ctx.close()

@@ -47,7 +47,7 @@ int ws_get(sgpu_ctx *ctx, int slot, size_t bytes, void **out)
             w.bytes = 0;
         }
         size_t nb = bytes + bytes / 8 + 256;
-        if ((ctx->inject & 1) && ws_optional(slot)) nb = (size_t)1 << 60;
+        if ((ctx->inject & 1) && (ws_optional(slot) || slot == WS_ALPHA2)) nb = (size_t)1 << 60;
         cudaError_t e = cudaMalloc(&w.ptr, nb);
         if (e != cudaSuccess) {
             cudaGetLastError();  // the callers' launch checks must not meet it
@@ -440,7 +440,8 @@ int sgpu_Hamiltonian_vectors_mult(sgpu_ctx *ctx, int spin, int ncol, double c, c
 // so the block is cut into chunks that move through three device slots: while chunk i is
 // filtered on the context stream, chunk i+1 is copied in on one copy stream and chunk i-1
 // copied out on another. The host-device copies then hide behind the filter instead of
-// adding to it. Each column's arithmetic is the one of the unchunked call.
+// adding to it. Each column goes through the operations of the unchunked call; in fixed point the
+// tiles, and with them the scales that values are rounded to, follow the chunk's width.
 // return_x false: X is input only (its chunks are not copied back).
 static int filter_pipelined(sgpu_ctx *ctx, int spin, double *X, int ldi, double *Y, int ldo,
                             int ncol, int nc, int m, double a, double b, double a0, bool f32,

@@ -85,7 +85,12 @@ static int carried_alpha(sgpu_ctx *ctx, int ncol, const T *X, long ldx, T **A, T
     const long lda = nonlocal_alpha_ld(ncol, (int)sizeof(T));
     const size_t bytes = sizeof(T) * (size_t)ctx->nl.ntot * lda;
     SGPU_TRY(ws_get(ctx, WS_ALPHA, bytes, (void **)A));
-    SGPU_TRY(ws_get(ctx, WS_ALPHA2, bytes, (void **)B));
+    const int rc = ws_get(ctx, WS_ALPHA2, bytes, (void **)B);
+    if (rc == SGPU_ERR_NOMEM && sizeof(T) == 8) {  // each degree projects for itself
+        *A = *B = nullptr;
+        return SGPU_OK;
+    }
+    SGPU_TRY(rc);
     if (sizeof(T) == 4) SGPU_CUDA_TRY(cudaMemsetAsync(*A, 0, bytes, st));
     return launch_nonlocal_project<T>(ctx, ncol, X, ldx, *A, lda, st);
 }

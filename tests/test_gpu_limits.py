@@ -407,3 +407,47 @@ def test_other_allocations_take_scratch_back(gpu_available):
     ctx.Hamiltonian_vectors_mult(0.2, x, y, spin=1)
     _close(y, o.hamiltonian(0.5 * v, 0.2, x))
     ctx.close()
+
+
+def _padded(x, pad):
+    """The rows of x in a device block of longer, poisoned rows."""
+    import torch
+    b = torch.full((x.shape[0], x.shape[1] + pad), float("nan"), dtype=torch.float64, device="cuda")
+    b[:, :x.shape[1]] = torch.from_numpy(x).cuda()
+    return b[:, :x.shape[1]]
+
+
+@pytest.mark.parametrize("ncol,pad", [(5, 1), (33, 7), (70, 64)])
+def test_padded_device_blocks(gpu_available, ncol, pad):
+    """Leading dimensions above Nd, odd ones among them, in the real FP64 calls above the size of the
+    point-per-thread kernel; the second spin of two."""
+    N, h = (29, 27, 31), 0.4
+    ctx, v, nl, grid, rng = _system(N, h, nspin=2)
+    o, Nd = Oracle(grid, nl), ctx.Nd
+    v1 = v[Nd:]
+    x = rng.uniform(-1, 1, (ncol, Nd))
+    X, Y = _padded(x, pad), _padded(np.zeros_like(x), pad)
+    assert X.stride(0) == Nd + pad
+    ctx.Hamiltonian_vectors_mult(0.3, X, Y, spin=1)
+    _close(Y.cpu().numpy(), o.hamiltonian(v1, 0.3, x))
+    Y.zero_()
+    ctx.Vnl_vec_mult(X, Y)
+    _close(Y.cpu().numpy(), o.vnl(x))
+    ctx.ChebyshevFiltering(X, Y, 6, 0.5, 40.0, -0.8, spin=1)
+    Xo, Yo = o.chebyshev(v1, 6, 0.5, 40.0, -0.8, x)
+    _close(Y.cpu().numpy(), Yo)
+    _close(X.cpu().numpy(), Xo)
+    HY, Z = _padded(np.zeros_like(x), pad), _padded(np.zeros_like(x), pad)
+    Hp, Mp = np.zeros((ncol, ncol)), np.zeros((ncol, ncol))
+    Q = rng.normal(size=(ncol, ncol))
+    ctx.Project_Hamiltonian(Y, HY, Hp, Mp, spin=1)
+    ctx.Subspace_Rotation(Y, Q, Z)
+    y, hy = Y.cpu().numpy(), HY.cpu().numpy()
+    _close(hy, o.hamiltonian(v1, 0.0, y))
+    _close(Mp, y @ y.T)
+    _close(Hp, y @ hy.T)
+    _close(Z.cpu().numpy(), Q @ y)
+    for b in (X, Y, HY, Z):  # nothing was written between the columns
+        full = b.as_strided((ncol, Nd + pad), (Nd + pad, 1))
+        assert np.isnan(full[:, Nd:].cpu().numpy()).all()
+    ctx.close()

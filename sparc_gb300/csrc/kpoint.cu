@@ -566,6 +566,9 @@ __global__ void __launch_bounds__(32 * nlfx::kWarps, 2)
     extern __shared__ __align__(16) unsigned char nlfxz_smem[];
     const int b = blockIdx.x / gx, g0 = blockIdx.x - b * gx;
     const BBlock<double2> &B = blocks[b];
+    // the launch has as many blocks per range as its widest member needs; the others leave before they
+    // have copies in flight (nlfx::block waits for those in its first group)
+    if (g0 * (nlfx::kLanes / 2) >= B.ncol) return;
     double *buf = reinterpret_cast<double *>(B.buf[sel]);
     nlfx::block<true, APPLY, PROJ, MAXJ>(
         T, blockIdx.y, g0, gx, B.ncol, reinterpret_cast<const double *>(second ? B.alpha2 : B.alpha),
@@ -1059,7 +1062,7 @@ static int nonlocal_z(sgpu_ctx *ctx, int ncol, const CT *x, long ldx, CT *out, l
             const int groups = (ncol + FG - 1) / FG;
             const NlFx &X = nonlocal_fx_pick(nl, groups);
             const nlfx::Tables T = nonlocal_fx_tables(nl, X);
-            const int sm = (int)T.L.bytes;
+            const int sm = (int)nlfx::shared_bytes(T);
             CT *part = nullptr;
             int chunk = groups;
             const int rc = X.nrange > 65535
@@ -1413,7 +1416,7 @@ static int chebyshev_batched(sgpu_ctx *ctx, int nblk, const sgpu_filter_block *b
     int fsm = 0, fgx = 1;
     if (fx_nl) {  // attributes set before any capture
         fT = nonlocal_fx_tables(nl, *fxt);
-        fsm = (int)fT.L.bytes;
+        fsm = (int)nlfx::shared_bytes(fT);
         const int groups = (maxcol + FG - 1) / FG;
         fgx = std::min(groups, std::max(1, (int)(152L * 8 / ((long)fxt->nrange * nblk))));
         auto attr = [&](auto k9, auto k18) {

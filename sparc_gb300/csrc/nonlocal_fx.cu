@@ -63,7 +63,7 @@ int launch(sgpu_ctx *ctx, int ncol, const double *alpha, double scale, double *o
     const int groups = (ncol + nlfx::kLanes - 1) / nlfx::kLanes;
     const NlFx &X = nonlocal_fx_pick(nl, groups);
     const nlfx::Tables T = nonlocal_fx_tables(nl, X);
-    const size_t smem = T.L.bytes;
+    const size_t smem = nlfx::shared_bytes(T);
     auto kern = nl.max_np <= 9 ? k_nl_fx<APPLY, PROJ, 9> : k_nl_fx<APPLY, PROJ, 18>;
     SGPU_CUDA_TRY(allow_smem(kern));
     double *part = nullptr;
@@ -114,7 +114,7 @@ int project_fp64(sgpu_ctx *ctx, int ncol, const double *x, long ldx, double *alp
 nlfx::Tables nonlocal_fx_tables(const Nonlocal &nl, const NlFx &x)
 {
     return {x.pt0, x.pts, x.item0, x.items, x.ent0, x.wsplit, x.lp, x.chi, x.rows, x.row0, nl.fx_jp,
-            nlfx::layout(x.max_rows, x.max_ent, x.max_items, nl.fx_jp)};
+            x.max_rows, x.max_ent, x.max_items};
 }
 
 // The large ranges when they and the column groups make two blocks per SM, else the small ones:

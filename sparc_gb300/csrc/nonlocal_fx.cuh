@@ -56,9 +56,13 @@ struct Tables {
     const int4 *chi;    // entry: jp / 2 pairs of digits (h, l, h, l)
     const int4 *rows;   // row of a range: (alpha row, image, er), |Chi| of the row < 2^er
     const int *row0;    // nrange + 1: first row of each range (rows, partial buffer)
-    int jp;
-    Layout L;           // shared memory for the largest of the ranges
+    int jp, max_rows, max_ent, max_items;
 };
+
+inline size_t shared_bytes(const Tables &T)
+{
+    return shared_bytes(T.max_rows, T.max_ent, T.max_items, T.jp);
+}
 
 // raw sum in units of 2^57. A product is below 2^113, so 128 of them end below 2^63 units (what an
 // intermediate sum wraps, a later one wraps back); mid alone must not wrap: 64 products at most
@@ -72,7 +76,7 @@ __device__ __forceinline__ double chi_value(int2 c, int er)
     return ldexp((double)c.x * 536870912.0 + (double)c.y, er - kChiBits);
 }
 
-// Block (range r; column groups g0, g0 + gstep, ...) of x / out (column-major, ld in elements:
+// Block (range r; column groups g0, g0 + gstep, ..., g0 among them) of x / out (column-major, ld in elements:
 // doubles, or complex pairs when CPLX) with ncol columns in all; alpha: projector-major rows of
 // lda elements; part: the ranges' projections (dV and Gamma not applied), rows of ldp elements.
 // phase (CPLX): cos and sin of each image's phase.
@@ -89,14 +93,15 @@ __device__ __forceinline__ void block(const Tables &T, int r, int g0, int gstep,
     constexpr int NV = kPts / 32;                   // points per lane
     constexpr int NA = kRows / kWarps;              // alpha rows per warp
     const int hp = T.jp >> 1;                                    // digit pairs per entry
-    long long *tile = reinterpret_cast<long long *>(smem);       // [kPts][kPitch]
-    int2 *al = reinterpret_cast<int2 *>(smem + T.L.al);            // [rows][kLanes]
-    int4 *chi = reinterpret_cast<int4 *>(smem + T.L.chi);
-    unsigned char *lps = smem + T.L.lps;
-    int4 *rows = reinterpret_cast<int4 *>(smem + T.L.rows);
-    int4 *items = reinterpret_cast<int4 *>(smem + T.L.items);
-    int *ent0 = reinterpret_cast<int *>(smem + T.L.ent0);
-    int *wsplit = reinterpret_cast<int *>(smem + T.L.wsplit);
+    const auto R = regions(smem, T.max_rows, T.max_ent, T.max_items, T.jp);
+    long long *tile = reinterpret_cast<long long *>(R.tile);     // [kPts][kPitch]
+    int2 *al = reinterpret_cast<int2 *>(R.al);                   // [rows][kLanes]
+    int4 *chi = reinterpret_cast<int4 *>(R.chi);
+    unsigned char *lps = R.lps;
+    int4 *rows = reinterpret_cast<int4 *>(R.rows);
+    int4 *items = reinterpret_cast<int4 *>(R.items);
+    int *ent0 = reinterpret_cast<int *>(R.ent0);
+    int *wsplit = reinterpret_cast<int *>(R.wsplit);
     __shared__ unsigned s_key[kLanes];
     __shared__ int s_bad, s_E[kLanes];
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
@@ -105,9 +110,6 @@ __device__ __forceinline__ void block(const Tables &T, int r, int g0, int gstep,
     const int q0 = T.row0[r], nrow = T.row0[r + 1] - q0;
     const int b0 = T.ent0[i0], nent = T.ent0[i0 + nit] - b0;
     const int ngroup = (ncol + NC - 1) / NC;
-    // a batched launch has as many blocks per range as its widest member needs; the others leave
-    // before they have copies in flight (the wait for those is in the first group)
-    if (g0 >= ngroup) return;
 
     // ---- the range's tables and Chi digits
     {

@@ -23,22 +23,23 @@ int main()
         for (int rows = 1; rows <= 128; rows++)
             for (int ent : {1, 2, 15, 16, 17, 31, 128, 226, 227, 408, 409})
                 for (int items = 1; items <= 128; items++) {
-                    const Layout L = layout(rows, ent, items, jp);
-                    const unsigned r = rows, e = ent, i = items;
+                    const auto L = regions<std::size_t>(0, rows, ent, items, jp);
+                    const unsigned bytes = shared_bytes(rows, ent, items, jp);
+                    const std::size_t r = rows, e = ent, i = items;
                     // start, bytes used and alignment of each region, in the order of the layout
-                    const unsigned reg[][3] = {
-                        {0, 8 * 128 * 33, 16},       {L.al, r * 32 * 8, 8},
+                    const std::size_t reg[][3] = {
+                        {L.tile, 8 * 128 * 33, 16},       {L.al, r * 32 * 8, 8},
                         {L.chi, e * jp * 8, 16},     {L.lps, e, 1},
                         {L.rows, r * 16, 16},        {L.items, i * 16, 16},
                         {L.ent0, (i + 1) * 4, 4},    {L.wsplit, i * 9 * 4, 4},
-                        {L.bytes, 0, 16}};
+                        {bytes, 0, 16}};
                     for (int k = 0; k < 9; k++) {
                         if (reg[k][0] % reg[k][2]) bad++;
                         if (k < 8 && reg[k][0] + reg[k][1] > reg[k + 1][0]) bad++;
                     }
                     // the largest ranges that are built: 128 rows, 32 KB of Chi digits, an item
                     // per row at most
-                    if (e * jp * 8 <= 32 * 1024 && items <= rows && L.bytes > 227 * 1024) bad++;
+                    if (e * jp * 8 <= 32 * 1024 && items <= rows && bytes > 227 * 1024) bad++;
                     n++;
                 }
     std::printf("%ld of %ld\n", bad, n);

@@ -531,12 +531,13 @@ int sgpu_kernel_status(sgpu_ctx *ctx, int *status);
  * bound works) and leaves it cleared. No copy is in flight and nothing faults. */
 int sgpu_check_wait_bound(sgpu_ctx *ctx, int *status);
 
-/* Failures made on the host, for tests of what a call does about them; mask 0 ends them. 1: device
- * scratch that a call can do without cannot be allocated; 2: the fixed-point tables of set_veff
- * and set_nonlocal cannot be; 4: a bounded wait of the FP64 Rayleigh-Ritz products is reported as
- * run out, with part of their output unwritten; 8: an operand's scratch is held to 1 MB;
- * 16: the first try of every other allocation fails, as on a device that the scratch fills. A call then takes the form that needs none of
- * these, with the same result. */
+/* Failures made on the host, for tests of what a call does about them; mask 0 ends them. 1: scratch
+ * that FP64 calls can do without cannot be allocated (FP32 Rayleigh-Ritz products, which cannot do
+ * without their slices, return SGPU_ERR_NOMEM); 2: the fixed-point tables of set_veff and
+ * set_nonlocal cannot be; 4: a bounded wait of the FP64 Rayleigh-Ritz products is reported as run
+ * out, with part of their output unwritten; 8: an operand's scratch is held to 1 MB; 16: the first
+ * try of every other allocation fails, as on a device that the scratch fills. FP64 calls then take
+ * the form that needs none of these, with the same result. */
 int sgpu_inject_failure(sgpu_ctx *ctx, int mask);
 
 /* Measures this GPU's FP64 FMA rate (TFLOP/s, an FMA counted as two flops) with one
@@ -646,10 +647,12 @@ int sgpu_set_rr_products(sgpu_ctx *ctx, int mode);
  * filters of degree 20 with projectors, in the norm of a column, are at 0.6 to 0.9 of the error of
  * the FP64 kernels for uniform and for smooth columns, at 1.0 to 2.0 for columns that fall off by
  * exp(-0.9 r) (Bohr) from a point. Tiles and ranges depend on the number of columns, and with
- * them the last bits of a column. Potentials above 16 times the largest power of two in the sum
- * of the coefficients (a launch then takes 7 times as long), more than 18 projectors per atom and
- * values outside about 1e-230 .. 1e230 take the FP64 kernels with either. The Rayleigh-Ritz
- * products have sgpu_set_rr_products. */
+ * them the last bits of a column. Potentials of 16 times the next power of two above the sum of the
+ * coefficients or more (one such point decides for all spins and columns of a launch, which then
+ * takes 7 times as long), more than 18 projectors per atom, projectors of more than 128 rows over
+ * one point and values outside about 1e-230 .. 1e230 take the FP64 kernels with either, and so
+ * does a call without room for its scratch. The Rayleigh-Ritz products have
+ * sgpu_set_rr_products. */
 int sgpu_set_fixed_point(sgpu_ctx *ctx, int on);
 
 /* complex64 stencil form: 1 (default) tiles with packed FP32 arithmetic and a per-k table of

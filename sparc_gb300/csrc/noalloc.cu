@@ -5,9 +5,11 @@
 // library do that: a host application that hands all of the GPU's memory to its own pool
 // allocator up front leaves nothing for cudaMalloc to return, and a caller that overlaps this
 // call with other work on other streams cannot accept cudaFree, which synchronises the whole
-// device. sgpu_Vnl_vec_mult_noalloc serves them: the same kernels, with alpha in a fixed
-// scratch array that lives in this library's own device image (every GPU that loads the
-// library holds it until the process exits), so the call itself allocates nothing.
+// device. sgpu_Vnl_vec_mult_noalloc serves them: the apply kernel of sgpu_Vnl_vec_mult and the FP64
+// segment projection, which adds up in alpha itself (the fixed-point projection needs partial
+// rows), with alpha in a fixed scratch array that lives in this library's own device image (every
+// GPU that loads the library holds it until the process exits), so the call itself allocates
+// nothing.
 //
 // Limits and rules:
 //  * scratch holds kNoallocScratchDoubles doubles (8 MiB): n_proj * round_up(ncol, 8) must fit,

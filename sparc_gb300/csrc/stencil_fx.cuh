@@ -14,16 +14,16 @@
 // value within 2^-4 of the scale: the scale follows the data along z both ways. (With a scale that
 // only grew, a column that falls off into a vacuum was rounded to 2^-57 of its largest value
 // everywhere: after 85 planes of exp(-0.35) that is 1e-5 of the values there.) Values that the
-// fixed-point range does not cover (infinities, NaN, extreme exponents) send the rest of the slab through the
-// FP64 path.
+// fixed-point range does not cover (infinities, NaN, extreme exponents) send the rest of the slab
+// through the FP64 path.
 //
-// What bounds it: instruction issue (61 % of the slots busy, 60 % of the integer multiply pipe, 59 %
-// of the shared-memory wavefronts, HBM 29 %). Per point about 36 integer adds, 24 wide
+// What bounds it: instruction issue (58 % of the slots busy, 53 % of the shared-memory wavefronts,
+// HBM 24 %) between barriers at 15 warps per SM. Per point about 36 integer adds, 24 wide
 // multiply-adds and 7 high products (60 and 19 with three spacings), 21 instructions per converted
 // value (2.5 of them on a 16 x 16 tile) and 40 for the way back, against 42 FP64 instructions at
 // two lanes per clock in k_stencil_orth. 96^3, 512 columns: 37.3 -> 5.44 ms per launch (5.29 without
 // the lowering of the scale; 4.75 with coefficients of two digits as well, whose rounding cost a
-// filter its accuracy; the shares above were taken at 4.75).
+// filter its accuracy).
 #pragma once
 
 #include <algorithm>
@@ -406,10 +406,11 @@ inline void fx_plan(int Nx, int Ny, int Nz, int ncol, int nsm, int &TX, int &TY,
 }
 
 // Coefficient digits of a launch; vkey: exponent key of the largest |bv v| (0 without a
-// potential). False when the coefficients do not fit: the caller takes the FP64 kernel. All terms
-// of a point share one scale, the sum S of the coefficients' magnitudes, so a potential far
-// above the stencil's own weights (8 times: six bits of the scale) goes there too: its largest
-// values would take the precision of the points where it is small.
+// potential). False when the coefficients do not fit: the caller takes the FP64 kernel, 37.3 ms per
+// launch at 96^3 x 512 where this form takes 5.44. All terms of a point share one scale, the next
+// power of two above the sum S of the coefficients' magnitudes, so a potential of 16 times that or
+// more (it would take six bits of the scale from the points where it is small) goes there too,
+// with all spins and columns of the launch.
 inline bool fx_setup(StencilFxParams &p, int FDn, unsigned vkey)
 {
     double S = std::fabs(p.c0);

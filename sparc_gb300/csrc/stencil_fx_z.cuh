@@ -3,8 +3,8 @@
 // side, and the Bloch factor of a value's unwrapped position applied in FP64 before it becomes
 // digits (only to values from outside the cell).
 //
-// What bounds it: latency at the 15 warps that 128 registers leave (46 % of the issue slots busy, the
-// FP64 pipe, which has the output scale, the recurrence term and the factors, 37 %; with the
+// What bounds it: latency at the 15 warps that 128 registers leave (47 % of the issue slots busy, the
+// FP64 pipe, which has the output scale, the recurrence term and the factors, 35 %; with the
 // factors as selects on every value it was the bound at 75 %, and 2.9 ms). 34^3, 20 blocks of 64
 // columns: 12.6 ms per degree in k_stencil_zb<double2>, 2.05 here.
 #pragma once

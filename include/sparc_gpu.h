@@ -642,14 +642,15 @@ int sgpu_set_rr_products(sgpu_ctx *ctx, int mode);
  * the planes that its stencil reaches, and the potential and the coefficients against the sum of
  * the coefficients; for the nonlocal products a column's values and projections over a range of
  * 128 neighbouring points, and a projector row's Chi values. In the norm of such a block a product
- * is at least as accurate as in FP64. A value 2^-k of its block's largest keeps 57 - k bits, so a
- * column that falls off within a few points may be off by more than in FP64 far from its centre:
- * filters of degree 20 with projectors, in the norm of a column, are at 0.6 to 0.9 of the error of
- * the FP64 kernels for uniform and for smooth columns, at 1.0 to 2.0 for columns that fall off by
- * exp(-0.9 r) (Bohr) from a point. Tiles and ranges depend on the number of columns, and with
- * them the last bits of a column. Potentials of 16 times the next power of two above the sum of the
- * coefficients or more (one such point decides for all spins and columns of a launch, which then
- * takes 7 times as long), more than 18 projectors per atom, projectors of more than 128 rows over
+ * is at least as accurate as in FP64: filters of degree 18 to 20 with projectors, in the norm of a
+ * column and against extended precision, are at 0.5 to 0.65 of the error of the FP64 kernels for
+ * uniform and smooth columns and for columns that fall off by exp(-0.9 r) (Bohr) from a point. At
+ * a single point it need not be: a value 2^-k of its block's largest keeps 57 - k bits. (A filter
+ * whose upper bound lies below the end of the spectrum amplifies the roundings themselves; there
+ * columns of the last kind were at 0.6 to 1.9.) Tiles and ranges depend on the number of columns,
+ * and with them the last bits of a column. Potentials of 16 times the next power of two above the
+ * sum of the coefficients or more (one such point decides for all spins and columns of a launch,
+ * which then takes 7 times as long), more than 18 projectors per atom, projectors of more than 128 rows over
  * one point and values outside about 1e-230 .. 1e230 take the FP64 kernels with either, and so
  * does a call without room for its scratch. The Rayleigh-Ritz products have
  * sgpu_set_rr_products. */

@@ -11,10 +11,12 @@
 // this way is at least as accurate, in the norm of the block, as the FP64 one. What repeats in
 // every application has to be finer, as it adds up over the degrees of a filter: values cut
 // toward zero and coefficients of two digits each made a filter of 20 degrees 1.5 to 2 times less
-// accurate than FP64; rounded, and with a third coefficient digit, the error of a filter with
-// projectors, in the norm of a column and against extended precision, is 0.6 to 0.9 of FP64's for
-// uniform and smooth columns. Values far below their block's largest are the price: 1.0 to 2.0 times
-// FP64's error for columns that fall off by exp(-0.9 r) (Bohr) from a point.
+// accurate than FP64, and ties rounded to one side (values and results away from zero, a potential's
+// products up) 1.4 to 1.6 times for columns that fall off from a point, as their errors then have one
+// sign. With ties to even and a third coefficient digit the error of a filter with projectors, in
+// the norm of a column and against extended precision, is 0.5 to 0.65 of FP64's for uniform and
+// smooth columns and for those that fall off by exp(-0.9 r) (Bohr) from a point. What is lost is
+// accuracy at a single point whose values are far below their block's largest.
 // Sums of six digits fit 32 bits; products with coefficient digits accumulate exactly in 64 bits.
 #pragma once
 
@@ -44,11 +46,15 @@ __device__ __forceinline__ int2 to_digits(double x, int E)
     const int ex = (int)((hi >> 20) & 0x7ffu);
     const int d = min(E - ex, 63);  // ex = 0 (zero, denormal): everything is shifted out
     unsigned long long M = ((unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32) | lo;
-    // twice U, a half for the rounding and the half digit that rounds h
-    M = ((M << (kBits + 1 - 53)) >> d) + (1ull + (1ull << kDigit));
+    // 8 U, so that h is the upper word; then a half for the rounding, ties to even, and the half digit
+    // that rounds h. Values 2^-5 to 2^-7 below the scale lose one to three bits and end in a tie that
+    // often; further down ties are rare, and the bits below 8 U make them look like ones.
+    M = (M << (kBits + 3 - 53)) >> d;
+    const unsigned odd = (((unsigned)M >> 3) | ((unsigned)(d + 120) >> 7)) & 1u;  // or d > 7
+    M += (1ull << 31) + 3u + odd;
     const int sg = 1 | ((int)hi >> 31);
-    const int l = (int)(((unsigned)M ^ (1u << kDigit)) << (31 - kDigit)) >> (32 - kDigit);
-    const int h = (int)(M >> (kDigit + 1));
+    const int l = (int)((unsigned)M ^ 0x80000000u) >> (32 - kDigit);
+    const int h = (int)(M >> 32);
     return make_int2(h * sg, l * sg);
 }
 
@@ -87,7 +93,7 @@ __device__ __forceinline__ long long total(long long hh, long long mid, int lo)
     return total(hh, mid + (long long)lo * 4);
 }
 
-// T 2^K as a double, rounded to nearest; the result's exponent must be normal
+// T 2^K as a double, rounded to nearest, ties to even; the result's exponent must be normal
 __device__ __forceinline__ double to_double(long long T, int K)
 {
     const int sg = (int)(T >> 63);
@@ -95,7 +101,8 @@ __device__ __forceinline__ double to_double(long long T, int K)
     const unsigned ah = (unsigned)(A >> 32);
     const int n = __clz((int)(ah ? ah : (unsigned)A)) + (ah ? 0 : 32);
     const int sh = n - 1;  // |T| < 2^63: n >= 1
-    A = (A << sh) + 0x200ull;  // leading one at bit 62, rounded at bit 10
+    A <<= sh;  // leading one at bit 62; rounded at bit 10, ties to even
+    A += 0x1ffull + (((unsigned)A >> 10) & 1u);
     const unsigned be1 = (unsigned)(1023 + 62 - sh + K - 1);  // the leading one adds 1
     const unsigned long long b = (A >> 10) + ((unsigned long long)be1 << 52);
     const unsigned rh = (unsigned)(b >> 32) | ((unsigned)sg & 0x80000000u);

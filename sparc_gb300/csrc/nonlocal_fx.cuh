@@ -30,7 +30,7 @@
 // and product of a 9-projector set) at 16 warps per SM; HBM 13 %. Chi digits staged in shared
 // memory: read through L1 instead a launch waits for them (11.8 against 7.6 ms). 96^3, 512
 // columns, 64 atoms of 9 projectors on 6 Bohr spheres: apply 17.6 + projection 11.0 ms per
-// degree in FP64, 7.6 + 0.5 (reduction) ms here; 26^3, 32 columns: 78 + 163 us, 20 + 5 us here.
+// degree in FP64, 7.8 + 0.45 (reduction) ms here; 26^3, 32 columns: 78 + 163 us, 20 + 5 us here.
 #pragma once
 
 #include "fixed64.cuh"

@@ -44,7 +44,7 @@ __device__ __forceinline__ int wrapi(int i, int n)
 }
 
 // FP64 kernel: one point per thread. The FP64 pipe (2 lanes per clock and SM) bounds it, 37.3 ms per
-// launch at 96^3 x 512 against 5.44 of the fixed-point form (stencil_fx.cuh); it serves the AAR
+// launch at 96^3 x 512 against 5.58 of the fixed-point form (stencil_fx.cuh); it serves the AAR
 // solves, the coefficients and potentials that the fixed-point form does not take, potentials
 // without digits, and callers that ask for FP64 arithmetic (sgpu_set_fixed_point).
 template <typename T, int R, int BX, int BY>

@@ -21,9 +21,9 @@
 // HBM 24 %) between barriers at 15 warps per SM. Per point about 36 integer adds, 24 wide
 // multiply-adds and 7 high products (60 and 19 with three spacings), 21 instructions per converted
 // value (2.5 of them on a 16 x 16 tile) and 40 for the way back, against 42 FP64 instructions at
-// two lanes per clock in k_stencil_orth. 96^3, 512 columns: 37.3 -> 5.44 ms per launch (5.29 without
-// the lowering of the scale; 4.75 with coefficients of two digits as well, whose rounding cost a
-// filter its accuracy).
+// two lanes per clock in k_stencil_orth. 96^3, 512 columns: 37.3 -> 5.58 ms per launch (5.44 with
+// ties rounded to one side, 5.29 without the lowering of the scale as well, 4.75 with coefficients of
+// two digits: all cost a filter its accuracy).
 #pragma once
 
 #include <algorithm>
@@ -266,7 +266,8 @@ __global__ void __launch_bounds__(kFxThreads, 1) k_stencil_fx(const StencilFxPar
             long long a0 = 0, b0 = 0, a1 = 0, b1 = 0;
             fx::mac(a0, b0, cen.x, cen.y, v0.x, v0.y);
             fx::mac(a1, b1, cen.z, cen.w, v1.x, v1.y);
-            const long long half = (1ll << p.dv) >> 1;
+            // a half, ties up on even steps and down on odd ones
+            const long long half = ((1ll << p.dv) >> 1) - (U == 1 && p.dv > 0);
             T0 += (fx::total(a0, b0) + half) >> p.dv;
             T1 += (fx::total(a1, b1) + half) >> p.dv;
         }
@@ -407,7 +408,7 @@ inline void fx_plan(int Nx, int Ny, int Nz, int ncol, int nsm, int &TX, int &TY,
 
 // Coefficient digits of a launch; vkey: exponent key of the largest |bv v| (0 without a
 // potential). False when the coefficients do not fit: the caller takes the FP64 kernel, 37.3 ms per
-// launch at 96^3 x 512 where this form takes 5.44. All terms of a point share one scale, the next
+// launch at 96^3 x 512 where this form takes 5.58. All terms of a point share one scale, the next
 // power of two above the sum S of the coefficients' magnitudes, so a potential of 16 times that or
 // more (it would take six bits of the scale from the points where it is small) goes there too,
 // with all spins and columns of the launch.

@@ -6,7 +6,7 @@
 // What bounds it: latency at the 15 warps that 128 registers leave (47 % of the issue slots busy, the
 // FP64 pipe, which has the output scale, the recurrence term and the factors, 35 %; with the
 // factors as selects on every value it was the bound at 75 %, and 2.9 ms). 34^3, 20 blocks of 64
-// columns: 12.6 ms per degree in k_stencil_zb<double2>, 2.05 here.
+// columns: 12.6 ms per degree in k_stencil_zb<double2>, 2.08 here.
 #pragma once
 
 #include "stencil_fx.cuh"
@@ -253,7 +253,8 @@ __device__ __forceinline__ void stencil_fxz(const FxZConst &p, const FxZCol &c, 
             long long a0 = 0, b0 = 0, a1 = 0, b1 = 0;
             fx::mac(a0, b0, cen.x, cen.y, v.x, v.y);
             fx::mac(a1, b1, cen.z, cen.w, v.x, v.y);
-            const long long half = (1ll << p.dv) >> 1;
+            // a half, ties up on even steps and down on odd ones
+            const long long half = ((1ll << p.dv) >> 1) - (U == 1 && p.dv > 0);
             Tr += (fx::total(a0, b0) + half) >> p.dv;
             Ti += (fx::total(a1, b1) + half) >> p.dv;
         }
